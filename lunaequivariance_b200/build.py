@@ -34,8 +34,29 @@ def find_nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or CUDA_HOME")
 
 
-def sources() -> list[str]:
-    return sorted(os.path.join(CSRC, name) for name in os.listdir(CSRC) if name.endswith(".cu"))
+# uvu_edge_inst.cu is compiled once per (element type, channels per lane, shape); the shapes are those of uvu_edge.cuh
+EDGE_SOURCE = "uvu_edge_inst.cu"
+EDGE_LANES = (("float", 1), ("float", 2), ("float", 4), ("double", 1), ("double", 2))
+EDGE_SHAPES = 11
+
+
+def units() -> list[tuple[str, str, list[str]]]:
+    """(source, object, extra flags) of everything the library is made of."""
+    found = []
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith(".cu"):
+            continue
+        source = os.path.join(CSRC, name)
+        if name != EDGE_SOURCE:
+            found.append((source, os.path.join(BUILD_DIR, name[:-3] + ".o"), []))
+            continue
+        for shape in reversed(range(EDGE_SHAPES)):
+            for kind, lanes in EDGE_LANES:
+                obj = os.path.join(BUILD_DIR, f"{name[:-3]}_{kind}{lanes}_{shape}.o")
+                found.append((source, obj, [f"-DLUNA_EDGE_T={kind}", f"-DLUNA_EDGE_CPL={lanes}",
+                                            f"-DLUNA_EDGE_SHAPE={shape}"]))
+    # the longest to compile first
+    return sorted(found, key=lambda unit: not unit[2])
 
 
 def headers_mtime() -> float:
@@ -44,14 +65,14 @@ def headers_mtime() -> float:
     return max(os.path.getmtime(p) for p in paths if os.path.exists(p))
 
 
-def compile_one(nvcc: str, source: str, verbose: bool, ptxas_info: bool) -> tuple[str, str]:
-    obj = os.path.join(BUILD_DIR, os.path.basename(source)[:-3] + ".o")
-    command = [nvcc, *NVCC_FLAGS, "-c", source, "-o", obj]
+def compile_one(nvcc: str, unit: tuple[str, str, list[str]], verbose: bool, ptxas_info: bool) -> tuple[str, str]:
+    source, obj, flags = unit
+    command = [nvcc, *NVCC_FLAGS, *flags, "-c", source, "-o", obj]
     if ptxas_info:
         command[1:1] = ["-Xptxas", "-v"]
     result = subprocess.run(command, capture_output=True, text=True)
     if result.returncode != 0:
-        raise RuntimeError(f"nvcc failed for {source}:\n{result.stdout}\n{result.stderr}")
+        raise RuntimeError(f"nvcc failed for {source} {flags}:\n{result.stdout}\n{result.stderr}")
     return obj, result.stderr if (verbose or ptxas_info) else ""
 
 
@@ -60,17 +81,16 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     os.makedirs(BUILD_DIR, exist_ok=True)
     newest_header = headers_mtime()
     todo, objects = [], []
-    for source in sources():
-        obj = os.path.join(BUILD_DIR, os.path.basename(source)[:-3] + ".o")
+    for source, obj, flags in units():
         objects.append(obj)
         stale = (force or ptxas_info or not os.path.exists(obj)
                  or os.path.getmtime(obj) < max(os.path.getmtime(source), newest_header))
         if stale:
-            todo.append(source)
+            todo.append((source, obj, flags))
     if todo:
         workers = min(len(todo), max(1, (os.cpu_count() or 2)))
         with concurrent.futures.ThreadPoolExecutor(max_workers=workers) as pool:
-            for obj, log in pool.map(lambda s: compile_one(nvcc, s, verbose, ptxas_info), todo):
+            for obj, log in pool.map(lambda unit: compile_one(nvcc, unit, verbose, ptxas_info), todo):
                 if log:
                     print(log, file=sys.stderr)
     wanted = {os.path.basename(o) for o in objects}

@@ -37,7 +37,7 @@ int check_ptr(const luna_uvu_plan* plan, const void* p, const char* name, bool r
 }
 
 bool use_fast(const luna_uvu_plan* plan, std::initializer_list<const void*> pointers) {
-  if (!plan->fast_ok || plan->force_generic || !fast_available()) return false;
+  if ((!plan->fast_ok && plan->edge.shape < 0) || plan->force_generic || !fast_available()) return false;
   for (const void* p : pointers)
     if (p && !aligned_to(p, 16)) return false;  // bulk copies and 128-bit accesses need 16-byte rows
   return true;
@@ -59,7 +59,7 @@ int zero_fill(void* p, int64_t numel, size_t elem, cudaStream_t stream) {
 extern "C" int64_t luna_uvu_plan_query(const luna_uvu_plan* plan, int what) {
   if (!plan) return -1;
   switch (what) {
-    case LUNA_PLAN_FAST_PATH: return plan->fast_ok && !plan->force_generic;
+    case LUNA_PLAN_FAST_PATH: return (plan->fast_ok || plan->edge.shape >= 0) && !plan->force_generic;
     case LUNA_PLAN_CHANNELS_PER_LANE: return plan->fast_ok ? plan->fast.cpl : 0;
     case LUNA_PLAN_CHANNEL_CHUNKS: return plan->fast_ok ? plan->fast.chunks : 0;
     case LUNA_PLAN_FWD_SMEM_BYTES: return fast_smem_bytes(plan, 0);

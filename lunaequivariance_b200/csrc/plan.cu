@@ -199,12 +199,9 @@ bool fill_layout(luna_uvu_plan* plan, FastMeta& f, int cpl) {
     if (canon) f.canon_l2 = L2;
     // sparse term list: every path's terms must have exactly the compiled-in pattern
     f.sparse_terms = 0;
-    plan->sp_c.clear();
-    plan->sp_j.clear();
     if (canon && L2 <= 3 && f.LX <= 3 && f.LO <= 3) {
       const int total_terms = fastk::canon_toff(f.LX, L2, f.LO, -1, -1, -1);
-      std::vector<double> sc(static_cast<size_t>(total_terms), 0.0);
-      std::vector<unsigned char> sj(static_cast<size_t>(total_terms), 0);
+      std::vector<char> seen(static_cast<size_t>(total_terms), 0);
       bool match = true;
       for (size_t q = 0; q < order.size() && match; ++q) {
         const PathRec& p = paths[order[q]];
@@ -220,21 +217,16 @@ bool fill_layout(luna_uvu_plan* plan, FastMeta& f, int cpl) {
             int slot = -1;
             for (int u = 0; u < n; ++u)
               if (pattern[u].i == term.a && pattern[u].j == term.b && pattern[u].k == k) slot = u;
-            if (slot < 0 || sc[toff + slot] != 0.0) {
+            if (slot < 0 || seen[toff + slot]) {
               match = false;
             } else {
-              sc[toff + slot] = term.c;
-              sj[toff + slot] = static_cast<unsigned char>(p.y_off + term.b);
+              seen[toff + slot] = 1;
               ++found;
             }
           }
         if (found != n) match = false;  // a pattern entry the plan does not have would be a wasted (zero) term
       }
-      if (match) {
-        f.sparse_terms = total_terms;
-        plan->sp_c = sc;
-        plan->sp_j = sj;
-      }
+      if (match) f.sparse_terms = total_terms;
     }
   }
 
@@ -327,14 +319,10 @@ Tuning tuning_from_environment() {
     return value ? std::atoll(value) : 0;
   };
   t.no_canon = std::getenv("LUNA_B200_NO_CANON") != nullptr;
-  t.no_sparse = std::getenv("LUNA_B200_NO_SPARSE") != nullptr;
-  t.no_plain = std::getenv("LUNA_B200_NO_PLAIN") != nullptr;
-  if (const char* kind = std::getenv("LUNA_B200_BWD_KERNEL"))
-    t.bwd_kernel = kind[0] == 'r' ? 1 : (kind[0] == 'u' ? 2 : 0);
   t.max_warps = static_cast<int>(std::max(0ll, number("LUNA_B200_MAXW")));
-  t.row_stages = static_cast<int>(std::max(0ll, number("LUNA_B200_ROW_STAGES")));
   t.edges_per_warp = std::max(0ll, number("LUNA_B200_EPW"));
   t.fwd_tile_edges = std::max(0ll, number("LUNA_B200_FWD_TILE"));
+  t.lane_channels = static_cast<int>(std::max(0ll, number("LUNA_B200_LANE_CHANNELS")));
   return t;
 }
 
@@ -421,17 +409,17 @@ int get_device_tables(luna_uvu_plan* plan, const DeviceTables** out) {
     std::memcpy(blob.data() + f.tb_ellj, plan->ell_j.data(), plan->ell_j.size());
   }
   const size_t o_blob = append(blob.data(), blob.size());
-  std::vector<unsigned char> spc(plan->sp_c.size() * scalar);
-  for (size_t i = 0; i < plan->sp_c.size(); ++i) {
-    if (f64) {
-      std::memcpy(spc.data() + i * 8, &plan->sp_c[i], 8);
-    } else {
-      float v = static_cast<float>(plan->sp_c[i]);
-      std::memcpy(spc.data() + i * 4, &v, 4);
+  auto append_scalars = [&](const std::vector<double>& values) {
+    std::vector<unsigned char> raw(values.size() * scalar);
+    for (size_t i = 0; i < values.size(); ++i) {
+      const float narrow = static_cast<float>(values[i]);
+      std::memcpy(raw.data() + i * scalar, f64 ? static_cast<const void*>(&values[i]) : &narrow, scalar);
     }
-  }
-  const size_t o_spc = append(spc.data(), spc.size());
-  const size_t o_spj = append(plan->sp_j.data(), plan->sp_j.size());
+    return append(raw.data(), raw.size());
+  };
+  const EdgePlan& edge = plan->edge;
+  const size_t o_epc = append_scalars(edge.prog_c), o_etc = append_scalars(edge.term_c);
+  const size_t o_epj = append(edge.prog_j.data(), edge.prog_j.size() * sizeof(unsigned short));
 
   DeviceTables dt;
   dt.bytes = host.size();
@@ -461,8 +449,9 @@ int get_device_tables(luna_uvu_plan* plan, const DeviceTables** out) {
   dt.ell_j = base + o_mj;
   dt.ell_c = base + o_mc;
   dt.bwd_tables = base + o_blob;
-  dt.sp_c = base + o_spc;
-  dt.sp_j = base + o_spj;
+  dt.edge_prog_c = base + o_epc;
+  dt.edge_term_c = base + o_etc;
+  dt.edge_prog_j = reinterpret_cast<const unsigned short*>(base + o_epj);
   LUNA_CUDA_CHECK(cudaDeviceGetAttribute(&dt.sm_count, cudaDevAttrMultiProcessorCount, device));
   LUNA_CUDA_CHECK(cudaDeviceGetAttribute(&dt.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   auto inserted = plan->device_tables.emplace(device, dt);
@@ -588,6 +577,7 @@ extern "C" int luna_uvu_plan_create(const luna_uvu_desc* desc, luna_uvu_plan** o
   }
   plan->out_fully_covered = std::all_of(out_cover.begin(), out_cover.end(), [](char c) { return c != 0; });
   analyse_fast(plan);
+  edgek::analyse(plan);
   *out = plan;
   return LUNA_OK;
 }

@@ -66,8 +66,8 @@ struct CopyPiece {
 struct FastMeta {
   int LX, LO;                 // highest degree present in x / out
   int canon_l2;               // highest edge-harmonic degree if the path list is the canonical full list, else -1
-  int sparse_terms;           // length of the sparse term list (canon_toff total) if the plan's coupling terms have
-                              // the compiled-in patterns and y is laid out as degrees 0..L2 in order, else 0
+  int sparse_terms;           // length of the term list (canon_toff total) if the plan's coupling terms have the
+                              // patterns of cg_patterns.h and y is laid out as degrees 0..L2 in order, else 0
   int cpl;                    // channels per lane
   int chunks;                 // channel chunks per feature block (a warp handles 32 * cpl channels)
   int ch;                     // channels per block (uniform)
@@ -104,22 +104,18 @@ struct FastMeta {
 // ------------------------------------------------------------------------------------------------ the plan
 // Settings that select kernel variants or override a launch policy.  They come from LUNA_B200_* environment
 // variables, read once when the plan is created (never on a launch path):
-//   LUNA_B200_NO_CANON=1        canonical path lists run the kernels that loop over run-time path tables
-//   LUNA_B200_NO_SPARSE=1       backward without the compiled-in coupling patterns
-//   LUNA_B200_NO_PLAIN=1        backward without the kernels that have the layout compiled in
-//   LUNA_B200_BWD_KERNEL=row|units   data-movement variant of the backward kernel with compiled-in patterns
+//   LUNA_B200_NO_CANON=1        path lists with compiled kernels run the kernels that loop over run-time path tables
 //   LUNA_B200_MAXW=n            cap on warps per CTA
-//   LUNA_B200_ROW_STAGES=n      cap on weight-row stages of the row-staged backward
-//   LUNA_B200_EPW=n             backward: edges per tile of source nodes (kernels with a compile-time layout), target
-//                               edges per warp when a graph needs several waves (the others)
-//   LUNA_B200_FWD_TILE=n        forward: edges per tile of destination nodes
+//   LUNA_B200_EPW=n             backward: edges per tile of source rows (edge kernels), target edges per warp when a
+//                               graph needs several waves (table kernels)
+//   LUNA_B200_FWD_TILE=n        forward of the table kernels: edges per tile of destination nodes
+//   LUNA_B200_LANE_CHANNELS=n   channels per lane of the edge kernels
 struct Tuning {
-  bool no_canon = false, no_sparse = false, no_plain = false;
-  int bwd_kernel = 0;  // 0 automatic, 1 row stages, 2 unit ring
+  bool no_canon = false;
   int max_warps = 0;   // 0: no cap
-  int row_stages = 0;  // 0: no cap
   int64_t edges_per_warp = 0;  // 0: the kernel's default
   int64_t fwd_tile_edges = 0;  // 0: the kernel's default
+  int lane_channels = 0;       // 0: chosen by the channel count
 };
 Tuning tuning_from_environment();
 
@@ -147,11 +143,22 @@ struct DeviceTables {
   // entry indices of the edge-attribute gradient's program (gy[j] = sum_t c[t] * G[m[t]]), y indices of the
   // padded program; offsets in FastMeta::tb_*
   const unsigned char* bwd_tables = nullptr;
-  // sparse term list of a canonical plan (FastMeta::sparse_terms entries): coefficient and y index of each term
-  const void* sp_c = nullptr;
-  const unsigned char* sp_j = nullptr;
+  // edge kernels (EdgePlan): the coupling-matrix program and the term list
+  const void* edge_prog_c = nullptr;
+  const unsigned short* edge_prog_j = nullptr;
+  const void* edge_term_c = nullptr;
   int sm_count = 0;
   int max_smem_optin = 0;
+};
+
+// What the edge kernels (uvu_edge.cuh) need of a plan whose path list has one of their compiled shapes.
+struct EdgePlan {
+  int shape = -1;      // index of the compiled shape, -1 if the plan has none or is kept from its kernels
+  int ch = 0;          // channels per block
+  int cpl = 0;         // channels per lane
+  int team_warps = 0;  // warps that share an edge
+  std::vector<double> prog_c, term_c;
+  std::vector<unsigned short> prog_j;
 };
 
 }  // namespace luna
@@ -176,12 +183,11 @@ struct luna_uvu_plan {
   bool force_generic = false;
   luna::Tuning tuning{};
   luna::FastMeta fast{};
+  luna::EdgePlan edge{};
   std::vector<double> ell_c;
   std::vector<unsigned char> ell_j;
   std::vector<int> gy_ptr, gy_m;
   std::vector<double> gy_c;
-  std::vector<double> sp_c;
-  std::vector<unsigned char> sp_j;
 
   std::mutex mutex;
   std::map<int, luna::DeviceTables> device_tables;
@@ -234,6 +240,16 @@ enum FreeSlot { kFreeG = 0, kFreeX = 1, kFreeY = 2, kFreeW = 3 };
 // pointers of the plan's dtype; the pointer in the free position is ignored.
 int generic_contract(luna_uvu_plan* plan, const luna_graph* graph, int free_slot, const void* x, const void* y,
                      const void* w, const void* g, void* out, bool accumulate, cudaStream_t stream);
+
+// Edge kernels (uvu_edge.cu): analyse() decides at plan creation whether they serve the plan.
+namespace edgek {
+void analyse(luna_uvu_plan* plan);
+int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
+            const void* w, void* out, bool accumulate, cudaStream_t stream);
+int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
+             const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w,
+             cudaStream_t stream);
+}  // namespace edgek
 
 // Staged kernels (bulk-copy pipeline).  fast_available() is false in a build without them.
 bool fast_available();

@@ -1,0 +1,133 @@
+// Which plans the edge kernels serve, the tables they read, and the choice of the compiled instance.
+#include "uvu_edge.cuh"
+
+namespace luna {
+namespace edgek {
+
+namespace {
+
+// Channels per lane and warps per team: a warp's pass over an edge costs about one unit of fixed work plus one per
+// channel of a lane, so 48 channels take one warp with two channels on 24 lanes, 96 one warp with four on 24 lanes.
+bool choose_lanes(luna_uvu_plan* plan, int ch) {
+  const int widest = plan->dtype == LUNA_F64 ? 2 : 4;
+  int best = 0;
+  for (int cpl = widest; cpl >= 1; cpl /= 2) {
+    if (plan->tuning.lane_channels > 0 && cpl != plan->tuning.lane_channels) continue;
+    const int team = (ch + 32 * cpl - 1) / (32 * cpl);
+    if (team > 8 || ch % (team * cpl) != 0) continue;
+    const int cost = team * (1 + cpl);
+    if (best != 0 && cost >= best) continue;
+    best = cost;
+    plan->edge.cpl = cpl;
+    plan->edge.team_warps = team;
+  }
+  return best != 0;
+}
+
+template <typename S>
+bool match_shape(luna_uvu_plan* plan) {
+  const auto& paths = plan->paths;
+  const int ch = paths[0].ch;
+  if (static_cast<int>(paths.size()) != S::paths || plan->X != S::XD * ch || plan->O != S::OD * ch || plan->Y != S::YD ||
+      plan->W != S::paths * ch)
+    return false;
+  std::vector<double> term_c(S::terms, 0.0), prog_c(2 * S::m_total, 0.0);
+  std::vector<unsigned short> prog_j(S::m_total, 0);
+  std::vector<int> entry_terms(S::m_total, 0);
+  for (const PathRec& p : paths) {
+    const int l1 = (p.d1 - 1) / 2, l2 = (p.d2 - 1) / 2, l3 = (p.d3 - 1) / 2;
+    if (p.ch != ch || p.w_stride != 1 || l1 > 3 || l2 > 3 || l3 > 3 || !S::ok(l1, l2, l3)) return false;
+    if (p.x_off != ch * S::xoff(l1) || p.y_off != S::yoff(l2) || p.out_off != ch * S::ooff(l3) ||
+        p.w_off != ch * S::rank(l1, l2, l3))
+      return false;
+    // the terms: exactly the compiled-in pattern
+    const CgTerm* pattern = cg_pattern(l1, l2, l3);
+    const int n = cg_count(l1, l2, l3), toff = S::toff(l1, l2, l3), moff = S::moff(l1, l2, l3);
+    std::vector<char> seen(n, 0);
+    int found = 0;
+    for (int k = 0; k < p.d3; ++k)
+      for (int t = plan->rowptr_k[p.byk_ptr + k]; t < plan->rowptr_k[p.byk_ptr + k + 1]; ++t) {
+        const auto& term = plan->terms_k[t];  // (a, b) = (i, j)
+        int slot = -1;
+        for (int u = 0; u < n; ++u)
+          if (pattern[u].i == term.a && pattern[u].j == term.b && pattern[u].k == k) slot = u;
+        if (slot < 0 || seen[slot]) return false;
+        seen[slot] = 1;
+        ++found;
+        term_c[toff + slot] = term.c;
+        int entry = moff - 1;  // the term's (i, k) among the pattern's distinct ones
+        for (int u = 0; u <= slot; ++u)
+          entry += u == 0 || pattern[u].i != pattern[u - 1].i || pattern[u].k != pattern[u - 1].k;
+        const int which = entry_terms[entry]++;
+        if (which > 1) return false;  // degrees up to 3 have at most two terms per entry
+        prog_c[which * S::m_total + entry] = term.c;
+        prog_j[entry] = static_cast<unsigned short>(prog_j[entry] | (p.y_off + term.b) << (8 * which));
+      }
+    if (found != n) return false;
+  }
+  plan->edge.ch = ch;
+  plan->edge.term_c = term_c;
+  plan->edge.prog_c = prog_c;
+  plan->edge.prog_j = prog_j;
+  return true;
+}
+
+template <int ID>
+int find_shape(luna_uvu_plan* plan) {
+  if constexpr (ID < kEdgeShapes) {
+    return match_shape<ShapeOf<ID>>(plan) ? ID : find_shape<ID + 1>(plan);
+  } else {
+    return -1;
+  }
+}
+
+// Calls body with the compiled instance of a plan.
+template <typename T, int CPL, int ID, typename F>
+int with_shape(int shape, F&& body) {
+  if constexpr (ID < kEdgeShapes) {
+    if (shape == ID) return body(EdgeKernels<T, CPL, ID>{});
+    return with_shape<T, CPL, ID + 1>(shape, body);
+  } else {
+    return fail(LUNA_ERR_UNSUPPORTED, "no edge kernel of shape %d", shape);
+  }
+}
+template <typename F>
+int with_instance(const luna_uvu_plan* plan, F&& body) {
+  const EdgePlan& ep = plan->edge;
+  if (plan->dtype == LUNA_F64)
+    return ep.cpl == 2 ? with_shape<double, 2, 0>(ep.shape, body) : with_shape<double, 1, 0>(ep.shape, body);
+  if (ep.cpl == 4) return with_shape<float, 4, 0>(ep.shape, body);
+  return ep.cpl == 2 ? with_shape<float, 2, 0>(ep.shape, body) : with_shape<float, 1, 0>(ep.shape, body);
+}
+
+}  // namespace
+
+void analyse(luna_uvu_plan* plan) {
+  plan->edge = EdgePlan{};
+  if (plan->paths.empty() || plan->tuning.no_canon) return;
+  const int ch = plan->paths[0].ch;
+  const int elem = plan->dtype == LUNA_F64 ? 8 : 4;
+  if (ch * elem % 16 != 0) return;  // bulk copies move whole 16-byte pieces
+  if (!choose_lanes(plan, ch)) return;
+  // one team with two stages must fit an SM's shared memory in either direction
+  const size_t room = 200 * 1024, W = static_cast<size_t>(plan->W) * elem, X = static_cast<size_t>(plan->X) * elem,
+               O = static_cast<size_t>(plan->O) * elem;
+  if (std::max(std::max(2 * W + O, 2 * (W + X)), std::max(X, O)) + plan->edge.team_warps * 8192 > room) return;
+  plan->edge.shape = find_shape<0>(plan);
+}
+
+int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
+            const void* w, void* out, bool accumulate, cudaStream_t stream) {
+  const EdgeForwardArgs args{x, y, w, out, accumulate};
+  return with_instance(plan, [&](auto kernels) { return kernels.forward(plan, dt, graph, args, stream); });
+}
+
+int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
+             const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w,
+             cudaStream_t stream) {
+  const EdgeBackwardArgs args{x, y, w, g, gx, gy, gw, acc_x, acc_y, acc_w};
+  return with_instance(plan, [&](auto kernels) { return kernels.backward(plan, dt, graph, args, stream); });
+}
+
+}  // namespace edgek
+}  // namespace luna

@@ -1,0 +1,348 @@
+// Common parts of the edge kernels: the convolution's forward and first derivatives for path lists that are complete
+// over three sets of degrees, with everything about the list compiled in.
+//
+// A shape is three sets of degrees (x, edge attributes, out) as bit masks.  Its list is every (l1, l2, l3) from the
+// sets that satisfies the triangle rule and has an even degree sum, in that order, which is also the order of the
+// weight blocks: first layers (scalars in), interior layers and last layers (scalars out) of the usual networks, and
+// single couplings.  The number of channels is not compiled in.
+//
+// Teams.  A team of one or more warps of a CTA walks the edges of a row (a destination in the forward, a source in the
+// backward kernel); warp t of a team of n owns channels [t, t + 1) * ch / n of every block, and a lane owns CPL of them
+// (lanes beyond the warp's channels repeat the last lane's addresses and contribute zeros).
+// One lane of the team stages an edge's rows - the whole weight row, the whole gathered node row - with one bulk copy
+// each, whatever the number of warps: DRAM sees requests of full rows.
+//
+// Two ways of handing out rows.  Large launches: a team takes tiles of consecutive rows from a counter.  Small
+// launches, in which a row per team would leave the chip waiting for the longest rows: `group` teams of a CTA share a
+// row, each a contiguous part of its edges, and the parts are summed in a fixed order through shared memory.  A row's
+// sum depends on its own edges and on `group`, not on which team got it.
+#pragma once
+
+#include <atomic>
+
+#include "uvu_fast.cuh"
+#include "uvu_packets.cuh"
+
+namespace luna {
+namespace edgek {
+
+using namespace fastk;
+
+constexpr int kEdgeMaxStages = 4;
+constexpr int kEdgeMaxWarps = 32;
+
+// ---- shapes ---------------------------------------------------------------------------------------------------------
+template <int MX_, int MY_, int MO_>
+struct Shape {
+  static constexpr int MX = MX_, MY = MY_, MO = MO_;
+  static constexpr bool has(int mask, int l) { return ((mask >> l) & 1) != 0; }
+  // components of the degrees below l
+  static constexpr int below(int mask, int l) {
+    int n = 0;
+    for (int a = 0; a < l; ++a)
+      if (has(mask, a)) n += 2 * a + 1;
+    return n;
+  }
+  static constexpr int XD = below(MX, 4), YD = below(MY, 4), OD = below(MO, 4);
+  static constexpr int xoff(int l) { return below(MX, l); }
+  static constexpr int yoff(int l) { return below(MY, l); }
+  static constexpr int ooff(int l) { return below(MO, l); }
+  static constexpr bool ok(int l1, int l2, int l3) {
+    const int lo = l1 > l2 ? l1 - l2 : l2 - l1;
+    return has(MX, l1) && has(MY, l2) && has(MO, l3) && l3 >= lo && l3 <= l1 + l2 && (l1 + l2 + l3) % 2 == 0;
+  }
+  // position of a path's weight block; past-the-end arguments give the number of paths
+  static constexpr int rank(int a, int b, int c) {
+    int r = 0;
+    for (int l1 = 0; l1 < 4; ++l1)
+      for (int l2 = 0; l2 < 4; ++l2)
+        for (int l3 = 0; l3 < 4; ++l3) {
+          if (l1 == a && l2 == b && l3 == c) return r;
+          if (ok(l1, l2, l3)) ++r;
+        }
+    return r;
+  }
+  static constexpr int paths = rank(-1, -1, -1);
+  // first entry of a path in an edge's coupling-matrix buffer: the entries that some edge attribute reaches, in (i, k)
+  // order, paths in (l3, l1, l2) order, every path padded to a multiple of four
+  static constexpr int moff(int a, int b, int c) {
+    int m = 0;
+    for (int l3 = 0; l3 < 4; ++l3)
+      for (int l1 = 0; l1 < 4; ++l1)
+        for (int l2 = 0; l2 < 4; ++l2) {
+          if (!ok(l1, l2, l3)) continue;
+          if (l1 == a && l2 == b && l3 == c) return m;
+          m += (cg_pair_count(l1, l2, l3) + 3) / 4 * 4;
+        }
+    return m;
+  }
+  static constexpr int m_total = moff(-1, -1, -1);
+  static constexpr int m_rounds = (m_total + 31) / 32;
+  // first coupling term of a path in the term list: (l3, l1, l2) order, every path's terms padded to a multiple of four
+  static constexpr int toff(int a, int b, int c) {
+    int t = 0;
+    for (int l3 = 0; l3 < 4; ++l3)
+      for (int l1 = 0; l1 < 4; ++l1)
+        for (int l2 = 0; l2 < 4; ++l2) {
+          if (!ok(l1, l2, l3)) continue;
+          if (l1 == a && l2 == b && l3 == c) return t;
+          t += (cg_count(l1, l2, l3) + 3) / 4 * 4;
+        }
+    return t;
+  }
+  static constexpr int terms = toff(-1, -1, -1);
+  static constexpr int top(int mask) { return mask >= 8 ? 3 : (mask >= 4 ? 2 : (mask >= 2 ? 1 : 0)); }
+  static constexpr int LO = top(MO);
+};
+
+// The compiled shapes: network layers with edge harmonics to degree 1, 2 or 3 - first, interior, last - and the single
+// vector-vector-scalar coupling.
+constexpr int kEdgeShapes = 11;
+constexpr int kEdgeShapeMasks[kEdgeShapes][3] = {{1, 3, 3},  {1, 7, 7},   {1, 15, 15}, {3, 3, 3},   {7, 7, 7}, {15, 15, 15},
+                                                 {7, 15, 15}, {3, 3, 1},  {7, 7, 1},   {15, 15, 1}, {2, 2, 1}};
+template <int ID>
+using ShapeOf = Shape<kEdgeShapeMasks[ID][0], kEdgeShapeMasks[ID][1], kEdgeShapeMasks[ID][2]>;
+
+// ---- launch arguments, type-erased ------------------------------------------------------------------------------------
+struct EdgeForwardArgs {
+  const void *x, *y, *w;
+  void* out;
+  bool accumulate;
+};
+struct EdgeBackwardArgs {
+  const void *x, *y, *w, *g;
+  void *gx, *gy, *gw;
+  bool acc_x, acc_y, acc_w;
+};
+// The kernels of one (element type, channels per lane, shape), compiled in a file of their own.
+template <typename T, int CPL, int ID>
+struct EdgeKernels {
+  static int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
+                     const EdgeForwardArgs& a, cudaStream_t stream);
+  static int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
+                      const EdgeBackwardArgs& a, cudaStream_t stream);
+};
+
+// ---- how a launch is laid out -----------------------------------------------------------------------------------------
+struct EdgeLaunch {
+  int warps = 0;   // per CTA
+  int stages = 0;  // per team
+  int split = 0;   // backward: g in one slot per degree instead of in the stages
+  size_t bytes = 0;
+};
+// Rows shared by `group` teams, or 1: rows are handed out in tiles.
+struct EdgeSplit {
+  int group = 1;
+  int64_t blocks = 1;
+  int64_t tile_rows = 1;
+};
+
+constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
+
+// Small launches.  With R rows of d edges and T teams on the chip, a row per team takes d * ceil(R / T) edge steps of
+// the last team; parts of a row per team take about d * R / T.  Sharing costs two barriers and a pass through shared
+// memory per row, so it stops where the tiles of the large launches are even enough.
+inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps) {
+  EdgeSplit s;
+  const int64_t all = static_cast<int64_t>(sm_count) * teams;
+  const double degree = static_cast<double>(edges) / static_cast<double>(std::max<int64_t>(rows, 1));
+  if (rows <= 4 * all && degree >= 4.0) {
+    // enough parts that every SM has work, and at least two edges in a part
+    int want = rows * 2 <= all ? 8 : (rows <= 2 * all ? 4 : 2);
+    while (want > 1 && (want > teams || teams % want != 0 || degree < 2.0 * want)) want /= 2;
+    if (want > 1 && team_warps > 1 && teams + teams / want > kNamedBarriers) want = 1;
+    s.group = want;
+  }
+  if (s.group > 1) {
+    s.blocks = std::max<int64_t>(1, std::min<int64_t>(sm_count, rows));
+    return s;
+  }
+  const int64_t tile_edges = tile_edges_for(edges, all, 64);
+  s.tile_rows = std::min<int64_t>(1 << 20, std::max<int64_t>(1, static_cast<int64_t>(tile_edges / std::max(degree, 1e-3) + 0.5)));
+  const int64_t tiles = ceil_div(std::max<int64_t>(rows, 1), s.tile_rows);
+  s.blocks = std::max<int64_t>(1, std::min<int64_t>(sm_count, ceil_div(tiles, teams)));
+  return s;
+}
+
+// ---- coupling patterns --------------------------------------------------------------------------------------------------
+// Terms of a pattern are sorted by (i, k, j).  The end of the row of term t0, and the position of term t's (i, k) among
+// the pattern's distinct ones.
+template <typename PT>
+__host__ __device__ constexpr int edge_row_end(int t0) {
+  int t = t0;
+  while (t < PT::n && PT::t[t].i == PT::t[t0].i) ++t;
+  return t;
+}
+template <typename PT>
+__host__ __device__ constexpr bool edge_new_entry(int t) {
+  return t == 0 || PT::t[t].i != PT::t[t - 1].i || PT::t[t].k != PT::t[t - 1].k;
+}
+template <typename PT>
+__host__ __device__ constexpr bool edge_new_row(int t) {
+  return t == 0 || PT::t[t].i != PT::t[t - 1].i;
+}
+template <typename PT>
+__host__ __device__ constexpr int edge_entry(int t) {
+  int e = -1;
+  for (int q = 0; q <= t; ++q) e += edge_new_entry<PT>(q) ? 1 : 0;
+  return e;
+}
+
+// ---- device helpers ---------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// Synchronises the warps of a team (its own barrier, unless it is one warp).
+__device__ __forceinline__ void team_sync(int team_warps, int team_id) {
+  if (team_warps == 1)
+    __syncwarp();
+  else
+    named_barrier(1 + team_id, team_warps * 32);
+}
+// After one wait has run out the kernel keeps its control flow (other warps may be waiting for it at a barrier), writes
+// nothing more to rely on, and stops spending time on waits.
+constexpr uint32_t kWaitAfterFailure = 64;
+__device__ __forceinline__ bool edge_wait(uint64_t* bar, uint32_t parity, bool alive) {
+  const uint32_t limit = alive ? kWaitLimit : kWaitAfterFailure;
+#pragma unroll 1
+  for (uint32_t spin = 0; spin < limit; ++spin)
+    if (mbar_try_wait(bar, parity)) return true;
+  return false;
+}
+__device__ __forceinline__ void bulk_reduce_add_s2g(float* dst, const float* src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst),
+               "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_reduce_add_s2g(double* dst, const double* src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(dst),
+               "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
+// Four consecutive entries of a 16-byte aligned table; every lane reads the same address.
+template <typename T>
+__device__ __forceinline__ void edge_load_four(const T* p, T* out) {
+  constexpr int per = 16 / static_cast<int>(sizeof(T));
+#pragma unroll
+  for (int v = 0; v < 4 / per; ++v) {
+    const Vec<T, per> t = reinterpret_cast<const Vec<T, per>*>(p)[v];
+#pragma unroll
+    for (int c = 0; c < per; ++c) out[v * per + c] = t.a[c];
+  }
+}
+
+// A lane's channels.  Packet q of a lane holds PK::W consecutive channels, and the packets of the warp's lanes lie side
+// by side: packet q of lane l starts at channel  own + q * stride  with  own = first + W * l  and  stride = W * lanes.
+// Weights then arrive as ready-made packets, and the scalar loads that assemble the packets of a node row (channel-
+// major, 2l + 1 components) meet two-way bank conflicts at most (with four consecutive channels per lane: four-way).
+template <typename PK, typename T>
+__device__ __forceinline__ void lane_load(const T* p, int stride, typename PK::V* out) {
+#pragma unroll
+  for (int q = 0; q < PK::NP; ++q) {
+    if constexpr (PK::W == 2)
+      out[q].v = *reinterpret_cast<const unsigned long long*>(p + q * stride);
+    else
+      out[q] = p[q * stride];
+  }
+}
+template <typename PK, typename T>
+__device__ __forceinline__ void lane_store(T* p, int stride, const typename PK::V* in) {
+#pragma unroll
+  for (int q = 0; q < PK::NP; ++q) {
+    if constexpr (PK::W == 2)
+      *reinterpret_cast<unsigned long long*>(p + q * stride) = in[q].v;
+    else
+      p[q * stride] = in[q];
+  }
+}
+// Components of a node row's block of D components per channel -> packets [component][packet]; p: the block plus
+// own * D, stride as above.  Scalar loads on purpose: the two halves then land in the pair's registers, while halves
+// taken from vector loads are put together again in front of every packed instruction that uses the pair (measured on
+// the 128-channel degree-(2,3,3) backward: 18.9 ms against 11.4).
+template <typename PK, typename T, int D>
+__device__ __forceinline__ void lane_load_block(const T* p, int stride, typename PK::V* out) {
+  using V = typename PK::V;
+#pragma unroll
+  for (int q = 0; q < PK::NP; ++q)
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      T vals[PK::W];
+#pragma unroll
+      for (int c = 0; c < PK::W; ++c) vals[c] = p[q * stride * D + c * D + i];
+      out[i * PK::NP + q] = make_packet(vals, V{});
+    }
+}
+// Packets [component][packet] to such a block in memory, added to what is there if `add`.
+template <typename PK, typename T, int D>
+__device__ __forceinline__ void lane_store_block(T* p, int stride, const typename PK::V* in, bool add) {
+#pragma unroll
+  for (int q = 0; q < PK::NP; ++q) {
+    T row[PK::W * D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      T vals[PK::W];
+      split_packet(in[i * PK::NP + q], vals);
+#pragma unroll
+      for (int c = 0; c < PK::W; ++c) row[c * D + i] = vals[c];
+    }
+    T* to = p + q * stride * D;
+    if (add) {
+      T old[PK::W * D];
+      load_vectors<T, PK::W, D>(to, old);
+#pragma unroll
+      for (int a = 0; a < PK::W * D; ++a) row[a] += old[a];
+    }
+    store_vectors<T, PK::W, D>(to, row);
+  }
+}
+
+// The program that turns an edge's attributes, one per lane, into its coupling matrices: entry m is a_m y[ja] + b_m
+// y[jb].  Lane l makes entries l, l + 32, ...
+template <typename T, typename S>
+struct MatrixProgram {
+  T a[S::m_rounds], b[S::m_rounds];
+  unsigned j[(S::m_rounds + 1) / 2];  // two attribute indices of 8 bits per round
+  __device__ __forceinline__ void load(const T* coefficients, const unsigned short* attributes, int lane) {
+#pragma unroll
+    for (int r = 0; r < (S::m_rounds + 1) / 2; ++r) j[r] = 0u;
+#pragma unroll
+    for (int r = 0; r < S::m_rounds; ++r) {
+      const int m = r * 32 + lane;
+      a[r] = m < S::m_total ? coefficients[m] : T(0);
+      b[r] = m < S::m_total ? coefficients[S::m_total + m] : T(0);
+      j[r / 2] |= (m < S::m_total ? static_cast<unsigned>(attributes[m]) : 0u) << (16 * (r % 2));
+    }
+  }
+  __device__ __forceinline__ void run(T y, T* to, int lane) const {
+#pragma unroll
+    for (int r = 0; r < S::m_rounds; ++r) {
+      const T ya = __shfl_sync(0xffffffffu, y, static_cast<int>((j[r / 2] >> (16 * (r % 2))) & 255u));
+      const T yb = __shfl_sync(0xffffffffu, y, static_cast<int>((j[r / 2] >> (16 * (r % 2) + 8)) & 255u));
+      to[r * 32 + lane] = fma(b[r], yb, a[r] * ya);
+    }
+  }
+};
+
+// Warps per CTA by the registers a lane is going to need (an estimate from the state it keeps): the launch bound caps
+// the registers at 65,536 / threads.
+__host__ __device__ constexpr int warps_for(int regs) {
+  return regs <= 60 ? 24 : (regs <= 120 ? 16 : (regs <= 150 ? 12 : 8));
+}
+
+// Attributes a kernel needs set once per device, not on every launch.
+struct KernelSetup {
+  std::atomic<uint64_t> done{0};
+  int once(const void* kernel, int max_smem) {
+    int device = 0;
+    LUNA_CUDA_CHECK(cudaGetDevice(&device));
+    const uint64_t bit = 1ull << (device & 63);
+    if (device < 64 && (done.load(std::memory_order_acquire) & bit)) return LUNA_OK;
+    LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+    LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (device < 64) done.fetch_or(bit, std::memory_order_release);
+    return LUNA_OK;
+  }
+};
+
+}  // namespace edgek
+}  // namespace luna

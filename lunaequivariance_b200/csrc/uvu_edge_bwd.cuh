@@ -1,0 +1,605 @@
+// Backward kernel of the edge family: gx, gy and gw of one pass over the edges, grouped by source row.
+//
+// With the pattern of every coupling tensor compiled in, a path is a straight line over its terms t = (i, j, k):
+//     s_i   = sum_k M_ik g_k                 M_ik = sum_j c_ijk y_j is made by the warp, one edge ahead
+//     gx_i += w_p s_i,   gw_p = sum_i x_i s_i
+//     P_ik  = sum over the lane's channels of (x_i w_p) g_k,    gy_j += c_t P_ik
+// so gx stays in registers for the whole row, gy is contracted inside each lane and only its few values cross lanes,
+// and the weight gradients overwrite the weights in shared memory and leave as one row with one bulk store (or one bulk
+// add, when a call accumulates).
+//
+// Staging.  A stage holds an edge's weight row and, where two such stages per team fit, its g[dst] row.  Where they do
+// not, g goes through two slots, one for the highest output degree and one for the others, each refilled for the next
+// edge as soon as its degrees are done (one slot per degree: 2 % slower, for the two more waits and copies per edge).
+// Weights are not read at all by calls that want gw alone: gw does not depend on them.
+//
+// Every wait is bounded; a wait that runs out sets the plan's status word.
+#pragma once
+
+#include "uvu_edge.cuh"
+
+namespace luna {
+namespace edgek {
+
+constexpr int kEdgeMaxSlots = 2;
+
+template <typename T>
+struct EdgeBwdParams {
+  const T *x, *y, *w, *g;
+  T *gx, *gy, *gw;
+  const int *dst, *src_rowptr, *edge_ids;
+  const T* prog_c;               // [2][m_total] coefficients of the two attributes a matrix entry depends on
+  const unsigned short* prog_j;  // [m_total] the two attributes, 8 bits each
+  const T* term_c;               // [terms] coefficients of the coupling terms
+  int* status;
+  unsigned* tile_counters;
+  int64_t num_rows, tile_rows, tile_edges, num_tiles;  // tile_rows 0: tiles are stretches of tile_edges edges
+  float rows_per_edge;
+  int ch, team_warps, teams, group;
+  int stages, split;
+  int team_elems;  // shared memory per team
+  int need_w;
+  int acc_x, acc_y, acc_w;
+};
+
+template <typename T, int CPL, typename S, bool WXW, bool WY>
+struct EdgeBwd {
+  static constexpr int words = sizeof(T) / 4;
+  static constexpr int pair = PkT<T, CPL, UsePairs<T, CPL>::value>::W;
+  static constexpr int max_warps =
+      warps_for((S::XD * CPL * (WXW ? 2 : 1) + (WY ? S::YD * pair : 0) + (2 * S::LO + 1) * CPL) * words +
+                (WXW ? S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 : 0) + 48);
+  // slots of g: the highest degree has one, the others share one
+  static constexpr int slot_of(int l3) { return l3 == S::LO && S::ooff(S::LO) > 0 ? 1 : 0; }
+  static constexpr int slots = slot_of(S::LO) + 1;
+  static constexpr int slot_begin(int h) {  // first component
+    for (int l = 0; l <= S::LO; ++l)
+      if (S::has(S::MO, l) && slot_of(l) == h) return S::ooff(l);
+    return S::OD;
+  }
+  static constexpr int red_rows = WY ? (S::YD + 1) / 2 : 0;
+  static constexpr int red_pass = red_rows > 4 && sizeof(T) == 8 ? 4 : red_rows;  // rows of the tile at a time
+  static constexpr int red_row = 64 + 16 / static_cast<int>(sizeof(T));
+  static constexpr int m_elems = WXW ? S::m_rounds * 32 : 0;
+  // per warp: coupling matrices, reduction tile and, in teams of several warps, two reduced gy rows
+  static constexpr int warp_elems(int team_warps) {
+    return m_elems + (WY ? red_pass * red_row + (team_warps > 1 ? 64 : 0) : 0);
+  }
+  static constexpr int table_elems = (S::terms + 3) / 4 * 4;
+};
+
+// One path for a lane's packets.  xl / gxl: the lane's x and gx packets of degree l1; g2: its g packets of degree l3;
+// w2: its weights; dot receives sum_i x_i s_i; gyl: the accumulators of degree l2.  The arithmetic of a row i is issued
+// in batches of independent instructions, so that the latency of one is covered by the others with few warps resident.
+template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WXW, bool WY, typename V>
+__device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* g2, const V* w2, V* dot, const T* mbuf,
+                                          const T* ctab) {
+  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  constexpr int NP = PK::NP;
+  using PT = CgPattern<l1, l2, l3>;
+  constexpr int n = PT::n;
+  constexpr int toff = S::toff(l1, l2, l3), moff = S::moff(l1, l2, l3);
+  static_for<0, n>([&](auto tc) {
+    constexpr int t0 = decltype(tc)::value;
+    if constexpr (edge_new_row<PT>(t0)) {
+      constexpr int i = PT::t[t0].i;
+      constexpr int t1 = edge_row_end<PT>(t0);
+      // groups of four table entries that cover the row
+      constexpr int e0 = edge_entry<PT>(t0), e1 = edge_entry<PT>(t1 - 1);
+      constexpr int m_lo = e0 / 4, m_hi = e1 / 4, c_lo = t0 / 4, c_hi = (t1 - 1) / 4;
+      T mm[WXW ? 4 * (m_hi - m_lo + 1) : 1], cc[WY ? 4 * (c_hi - c_lo + 1) : 1];
+      if constexpr (WXW)
+        static_for<m_lo, m_hi + 1>([&](auto qc) {
+          constexpr int q = decltype(qc)::value;
+          edge_load_four<T>(mbuf + moff + 4 * q, mm + 4 * (q - m_lo));
+        });
+      if constexpr (WY)
+        static_for<c_lo, c_hi + 1>([&](auto qc) {
+          constexpr int q = decltype(qc)::value;
+          edge_load_four<T>(ctab + toff + 4 * q, cc + 4 * (q - c_lo));
+        });
+      if constexpr (WY) {
+        V xw[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) xw[p] = vmul(xl[i * NP + p], w2[p]);
+        V pik[e1 - e0 + 1];
+        static_for<t0, t1>([&](auto uc) {
+          constexpr int t = decltype(uc)::value;
+          if constexpr (edge_new_entry<PT>(t)) {
+            constexpr int k = PT::t[t].k, slot = edge_entry<PT>(t) - e0;
+            pik[slot] = vmul(xw[0], g2[k * NP]);
+#pragma unroll
+            for (int p = 1; p < NP; ++p) pik[slot] = vfma(xw[p], g2[k * NP + p], pik[slot]);
+          }
+        });
+        static_for<t0, t1>([&](auto uc) {
+          constexpr int t = decltype(uc)::value;
+          constexpr int j = PT::t[t].j, slot = edge_entry<PT>(t) - e0;
+          gyl[j] = vfma(bcast_packet(cc[t - 4 * c_lo], V{}), pik[slot], gyl[j]);
+        });
+      }
+      if constexpr (WXW) {
+        V sa[NP];
+        static_for<t0, t1>([&](auto uc) {
+          constexpr int t = decltype(uc)::value;
+          if constexpr (edge_new_entry<PT>(t)) {
+            constexpr int k = PT::t[t].k, e = edge_entry<PT>(t), r = e - e0;
+            const V c = bcast_packet(mm[e - 4 * m_lo], V{});
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+              if constexpr (r == 0) {
+                sa[p] = vmul(c, g2[k * NP + p]);
+              } else {
+                sa[p] = vfma(c, g2[k * NP + p], sa[p]);
+              }
+            }
+          }
+        });
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          gxl[i * NP + p] = vfma(w2[p], sa[p], gxl[i * NP + p]);
+          dot[p] = vfma(xl[i * NP + p], sa[p], dot[p]);
+        }
+      }
+    }
+  });
+}
+
+// FULL: one warp per edge and 32 * CPL channels, known to the compiler.
+template <typename T, int CPL, typename S, bool WXW, bool WY, bool FULL>
+__global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WXW, WY>::max_warps * 32, 1)
+    edge_bwd_kernel(const __grid_constant__ EdgeBwdParams<T> P) {
+  using K = EdgeBwd<T, CPL, S, WXW, WY>;
+  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  using V = typename PK::V;
+  constexpr int NP = PK::NP;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int team_warps = FULL ? 1 : P.team_warps;
+  const int team = FULL ? warp : warp / team_warps, member = warp - team * team_warps;
+  const int ch = FULL ? 32 * CPL : P.ch, stages = P.stages;
+  const int W = S::paths * ch, X = S::XD * ch, O = S::OD * ch;
+  const bool split = P.split != 0;
+  const int stage_elems = W + (split ? 0 : O);
+
+  T* const base = reinterpret_cast<T*>(smem_raw);
+  T* const ring = base + static_cast<size_t>(team) * P.team_elems;
+  T* const gslots = ring + static_cast<size_t>(stages) * stage_elems;  // split: the row of g, in slots
+  T* const warp_mem = base + static_cast<size_t>(P.teams) * P.team_elems;
+  const int warp_elems = K::warp_elems(team_warps);
+  T* const mbuf = warp_mem + static_cast<size_t>(warp) * warp_elems;
+  T* const red = mbuf + K::m_elems;
+  T* const gbuf = red + K::red_pass * K::red_row;
+  T* const ctab = warp_mem + static_cast<size_t>(blockDim.x >> 5) * warp_elems;
+  uint64_t* const all_bars = reinterpret_cast<uint64_t*>(ctab + K::table_elems);
+  uint64_t* const full = all_bars + team * (kEdgeMaxStages + kEdgeMaxSlots);
+  uint64_t* const gfull = full + kEdgeMaxStages;
+  unsigned* const tickets = reinterpret_cast<unsigned*>(all_bars + P.teams * (kEdgeMaxStages + kEdgeMaxSlots));
+
+  if (member == 0 && lane == 0) {
+    for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
+    for (int s = 0; s < K::slots; ++s) mbar_init(&gfull[s], 1);
+    fence_barrier_init();
+  }
+  if constexpr (WY)
+    for (int i = threadIdx.x; i < S::terms; i += blockDim.x) ctab[i] = P.term_c[i];
+
+  MatrixProgram<T, S> program;
+  if constexpr (WXW) program.load(P.prog_c, P.prog_j, lane);
+  __syncthreads();
+
+  const int cpw = ch / team_warps;  // channels of this warp
+  const int lanes = FULL ? 32 : cpw / CPL, stride = PK::W * lanes;
+  const int own = FULL ? PK::W * lane : member * cpw + PK::W * min(lane, lanes - 1);  // first channel of this lane
+  const bool active = FULL || lane < lanes;
+  const bool leader = member == 0 && lane == 0;
+  const bool want_x = WXW && P.gx != nullptr, storing = WXW && P.gw != nullptr;
+  const uint32_t w_bytes = P.need_w ? static_cast<uint32_t>(W * sizeof(T)) : 0u;
+  const uint32_t g_bytes = split ? 0u : static_cast<uint32_t>(O * sizeof(T));
+  const bool staged = w_bytes + g_bytes != 0u;
+
+  auto load_stage = [&](int e, int d, int st) {  // leader only
+    if (!staged) return;
+    T* to = ring + static_cast<size_t>(st) * stage_elems;
+    mbar_arrive_expect_tx(&full[st], w_bytes + g_bytes);
+    if (w_bytes)
+      bulk_copy_g2s_hint(to, P.w + static_cast<int64_t>(e) * W, w_bytes, &full[st], l2_policy_evict_first());
+    if (g_bytes) bulk_copy_g2s(to + W, P.g + static_cast<int64_t>(d) * O, g_bytes, &full[st]);
+  };
+  auto load_slot = [&](auto slot, int d) {  // leader only
+    constexpr int h = decltype(slot)::value, first = K::slot_begin(h), count = K::slot_begin(h + 1) - first;
+    const uint32_t bytes = static_cast<uint32_t>(count * ch * sizeof(T));
+    mbar_arrive_expect_tx(&gfull[h], bytes);
+    bulk_copy_g2s(gslots + first * ch, P.g + static_cast<int64_t>(d) * O + first * ch, bytes, &gfull[h]);
+  };
+
+  V xr[S::XD * NP], gxr[WXW ? S::XD * NP : 1], gy2[WY ? S::YD : 1];
+  int st = 0;                       // stage of the current edge; the ring keeps turning from one row to the next
+  uint32_t parity = 0, gparity = 0;  // phases of that stage's barrier and of the slots' barriers
+  bool alive = true;
+  int flip = 0;                     // which of the two reduced gy rows the current edge uses
+  auto wait = [&](uint64_t* bar, uint32_t phase, int code) {
+    if (!edge_wait(bar, phase, alive)) {
+      if (lane == 0) atomicExch(P.status, code);
+      alive = false;
+    }
+  };
+
+  auto unit_body = [&](auto l3c, const T* gblock, T* wrow) {
+    constexpr int l3 = decltype(l3c)::value;
+    constexpr int d3 = 2 * l3 + 1;
+    V g2[d3 * NP];
+    lane_load_block<PK, T, d3>(gblock + own * d3, stride, g2);
+    static_for<0, 4>([&](auto l1c) {
+      constexpr int l1 = decltype(l1c)::value;
+      static_for<0, 4>([&](auto l2c) {
+        constexpr int l2 = decltype(l2c)::value;
+        if constexpr (S::ok(l1, l2, l3)) {
+          T* wq = wrow + S::rank(l1, l2, l3) * ch + own;
+          V w2[NP], dot[NP];
+          lane_load<PK, T>(wq, stride, w2);
+#pragma unroll
+          for (int p = 0; p < NP; ++p) dot[p] = zero_packet<V>();
+          edge_path<T, CPL, S, l1, l2, l3, WXW, WY, V>(&xr[S::xoff(l1) * NP], &gxr[WXW ? S::xoff(l1) * NP : 0],
+                                                      &gy2[WY ? S::yoff(l2) : 0], g2, w2, dot, mbuf, ctab);
+          if (storing && active) lane_store<PK, T>(wq, stride, dot);  // the gradients leave with the row
+        }
+      });
+    });
+  };
+
+  const bool grouped = P.group > 1;
+  const int in_group = team % P.group, group_id = team / P.group, groups = P.teams / P.group;
+  const int64_t total = static_cast<int64_t>(gridDim.x) * (grouped ? groups : P.teams);
+  int64_t unit = grouped ? blockIdx.x + static_cast<int64_t>(gridDim.x) * group_id
+                         : static_cast<int64_t>(blockIdx.x) * P.teams + team;
+  const int64_t units = grouped ? P.num_rows : P.num_tiles;
+  int64_t seen_row = 0, seen_pos = 0;  // a row boundary this warp has seen, and where its edges begin
+#pragma unroll 1
+  while (unit < units) {
+    int64_t unit_after = unit + total;
+    int64_t n = unit, n_hi = unit + 1;
+    if (!grouped) {
+      if (team_warps == 1) {
+        unit_after = take_tile(P.tile_counters, total, lane);
+      } else {
+        if (leader) tickets[team] = atomicAdd(&P.tile_counters[0], 1u);
+        team_sync(team_warps, team);
+        unit_after = total + static_cast<int64_t>(tickets[team]);
+        team_sync(team_warps, team);
+      }
+      if (P.tile_rows > 0) {
+        n = unit * P.tile_rows;
+        n_hi = n + P.tile_rows < P.num_rows ? n + P.tile_rows : P.num_rows;
+      } else {
+        // tile t: the rows whose edges begin in [t, t + 1) * tile_edges of the source-sorted edge order (guessed from
+        // where the warp's previous tile ended, assuming rows of average length in between)
+        const int64_t guess =
+            seen_row + static_cast<int64_t>(static_cast<float>(unit * P.tile_edges - seen_pos) * P.rows_per_edge);
+        n = unit == 0 ? 0 : warp_lower_bound_guess(P.src_rowptr, P.num_rows, unit * P.tile_edges, guess, lane);
+        n_hi = unit + 1 == P.num_tiles
+                   ? P.num_rows
+                   : warp_lower_bound_near(P.src_rowptr, P.num_rows, (unit + 1) * P.tile_edges, n, lane);
+      }
+    }
+    const int64_t unit_now = unit;
+    unit = unit_after;
+    if (n >= n_hi) continue;  // a row with more edges than a tile spans several tile numbers
+    int64_t pos = P.src_rowptr[n], p_end = P.src_rowptr[n_hi];
+    seen_row = n_hi;
+    seen_pos = p_end;
+    if (grouped) {
+      const int64_t first = pos, count = p_end - pos;
+      pos = first + count * in_group / P.group;
+      p_end = first + count * (in_group + 1) / P.group;
+    }
+    // ids of the current and the next four edges, destinations of the first four of them
+    auto id_at = [&](int64_t p) { return p < p_end ? P.edge_ids[p] : -1; };
+    auto dst_of = [&](int e) { return e >= 0 ? P.dst[e] : 0; };
+    int e0 = id_at(pos), e1 = id_at(pos + 1), e2 = id_at(pos + 2), e3 = id_at(pos + 3), e4 = id_at(pos + 4);
+    int d0 = dst_of(e0), d1 = dst_of(e1), d2 = dst_of(e2), d3n = dst_of(e3);
+    auto id_ahead = [&](int k) { return k == 1 ? e1 : (k == 2 ? e2 : e3); };
+    auto dst_ahead = [&](int k) { return k == 1 ? d1 : (k == 2 ? d2 : d3n); };
+    if (leader && e0 >= 0) {
+      load_stage(e0, d0, st);
+      for (int k = 1, stage = st; k < stages; ++k) {
+        if (++stage == stages) stage = 0;
+        if (id_ahead(k) >= 0) load_stage(id_ahead(k), dst_ahead(k), stage);
+      }
+      if (split) static_for<0, K::slots>([&](auto h) { load_slot(h, d0); });
+    }
+    T y_next = lane < S::YD && e0 >= 0 ? P.y[static_cast<int64_t>(e0) * S::YD + lane] : T(0);
+    if constexpr (WXW) program.run(y_next, mbuf, lane);
+    if (WXW && e1 >= 0 && lane < S::YD) y_next = P.y[static_cast<int64_t>(e1) * S::YD + lane];
+    __syncwarp();
+    int refill_stage = -1;  // a stage whose row is on its way back, to be refilled with the edge `stages` after it
+#pragma unroll 1
+    for (; n < n_hi; ++n) {
+      const int64_t pe = min(static_cast<int64_t>(P.src_rowptr[n + 1]), p_end);
+      if (!grouped && P.tile_rows == 0 && pos >= pe) {
+        // A row without edges in a piece of a graph, which has long runs of them (their gx is cleared beforehand): jump
+        // to the row that holds the next edge instead of walking the run one dependent load at a time.
+        if (pos >= p_end) break;
+        n = warp_lower_bound(P.src_rowptr, P.num_rows, pos + 1, lane) - 2;
+        continue;
+      }
+      if (pos < pe) {
+        static_for<0, 4>([&](auto l1c) {
+          constexpr int l1 = decltype(l1c)::value;
+          if constexpr (S::has(S::MX, l1)) {
+            constexpr int d = 2 * l1 + 1;
+            lane_load_block<PK, T, d>(P.x + n * X + ch * S::xoff(l1) + own * d, stride, &xr[S::xoff(l1) * NP]);
+          }
+        });
+        if (!active) {
+#pragma unroll
+          for (int a = 0; a < S::XD * NP; ++a) xr[a] = zero_packet<V>();
+        }
+      }
+      if constexpr (WXW) {
+#pragma unroll
+        for (int a = 0; a < S::XD * NP; ++a) gxr[a] = zero_packet<V>();
+      }
+#pragma unroll 1
+      for (; pos < pe; ++pos) {
+        if constexpr (WY) {
+#pragma unroll
+          for (int j = 0; j < S::YD; ++j) gy2[j] = zero_packet<V>();
+        }
+        if (staged) wait(&full[st], parity, 3);
+        T* wrow = ring + static_cast<size_t>(st) * stage_elems;
+        const bool more = pos + 1 < p_end;
+        static_for<0, 4>([&](auto l3c) {
+          constexpr int l3 = decltype(l3c)::value;
+          if constexpr (S::has(S::MO, l3)) {
+            constexpr int slot = K::slot_of(l3);
+            if constexpr (S::ooff(l3) == K::slot_begin(slot)) {
+              if (split) wait(&gfull[slot], gparity, 2);
+            }
+            unit_body(l3c, (split ? gslots : wrow + W) + ch * S::ooff(l3), wrow);
+            if constexpr (l3 != S::LO && S::ooff(l3) + 2 * l3 + 1 == K::slot_begin(slot + 1)) {
+              if (split) {  // the slot is done with; the last one is refilled at the end of the edge
+                team_sync(team_warps, team);
+                if (leader && more) load_slot(std::integral_constant<int, slot>{}, d1);
+              }
+            }
+            if constexpr (S::ooff(l3) == 0) {  // after the first degree: the row sent back has left its stage by now
+              if (refill_stage >= 0 && leader) {
+                bulk_wait_group_read_all();
+                if (id_ahead(stages - 1) >= 0) load_stage(id_ahead(stages - 1), dst_ahead(stages - 1), refill_stage);
+              }
+              refill_stage = -1;
+            }
+          }
+        });
+        if (storing) fence_async_shared();  // gradient writes, before the bulk store reads the stage
+        team_sync(team_warps, team);      // every lane is done with the stage, the last slot and the scalars
+        if (leader) {
+          if (split && more) load_slot(std::integral_constant<int, K::slots - 1>{}, d1);
+          if (storing) {
+            T* row = P.gw + static_cast<int64_t>(e0) * W;
+            const uint32_t bytes = static_cast<uint32_t>(W * sizeof(T));
+            if (P.acc_w)
+              bulk_reduce_add_s2g(row, wrow, bytes);
+            else
+              bulk_copy_s2g_hint(row, wrow, bytes, l2_policy_evict_first());
+            bulk_commit_group();
+          } else if (pos + stages < p_end) {
+            const int k = stages;
+            load_stage(k == 2 ? e2 : (k == 3 ? e3 : e4), k == 2 ? d2 : d3n, st);
+          }
+        }
+        if (storing) refill_stage = st;
+        if constexpr (WXW) program.run(y_next, mbuf, lane);
+        if (WXW && pos + 2 < p_end && lane < S::YD) y_next = P.y[static_cast<int64_t>(e2) * S::YD + lane];
+        if constexpr (WY) {
+          // the lanes' partial gy rows through the reduction tile: entries 2r and 2r + 1 in tile row r; four lanes sum
+          // a row, a quarter each
+          constexpr int passes = (K::red_rows + K::red_pass - 1) / K::red_pass;
+          static_for<0, passes>([&](auto qc) {
+            constexpr int first = decltype(qc)::value * K::red_pass;
+            constexpr int rows = K::red_rows - first < K::red_pass ? K::red_rows - first : K::red_pass;
+            static_for<0, rows>([&](auto rc) {
+              constexpr int j = 2 * (first + decltype(rc)::value);
+              Vec<T, 2> pr;
+              pr.a[0] = hsum(gy2[j]);
+              if constexpr (j + 1 < S::YD) {
+                pr.a[1] = hsum(gy2[j + 1]);
+              } else {
+                pr.a[1] = T(0);
+              }
+              *reinterpret_cast<Vec<T, 2>*>(red + decltype(rc)::value * K::red_row + lane * 2) = pr;
+            });
+            __syncwarp();
+            constexpr int per = 16 / static_cast<int>(sizeof(T));
+            const int r = min(lane & 7, rows - 1);
+            const T* seg = red + r * K::red_row + (lane >> 3) * 16;
+            T s0 = T(0), s1 = T(0);
+#pragma unroll
+            for (int v = 0; v < 16 / per; ++v) {
+              const Vec<T, per> q = reinterpret_cast<const Vec<T, per>*>(seg)[v];
+#pragma unroll
+              for (int c = 0; c < per; c += 2) {
+                s0 += q.a[c];
+                s1 += q.a[c + 1];
+              }
+            }
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 8);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 8);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 16);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 16);
+            if (lane < rows) {
+              const int j = 2 * (first + lane);
+              if (team_warps > 1) {
+                *reinterpret_cast<Vec<T, 2>*>(gbuf + flip * 32 + j) = Vec<T, 2>{{s0, s1}};
+              } else {
+                T* to = P.gy + static_cast<int64_t>(e0) * S::YD + j;
+                to[0] = P.acc_y ? to[0] + s0 : s0;
+                if (j + 1 < S::YD) to[1] = P.acc_y ? to[1] + s1 : s1;
+              }
+            }
+            __syncwarp();
+          });
+          if (team_warps > 1) {
+            team_sync(team_warps, team);
+            if (member == 0 && lane < S::YD) {
+              T sum = gbuf[flip * 32 + lane];
+              for (int m = 1; m < team_warps; ++m) sum += gbuf[m * warp_elems + flip * 32 + lane];
+              T* to = P.gy + static_cast<int64_t>(e0) * S::YD + lane;
+              *to = P.acc_y ? *to + sum : sum;
+            }
+            flip ^= 1;
+          }
+        } else {
+          __syncwarp();
+        }
+        e0 = e1;
+        e1 = e2;
+        e2 = e3;
+        e3 = e4;
+        d0 = d1;
+        d1 = d2;
+        d2 = d3n;
+        if (pos + 4 < p_end) d3n = P.dst[e3];
+        e4 = pos + 5 < p_end ? P.edge_ids[pos + 5] : -1;
+        gparity ^= 1u;
+        if (++st == stages) {
+          st = 0;
+          parity ^= 1u;
+        }
+      }
+      if constexpr (WXW) {
+        if (grouped) {  // the part goes to shared memory: bulk stores must have read the ring
+          if (leader) bulk_wait_group_read_all();
+          team_sync(team_warps, team);
+        }
+        if (want_x && active) {
+          T* to = grouped ? ring : P.gx + n * X;
+          static_for<0, 4>([&](auto l1c) {
+            constexpr int l1 = decltype(l1c)::value, d = 2 * l1 + 1;
+            if constexpr (S::has(S::MX, l1))
+              lane_store_block<PK, T, d>(to + ch * S::xoff(l1) + own * d, stride, &gxr[S::xoff(l1) * NP],
+                                         !grouped && P.acc_x);
+          });
+        }
+      }
+    }
+    if (WXW && leader) bulk_wait_group_read_all();  // the next rows' copies reuse the stages
+    if constexpr (WXW) {
+      if (grouped) {  // the parts of the row, in order
+        const int barrier = 1 + (team_warps > 1 ? P.teams : 0) + group_id;
+        const int threads = P.group * team_warps * 32;
+        const T* parts = base + static_cast<size_t>(group_id * P.group) * P.team_elems;
+        named_barrier(barrier, threads);
+        if (want_x) {
+          T* to = P.gx + unit_now * X;
+          for (int a = static_cast<int>(threadIdx.x) - group_id * threads; a < X; a += threads) {
+            T sum = parts[a];
+            for (int q = 1; q < P.group; ++q) sum += parts[static_cast<size_t>(q) * P.team_elems + a];
+            to[a] = P.acc_x ? to[a] + sum : sum;
+          }
+        }
+        fence_async_shared();  // threads have written and read the ring; its next users are bulk copies
+        named_barrier(barrier, threads);
+      }
+    }
+  }
+  if (!grouped && member == 0) leave_tiles(P.tile_counters, total, lane);
+  if (WXW && leader) bulk_wait_group_read_all();
+  if (!alive) {  // let copies that are still in flight land before the CTA's shared memory is released
+    for (int d = 0; d < stages; ++d) edge_wait(&full[d], d < st ? parity : parity ^ 1u, false);
+    for (int d = 0; d < K::slots; ++d) edge_wait(&gfull[d], gparity ^ 1u, false);
+  }
+}
+
+template <typename T, int CPL, typename S, bool WXW, bool WY, bool FULL>
+int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
+                    const EdgeBackwardArgs& a, cudaStream_t stream) {
+  using K = EdgeBwd<T, CPL, S, WXW, WY>;
+  auto kernel = edge_bwd_kernel<T, CPL, S, WXW, WY, FULL>;
+  const EdgePlan& ep = plan->edge;
+  EdgeBwdParams<T> P;
+  P.x = static_cast<const T*>(a.x);
+  P.y = static_cast<const T*>(a.y);
+  P.w = static_cast<const T*>(a.w);
+  P.g = static_cast<const T*>(a.g);
+  P.gx = static_cast<T*>(a.gx);
+  P.gy = static_cast<T*>(a.gy);
+  P.gw = static_cast<T*>(a.gw);
+  P.dst = graph->dst;
+  P.src_rowptr = graph->src_rowptr;
+  P.edge_ids = graph->edge_ids_by_src;
+  P.term_c = static_cast<const T*>(dt.edge_term_c);
+  P.prog_c = static_cast<const T*>(dt.edge_prog_c);
+  P.prog_j = dt.edge_prog_j;
+  P.status = dt.status;
+  P.tile_counters = next_tile_counters(plan, dt);
+  P.num_rows = graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;
+  P.ch = ep.ch;
+  P.team_warps = ep.team_warps;
+  P.need_w = a.gx != nullptr || a.gy != nullptr;
+  P.acc_x = a.acc_x;
+  P.acc_y = a.acc_y;
+  P.acc_w = a.acc_w;
+  const size_t w_row = static_cast<size_t>(S::paths) * ep.ch * sizeof(T);
+  const size_t x_row = static_cast<size_t>(S::XD) * ep.ch * sizeof(T), g_row = static_cast<size_t>(S::OD) * ep.ch * sizeof(T);
+  EdgeLaunch launch;
+  const int max_teams = capped_warps(plan->tuning, K::max_warps) / ep.team_warps;
+  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
+    for (int option = 0; option < 3; ++option) {  // three or two stages with g in them, or two and g by degree
+      const int stages = option == 0 ? 3 : 2, split = option == 2;
+      size_t team = split ? stages * w_row + g_row : stages * (w_row + g_row);
+      team = (std::max(team, x_row) + 127) / 128 * 128;
+      const size_t bytes = teams * (team + (kEdgeMaxStages + kEdgeMaxSlots) * sizeof(uint64_t) + sizeof(unsigned)) +
+                           (static_cast<size_t>(teams) * ep.team_warps * K::warp_elems(ep.team_warps) + K::table_elems) * sizeof(T);
+      if (bytes > static_cast<size_t>(dt.max_smem_optin)) continue;
+      launch.warps = teams * ep.team_warps;
+      launch.stages = stages;
+      launch.split = split;
+      launch.bytes = bytes;
+      P.team_elems = static_cast<int>(team / sizeof(T));
+      break;
+    }
+  if (launch.warps == 0) return LUNA_ERR_UNSUPPORTED;
+  P.stages = launch.stages;
+  P.split = launch.split;
+  P.teams = launch.warps / ep.team_warps;
+  const int64_t edges = graph->num_edges;
+  P.rows_per_edge = static_cast<float>(static_cast<double>(P.num_rows) / static_cast<double>(std::max<int64_t>(edges, 1)));
+  EdgeSplit cut = edge_split(P.num_rows, edges, dt.sm_count, P.teams, ep.team_warps);
+  P.group = cut.group;
+  P.tile_rows = cut.tile_rows;
+  P.tile_edges = tile_edges_for(edges, static_cast<int64_t>(dt.sm_count) * P.teams, edges_per_warp(plan->tuning, 64));
+  P.num_tiles = ceil_div(std::max<int64_t>(P.num_rows, 1), P.tile_rows);
+  // A whole graph of some density, or a shard of one (its own rows plus a halo at most half as large), has hardly any
+  // rows without edges, and tiles of a fixed number of rows are even without any search.  A piece of a graph (a
+  // destination range against all source rows) has long runs of rows without edges: its tiles are cut by edge count,
+  // and the rows that are jumped over are cleared here.
+  const bool whole = graph->num_src_nodes <= 0 || graph->num_src_nodes <= graph->num_nodes + graph->num_nodes / 2;
+  if (P.group == 1 && !(whole && static_cast<double>(edges) >= 8.0 * static_cast<double>(P.num_rows))) {
+    P.tile_rows = 0;
+    P.num_tiles = ceil_div(std::max<int64_t>(edges, 1), P.tile_edges);
+    cut.blocks = std::max<int64_t>(1, std::min<int64_t>(dt.sm_count, ceil_div(P.num_tiles, P.teams)));
+    if (a.gx && !a.acc_x)
+      LUNA_CUDA_CHECK(cudaMemsetAsync(a.gx, 0, static_cast<size_t>(P.num_rows) * plan->X * sizeof(T), stream));
+  }
+  static KernelSetup setup;
+  const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
+  if (rc != LUNA_OK) return rc;
+  kernel<<<static_cast<unsigned>(cut.blocks), launch.warps * 32, launch.bytes, stream>>>(P);
+  LUNA_LAUNCH_CHECK("backward (edge family)");
+  return LUNA_OK;
+}
+
+template <typename T, int CPL, typename S, bool FULL>
+int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
+                      const EdgeBackwardArgs& a, cudaStream_t stream) {
+  const bool wxw = a.gx || a.gw, wy = a.gy != nullptr;
+  if (wxw && wy) return launch_edge_bwd<T, CPL, S, true, true, FULL>(plan, dt, graph, a, stream);
+  if (wxw) return launch_edge_bwd<T, CPL, S, true, false, FULL>(plan, dt, graph, a, stream);
+  if (wy) return launch_edge_bwd<T, CPL, S, false, true, FULL>(plan, dt, graph, a, stream);
+  return LUNA_OK;
+}
+
+}  // namespace edgek
+}  // namespace luna

@@ -1,0 +1,285 @@
+// Forward kernel of the edge family:  out[t] = sum_{e: dst e = t} sum_p w_p * (M^p(y_e)^T x[src e]).
+//
+// Per edge the warp turns the edge attributes into the coupling matrices M^p[i][k] = sum_j C^p_ijk y_j (the entries the
+// coupling tensors leave zero for every y are skipped, at compile time), a lane multiplies them into its channels:
+// out_k += sum_i M[i][k] * (x_i * w).  FP32 with an even number of channels per lane runs on packed two-wide FMAs.
+// The matrices of the next edge are made while the current edge is computed: its attributes sit one per lane and reach
+// the lane that needs them by shuffles, so nothing waits for shared memory in between.
+#pragma once
+
+#include "uvu_edge.cuh"
+
+namespace luna {
+namespace edgek {
+
+template <typename T>
+struct EdgeFwdParams {
+  const T *x, *y, *w;
+  T* out;
+  const int *src, *dst_rowptr;
+  const T* prog_c;               // [2][m_total] coefficients of the two attributes an entry depends on
+  const unsigned short* prog_j;  // [m_total] the two attributes, 8 bits each
+  int* status;
+  unsigned* tile_counters;
+  int64_t num_rows, tile_rows, num_tiles;
+  int ch;          // channels per block
+  int team_warps;  // warps per team
+  int teams;       // per CTA
+  int group;       // teams that share a row, 1: tiles
+  int stages;
+  int ring_elems;  // per team
+  int accumulate;
+};
+
+template <typename T, int CPL, typename S>
+struct EdgeFwd {
+  static constexpr int words = sizeof(T) / 4;
+  static constexpr int m_elems = S::m_rounds * 32;
+  static constexpr int max_warps =
+      warps_for((S::OD + S::XD) * CPL * words + S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 + 44);
+  static constexpr size_t warp_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
+};
+
+// FULL: one warp per edge and 32 * CPL channels, known to the compiler.
+template <typename T, int CPL, typename S, bool FULL>
+__global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
+    edge_fwd_kernel(const __grid_constant__ EdgeFwdParams<T> P) {
+  using K = EdgeFwd<T, CPL, S>;
+  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  using V = typename PK::V;
+  constexpr int NP = PK::NP;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int team_warps = FULL ? 1 : P.team_warps;
+  const int team = FULL ? warp : warp / team_warps, member = warp - team * team_warps;
+  const int ch = FULL ? 32 * CPL : P.ch, stages = P.stages;
+  const int W = S::paths * ch, X = S::XD * ch, O = S::OD * ch;
+  const int stage_elems = W + X;
+
+  T* ring = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(team) * P.ring_elems;
+  T* mbuf = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(P.teams) * P.ring_elems +
+            static_cast<size_t>(warp) * (2 * K::m_elems);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<T*>(smem_raw) +
+                                               static_cast<size_t>(P.teams) * P.ring_elems +
+                                               static_cast<size_t>(blockDim.x >> 5) * (2 * K::m_elems)) +
+                   team * kEdgeMaxStages;
+  unsigned* tickets = reinterpret_cast<unsigned*>(bars + (P.teams - team) * kEdgeMaxStages);
+  if (member == 0 && lane == 0) {
+    for (int s = 0; s < stages; ++s) mbar_init(&bars[s], 1);
+    fence_barrier_init();
+  }
+
+  MatrixProgram<T, S> program;
+  program.load(P.prog_c, P.prog_j, lane);
+  __syncthreads();
+
+  const int cpw = ch / team_warps;  // channels of this warp
+  const int lanes = FULL ? 32 : cpw / CPL, stride = PK::W * lanes;
+  const int own = FULL ? PK::W * lane : member * cpw + PK::W * min(lane, lanes - 1);  // first channel of this lane
+  const bool active = FULL || lane < lanes;
+  const bool leader = member == 0 && lane == 0;
+  const uint32_t w_bytes = static_cast<uint32_t>(W * sizeof(T)), x_bytes = static_cast<uint32_t>(X * sizeof(T));
+  auto issue = [&](int64_t e, int s_node, int s) {  // leader only
+    T* to = ring + static_cast<size_t>(s) * stage_elems;
+    mbar_arrive_expect_tx(&bars[s], w_bytes + x_bytes);
+    bulk_copy_g2s_hint(to, P.w + e * W, w_bytes, &bars[s], l2_policy_evict_first());
+    bulk_copy_g2s(to + W, P.x + static_cast<int64_t>(s_node) * X, x_bytes, &bars[s]);
+  };
+
+  V acc[S::OD * NP];
+  int s = 0;            // stage of the next edge; the ring keeps turning from one row to the next
+  uint32_t parity = 0;  // phase of that stage's barrier
+  bool alive = true;
+  int buf = 0;          // matrix buffer of the current edge
+
+  // out_k += sum_i M[i][k] * (x_i * w) for one path, over the entries of M that the pattern has
+  auto path_body = [&](auto l1c, auto l2c, auto l3c, const T* wq, const T* matrix, const V* xl, V* al) {
+    constexpr int l1 = decltype(l1c)::value, l2 = decltype(l2c)::value, l3 = decltype(l3c)::value;
+    using PT = CgPattern<l1, l2, l3>;
+    V w2[NP], xw[NP];
+    T m[4];
+    lane_load<PK, T>(wq, stride, w2);
+    static_for<0, PT::n>([&](auto tc) {
+      constexpr int t = decltype(tc)::value;
+      if constexpr (edge_new_entry<PT>(t)) {
+        constexpr int i = PT::t[t].i, k = PT::t[t].k, entry = edge_entry<PT>(t);
+        if constexpr (entry % 4 == 0) edge_load_four<T>(matrix + entry, m);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          if constexpr (edge_new_row<PT>(t)) xw[p] = vmul(xl[i * NP + p], w2[p]);
+          al[k * NP + p] = vfma(bcast_packet(m[entry % 4], V{}), xw[p], al[k * NP + p]);
+        }
+      }
+    });
+  };
+  const bool grouped = P.group > 1;
+  const int in_group = team % P.group, group_id = team / P.group, groups = P.teams / P.group;
+  const int64_t total = static_cast<int64_t>(gridDim.x) * (grouped ? groups : P.teams);
+  // a group takes every total-th row; a team's first tile is its own number, and further ones come from a counter, one
+  // ahead of need, so that a team that started late or met long rows simply takes fewer
+  int64_t unit = grouped ? blockIdx.x + static_cast<int64_t>(gridDim.x) * group_id
+                         : static_cast<int64_t>(blockIdx.x) * P.teams + team;
+  const int64_t units = grouped ? P.num_rows : P.num_tiles;
+#pragma unroll 1
+  while (unit < units) {
+    int64_t unit_after = unit + total;
+    int64_t n = unit, n_hi = unit + 1;
+    if (!grouped) {
+      if (team_warps == 1) {
+        unit_after = take_tile(P.tile_counters, total, lane);
+      } else {
+        if (leader) tickets[team] = atomicAdd(&P.tile_counters[0], 1u);
+        team_sync(team_warps, team);
+        unit_after = total + static_cast<int64_t>(tickets[team]);
+        team_sync(team_warps, team);
+      }
+      n = unit * P.tile_rows;
+      n_hi = n + P.tile_rows < P.num_rows ? n + P.tile_rows : P.num_rows;
+    }
+    int64_t e = P.dst_rowptr[n], e_end = P.dst_rowptr[n_hi];
+    if (grouped) {
+      const int64_t first = e, count = e_end - e;
+      e = first + count * in_group / P.group;
+      e_end = first + count * (in_group + 1) / P.group;
+    }
+    // all stages are empty here: fill them in ring order from the current one
+    if (leader) {
+      for (int d = 0, stage = s; d < stages; ++d) {
+        if (e + d < e_end) issue(e + d, P.src[e + d], stage);
+        if (++stage == stages) stage = 0;
+      }
+    }
+    // source node of the edge that is issued in the next iteration, attributes of the next edge
+    int src_ahead = leader && e + stages < e_end ? P.src[e + stages] : 0;
+    T y_next = lane < S::YD && e < e_end ? P.y[e * S::YD + lane] : T(0);
+    program.run(y_next, mbuf + buf * K::m_elems, lane);
+    if (lane < S::YD && e + 1 < e_end) y_next = P.y[(e + 1) * S::YD + lane];
+    __syncwarp();
+#pragma unroll 1
+    for (; n < n_hi; ++n) {
+      const int64_t row_end = min(static_cast<int64_t>(P.dst_rowptr[n + 1]), e_end);
+#pragma unroll
+      for (int a = 0; a < S::OD * NP; ++a) acc[a] = zero_packet<V>();
+#pragma unroll 1
+      for (; e < row_end; ++e) {
+        if (!edge_wait(&bars[s], parity, alive)) {
+          if (lane == 0) atomicExch(P.status, 1);
+          alive = false;
+        }
+        const T* ws = ring + static_cast<size_t>(s) * stage_elems + own;
+        const T* xs = ring + static_cast<size_t>(s) * stage_elems + W;
+        program.run(y_next, mbuf + (buf ^ 1) * K::m_elems, lane);  // of the next edge; of no use after the last one
+        if (lane < S::YD && e + 2 < e_end) y_next = P.y[(e + 2) * S::YD + lane];
+        const T* m_now = mbuf + buf * K::m_elems;
+        static_for<0, 4>([&](auto l1c) {
+          constexpr int l1 = decltype(l1c)::value;
+          if constexpr (S::has(S::MX, l1)) {
+            constexpr int d1 = 2 * l1 + 1;
+            V xl[d1 * NP];
+            lane_load_block<PK, T, d1>(xs + ch * S::xoff(l1) + own * d1, stride, xl);
+            static_for<0, 4>([&](auto l3c) {
+              constexpr int l3 = decltype(l3c)::value;
+              static_for<0, 4>([&](auto l2c) {
+                constexpr int l2 = decltype(l2c)::value;
+                if constexpr (S::ok(l1, l2, l3))
+                  path_body(l1c, l2c, l3c, ws + S::rank(l1, l2, l3) * ch, m_now + S::moff(l1, l2, l3), xl,
+                            &acc[S::ooff(l3) * NP]);
+              });
+            });
+          }
+        });
+        buf ^= 1;
+        team_sync(team_warps, team);  // every lane is done with this stage and with the matrices
+        if (leader && e + stages < e_end) {
+          issue(e + stages, src_ahead, s);
+          if (e + stages + 1 < e_end) src_ahead = P.src[e + stages + 1];
+        }
+        if (++s == stages) {
+          s = 0;
+          parity ^= 1u;
+        }
+      }
+      if (active) {
+        T* to = grouped ? ring : P.out + n * O;
+        static_for<0, 4>([&](auto l3c) {
+          constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
+          if constexpr (S::has(S::MO, l3))
+            lane_store_block<PK, T, d3>(to + ch * S::ooff(l3) + own * d3, stride, &acc[S::ooff(l3) * NP],
+                                        !grouped && P.accumulate);
+        });
+      }
+    }
+    if (grouped) {  // the parts of the row, in order
+      const int barrier = 1 + (team_warps > 1 ? P.teams : 0) + group_id;
+      const int threads = P.group * team_warps * 32;
+      const T* parts = reinterpret_cast<const T*>(smem_raw) + static_cast<size_t>(group_id * P.group) * P.ring_elems;
+      named_barrier(barrier, threads);
+      T* to = P.out + unit * O;
+      for (int a = static_cast<int>(threadIdx.x) - group_id * threads; a < O; a += threads) {
+        T sum = parts[a];
+        for (int g = 1; g < P.group; ++g) sum += parts[static_cast<size_t>(g) * P.ring_elems + a];
+        to[a] = P.accumulate ? to[a] + sum : sum;
+      }
+      fence_async_shared();  // threads have written and read the ring; its next users are bulk copies
+      named_barrier(barrier, threads);
+    }
+    unit = unit_after;
+  }
+  if (!grouped && member == 0) leave_tiles(P.tile_counters, total, lane);
+  if (!alive)  // let copies that are still in flight land before the CTA's shared memory is released
+    for (int d = 0; d < stages; ++d) edge_wait(&bars[d], d < s ? parity : parity ^ 1u, false);
+}
+
+template <typename T, int CPL, typename S, bool FULL>
+int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
+                    const EdgeForwardArgs& a, cudaStream_t stream) {
+  using K = EdgeFwd<T, CPL, S>;
+  auto kernel = edge_fwd_kernel<T, CPL, S, FULL>;
+  const EdgePlan& ep = plan->edge;
+  EdgeFwdParams<T> P;
+  P.x = static_cast<const T*>(a.x);
+  P.y = static_cast<const T*>(a.y);
+  P.w = static_cast<const T*>(a.w);
+  P.out = static_cast<T*>(a.out);
+  P.src = graph->src;
+  P.dst_rowptr = graph->dst_rowptr;
+  P.prog_c = static_cast<const T*>(dt.edge_prog_c);
+  P.prog_j = dt.edge_prog_j;
+  P.status = dt.status;
+  P.tile_counters = next_tile_counters(plan, dt);
+  P.num_rows = graph->num_nodes;
+  P.ch = ep.ch;
+  P.team_warps = ep.team_warps;
+  P.accumulate = a.accumulate ? 1 : 0;
+  const size_t stage = static_cast<size_t>(S::paths + S::XD) * ep.ch * sizeof(T);
+  const size_t row = static_cast<size_t>(S::OD) * ep.ch * sizeof(T);
+  EdgeLaunch launch;
+  const int max_teams = capped_warps(plan->tuning, K::max_warps) / ep.team_warps;
+  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
+    for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
+      const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
+      const size_t bytes = teams * (ring + ep.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned));
+      if (bytes > static_cast<size_t>(dt.max_smem_optin)) continue;
+      launch.warps = teams * ep.team_warps;
+      launch.stages = stages;
+      launch.bytes = bytes;
+      P.ring_elems = static_cast<int>(ring / sizeof(T));
+      break;
+    }
+  if (launch.warps == 0) return LUNA_ERR_UNSUPPORTED;
+  P.stages = launch.stages;
+  P.teams = launch.warps / ep.team_warps;
+  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, dt.sm_count, P.teams, ep.team_warps);
+  P.group = split.group;
+  P.tile_rows = split.tile_rows;
+  P.num_tiles = ceil_div(std::max<int64_t>(graph->num_nodes, 1), split.tile_rows);
+  static KernelSetup setup;
+  const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
+  if (rc != LUNA_OK) return rc;
+  kernel<<<static_cast<unsigned>(split.blocks), launch.warps * 32, launch.bytes, stream>>>(P);
+  LUNA_LAUNCH_CHECK("forward (edge family)");
+  return LUNA_OK;
+}
+
+}  // namespace edgek
+}  // namespace luna

@@ -1,0 +1,30 @@
+// The edge kernels of one element type, channels per lane and shape.  The build compiles this file once for each
+// combination (LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE), so that they compile in parallel.
+#include "uvu_edge_bwd.cuh"
+#include "uvu_edge_fwd.cuh"
+
+namespace luna {
+namespace edgek {
+
+template <>
+int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::forward(const luna_uvu_plan* plan, const DeviceTables& dt,
+                                                                      const luna_graph* graph, const EdgeForwardArgs& a,
+                                                                      cudaStream_t stream) {
+  using S = ShapeOf<LUNA_EDGE_SHAPE>;
+  if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
+    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true>(plan, dt, graph, a, stream);
+  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false>(plan, dt, graph, a, stream);
+}
+
+template <>
+int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const luna_uvu_plan* plan, const DeviceTables& dt,
+                                                                       const luna_graph* graph, const EdgeBackwardArgs& a,
+                                                                       cudaStream_t stream) {
+  using S = ShapeOf<LUNA_EDGE_SHAPE>;
+  if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
+    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true>(plan, dt, graph, a, stream);
+  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false>(plan, dt, graph, a, stream);
+}
+
+}  // namespace edgek
+}  // namespace luna

@@ -75,21 +75,9 @@ extern template int launch_fast_bwd<double, 2>(LUNA_BWD_SIG(double));
 bool fast_available() { return true; }
 
 int fast_bwd_variant(const luna_uvu_plan* plan) {
-  if (!plan->fast_ok || plan->force_generic) return LUNA_BWD_TABLE_DRIVEN;
-  const FastMeta& f = plan->fast;
-  const int lx = f.LX, lo = f.LO, l2 = f.canon_l2;
-  // shapes with kernels unrolled for the canonical full path list (see launch_fast_bwd)
-  const bool compiled_shape = !plan->tuning.no_canon && ((lx == 2 && l2 == 3 && lo == 3) || (lx == 2 && l2 == 2 && lo == 2) ||
-                                                         (lx == 3 && l2 == 3 && lo == 3) || (lx == 1 && l2 == 1 && lo == 1));
-  if (!compiled_shape || f.sparse_terms <= 0 || plan->tuning.no_sparse) return LUNA_BWD_STAGED_TABLES;
-  const size_t elem = plan->dtype == LUNA_F64 ? 8 : 4;
-  // Row stages pay off when an edge's weight row is one long contiguous piece for the CTA; short rows and rows
-  // split into channel chunks go through the unit ring.
-  const bool rows_ok = f.chunks == 1;
-  int variant = rows_ok && static_cast<size_t>(f.w_stage_elems) * elem >= 2560 ? LUNA_BWD_ROW_STAGES : LUNA_BWD_UNIT_RING;
-  if (plan->tuning.bwd_kernel == 1) variant = LUNA_BWD_ROW_STAGES;
-  if (plan->tuning.bwd_kernel == 2) variant = LUNA_BWD_UNIT_RING;
-  return variant;
+  if (plan->force_generic || (!plan->fast_ok && plan->edge.shape < 0)) return LUNA_BWD_TABLE_DRIVEN;
+  if (plan->edge.shape >= 0) return LUNA_BWD_ROW_STAGES;
+  return LUNA_BWD_STAGED_TABLES;
 }
 
 namespace {
@@ -137,6 +125,19 @@ int fast_forward(luna_uvu_plan* plan, const luna_graph* graph, const void* x, co
   const DeviceTables* dt = nullptr;
   int rc = get_device_tables(plan, &dt);
   if (rc != LUNA_OK) return rc;
+  if (plan->edge.shape >= 0) {
+    bool acc = false;
+    auto one = [&](const void* xa, const void* ya, const void* wa) -> int {
+      const int code = edgek::forward(plan, *dt, graph, xa, ya, wa, out, acc, stream);
+      acc = true;
+      return code;
+    };
+    if (!tangents) return one(x, y, w);
+    if (rx && (rc = one(rx, y, w)) != LUNA_OK) return rc;
+    if (ry && (rc = one(x, ry, w)) != LUNA_OK) return rc;
+    if (rw && (rc = one(x, y, rw)) != LUNA_OK) return rc;
+    return acc ? LUNA_OK : fail(LUNA_ERR_INVALID_ARGUMENT, "tangent forward needs at least one tangent");
+  }
   if (!plan->out_fully_covered) {
     const size_t elem = plan->dtype == LUNA_F64 ? 8 : 4;
     LUNA_CUDA_CHECK(cudaMemsetAsync(out, 0, static_cast<size_t>(graph->num_nodes) * plan->O * elem, stream));
@@ -170,6 +171,8 @@ int fast_backward(luna_uvu_plan* plan, const luna_graph* graph, const void* x, c
   const DeviceTables* dt = nullptr;
   int rc = get_device_tables(plan, &dt);
   if (rc != LUNA_OK) return rc;
+  if (plan->edge.shape >= 0)
+    return edgek::backward(plan, *dt, graph, x, y, w, g, gx, acc_x, gy, acc_y, gw, acc_w, stream);
   const int cpl = plan->fast.cpl;
   if (plan->dtype == LUNA_F64) {
     auto X = static_cast<const double*>(x), Y = static_cast<const double*>(y), W = static_cast<const double*>(w);

@@ -284,11 +284,8 @@ inline int capped_warps(const Tuning& tuning, int max_warps) {
 // ---- canonical path lists ---------------------------------------------------------------------------------------
 // Most models couple every degree of x with every degree of the edge harmonics into every degree of the output:
 // all (l1, l2, l3) with l1 <= LX, l2 <= L2, l3 <= LO that satisfy the triangle rule and have an even degree sum,
-// listed in (l1, l2, l3) order, which is also the order of their weight blocks.  For such a list everything the
-// inner loops need (which paths exist, where a path's weights sit in a stage, where its coupling matrix sits in
-// the per-edge buffer) is known at compile time, so the loops over paths unroll completely and the compiler can
-// move shared-memory loads ahead of the arithmetic of the previous path.  These functions define the list; the
-// plan checks a configuration against them (FastMeta::canon_l2) and the kernels use them as constants.
+// listed in (l1, l2, l3) order, which is also the order of their weight blocks.  The plan checks a configuration
+// against these functions (FastMeta::canon_l2).
 __host__ __device__ constexpr bool canon_ok(int LX, int L2, int LO, int l1, int l2, int l3) {
   const int lo = l1 > l2 ? l1 - l2 : l2 - l1;
   return l1 <= LX && l2 <= L2 && l3 <= LO && l3 >= lo && l3 <= l1 + l2 && ((l1 + l2 + l3) % 2 == 0);
@@ -317,18 +314,6 @@ __host__ __device__ constexpr int canon_moff(int LX, int L2, int LO, int a, int 
         while (m % 4) ++m;
       }
   return m;
-}
-
-// number of canonical paths into degree c that come before (a, b) in (l1, l2) order; past-the-end arguments give
-// the number of paths into that degree
-__host__ __device__ constexpr int canon_unit_index(int LX, int L2, int LO, int a, int b, int c) {
-  int r = 0;
-  for (int l1 = 0; l1 <= LX; ++l1)
-    for (int l2 = 0; l2 <= L2; ++l2) {
-      if (l1 == a && l2 == b) return r;
-      if (canon_ok(LX, L2, LO, l1, l2, c)) ++r;
-    }
-  return r;
 }
 
 // first coupling term of the path in the sparse term list: paths in (l3, l1, l2) order, every path's terms (in the

@@ -50,12 +50,9 @@ struct BwdParams {
   const int* src_rowptr;
   const int* edge_ids;
   const unsigned char* tables;  // blob described by FastMeta::tb_*
-  const T* sp_c;                // sparse term list of a canonical plan (coefficients, y indices), else null
-  const unsigned char* sp_j;
   int* status;
   int64_t num_src_nodes, num_edges;
   int slots;
-  int row_stages;  // kernel with compiled-in patterns: weight-row stages per warp
   int acc_x, acc_y, acc_w;
 };
 
@@ -122,26 +119,19 @@ __host__ __device__ inline size_t bwd_shared_bytes(const FastMeta& f) {
 
 // WXW: whether gx and/or gw are produced; WY: whether gy is.  Compiled in or out: each is about half of the kernel,
 // and only the first needs the coupling matrices.
-// L2 >= 0: canonical full path list for (LX, L2, LO), loops over units and paths unrolled from compile-time tables;
-// L2 < 0: any path list, loops read the tables in FastMeta.
 // MAXW warps per CTA at most and MINB CTAs per SM at least: together they cap the registers per thread.
-template <typename T, int CPL, int LX, int LO, int L2, bool WXW, bool WY, int MAXW, int MINB>
+template <typename T, int CPL, int LX, int LO, bool WXW, bool WY, int MAXW, int MINB>
 __global__ void __launch_bounds__(MAXW * 32, MINB) fast_bwd_kernel(const __grid_constant__ BwdParams<T> P) {
   using PK = Pk<T, CPL>;
   using V = typename PK::V;
   constexpr int NP = PK::NP;
   constexpr int L1S = kMaxFastL + 1;
-  constexpr bool kCanon = L2 >= 0;
-  constexpr int L2c = L2 < 0 ? 0 : L2;
-  constexpr int kCanonTotal = kCanon ? canon_moff(LX, L2c, LO, -1, -1, -1) : 0;
-  constexpr int kRounds = (kCanonTotal + 31) / 32;
-  constexpr bool kProgramInRegisters = kCanon && WXW && kRounds <= 12;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const FastMeta& F = P.meta;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int R = P.slots, nk = kCanon ? LO + 1 : F.nkinds;
+  const int R = P.slots, nk = F.nkinds;
   const int slot_elems = F.slot_elems;
-  const int m_total = kCanon ? kCanonTotal : F.m_total;
+  const int m_total = F.m_total;
   constexpr int chw = 32 * CPL;
   const int c0 = blockIdx.y * chw;
 
@@ -172,20 +162,6 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) fast_bwd_kernel(const __grid_
     fence_barrier_init();
   }
   __syncwarp();
-
-  // the lane's share of the coupling-matrix program: entries lane, lane + 32, ...
-  T prog_a[kProgramInRegisters ? kRounds : 1], prog_b[kProgramInRegisters ? kRounds : 1];
-  unsigned prog_j[kProgramInRegisters ? kRounds : 1];
-  if constexpr (kProgramInRegisters) {
-#pragma unroll
-    for (int r = 0; r < kRounds; ++r) {
-      const int m = r * 32 + lane;
-      const bool in = m < m_total;
-      prog_a[r] = in ? ell_c[m] : T(0);
-      prog_b[r] = in ? ell_c[m_total + m] : T(0);
-      prog_j[r] = in ? (static_cast<unsigned>(ell_j[m]) | (static_cast<unsigned>(ell_j[m_total + m]) << 8)) : 0u;
-    }
-  }
 
   const int64_t E = P.num_edges, N = P.num_src_nodes;
   const int nwarps = blockDim.x >> 5;
@@ -321,33 +297,17 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) fast_bwd_kernel(const __grid_
     constexpr int d3 = 2 * l3 + 1;
     V g2[d3 * NP];
     const int64_t w_row = static_cast<int64_t>(e0) * F.W + lane * CPL;
-    if constexpr (kCanon) {
-      constexpr int paths_here = canon_unit_index(LX, L2c, LO, -1, -1, l3);
-      load_packets_scalar<PK, T, CPL, d3>(unit + paths_here * chw + lane * (CPL * d3), g2);
-      settle_packets<d3 * NP>(g2, ones);
-      static_for<0, LX + 1>([&](auto l1c) {
-        constexpr int l1 = decltype(l1c)::value;
-        static_for<0, L2c + 1>([&](auto l2c) {
-          constexpr int l2 = decltype(l2c)::value;
-          if constexpr (canon_ok(LX, L2c, LO, l1, l2, l3))
-            path_body(l1c, l3c, g2, unit + canon_unit_index(LX, L2c, LO, l1, l2, l3) * chw + lane * CPL,
-                      canon_moff(LX, L2c, LO, l1, l2, l3),
-                      w_row + canon_wrank(LX, L2c, LO, l1, l2, l3) * F.ch + c0);
-        });
-      });
-    } else {
-      load_packets_scalar<PK, T, CPL, d3>(unit + F.ug_soff[l3] + lane * (CPL * d3), g2);
-      settle_packets<d3 * NP>(g2, ones);
-      static_for<0, LX + 1>([&](auto l1c) {
-        constexpr int l1 = decltype(l1c)::value;
-        const int q_end = F.pair_ptr[l3 * L1S + l1 + 1];
+    load_packets_scalar<PK, T, CPL, d3>(unit + F.ug_soff[l3] + lane * (CPL * d3), g2);
+    settle_packets<d3 * NP>(g2, ones);
+    static_for<0, LX + 1>([&](auto l1c) {
+      constexpr int l1 = decltype(l1c)::value;
+      const int q_end = F.pair_ptr[l3 * L1S + l1 + 1];
 #pragma unroll 1
-        for (int q = F.pair_ptr[l3 * L1S + l1]; q < q_end; ++q) {
-          const int4 rec = ptab[q];
-          path_body(l1c, l3c, g2, unit + rec.x + lane * CPL, rec.y, w_row + rec.z);
-        }
-      });
-    }
+      for (int q = F.pair_ptr[l3 * L1S + l1]; q < q_end; ++q) {
+        const int4 rec = ptab[q];
+        path_body(l1c, l3c, g2, unit + rec.x + lane * CPL, rec.y, w_row + rec.z);
+      }
+    });
   };
 
   // waits for the unit in slot s, runs it and refills the slot with the unit R places later
@@ -392,7 +352,7 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) fast_bwd_kernel(const __grid_
       static_for<0, LX + 1>([&](auto l1c) {
         constexpr int l1 = decltype(l1c)::value;
         constexpr int d1 = 2 * l1 + 1;
-        if (kCanon || F.x_off[l1] >= 0)
+        if (F.x_off[l1] >= 0)
           load_packets_scalar<PK, T, CPL, d1>(P.x + n * F.X + F.x_off[l1] + c0 * d1 + lane * (CPL * d1),
                                               &xr[l1 * l1 * NP]);
       });
@@ -406,42 +366,28 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) fast_bwd_kernel(const __grid_
       // coupling matrices of this edge, computed while its first unit may still be in flight
       if (lane < F.Y) ybuf[lane] = y_next;
       __syncwarp();
-      if constexpr (WXW) {
-        if constexpr (kProgramInRegisters) {
-#pragma unroll
-          for (int r = 0; r < kRounds; ++r)
-            mbuf[r * 32 + lane] = fma(prog_b[r], ybuf[prog_j[r] >> 8], prog_a[r] * ybuf[prog_j[r] & 255u]);
-        } else {
-          compute_m_share<T, false>(ell_c, ell_j, ybuf, mbuf, m_total, 0, 1, lane);
-        }
-      }
+      if constexpr (WXW) compute_m_share<T, false>(ell_c, ell_j, ybuf, mbuf, m_total, 0, 1, lane);
       if (pos + 1 < p_end && lane < F.Y) y_next = P.y[static_cast<int64_t>(e1) * F.Y + lane];
       __syncwarp();
       tile_base = 0;
       tile_end = 0;
 
-      if constexpr (kCanon) {
-        static_for<0, LO + 1>([&](auto l3c) {
-          if (alive) alive = run_unit(l3c, decltype(l3c)::value);
-        });
-      } else {
-        // the per-degree arithmetic is selected by a switch so that the wait and the refill exist once in the loop
+      // the per-degree arithmetic is selected by a switch so that the wait and the refill exist once in the loop
 #pragma unroll 1
-        for (int kind = 0; kind < nk && alive; ++kind) {
-          switch (F.kind_l3[kind]) {
-            case 0:
-              alive = run_unit(std::integral_constant<int, 0>{}, kind);
-              break;
-            case 1:
-              if constexpr (LO >= 1) alive = run_unit(std::integral_constant<int, 1>{}, kind);
-              break;
-            case 2:
-              if constexpr (LO >= 2) alive = run_unit(std::integral_constant<int, 2>{}, kind);
-              break;
-            default:
-              if constexpr (LO >= 3) alive = run_unit(std::integral_constant<int, 3>{}, kind);
-              break;
-          }
+      for (int kind = 0; kind < nk && alive; ++kind) {
+        switch (F.kind_l3[kind]) {
+          case 0:
+            alive = run_unit(std::integral_constant<int, 0>{}, kind);
+            break;
+          case 1:
+            if constexpr (LO >= 1) alive = run_unit(std::integral_constant<int, 1>{}, kind);
+            break;
+          case 2:
+            if constexpr (LO >= 2) alive = run_unit(std::integral_constant<int, 2>{}, kind);
+            break;
+          default:
+            if constexpr (LO >= 3) alive = run_unit(std::integral_constant<int, 3>{}, kind);
+            break;
         }
       }
       if (!alive) break;
@@ -519,22 +465,7 @@ __global__ void reduce_gy_partial(const T* __restrict__ partial, T* __restrict__
 }
 
 
-}  // namespace fastk
-}  // namespace luna
-
-#include "uvu_fast_bwd_sparse.cuh"
-#include "uvu_fast_bwd_units.cuh"
-
-namespace luna {
-namespace fastk {
-
-// Kernels with a compile-time layout (uvu_fast_bwd_plain.cuh), one translation unit per (T, CPL).  Returns
-// LUNA_ERR_UNSUPPORTED if the plan's layout is not the compile-time one.
-template <typename T, int CPL>
-int launch_fast_bwd_plain_any(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
-                              const BwdParams<T>& P, cudaStream_t stream);
-
-template <typename T, int CPL, int LX, int LO, int L2>
+template <typename T, int CPL, int LX, int LO>
 int launch_fast_bwd_one(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const T* x,
                         const T* y, const T* w, const T* g, T* gx, bool acc_x, T* gy, bool acc_y, T* gw, bool acc_w,
                         void* scratch, int64_t scratch_bytes, cudaStream_t stream) {
@@ -553,9 +484,6 @@ int launch_fast_bwd_one(const luna_uvu_plan* plan, const DeviceTables& dt, const
   P.src_rowptr = graph->src_rowptr;
   P.edge_ids = graph->edge_ids_by_src;
   P.tables = dt.bwd_tables;
-  P.sp_c = nullptr;
-  P.sp_j = nullptr;
-  P.row_stages = 0;
   P.status = dt.status;
   P.num_src_nodes = graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;
   P.num_edges = graph->num_edges;
@@ -577,56 +505,30 @@ int launch_fast_bwd_one(const luna_uvu_plan* plan, const DeviceTables& dt, const
   // would otherwise all land on one warp): their rows of gx are zero-filled here.
   if (gx != nullptr && !acc_x)
     LUNA_CUDA_CHECK(cudaMemsetAsync(gx, 0, static_cast<size_t>(P.num_src_nodes) * f.X * sizeof(T), stream));
-  bool launched = false;
-  if constexpr (L2 >= 0) {
-    // compiled-in coupling patterns, if the plan's terms have them
-    if constexpr (sparse_shape_ok<LX, (L2 < 0 ? 0 : L2), LO>()) {
-      const int variant = fast_bwd_variant(plan);
-      // The call training makes all the time - every gradient, gy and gw not accumulated, one warp pass per block -
-      // has kernels with a compile-time layout.
-      const bool plain = gx != nullptr && gy != nullptr && gw != nullptr && !acc_y && !acc_w &&
-                         f.chunks == 1 && variant == LUNA_BWD_ROW_STAGES && !plan->tuning.no_plain;
-      if (plain) {
-        const int rc = launch_fast_bwd_plain_any<T, CPL>(plan, dt, graph, P, stream);
-        if (rc == LUNA_OK) launched = true;
-        else if (rc != LUNA_ERR_UNSUPPORTED) return rc;
-      }
-      if (!launched && variant != LUNA_BWD_STAGED_TABLES) {
-        const bool rows = variant != LUNA_BWD_UNIT_RING;
-        const int rc = rows ? launch_fast_bwd_sparse<T, CPL, LX, (L2 < 0 ? 0 : L2), LO>(plan, dt, graph, P, gy != nullptr, wxw, stream)
-                            : launch_fast_bwd_units<T, CPL, LX, (L2 < 0 ? 0 : L2), LO>(plan, dt, graph, P, gy != nullptr, wxw, stream);
-        if (rc != LUNA_OK) return rc;
-        launched = true;
-      }
-    }
-  }
-  if (!launched) {
-    // Register budget by shape, through the launch bounds: FP32 with four channels per lane or degree-3 blocks runs
-    // up to 12 warps in a CTA (168 registers), smaller FP32 shapes up to 16 (128 registers); FP64 and the unrolled
-    // canonical kernels keep 8 warps (255).
-    constexpr int MAXW = (sizeof(T) == 8 || L2 >= 0) ? 8 : ((CPL == 4 || LX == 3 || LO == 3) ? 12 : 16);
-    constexpr int MINB = 1;
-    auto kernel = gy == nullptr ? fast_bwd_kernel<T, CPL, LX, LO, L2, true, false, MAXW, MINB>
-                                : (wxw ? fast_bwd_kernel<T, CPL, LX, LO, L2, true, true, MAXW, MINB>
-                                       : fast_bwd_kernel<T, CPL, LX, LO, L2, false, true, MAXW, MINB>);
-    cudaFuncAttributes attr;
-    LUNA_CUDA_CHECK(cudaFuncGetAttributes(&attr, kernel));
-    // between two units and two edges in a warp's ring
-    const Residency r = choose_residency(static_cast<size_t>(f.slot_elems) * sizeof(T), bwd_fixed_bytes<T, CPL>(f),
-                                         bwd_shared_bytes(f), dt.max_smem_optin, attr.numRegs, capped_warps(plan->tuning, MAXW), 2,
-                                         std::min(kMaxSlots, 2 * f.nkinds));
-    if (r.depth == 0) return fail(LUNA_ERR_UNSUPPORTED, "staged backward needs more shared memory than the device has");
-    P.slots = r.depth;
-    const size_t block_bytes = r.block_bytes;
-    const int nwarps = r.warps;
-    LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(block_bytes)));
-    // without this the driver may size the shared-memory carve-out for fewer CTAs than planned
-    LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    const int64_t blocks = grid_blocks(graph->num_edges, edges_per_warp(plan->tuning, 1024), r, dt.sm_count);
-    const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(f.chunks));
-    kernel<<<grid, nwarps * 32, block_bytes, stream>>>(P);
-    LUNA_LAUNCH_CHECK("staged backward");
-  }
+  // Register budget by shape, through the launch bounds: FP32 with four channels per lane or degree-3 blocks runs
+  // up to 12 warps in a CTA (168 registers), smaller FP32 shapes up to 16 (128 registers); FP64 keeps 8 warps (255).
+  constexpr int MAXW = sizeof(T) == 8 ? 8 : ((CPL == 4 || LX == 3 || LO == 3) ? 12 : 16);
+  constexpr int MINB = 1;
+  auto kernel = gy == nullptr ? fast_bwd_kernel<T, CPL, LX, LO, true, false, MAXW, MINB>
+                              : (wxw ? fast_bwd_kernel<T, CPL, LX, LO, true, true, MAXW, MINB>
+                                     : fast_bwd_kernel<T, CPL, LX, LO, false, true, MAXW, MINB>);
+  cudaFuncAttributes attr;
+  LUNA_CUDA_CHECK(cudaFuncGetAttributes(&attr, kernel));
+  // between two units and two edges in a warp's ring
+  const Residency r = choose_residency(static_cast<size_t>(f.slot_elems) * sizeof(T), bwd_fixed_bytes<T, CPL>(f),
+                                       bwd_shared_bytes(f), dt.max_smem_optin, attr.numRegs, capped_warps(plan->tuning, MAXW), 2,
+                                       std::min(kMaxSlots, 2 * f.nkinds));
+  if (r.depth == 0) return fail(LUNA_ERR_UNSUPPORTED, "staged backward needs more shared memory than the device has");
+  P.slots = r.depth;
+  const size_t block_bytes = r.block_bytes;
+  const int nwarps = r.warps;
+  LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(block_bytes)));
+  // without this the driver may size the shared-memory carve-out for fewer CTAs than planned
+  LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  const int64_t blocks = grid_blocks(graph->num_edges, edges_per_warp(plan->tuning, 1024), r, dt.sm_count);
+  const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(f.chunks));
+  kernel<<<grid, nwarps * 32, block_bytes, stream>>>(P);
+  LUNA_LAUNCH_CHECK("staged backward");
   if (P.gy_partial != nullptr) {
     const unsigned rb = static_cast<unsigned>(ceil_div(partial_count, 256));
     reduce_gy_partial<T><<<rb, 256, 0, stream>>>(P.gy_partial, gy, partial_count, f.chunks, acc_y ? 1 : 0);
@@ -639,18 +541,12 @@ template <typename T, int CPL>
 int launch_fast_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const T* x,
                     const T* y, const T* w, const T* g, T* gx, bool acc_x, T* gy, bool acc_y, T* gw, bool acc_w,
                     void* scratch, int64_t scratch_bytes, cudaStream_t stream) {
-  const int lx = plan->fast.LX, lo = plan->fast.LO, l2 = plan->fast.canon_l2;
+  const int lx = plan->fast.LX, lo = plan->fast.LO;
 #define LUNA_BWD_ARGS plan, dt, graph, x, y, w, g, gx, acc_x, gy, acc_y, gw, acc_w, scratch, scratch_bytes, stream
-  if (!plan->tuning.no_canon) {
-    if (lx == 2 && l2 == 3 && lo == 3) return launch_fast_bwd_one<T, CPL, 2, 3, 3>(LUNA_BWD_ARGS);
-    if (lx == 2 && l2 == 2 && lo == 2) return launch_fast_bwd_one<T, CPL, 2, 2, 2>(LUNA_BWD_ARGS);
-    if (lx == 3 && l2 == 3 && lo == 3) return launch_fast_bwd_one<T, CPL, 3, 3, 3>(LUNA_BWD_ARGS);
-    if (lx == 1 && l2 == 1 && lo == 1) return launch_fast_bwd_one<T, CPL, 1, 1, 1>(LUNA_BWD_ARGS);
-  }
-  if (lx <= 1 && lo <= 1) return launch_fast_bwd_one<T, CPL, 1, 1, -1>(LUNA_BWD_ARGS);
-  if (lx <= 2 && lo <= 2) return launch_fast_bwd_one<T, CPL, 2, 2, -1>(LUNA_BWD_ARGS);
-  if (lx <= 2 && lo <= 3) return launch_fast_bwd_one<T, CPL, 2, 3, -1>(LUNA_BWD_ARGS);
-  return launch_fast_bwd_one<T, CPL, 3, 3, -1>(LUNA_BWD_ARGS);
+  if (lx <= 1 && lo <= 1) return launch_fast_bwd_one<T, CPL, 1, 1>(LUNA_BWD_ARGS);
+  if (lx <= 2 && lo <= 2) return launch_fast_bwd_one<T, CPL, 2, 2>(LUNA_BWD_ARGS);
+  if (lx <= 2 && lo <= 3) return launch_fast_bwd_one<T, CPL, 2, 3>(LUNA_BWD_ARGS);
+  return launch_fast_bwd_one<T, CPL, 3, 3>(LUNA_BWD_ARGS);
 #undef LUNA_BWD_ARGS
 }
 

@@ -16,30 +16,15 @@
 // weights arrive as ready-made pairs, accumulators are unpacked only when a node is flushed.  The per-edge coupling
 // matrices are stored once; a matrix entry enters the packed FMA as a broadcast operand.  Every path is evaluated
 // as out_k += sum_i M[i][k] * (x_i * w): the accumulators are the only long-lived operands of the FMAs.
-//
-// What limits the kernel is the latency of a path's shared-memory loads in front of its arithmetic, with only two
-// warps per scheduler to hide it.  For the canonical full path lists (see canon_ok) the loops over paths are
-// therefore unrolled from compile-time tables, so that the loads of the next path are issued during the
-// arithmetic of the current one; a lane also keeps its share of the coupling-matrix program in registers.
 #pragma once
 
 #include <algorithm>
 #include <cstdlib>
 
-#include "cg_patterns.h"
 #include "uvu_packets.cuh"
 
 namespace luna {
 namespace fastk {
-
-// Whether the coupling tensor with pattern PT has a non-zero entry C[i][j][k] for some j: only those (i, k) have a
-// non-zero entry in an edge's coupling matrix.
-template <typename PT>
-__host__ __device__ constexpr bool pattern_has_ik(int i, int k) {
-  for (int t = 0; t < PT::n; ++t)
-    if (PT::t[t].i == i && PT::t[t].k == k) return true;
-  return false;
-}
 
 template <typename T>
 struct FwdParams {
@@ -71,27 +56,17 @@ __host__ __device__ inline size_t fwd_fixed_bytes(const FastMeta& f) {
   return (m_elems + 32) * sizeof(T) + kMaxStages * sizeof(uint64_t);
 }
 
-// Register budget of the coupling-matrix program: a lane keeps the two terms of up to this many entries in
-// registers (3 registers each); longer programs are read from shared memory.
-constexpr int kMaxProgramRounds = 12;
-
-// L2 >= 0: the path list is the canonical full list for (LX, L2, LO) and the loops over paths are unrolled from
-// compile-time tables.  L2 < 0: any path list, loops over paths read the tables in FastMeta.
-template <typename T, int CPL, int LX, int LO, int L2>
+template <typename T, int CPL, int LX, int LO>
 __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __grid_constant__ FwdParams<T> P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   using PK = FPk<T, CPL>;
   using V = typename PK::V;
   constexpr int NP = PK::NP;
-  constexpr bool kCanon = L2 >= 0;
-  constexpr int kCanonTotal = kCanon ? canon_moff(LX, L2 < 0 ? 0 : L2, LO, -1, -1, -1) : 0;
-  constexpr int kRounds = (kCanonTotal + 31) / 32;
-  constexpr bool kProgramInRegisters = kCanon && kRounds <= kMaxProgramRounds;
   const FastMeta& F = P.meta;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int stages = P.stages;
   const int stage_elems = F.w_stage_elems + F.x_stage_elems;
-  const int m_total = kCanon ? kCanonTotal : F.m_total;
+  const int m_total = F.m_total;
   const T* ell_c;
   const unsigned char* ell_j;
   load_ell<T>(smem_raw, P.ell_c, P.ell_j, m_total, F.m_terms, &ell_c, &ell_j);
@@ -107,20 +82,6 @@ __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __
     fence_barrier_init();
   }
   __syncwarp();
-
-  // the lane's share of the coupling-matrix program: entries lane, lane + 32, ...
-  T prog_a[kProgramInRegisters ? kRounds : 1], prog_b[kProgramInRegisters ? kRounds : 1];
-  unsigned prog_j[kProgramInRegisters ? kRounds : 1];
-  if constexpr (kProgramInRegisters) {
-#pragma unroll
-    for (int r = 0; r < kRounds; ++r) {
-      const int m = r * 32 + lane;
-      const bool in = m < m_total;
-      prog_a[r] = in ? ell_c[m] : T(0);
-      prog_b[r] = in ? ell_c[m_total + m] : T(0);
-      prog_j[r] = in ? (static_cast<unsigned>(ell_j[m]) | (static_cast<unsigned>(ell_j[m_total + m]) << 8)) : 0u;
-    }
-  }
 
   const int chw = 32 * CPL;
   const int c0 = blockIdx.y * chw;  // first channel of this warp's chunk
@@ -162,12 +123,9 @@ __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __
   bool alive = true;
 
   // out_k += sum_i M[i][k] * (x_i * w) for one path; the matrix is stored once and broadcast into both halves.
-  // With a compile-time degree l2 (canonical lists) the entries that the coupling tensor leaves zero for every y -
-  // about a quarter of them - are skipped.
-  auto path_body = [&](auto l1c, auto l2c, auto l3c, const T* wq, const T* matrix, const V* xl, V* al) {
-    constexpr int l1 = decltype(l1c)::value, l2 = decltype(l2c)::value, l3 = decltype(l3c)::value;
+  auto path_body = [&](auto l1c, auto l3c, const T* wq, const T* matrix, const V* xl, V* al) {
+    constexpr int l1 = decltype(l1c)::value, l3 = decltype(l3c)::value;
     constexpr int d1 = 2 * l1 + 1, d3 = 2 * l3 + 1, d3p = d3 + 1;
-    using PT = CgPattern<l1, (l2 < 0 ? 0 : l2), l3>;
     V w2[NP];  // a lane's consecutive channels are already adjacent in memory
     load_lane_packets<PK, T, CPL>(wq, w2);
     static_for<0, d1>([&](auto ic) {
@@ -179,8 +137,7 @@ __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __
         const V xw = vmul(xl[i * NP + p], w2[p]);
         static_for<0, d3>([&](auto kc) {
           constexpr int k = decltype(kc)::value;
-          if constexpr (l2 < 0 || pattern_has_ik<PT>(i, k))
-            al[k * NP + p] = vfma(bcast_packet(mrow[k], V{}), xw, al[k * NP + p]);
+          al[k * NP + p] = vfma(bcast_packet(mrow[k], V{}), xw, al[k * NP + p]);
         });
       }
     });
@@ -223,21 +180,15 @@ __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __
       // coupling matrices of this edge
       if (lane < F.Y) ybuf[lane] = y_next;
       __syncwarp();
-      if constexpr (kProgramInRegisters) {
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r)
-          mbuf[r * 32 + lane] = fma(prog_b[r], ybuf[prog_j[r] >> 8], prog_a[r] * ybuf[prog_j[r] & 255u]);
-      } else {
-        compute_m_share<T, false>(ell_c, ell_j, ybuf, mbuf, m_total, 0, 1, lane);
-      }
+      compute_m_share<T, false>(ell_c, ell_j, ybuf, mbuf, m_total, 0, 1, lane);
       if (e + 1 < e_end && lane < F.Y) y_next = P.y[(e + 1) * F.Y + lane];
       // this lane's x packets, formed once per edge: packet (l1, i, p) at l1 * l1 * NP + i * NP + p
       V xr[XR];
       static_for<0, LX + 1>([&](auto l1c) {
         constexpr int l1 = decltype(l1c)::value;
         constexpr int d1 = 2 * l1 + 1;
-        if (kCanon || F.x_off[l1] >= 0)
-          load_packets_scalar<PK, T, CPL, d1>(xs + (kCanon ? chw * l1 * l1 : F.xs_off[l1]) + lane * (CPL * d1),
+        if (F.x_off[l1] >= 0)
+          load_packets_scalar<PK, T, CPL, d1>(xs + F.xs_off[l1] + lane * (CPL * d1),
                                               &xr[l1 * l1 * NP]);
       });
       __syncwarp();
@@ -245,24 +196,15 @@ __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __
       const T* wl = ws + lane * CPL;
       static_for<0, LX + 1>([&](auto l1c) {
         constexpr int l1 = decltype(l1c)::value;
-        if (!kCanon && F.x_off[l1] < 0) return;
+        if (F.x_off[l1] < 0) return;
         const V* xl = &xr[l1 * l1 * NP];
         static_for<0, LO + 1>([&](auto l3c) {
           constexpr int l3 = decltype(l3c)::value;
           V* al = &acc[l3 * l3 * NP];
-          if constexpr (kCanon) {
-            static_for<0, (L2 < 0 ? 0 : L2) + 1>([&](auto l2c) {
-              constexpr int l2 = decltype(l2c)::value;
-              if constexpr (canon_ok(LX, L2, LO, l1, l2, l3))
-                path_body(l1c, l2c, l3c, wl + canon_wrank(LX, L2, LO, l1, l2, l3) * chw,
-                          mbuf + canon_moff(LX, L2, LO, l1, l2, l3), xl, al);
-            });
-          } else {
-            const int q_end = F.pair_ptr[l3 * (kMaxFastL + 1) + l1 + 1];
+          const int q_end = F.pair_ptr[l3 * (kMaxFastL + 1) + l1 + 1];
 #pragma unroll 1
-            for (int q = F.pair_ptr[l3 * (kMaxFastL + 1) + l1]; q < q_end; ++q)
-              path_body(l1c, std::integral_constant<int, -1>{}, l3c, wl + F.w_soff[q], mbuf + F.m_off[q], xl, al);
-          }
+          for (int q = F.pair_ptr[l3 * (kMaxFastL + 1) + l1]; q < q_end; ++q)
+            path_body(l1c, l3c, wl + F.w_soff[q], mbuf + F.m_off[q], xl, al);
         });
       });
       __syncwarp();  // every lane is done with this stage, mbuf and ybuf
@@ -309,7 +251,7 @@ __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __
 }
 
 
-template <typename T, int CPL, int LX, int LO, int L2>
+template <typename T, int CPL, int LX, int LO>
 int launch_fast_fwd_one(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const T* x,
                         const T* y, const T* w, T* out, bool accumulate, cudaStream_t stream) {
   const FastMeta& f = plan->fast;
@@ -329,7 +271,7 @@ int launch_fast_fwd_one(const luna_uvu_plan* plan, const DeviceTables& dt, const
   P.accumulate = accumulate ? 1 : 0;
   P.tile_counters = next_tile_counters(plan, dt);
   const size_t stage = static_cast<size_t>(f.w_stage_elems + f.x_stage_elems) * sizeof(T);
-  auto kernel = fast_fwd_kernel<T, CPL, LX, LO, L2>;
+  auto kernel = fast_fwd_kernel<T, CPL, LX, LO>;
   cudaFuncAttributes attr;
   LUNA_CUDA_CHECK(cudaFuncGetAttributes(&attr, kernel));
   const Residency r = choose_residency(stage, fwd_fixed_bytes<T, CPL>(f), ell_bytes<T>(f.m_total, f.m_terms),
@@ -356,23 +298,16 @@ int launch_fast_fwd_one(const luna_uvu_plan* plan, const DeviceTables& dt, const
   return LUNA_OK;
 }
 
-// Dispatch: a kernel unrolled for the canonical full path list if the plan has one of the compiled shapes, else
-// the smallest compiled degree class (LX, LO) that covers the plan, with loops over the plan's path tables.
+// Dispatch: the smallest compiled degree class (LX, LO) that covers the plan.
 template <typename T, int CPL>
 int launch_fast_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const T* x,
                     const T* y, const T* w, T* out, bool accumulate, cudaStream_t stream) {
-  const int lx = plan->fast.LX, lo = plan->fast.LO, l2 = plan->fast.canon_l2;
+  const int lx = plan->fast.LX, lo = plan->fast.LO;
 #define LUNA_FWD_ARGS plan, dt, graph, x, y, w, out, accumulate, stream
-  if (!plan->tuning.no_canon) {
-    if (lx == 2 && l2 == 3 && lo == 3) return launch_fast_fwd_one<T, CPL, 2, 3, 3>(LUNA_FWD_ARGS);
-    if (lx == 2 && l2 == 2 && lo == 2) return launch_fast_fwd_one<T, CPL, 2, 2, 2>(LUNA_FWD_ARGS);
-    if (lx == 3 && l2 == 3 && lo == 3) return launch_fast_fwd_one<T, CPL, 3, 3, 3>(LUNA_FWD_ARGS);
-    if (lx == 1 && l2 == 1 && lo == 1) return launch_fast_fwd_one<T, CPL, 1, 1, 1>(LUNA_FWD_ARGS);
-  }
-  if (lx <= 1 && lo <= 1) return launch_fast_fwd_one<T, CPL, 1, 1, -1>(LUNA_FWD_ARGS);
-  if (lx <= 2 && lo <= 2) return launch_fast_fwd_one<T, CPL, 2, 2, -1>(LUNA_FWD_ARGS);
-  if (lx <= 2 && lo <= 3) return launch_fast_fwd_one<T, CPL, 2, 3, -1>(LUNA_FWD_ARGS);
-  return launch_fast_fwd_one<T, CPL, 3, 3, -1>(LUNA_FWD_ARGS);
+  if (lx <= 1 && lo <= 1) return launch_fast_fwd_one<T, CPL, 1, 1>(LUNA_FWD_ARGS);
+  if (lx <= 2 && lo <= 2) return launch_fast_fwd_one<T, CPL, 2, 2>(LUNA_FWD_ARGS);
+  if (lx <= 2 && lo <= 3) return launch_fast_fwd_one<T, CPL, 2, 3>(LUNA_FWD_ARGS);
+  return launch_fast_fwd_one<T, CPL, 3, 3>(LUNA_FWD_ARGS);
 #undef LUNA_FWD_ARGS
 }
 

@@ -1,0 +1,67 @@
+"""The edge kernels at the sizes where they can go wrong, against the CPU oracle: every compiled shape, channel counts
+that leave lanes idle or need several warps per edge, rows shared by several teams and rows handed out in tiles."""
+
+import pytest
+import torch
+
+import lunaequivariance_b200 as luna
+from oracle import uvu_conv as oracle_conv
+from tests.helpers import all_paths, assert_close, random_problem
+from tests.test_gpu_random_shapes import skewed_graph
+
+pytestmark = pytest.mark.gpu
+DEVICE = "cuda"
+# degrees of x, of the edge attributes and of the output
+SHAPES = [((0,), (0, 1), (0, 1)), ((0,), (0, 1, 2), (0, 1, 2)), ((0,), (0, 1, 2, 3), (0, 1, 2, 3)),
+          ((0, 1), (0, 1), (0, 1)), ((0, 1, 2), (0, 1, 2), (0, 1, 2)), ((0, 1, 2, 3), (0, 1, 2, 3), (0, 1, 2, 3)),
+          ((0, 1, 2), (0, 1, 2, 3), (0, 1, 2, 3)), ((0, 1), (0, 1), (0,)), ((0, 1, 2), (0, 1, 2), (0,)),
+          ((0, 1, 2, 3), (0, 1, 2, 3), (0,)), ((1,), (1,), (0,))]
+
+
+def irreps(mul, degrees):
+    return "+".join(f"{mul}x{l}{'o' if l % 2 else 'e'}" for l in degrees)
+
+
+def check(shape, mul, dtype, nodes, edges, skew, seed):
+    in1, in2, out = irreps(mul, shape[0]), irreps(1, shape[1]), irreps(mul, shape[2])
+    instructions = all_paths(in1, in2, out)
+    module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False,
+                                    dtype=dtype)
+    assert module.op.backward_variant == "row"  # the edge kernels serve the plan
+    meta = oracle_conv.build_specs(in1, in2, out, instructions)
+    generator = torch.Generator().manual_seed(seed)
+    src, dst = skewed_graph(nodes, edges, generator, skew)
+    p = random_problem((meta["in1_dim"], meta["in2_dim"], meta["out_dim"], meta["weight_numel"]), nodes, src, dtype,
+                       generator)
+    ref = oracle_conv.conv_derivatives(meta, *(p[k].double() for k in ("x", "y", "w")), src, dst, nodes,
+                                       p["g"].double(), *(p[k].double() for k in ("rx", "ry", "rw")))
+    graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+    x, y, w, g = (p[k].to(DEVICE).requires_grad_(True) for k in ("x", "y", "w", "g"))
+    result = module(x, y, w, graph=graph)
+    gx, gy, gw = torch.autograd.grad(result, (x, y, w), g, create_graph=True)
+    hx, hy, hw, hg = torch.autograd.grad((gx, gy, gw), (x, y, w, g), tuple(p[k].to(DEVICE) for k in ("rx", "ry", "rw")))
+    module.op.check_status()
+    for key, value in dict(out=result, gx=gx, gy=gy, gw=gw, hx=hx, hy=hy, hw=hw, hg=hg).items():
+        assert_close(value, ref[key], dtype, f"{shape} x{mul} {dtype} {key}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+def test_every_shape(shape, dtype):
+    mul = (32, 48, 64)[shape % 3]
+    check(SHAPES[shape], mul, dtype, 29, 400, 0.0, shape)  # long rows: shared by teams
+    check(SHAPES[shape], mul, dtype, 150, 190, 1.5, shape + 50)  # short rows: tiles, many rows without edges
+
+
+# idle lanes (4, 12, 16, 48, 80, 96), all lanes (32, 64, 128), several warps per edge (160 and more; FP64: 96 and more)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("mul", [4, 12, 16, 32, 48, 64, 80, 96, 128, 160, 256, 320])
+def test_channel_counts(mul, dtype):
+    check(SHAPES[3], mul, dtype, 23, 260, 0.0, mul)
+    check(SHAPES[4], mul, dtype, 60, 90, 1.0, mul + 1)
+
+
+@pytest.mark.parametrize("nodes,edges", [(1, 1), (1, 2), (1, 77), (2, 9), (3, 1000), (700, 4000), (1300, 5300)])
+def test_row_splits(nodes, edges):
+    for mul in (16, 128):
+        check(SHAPES[3], mul, torch.float32, nodes, edges, 0.0, nodes + edges)
