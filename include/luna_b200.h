@@ -93,7 +93,8 @@ typedef enum {
                                    (l1, l2, l3) couplings in standard order (kernels unrolled at compile time), else -1 */
   LUNA_PLAN_SPARSE_TERMS = 6,   /* > 0 if the plan's coupling terms have the compiled-in non-zero patterns, so the
                                    backward kernel with per-lane contraction of the edge-attribute gradient applies */
-  LUNA_PLAN_BWD_VARIANT = 7     /* which first-order backward kernel aligned inputs get: a luna_bwd_variant */
+  LUNA_PLAN_BWD_VARIANT = 7,    /* which first-order backward kernel aligned inputs get: a luna_bwd_variant */
+  LUNA_PLAN_NEEDS_SCRATCH = 8   /* 1 if backward calls that produce gy use the scratch buffer, 0 if they take none */
 } luna_plan_query;
 typedef enum {
   LUNA_BWD_TABLE_DRIVEN = 0, /* one thread per output element, any configuration */

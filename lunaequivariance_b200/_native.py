@@ -8,6 +8,7 @@ point fails, callers get an exception.  The reference reaches its own generated 
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 
@@ -16,6 +17,8 @@ import torch
 _PACKAGE_DIR = os.path.dirname(os.path.abspath(__file__))
 # LUNA_B200_LIBRARY selects another build of the same library (kernel tuning experiments).
 LIBRARY_PATH = os.environ.get("LUNA_B200_LIBRARY") or os.path.join(_PACKAGE_DIR, "_lib", "libluna_b200.so")
+
+BINDING_PATH = os.path.join(_PACKAGE_DIR, "_lib", "luna_torch.so")
 
 LUNA_OK = 0
 LUNA_ERR_INVALID_ARGUMENT = -1
@@ -111,8 +114,9 @@ _SIGNATURES = {
 
 EXPORTED_SYMBOLS = tuple(_SIGNATURES)
 
-_lock = threading.Lock()
+_lock = threading.RLock()
 _library = None
+_binding = None
 
 
 def library() -> ctypes.CDLL:
@@ -134,6 +138,25 @@ def library() -> ctypes.CDLL:
                 function.argtypes = argtypes
             _library = handle
     return _library
+
+
+def binding():
+    """The launch path in C++ (``csrc/torch_binding.cpp``): checks, allocation and the autograd chain.  Loaded once, bound
+    to the same library as ``library()``; raises if it has not been built."""
+    global _binding
+    if _binding is not None:
+        return _binding
+    with _lock:
+        if _binding is None:
+            library()
+            if not os.path.exists(BINDING_PATH):
+                raise RuntimeError(f"{BINDING_PATH} is missing: build it with `python -m lunaequivariance_b200.build`")
+            spec = importlib.util.spec_from_file_location("luna_torch", BINDING_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            module.load(LIBRARY_PATH)
+            _binding = module
+    return _binding
 
 
 def last_error() -> str:
@@ -163,5 +186,5 @@ def dtype_code(dtype: torch.dtype) -> int:
     raise ValueError(f"float32 or float64 required, got {dtype}")
 
 
-__all__ = ["library", "check", "last_error", "pointer", "current_stream", "dtype_code", "UvuPath", "UvuDesc",
+__all__ = ["library", "binding", "check", "last_error", "pointer", "current_stream", "dtype_code", "UvuPath", "UvuDesc",
            "Graph", "GraphOut", "ShDesc", "EXPORTED_SYMBOLS", "LIBRARY_PATH"]

@@ -1,4 +1,5 @@
-"""Builds the C-ABI shared library ``_lib/libluna_b200.so`` from ``csrc/*.cu`` with nvcc for sm_100a.
+"""Builds the C-ABI shared library ``_lib/libluna_b200.so`` from ``csrc/*.cu`` with nvcc for sm_100a, and the PyTorch
+launch path ``_lib/luna_torch.so`` from ``csrc/torch_binding.cpp`` with the host compiler.
 
 Usage: ``python -m lunaequivariance_b200.build [--force] [--verbose]``.  Objects are rebuilt only when a source or
 header is newer; files compile in parallel.  No GPU is needed to build.
@@ -18,6 +19,7 @@ CSRC = os.path.join(PACKAGE_DIR, "csrc")
 LIB_DIR = os.path.join(PACKAGE_DIR, "_lib")
 BUILD_DIR = os.path.join(PACKAGE_DIR, "_lib", "obj")
 LIBRARY = os.path.join(LIB_DIR, "libluna_b200.so")
+BINDING = os.path.join(LIB_DIR, "luna_torch.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -76,6 +78,29 @@ def compile_one(nvcc: str, unit: tuple[str, str, list[str]], verbose: bool, ptxa
     return obj, result.stderr if (verbose or ptxas_info) else ""
 
 
+def build_binding(nvcc: str, newest_header: float, force: bool) -> None:
+    """The torch extension: host code only; it finds the library's entry points at load time."""
+    import sysconfig
+
+    import torch
+
+    source = os.path.join(CSRC, "torch_binding.cpp")
+    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) >= max(os.path.getmtime(source), newest_header):
+        return
+    root = torch.__path__[0]
+    cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               cuda_include, "/usr/local/cuda/include", sysconfig.get_paths()["include"]]
+    command = [os.environ.get("CXX") or shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared",
+               "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=luna_torch",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{path}" for path in include),
+               source, "-o", BINDING, f"-L{os.path.join(root, 'lib')}", "-ltorch", "-ltorch_cpu", "-ltorch_python",
+               "-lc10", "-lc10_cuda", "-ldl"]
+    result = subprocess.run(command, capture_output=True, text=True)
+    if result.returncode != 0:
+        raise RuntimeError(f"building {BINDING} failed:\n{result.stdout}\n{result.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
     nvcc = find_nvcc()
     os.makedirs(BUILD_DIR, exist_ok=True)
@@ -87,12 +112,14 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
                  or os.path.getmtime(obj) < max(os.path.getmtime(source), newest_header))
         if stale:
             todo.append((source, obj, flags))
-    if todo:
-        workers = min(len(todo), max(1, (os.cpu_count() or 2)))
-        with concurrent.futures.ThreadPoolExecutor(max_workers=workers) as pool:
+    workers = max(1, os.cpu_count() or 2)
+    with concurrent.futures.ThreadPoolExecutor(max_workers=workers) as pool:
+        binding = pool.submit(build_binding, nvcc, newest_header, force)
+        if todo:
             for obj, log in pool.map(lambda unit: compile_one(nvcc, unit, verbose, ptxas_info), todo):
                 if log:
                     print(log, file=sys.stderr)
+        binding.result()
     wanted = {os.path.basename(o) for o in objects}
     for name in os.listdir(BUILD_DIR):  # drop objects of deleted sources
         if name.endswith(".o") and name not in wanted:

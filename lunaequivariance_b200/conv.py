@@ -33,6 +33,8 @@ from functools import lru_cache
 
 import numpy as np
 import torch
+from torch.fx.experimental.proxy_tensor import get_proxy_mode
+from torch.utils._python_dispatch import is_in_torch_dispatch_mode
 
 from . import _native
 from .graph import LunaTPGraph, make_graph
@@ -43,9 +45,6 @@ _DTYPE_NAMES = {torch.float32: "float32", torch.float64: "float64"}
 
 def is_compiling() -> bool:
     """True while Dynamo or make_fx records a graph (``src/utils/__init__.py:8-12``)."""
-    from torch.fx.experimental.proxy_tensor import get_proxy_mode
-    from torch.utils._python_dispatch import is_in_torch_dispatch_mode
-
     return torch.compiler.is_compiling() or (is_in_torch_dispatch_mode() and get_proxy_mode() is not None)
 
 
@@ -87,18 +86,12 @@ class _Plan:
         handle = ctypes.c_void_p()
         _native.check(lib.luna_uvu_plan_create(ctypes.byref(desc), ctypes.byref(handle)))
         self.handle = handle
-        self._destroy = lib.luna_uvu_plan_destroy
+        # owns the plan: it is destroyed with the last reference, of which autograd graphs hold some
+        self.op = _native.binding().Op(handle.value, desc.in1_dim, desc.in2_dim, desc.out_dim, desc.weight_numel,
+                                       dtype == torch.float64)
 
     def query(self, what: int) -> int:
         return int(_native.library().luna_uvu_plan_query(self.handle, what))
-
-    def __del__(self):
-        handle, self.handle = getattr(self, "handle", None), None
-        if handle:
-            try:
-                self._destroy(handle)
-            except Exception:  # interpreter shutdown
-                pass
 
 
 class LunaTPUVUConv:
@@ -301,6 +294,8 @@ def _check_inputs(op: LunaTPUVUConv, x, y, w, source_rows, num_edges, *, g=None,
 
 
 def _scratch(op: LunaTPUVUConv, num_nodes: int, num_edges: int, device) -> tuple[torch.Tensor | None, int]:
+    if op._plan.query(8) <= 0:
+        return None, 0
     size = int(_native.library().luna_uvu_conv_scratch_bytes(op._plan.handle, num_nodes, num_edges))
     if size <= 0:
         return None, 0
@@ -750,6 +745,8 @@ def _conv(op: LunaTPUVUConv, x, edge_attr, weight, graph: LunaTPGraph):
             x.contiguous(), edge_attr.contiguous(), weight.contiguous(), None, graph.table_list(),
             graph.num_nodes, False, op.torch_config)
         return out
+    if x.is_cuda and graph.src.is_cuda and graph.split_rows() is None:
+        return _native.binding().conv(op._plan.op, graph.native_holder(), x, edge_attr, weight)
     return UVUConvForward.apply(op, _through_view(x), _through_view(edge_attr), _through_view(weight), graph)
 
 

@@ -1,0 +1,533 @@
+// PyTorch side of the launch path in C++: argument checks, output allocation, the stream lookup and the autograd chain of
+// the convolution and of the spherical harmonics.  A small convolution takes a few microseconds on the GPU; the same
+// chain in Python costs some two hundred per forward and backward.
+//
+// The C-ABI library stays the product: this module only calls its entry points (resolved at load time from the path
+// Python passes, so that both use the same build) and has no kernels of its own.
+//
+// Autograd.  F(x, y, w, g) is linear in every operand; ConvForward is dF/dg, ConvBackward the other three first
+// derivatives, ConvDouble the derivatives of ConvBackward, and everything beyond is made of ConvPartial, the derivative
+// of F with respect to one operand, whose own derivatives are again ConvPartial.  Which gradients are worth computing is
+// asked from the running graph task (needs_input_grad).
+#include <dlfcn.h>
+
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <array>
+#include <mutex>
+#include <optional>
+
+#include "../../include/luna_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+// ---- the library ------------------------------------------------------------------------------------------------------
+struct Api {
+  decltype(&luna_last_error) last_error = nullptr;
+  decltype(&luna_uvu_plan_destroy) plan_destroy = nullptr;
+  decltype(&luna_uvu_plan_query) plan_query = nullptr;
+  decltype(&luna_uvu_conv_scratch_bytes) scratch_bytes = nullptr;
+  decltype(&luna_uvu_conv_fwd) fwd = nullptr;
+  decltype(&luna_uvu_conv_bwd) bwd = nullptr;
+  decltype(&luna_uvu_conv_dbl_bwd) dbl_bwd = nullptr;
+  decltype(&luna_sh_fwd) sh_fwd = nullptr;
+  decltype(&luna_sh_bwd) sh_bwd = nullptr;
+  decltype(&luna_sh_dbl_bwd) sh_dbl_bwd = nullptr;
+} api;
+
+template <typename F>
+void resolve(void* library, const char* name, F& function) {
+  function = reinterpret_cast<F>(dlsym(library, name));
+  TORCH_CHECK(function != nullptr, "symbol ", name, " is missing from the library");
+}
+
+void load(const std::string& path) {
+  void* library = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  TORCH_CHECK(library != nullptr, "cannot load ", path, ": ", dlerror());
+  resolve(library, "luna_last_error", api.last_error);
+  resolve(library, "luna_uvu_plan_destroy", api.plan_destroy);
+  resolve(library, "luna_uvu_plan_query", api.plan_query);
+  resolve(library, "luna_uvu_conv_scratch_bytes", api.scratch_bytes);
+  resolve(library, "luna_uvu_conv_fwd", api.fwd);
+  resolve(library, "luna_uvu_conv_bwd", api.bwd);
+  resolve(library, "luna_uvu_conv_dbl_bwd", api.dbl_bwd);
+  resolve(library, "luna_sh_fwd", api.sh_fwd);
+  resolve(library, "luna_sh_bwd", api.sh_bwd);
+  resolve(library, "luna_sh_dbl_bwd", api.sh_dbl_bwd);
+}
+
+// A failed status as the exception Python raises for it.
+void check(int status) {
+  if (C10_LIKELY(status == LUNA_OK)) return;
+  const char* text = api.last_error();
+  switch (status) {
+    case LUNA_ERR_INVALID_ARGUMENT:
+    case LUNA_ERR_MISALIGNED:
+      TORCH_CHECK_VALUE(false, text);
+    case LUNA_ERR_UNSUPPORTED:
+      TORCH_CHECK_NOT_IMPLEMENTED(false, text);
+    default:
+      TORCH_CHECK(false, text, " (status ", status, ")");
+  }
+}
+
+// ---- handles kept by Python and by autograd nodes -----------------------------------------------------------------------
+struct Op : torch::CustomClassHolder {
+  luna_uvu_plan* plan;
+  int64_t X, Y, O, W;
+  at::ScalarType dtype;
+  Op(int64_t handle, int64_t x, int64_t y, int64_t o, int64_t w, bool f64)
+      : plan(reinterpret_cast<luna_uvu_plan*>(handle)), X(x), Y(y), O(o), W(w), dtype(f64 ? at::kDouble : at::kFloat) {}
+  ~Op() override { api.plan_destroy(plan); }
+};
+
+struct Graph : torch::CustomClassHolder {
+  std::array<Tensor, 5> tables;  // src, dst, dst_rowptr, src_rowptr, edge_ids_by_src
+  luna_graph native{};
+  Graph(std::array<Tensor, 5> t, int64_t nodes, int64_t source_rows) : tables(std::move(t)) {
+    native.num_nodes = nodes;
+    native.num_src_nodes = source_rows;
+    native.num_edges = tables[0].numel();
+    native.src = tables[0].data_ptr<int32_t>();
+    native.dst = tables[1].data_ptr<int32_t>();
+    native.dst_rowptr = tables[2].data_ptr<int32_t>();
+    native.src_rowptr = tables[3].data_ptr<int32_t>();
+    native.edge_ids_by_src = tables[4].data_ptr<int32_t>();
+  }
+};
+
+using OpPtr = c10::intrusive_ptr<Op>;
+using GraphPtr = c10::intrusive_ptr<Graph>;
+
+template <typename H>
+void keep(AutogradContext* ctx, const char* name, const c10::intrusive_ptr<H>& holder) {
+  ctx->saved_data[name] = c10::IValue::make_capsule(holder);
+}
+template <typename H>
+c10::intrusive_ptr<H> kept(AutogradContext* ctx, const char* name) {
+  return c10::static_intrusive_pointer_cast<H>(ctx->saved_data[name].toCapsule());
+}
+
+// ---- launch wrappers ----------------------------------------------------------------------------------------------------
+// Contiguous and 16-byte aligned (the staged kernels move 16-byte pieces of rows).
+Tensor prepared(const Tensor& t) {
+  if (!t.defined()) return t;
+  Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+}
+
+void check_operand(const Op& op, const Tensor& x, const Tensor& t, const char* name, int64_t rows, int64_t columns) {
+  if (!t.defined()) return;
+  TORCH_CHECK_TYPE(t.scalar_type() == op.dtype, name, " must be ", op.dtype == at::kDouble ? "torch.float64" : "torch.float32",
+                   ", got ", t.scalar_type());
+  TORCH_CHECK_VALUE(t.device() == x.device(), "features, weights and graph must share one CUDA device");
+  TORCH_CHECK_VALUE(t.dim() == 2 && t.size(0) == rows && t.size(1) == columns, name, " must have shape (", rows, ", ",
+                    columns, "), got ", t.sizes());
+}
+
+void check_operands(const Op& op, const Graph& graph, const Tensor& x, const Tensor& y, const Tensor& w, const Tensor& g) {
+  TORCH_CHECK(x.is_cuda(), "CUDA is required for SO3 LunaTP.");
+  check_operand(op, x, x, "x", graph.native.num_src_nodes, op.X);
+  check_operand(op, x, y, "edge_attr", graph.native.num_edges, op.Y);
+  check_operand(op, x, w, "weight", graph.native.num_edges, op.W);
+  check_operand(op, x, g, "grad_out", graph.native.num_nodes, op.O);
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+void* pointer(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+
+Tensor scratch_for(const Op& op, const Graph& graph, const Tensor& like, int64_t* bytes) {
+  *bytes = 0;
+  if (!api.plan_query(op.plan, LUNA_PLAN_NEEDS_SCRATCH)) return Tensor();
+  *bytes = api.scratch_bytes(op.plan, graph.native.num_nodes, graph.native.num_edges);
+  return *bytes > 0 ? at::empty({*bytes}, like.options().dtype(at::kByte)) : Tensor();
+}
+
+Tensor run_forward(const Op& op, const Graph& graph, const Tensor& x_, const Tensor& y_, const Tensor& w_) {
+  check_operands(op, graph, x_, y_, w_, Tensor());
+  const c10::cuda::CUDAGuard guard(x_.device());
+  const Tensor x = prepared(x_), y = prepared(y_), w = prepared(w_);
+  Tensor out = at::empty({graph.native.num_nodes, op.O}, x.options());
+  check(api.fwd(op.plan, &graph.native, x.data_ptr(), y.data_ptr(), w.data_ptr(), out.data_ptr(), stream_of(x)));
+  return out;
+}
+
+enum : int { kX = 1, kY = 2, kW = 4, kG = 8 };
+
+// The first derivatives named in `mask`; the others stay undefined.
+std::array<Tensor, 3> run_backward(const Op& op, const Graph& graph, const Tensor& x_, const Tensor& y_, const Tensor& w_,
+                                   const Tensor& g_, int mask) {
+  std::array<Tensor, 3> out;
+  if (!mask) return out;
+  check_operands(op, graph, x_, y_, w_, g_);
+  const c10::cuda::CUDAGuard guard(x_.device());
+  const Tensor x = prepared(x_), y = prepared(y_), w = prepared(w_), g = prepared(g_);
+  const Tensor* like[3] = {&x, &y, &w};
+  const bool empty = graph.native.num_edges == 0 || graph.native.num_nodes == 0;
+  for (int s = 0; s < 3; ++s)
+    if (mask >> s & 1) out[s] = empty ? at::zeros_like(*like[s]) : at::empty_like(*like[s]);
+  if (empty) return out;
+  int64_t bytes = 0;
+  const Tensor scratch = scratch_for(op, graph, x, &bytes);
+  check(api.bwd(op.plan, &graph.native, x.data_ptr(), y.data_ptr(), w.data_ptr(), g.data_ptr(), pointer(out[0]),
+                pointer(out[1]), pointer(out[2]), pointer(scratch), bytes, stream_of(x)));
+  return out;
+}
+
+// The second derivatives named in `mask` (x, y, w, g) for the cotangents rx, ry, rw, each of which may be undefined.
+std::array<Tensor, 4> run_double(const Op& op, const Graph& graph, const Tensor& x_, const Tensor& y_, const Tensor& w_,
+                                 const Tensor& g_, const Tensor& rx_, const Tensor& ry_, const Tensor& rw_, int mask) {
+  std::array<Tensor, 4> out;
+  if (!mask) return out;
+  check_operands(op, graph, x_, y_, w_, g_);
+  check_operand(op, x_, rx_, "rx", graph.native.num_src_nodes, op.X);
+  check_operand(op, x_, ry_, "ry", graph.native.num_edges, op.Y);
+  check_operand(op, x_, rw_, "rw", graph.native.num_edges, op.W);
+  const c10::cuda::CUDAGuard guard(x_.device());
+  const Tensor x = prepared(x_), y = prepared(y_), w = prepared(w_), g = prepared(g_), rx = prepared(rx_),
+               ry = prepared(ry_), rw = prepared(rw_);
+  const Tensor* like[4] = {&x, &y, &w, &g};
+  const bool empty = graph.native.num_edges == 0 || graph.native.num_nodes == 0;
+  for (int s = 0; s < 4; ++s)
+    if (mask >> s & 1) out[s] = empty ? at::zeros_like(*like[s]) : at::empty_like(*like[s]);
+  if (empty) return out;
+  int64_t bytes = 0;
+  const Tensor scratch = scratch_for(op, graph, x, &bytes);
+  check(api.dbl_bwd(op.plan, &graph.native, x.data_ptr(), y.data_ptr(), w.data_ptr(), g.data_ptr(), pointer(rx), pointer(ry),
+                    pointer(rw), pointer(out[0]), pointer(out[1]), pointer(out[2]), pointer(out[3]), pointer(scratch), bytes,
+                    stream_of(x)));
+  return out;
+}
+
+// ---- the autograd chain of the convolution --------------------------------------------------------------------------------
+template <size_t N>
+variable_list only(const std::array<Tensor, N>& tensors, int mask) {
+  variable_list list;
+  for (size_t s = 0; s < N; ++s)
+    if (mask >> s & 1) list.push_back(tensors[s]);
+  return list;
+}
+// The reverse: a list that holds the entries of `mask` only.
+template <size_t N>
+std::array<Tensor, N> spread(const variable_list& list, int mask) {
+  std::array<Tensor, N> tensors;
+  size_t next = 0;
+  for (size_t s = 0; s < N; ++s)
+    if (mask >> s & 1) tensors[s] = list[next++];
+  return tensors;
+}
+Tensor contiguous(const Tensor& t) { return t.defined() ? t.contiguous() : t; }
+
+// dF/d(operand `slot`), slots 0..3 = x, y, w, g; a, b, c: the other three operands in that order.
+struct ConvPartial : Function<ConvPartial> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& a, const Tensor& b, const Tensor& c, int64_t slot, const OpPtr& op,
+                        const GraphPtr& graph) {
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({a, b, c});
+    ctx->saved_data["slot"] = slot;
+    keep(ctx, "op", op);
+    keep(ctx, "graph", graph);
+    const auto full = operands({a, b, c}, slot, Tensor());
+    if (slot == 3) return run_forward(*op, *graph, full[0], full[1], full[2]);
+    // the kernels take all four operands; the one in the free slot is only looked at for its shape
+    const at::TensorOptions options = a.options();
+    const luna_graph& n = graph->native;
+    Tensor stand_in;
+    if (slot == 0) stand_in = at::empty({n.num_src_nodes, op->X}, options);
+    if (slot == 1) stand_in = at::empty({n.num_edges, op->Y}, options);
+    if (slot == 2) stand_in = at::empty({n.num_edges, op->W}, options);
+    const auto all = operands({a, b, c}, slot, stand_in);
+    return run_backward(*op, *graph, all[0], all[1], all[2], all[3], 1 << slot)[slot];
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    variable_list out(6);
+    if (!grads[0].defined()) return out;
+    const auto saved = ctx->get_saved_variables();
+    const int64_t slot = ctx->saved_data["slot"].toInt();
+    const auto op = kept<Op>(ctx, "op");
+    const auto graph = kept<Graph>(ctx, "graph");
+    // <r, dF/ds(a, b, c)> = F with r in slot s: the gradient of another operand is its partial at the rest
+    const auto full = operands({saved[0], saved[1], saved[2]}, slot, grads[0].contiguous());
+    for (int64_t other = 0, position = 0; other < 4; ++other) {
+      if (other == slot) continue;
+      if (ctx->needs_input_grad(position)) out[position] = of(full, other, op, graph);
+      ++position;
+    }
+    return out;
+  }
+  static std::array<Tensor, 4> operands(const std::array<Tensor, 3>& others, int64_t slot, const Tensor& free) {
+    std::array<Tensor, 4> full;
+    for (int64_t s = 0, next = 0; s < 4; ++s) full[s] = s == slot ? free : others[next++];
+    return full;
+  }
+  static Tensor of(const std::array<Tensor, 4>& full, int64_t slot, const OpPtr& op, const GraphPtr& graph) {
+    std::array<Tensor, 3> others;
+    for (int64_t s = 0, next = 0; s < 4; ++s)
+      if (s != slot) others[next++] = full[s];
+    return apply(others[0], others[1], others[2], slot, op, graph);
+  }
+};
+
+struct ConvDouble : Function<ConvDouble> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& y, const Tensor& w, const Tensor& g,
+                               const std::optional<Tensor>& rx, const std::optional<Tensor>& ry,
+                               const std::optional<Tensor>& rw, int64_t mask, const OpPtr& op, const GraphPtr& graph) {
+    const Tensor none;
+    const Tensor &tx = rx ? *rx : none, &ty = ry ? *ry : none, &tw = rw ? *rw : none;
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({x, y, w, g, tx, ty, tw});
+    ctx->saved_data["mask"] = mask;
+    keep(ctx, "op", op);
+    keep(ctx, "graph", graph);
+    return only(run_double(*op, *graph, x, y, w, g, tx, ty, tw, static_cast<int>(mask)), static_cast<int>(mask));
+  }
+  // The outputs contracted with their cotangents b are a sum of F with three of its operands replaced; the gradient of
+  // a tensor is the sum of the partials over the terms it appears in.
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    variable_list out(10);
+    const auto saved = ctx->get_saved_variables();
+    const auto op = kept<Op>(ctx, "op");
+    const auto graph = kept<Graph>(ctx, "graph");
+    const auto b = spread<4>(grads, static_cast<int>(ctx->saved_data["mask"].toInt()));
+    // tensors by number: 0..6 = x, y, w, g, rx, ry, rw (saved), 7..10 = bx, by, bw, bg
+    std::array<Tensor, 11> t;
+    for (int s = 0; s < 7; ++s) t[s] = saved[s];
+    for (int s = 0; s < 4; ++s) t[7 + s] = contiguous(b[s]);
+    static constexpr int terms[9][4] = {{7, 5, 2, 3}, {7, 1, 6, 3}, {4, 8, 2, 3}, {0, 8, 6, 3}, {4, 1, 9, 3},
+                                        {0, 5, 9, 3}, {4, 1, 2, 10}, {0, 5, 2, 10}, {0, 1, 6, 10}};
+    for (int v = 0, edge = 0; v < 7; ++v) {
+      if (!t[v].defined()) continue;  // a missing tangent has no edge
+      if (!ctx->needs_input_grad(edge++)) continue;
+      Tensor sum;
+      for (const auto& term : terms) {
+        bool whole = true;
+        int slot = -1;
+        for (int s = 0; s < 4; ++s) {
+          whole = whole && t[term[s]].defined();
+          if (term[s] == v) slot = s;
+        }
+        if (!whole || slot < 0) continue;
+        const Tensor part = ConvPartial::of({t[term[0]], t[term[1]], t[term[2]], t[term[3]]}, slot, op, graph);
+        sum = sum.defined() ? sum + part : part;
+      }
+      out[v] = sum;
+    }
+    return out;
+  }
+};
+
+struct ConvBackward : Function<ConvBackward> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& y, const Tensor& w, const Tensor& g,
+                               int64_t mask, const OpPtr& op, const GraphPtr& graph) {
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({x, y, w, g});
+    ctx->saved_data["mask"] = mask;
+    keep(ctx, "op", op);
+    keep(ctx, "graph", graph);
+    return only(run_backward(*op, *graph, x, y, w, g, static_cast<int>(mask)), static_cast<int>(mask));
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    variable_list out(7);
+    const auto r = spread<3>(grads, static_cast<int>(ctx->saved_data["mask"].toInt()));
+    if (!r[0].defined() && !r[1].defined() && !r[2].defined()) return out;
+    int mask = 0;
+    for (int s = 0; s < 4; ++s) mask |= ctx->needs_input_grad(s) ? 1 << s : 0;
+    if (!mask) return out;
+    const auto saved = ctx->get_saved_variables();
+    const auto op = kept<Op>(ctx, "op");
+    const auto graph = kept<Graph>(ctx, "graph");
+    std::array<Tensor, 4> h;
+    if (at::GradMode::is_enabled()) {
+      auto optional = [](const Tensor& t) { return t.defined() ? std::optional<Tensor>(t.contiguous()) : std::nullopt; };
+      h = spread<4>(ConvDouble::apply(saved[0], saved[1], saved[2], saved[3], optional(r[0]), optional(r[1]),
+                                      optional(r[2]), static_cast<int64_t>(mask), op, graph),
+                    mask);
+    } else {
+      h = run_double(*op, *graph, saved[0], saved[1], saved[2], saved[3], r[0], r[1], r[2], mask);
+    }
+    for (int s = 0; s < 4; ++s) out[s] = h[s];
+    return out;
+  }
+};
+
+struct ConvForward : Function<ConvForward> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& y, const Tensor& w, const OpPtr& op,
+                        const GraphPtr& graph) {
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({x, y, w});
+    keep(ctx, "op", op);
+    keep(ctx, "graph", graph);
+    return run_forward(*op, *graph, x, y, w);
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    variable_list out(5);
+    if (!grads[0].defined()) return out;
+    int mask = 0;
+    for (int s = 0; s < 3; ++s) mask |= ctx->needs_input_grad(s) ? 1 << s : 0;
+    if (!mask) return out;
+    const auto saved = ctx->get_saved_variables();
+    const auto op = kept<Op>(ctx, "op");
+    const auto graph = kept<Graph>(ctx, "graph");
+    const Tensor g = grads[0].contiguous();
+    const auto d = at::GradMode::is_enabled()
+                       ? spread<3>(ConvBackward::apply(saved[0], saved[1], saved[2], g, static_cast<int64_t>(mask), op, graph), mask)
+                       : run_backward(*op, *graph, saved[0], saved[1], saved[2], g, mask);
+    for (int s = 0; s < 3; ++s) out[s] = d[s];
+    return out;
+  }
+};
+
+bool tracked(std::initializer_list<const Tensor*> tensors) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : tensors)
+    if (t->requires_grad()) return true;
+  return false;
+}
+
+Tensor conv(const OpPtr& op, const GraphPtr& graph, const Tensor& x, const Tensor& y, const Tensor& w) {
+  pybind11::gil_scoped_release release;
+  return tracked({&x, &y, &w}) ? ConvForward::apply(x, y, w, op, graph) : run_forward(*op, *graph, x, y, w);
+}
+
+// ---- spherical harmonics --------------------------------------------------------------------------------------------------
+struct Harmonics : torch::CustomClassHolder {
+  luna_sh_desc desc{};
+  int64_t columns;
+  bool constant;
+  Harmonics(const std::vector<int64_t>& degrees, bool normalize, int64_t normalization, int64_t out_dim, bool f64)
+      : columns(out_dim), constant(true) {
+    TORCH_CHECK_NOT_IMPLEMENTED(degrees.size() <= 32, "at most 32 degree entries are supported");
+    desc.dtype = f64 ? LUNA_F64 : LUNA_F32;
+    desc.num_degrees = static_cast<int32_t>(degrees.size());
+    for (size_t i = 0; i < degrees.size(); ++i) {
+      desc.degrees[i] = static_cast<int32_t>(degrees[i]);
+      constant = constant && degrees[i] == 0;
+    }
+    desc.normalize = normalize;
+    desc.normalization = static_cast<int32_t>(normalization);
+  }
+};
+using HarmonicsPtr = c10::intrusive_ptr<Harmonics>;
+
+Tensor rows_of(const Tensor& t) { return t.reshape({-1, t.size(-1)}).contiguous(); }
+
+void check_vectors(const Harmonics& h, const Tensor& v) {
+  TORCH_CHECK(v.is_cuda(), "CUDA is required for spherical harmonics in this library");
+  TORCH_CHECK_TYPE(v.scalar_type() == (h.desc.dtype == LUNA_F64 ? at::kDouble : at::kFloat),
+                   "spherical harmonics require float32 or float64 input");
+  TORCH_CHECK_VALUE(v.dim() > 0 && v.size(-1) == 3, "SphericalHarmonics input must have shape (...,3)");
+}
+
+Tensor sh_forward(const Harmonics& h, const Tensor& v) {
+  check_vectors(h, v);
+  const c10::cuda::CUDAGuard guard(v.device());
+  const Tensor flat = rows_of(v);
+  auto shape = v.sizes().vec();
+  shape.back() = h.columns;
+  Tensor out = at::empty(shape, v.options());
+  check(api.sh_fwd(&h.desc, flat.data_ptr(), out.data_ptr(), flat.size(0), stream_of(v)));
+  return out;
+}
+
+Tensor sh_backward(const Harmonics& h, const Tensor& v, const Tensor& g) {
+  check_vectors(h, v);
+  const c10::cuda::CUDAGuard guard(v.device());
+  const Tensor flat = rows_of(v), cotangents = rows_of(g);
+  Tensor dv = at::empty(v.sizes(), v.options());
+  check(api.sh_bwd(&h.desc, flat.data_ptr(), cotangents.data_ptr(), dv.data_ptr(), flat.size(0), stream_of(v)));
+  return dv;
+}
+
+std::array<Tensor, 2> sh_double(const Harmonics& h, const Tensor& v, const Tensor& g, const Tensor& r, int mask) {
+  check_vectors(h, v);
+  const c10::cuda::CUDAGuard guard(v.device());
+  const Tensor flat = rows_of(v), cotangents = rows_of(g), tangents = rows_of(r);
+  std::array<Tensor, 2> out;
+  if (mask & 1) out[0] = at::empty(v.sizes(), v.options());
+  if (mask & 2) out[1] = at::empty(g.sizes(), g.options());
+  check(api.sh_dbl_bwd(&h.desc, flat.data_ptr(), cotangents.data_ptr(), tangents.data_ptr(), pointer(out[0]),
+                       pointer(out[1]), flat.size(0), stream_of(v)));
+  return out;
+}
+
+struct ShDouble : Function<ShDouble> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& v, const Tensor& g, const Tensor& r,
+                               const HarmonicsPtr& h) {
+    ctx->set_materialize_grads(false);
+    return only(sh_double(*h, v, g, r, 3), 3);
+  }
+  static variable_list backward(AutogradContext*, const variable_list& grads) {
+    TORCH_CHECK_NOT_IMPLEMENTED(!grads[0].defined() && !grads[1].defined(),
+                                "third-order derivatives of the spherical harmonics are not provided");
+    return variable_list(4);
+  }
+};
+
+struct ShBackward : Function<ShBackward> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& v, const Tensor& g, const HarmonicsPtr& h) {
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({v, g});
+    keep(ctx, "op", h);
+    return sh_backward(*h, v, g);
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    const auto saved = ctx->get_saved_variables();
+    const auto h = kept<Harmonics>(ctx, "op");
+    const int mask = (ctx->needs_input_grad(0) ? 1 : 0) | (ctx->needs_input_grad(1) ? 2 : 0);
+    if (!mask) return out;
+    if (at::GradMode::is_enabled()) {
+      const auto d = ShDouble::apply(saved[0], saved[1], grads[0], h);
+      if (mask & 1) out[0] = d[0];
+      if (mask & 2) out[1] = d[1];
+    } else {
+      const auto d = sh_double(*h, saved[0], saved[1], grads[0], mask);
+      out[0] = d[0];
+      out[1] = d[1];
+    }
+    return out;
+  }
+};
+
+struct ShForward : Function<ShForward> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& v, const HarmonicsPtr& h) {
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({v});
+    keep(ctx, "op", h);
+    return sh_forward(*h, v);
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    variable_list out(2);
+    const auto h = kept<Harmonics>(ctx, "op");
+    if (!grads[0].defined() || h->constant || !ctx->needs_input_grad(0)) return out;
+    const auto saved = ctx->get_saved_variables();
+    out[0] = at::GradMode::is_enabled() ? ShBackward::apply(saved[0], grads[0], h) : sh_backward(*h, saved[0], grads[0]);
+    return out;
+  }
+};
+
+Tensor harmonics(const HarmonicsPtr& h, const Tensor& v) {
+  pybind11::gil_scoped_release release;
+  return !h->constant && tracked({&v}) ? ShForward::apply(v, h) : sh_forward(*h, v);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(luna_torch, m) {
+  m.def("load", torch::wrap_pybind_function(load));
+  py::class_<Op, OpPtr>(m, "Op").def(py::init<int64_t, int64_t, int64_t, int64_t, int64_t, bool>());
+  py::class_<Graph, GraphPtr>(m, "Graph").def(py::init<std::array<Tensor, 5>, int64_t, int64_t>());
+  py::class_<Harmonics, HarmonicsPtr>(m, "Harmonics")
+      .def(py::init<const std::vector<int64_t>&, bool, int64_t, int64_t, bool>());
+  m.def("conv", torch::wrap_pybind_function(conv));
+  m.def("harmonics", torch::wrap_pybind_function(harmonics));
+}

@@ -126,6 +126,15 @@ class LunaTPGraph:
             self._tables["native"] = view
         return view
 
+    def native_holder(self):
+        """The same for the C++ launch path: it keeps the tables alive for the autograd graphs that need them."""
+        holder = self._tables.get("holder")
+        if holder is None:
+            holder = self._tables["holder"] = _native.binding().Graph(
+                [self.src, self.dst, self.dst_rowptr, self.src_rowptr, self.edge_ids_by_src], self.num_nodes,
+                self.source_rows)
+        return holder
+
     def destination_range(self, begin: int, end: int) -> "tuple[LunaTPGraph, int, int]":
         """The graph of the edges whose destination lies in ``[begin, end)``, and that slice ``[e0, e1)`` of the edge
         list: destinations renumbered from zero, sources as they are.
@@ -148,14 +157,16 @@ class LunaTPGraph:
     def split_rows(self) -> "SplitGraph | None":
         """The virtual-row form of this graph if a node has more than ``ROW_SPLIT_EDGES`` edges on either side, else
         ``None``.  Decided once per graph (one read of the largest degree) and cached."""
-        if "split" not in self._tables:
+        try:
+            return self._tables["split"]
+        except KeyError:
             split = None
             if self.can_split and self.num_edges:
                 longest = int(torch.maximum(self.dst_rowptr.diff().max(), self.src_rowptr.diff().max()))
                 if longest > ROW_SPLIT_EDGES:
                     split = SplitGraph(self, ROW_SPLIT_EDGES)
             self._tables["split"] = split
-        return self._tables["split"]
+            return split
 
     def table_list(self) -> list:
         """The 13 tensors the reference passes to its custom ops (``src/lunatp/uvu_conv/interface.py:186-192``)."""

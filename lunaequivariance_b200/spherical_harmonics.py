@@ -1,9 +1,9 @@
-"""``spherical_harmonics`` function, its configuration object and the recomputing autograd chain.
+"""``spherical_harmonics`` function, its configuration object and its custom ops.
 
 Follows the reference's ``src/o3/spherical_harmonics/interface.py``: ``parse_irreps`` (:27-55) for the accepted
 forms of ``irreps_out`` / degree lists and their errors, ``SphericalHarmonicsConfig`` (:256-279), the eager chain
 forward -> backward -> double-backward (:282-377, nothing but the inputs is saved; derivatives are recomputed from
-``x``) and the custom ops ``lunaeq::spherical_harmonics_{forward,backward,double_backward}`` (:75-126).
+``x``; here in ``csrc/torch_binding.cpp``) and the custom ops ``lunaeq::spherical_harmonics_{forward,backward,double_backward}`` (:75-126).
 CUDA float32/float64 inputs only: there is no CPU path in this library.
 """
 
@@ -16,6 +16,7 @@ from functools import lru_cache
 import torch
 
 from . import _native
+from .conv import is_compiling
 from .irreps import Irrep, Irreps, as_irreps
 
 UNSET = object()
@@ -62,6 +63,7 @@ class SphericalHarmonicsConfig:
                          out_dim=self.irreps_out.dim)
         self.last_execution_backend = "uninitialized"
         self.backward_backend = None
+        self._holders = {}
         # encoded now: a traced program carries it as a string constant and must not run the encoder
         self._descriptor = json.dumps([list(self._ls_list), self.normalize, self.normalization, self.index_bits,
                                        str(self.compute_dtype).removeprefix("torch.")])
@@ -84,6 +86,19 @@ class SphericalHarmonicsConfig:
         desc.normalize = int(self.normalize)
         desc.normalization = _NORMALIZATIONS[self.normalization]
         return desc
+
+
+    def holder(self, dtype):
+        """This evaluation for the C++ launch path."""
+        holder = self._holders.get(dtype)
+        if holder is None:
+            holder = self._holders[dtype] = _native.binding().Harmonics(
+                list(self._ls_list), self.normalize, _NORMALIZATIONS[self.normalization], self.out_dim,
+                dtype == torch.float64)
+        return holder
+
+    def __getstate__(self):
+        return dict(self.__dict__, _holders={})
 
 
 @lru_cache(maxsize=128)
@@ -138,58 +153,6 @@ def run_double_backward(op: SphericalHarmonicsConfig, x, g, rx, needs=(True, Tru
             ctypes.byref(desc), flat.data_ptr(), gflat.data_ptr(), rflat.data_ptr(), _native.pointer(sx),
             _native.pointer(sg), flat.shape[0], _native.current_stream(x.device)))
     return (None if sx is None else sx.reshape(x.shape), None if sg is None else sg.reshape(g.shape))
-
-
-class SphericalHarmonicsFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, op, x):
-        ctx.op = op
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(x)
-        return run_forward(op, x)
-
-    @staticmethod
-    def backward(ctx, g):
-        if g is None or ctx.op._lmax == 0:
-            return None, None
-        (x,) = ctx.saved_tensors
-        if torch.is_grad_enabled():
-            return None, SphericalHarmonicsBackward.apply(ctx.op, x, g)
-        return None, run_backward(ctx.op, x, g.contiguous())
-
-
-class SphericalHarmonicsBackward(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, op, x, g):
-        ctx.op = op
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(x, g)
-        return run_backward(op, x, g.contiguous())
-
-    @staticmethod
-    def backward(ctx, rx):
-        if rx is None:
-            return None, None, None
-        x, g = ctx.saved_tensors
-        needs = ctx.needs_input_grad[1:3]
-        if torch.is_grad_enabled():
-            sx, sg = SphericalHarmonicsDoubleBackward.apply(ctx.op, x, g, rx)
-        else:
-            sx, sg = run_double_backward(ctx.op, x, g, rx.contiguous(), needs=needs)
-        return None, sx if needs[0] else None, sg if needs[1] else None
-
-
-class SphericalHarmonicsDoubleBackward(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, op, x, g, rx):
-        ctx.set_materialize_grads(False)
-        return run_double_backward(op, x, g, rx.contiguous(), needs=(True, True))
-
-    @staticmethod
-    def backward(ctx, bx, bg):
-        if bx is None and bg is None:
-            return None, None, None, None
-        raise NotImplementedError("third-order derivatives of the spherical harmonics are not provided")
 
 
 # ----------------------------------------------------------------------------------------------- custom ops
@@ -269,14 +232,12 @@ def spherical_harmonics(l, x, normalize, normalization="integral", *, config=Non
     if x.ndim == 0 or x.shape[-1] < 3:
         raise ValueError("SphericalHarmonics input must have shape (...,3)")
     _check(x)
-    from .conv import is_compiling
-
     if is_compiling():
         return torch.ops.lunaeq.spherical_harmonics_forward.default(x, config.descriptor())
     config.last_execution_backend = "cuda_fused"
     tracked = torch.is_grad_enabled() and x.requires_grad and config._lmax > 0
     config.backward_backend = "cuda_fused_recompute" if tracked else None
-    return SphericalHarmonicsFunction.apply(config, x) if tracked else run_forward(config, x)
+    return _native.binding().harmonics(config.holder(x.dtype), x)
 
 
 # The composite op a traced or exported program can carry instead of the Python call; it decomposes into the ops
