@@ -196,6 +196,19 @@ typedef struct {
   int32_t* node_order;        /* [num_nodes] in-degree descending, stable */
   int32_t* source_node_order; /* [num_src_nodes] out-degree descending, stable */
 } luna_graph_out;
+/* The further tables of luna_graph_build_all: the identity permutation, the node_order positions at which one, two and
+ * three quarters of the edges are reached, and the source rows cut into pieces of at most 32 edges (at least one per row;
+ * begin and end count positions of edge_ids_by_src; the order is by length, then by row length, descending, then by
+ * number).  segment_nodes, _begin, _end, _order: room for num_src_nodes + num_edges / 32 entries. */
+typedef struct {
+  int32_t* edge_ids_by_dst; /* [E] */
+  int32_t* node_tiers;      /* [3] */
+  int32_t* segment_nodes;
+  int32_t* segment_begin;
+  int32_t* segment_end;
+  int32_t* segment_rowptr; /* [num_src_nodes+1] */
+  int32_t* segment_order;
+} luna_graph_pieces;
 LUNA_API int64_t luna_graph_scratch_bytes(int64_t num_nodes, int64_t num_edges);
 LUNA_API int luna_graph_bounds(const void* src, const void* dst, int index_bits, int64_t num_edges, int64_t* min_index,
                       int64_t* max_src, int64_t* max_dst, int* unsorted, void* scratch, int64_t scratch_bytes,
@@ -203,6 +216,12 @@ LUNA_API int luna_graph_bounds(const void* src, const void* dst, int index_bits,
 LUNA_API int luna_graph_build(const void* src, const void* dst, int index_bits, int64_t num_nodes, int64_t num_src_nodes,
                      int64_t num_edges, const luna_graph_out* out, void* scratch, int64_t scratch_bytes,
                      void* stream);
+/* All tables in one go, for a graph with nodes and edges, and one synchronisation at the end.  Checks the indices on the
+ * way: *bad is 1, and the tables are not to be used, if one is out of range or dst is not ascending. */
+LUNA_API int luna_graph_build_all(const void* src, const void* dst, int index_bits, int64_t num_nodes,
+                         int64_t num_src_nodes, int64_t num_edges, const luna_graph_out* out,
+                         const luna_graph_pieces* pieces, int* bad, int64_t* num_segments, void* scratch,
+                         int64_t scratch_bytes, void* stream);
 
 /* --------------------------------------------------------------------------------------------------------------
  * Real spherical harmonics (e3nn convention), degrees <= 12.  v[n,3] -> out[n, sum(2l+1)] for the listed

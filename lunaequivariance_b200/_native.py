@@ -71,6 +71,12 @@ class GraphOut(ctypes.Structure):
         "src", "dst", "dst_rowptr", "src_rowptr", "edge_ids_by_src", "node_order", "source_node_order")]
 
 
+class GraphPieces(ctypes.Structure):
+    _fields_ = [(name, ctypes.c_void_p) for name in (
+        "edge_ids_by_dst", "node_tiers", "segment_nodes", "segment_begin", "segment_end", "segment_rowptr",
+        "segment_order")]
+
+
 class ShDesc(ctypes.Structure):
     _fields_ = [
         ("dtype", ctypes.c_int32), ("num_degrees", ctypes.c_int32), ("degrees", ctypes.c_int32 * 32),
@@ -106,6 +112,10 @@ _SIGNATURES = {
                                          ctypes.POINTER(ctypes.c_int), _P, ctypes.c_int64, _P]),
     "luna_graph_build": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64,
                                         ctypes.POINTER(GraphOut), _P, ctypes.c_int64, _P]),
+    "luna_graph_build_all": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64,
+                                            ctypes.POINTER(GraphOut), ctypes.POINTER(GraphPieces),
+                                            ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int64), _P,
+                                            ctypes.c_int64, _P]),
     "luna_probe_fma": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _P, ctypes.POINTER(ctypes.c_double), _P]),
     "luna_sh_fwd": (ctypes.c_int, [ctypes.POINTER(ShDesc), _P, _P, ctypes.c_int64, _P]),
     "luna_sh_bwd": (ctypes.c_int, [ctypes.POINTER(ShDesc), _P, _P, _P, ctypes.c_int64, _P]),
@@ -187,4 +197,4 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 __all__ = ["library", "binding", "check", "last_error", "pointer", "current_stream", "dtype_code", "UvuPath", "UvuDesc",
-           "Graph", "GraphOut", "ShDesc", "EXPORTED_SYMBOLS", "LIBRARY_PATH"]
+           "Graph", "GraphOut", "GraphPieces", "ShDesc", "EXPORTED_SYMBOLS", "LIBRARY_PATH"]

@@ -38,6 +38,8 @@ struct Api {
   decltype(&luna_uvu_conv_fwd) fwd = nullptr;
   decltype(&luna_uvu_conv_bwd) bwd = nullptr;
   decltype(&luna_uvu_conv_dbl_bwd) dbl_bwd = nullptr;
+  decltype(&luna_graph_scratch_bytes) graph_scratch_bytes = nullptr;
+  decltype(&luna_graph_build_all) graph_build_all = nullptr;
   decltype(&luna_sh_fwd) sh_fwd = nullptr;
   decltype(&luna_sh_bwd) sh_bwd = nullptr;
   decltype(&luna_sh_dbl_bwd) sh_dbl_bwd = nullptr;
@@ -59,6 +61,8 @@ void load(const std::string& path) {
   resolve(library, "luna_uvu_conv_fwd", api.fwd);
   resolve(library, "luna_uvu_conv_bwd", api.bwd);
   resolve(library, "luna_uvu_conv_dbl_bwd", api.dbl_bwd);
+  resolve(library, "luna_graph_scratch_bytes", api.graph_scratch_bytes);
+  resolve(library, "luna_graph_build_all", api.graph_build_all);
   resolve(library, "luna_sh_fwd", api.sh_fwd);
   resolve(library, "luna_sh_bwd", api.sh_bwd);
   resolve(library, "luna_sh_dbl_bwd", api.sh_dbl_bwd);
@@ -397,6 +401,38 @@ Tensor conv(const OpPtr& op, const GraphPtr& graph, const Tensor& x, const Tenso
   return tracked({&x, &y, &w}) ? ConvForward::apply(x, y, w, op, graph) : run_forward(*op, *graph, x, y, w);
 }
 
+// ---- graph tables ---------------------------------------------------------------------------------------------------------
+// Every table of a graph with nodes and edges: src, dst, dst_rowptr, src_rowptr, edge_ids_by_src, edge_ids_by_dst,
+// node_order, source_node_order, node_tiers and the five of the segments; nothing if an index is out of range or dst is
+// not ascending.  src, dst: contiguous, int32 or int64, on one CUDA device, of one length.
+std::vector<Tensor> graph_tables(const Tensor& src, const Tensor& dst, int64_t nodes, int64_t source_rows) {
+  pybind11::gil_scoped_release release;
+  const c10::cuda::CUDAGuard guard(src.device());
+  const int64_t edges = src.numel();
+  const auto options = src.options().dtype(at::kInt);
+  auto table = [&](int64_t entries) { return at::empty({entries}, options); };
+  const int64_t room = source_rows + edges / 32;  // a segment per row at least, and one per 32 edges at most beyond that
+  Tensor by_src = table(edges), by_dst = table(edges), src_out = table(edges), dst_out = table(edges);
+  Tensor dst_rowptr = table(nodes + 1), src_rowptr = table(source_rows + 1), order = table(nodes);
+  Tensor source_order = table(source_rows), tiers = table(3), seg_rowptr = table(source_rows + 1);
+  Tensor seg_nodes = table(room), seg_begin = table(room), seg_end = table(room), seg_order = table(room);
+  const int64_t bytes = api.graph_scratch_bytes(std::max(nodes, source_rows), edges);
+  const Tensor scratch = at::empty({bytes}, options.dtype(at::kByte));
+  auto ints = [](const Tensor& t) { return t.data_ptr<int32_t>(); };
+  const luna_graph_out out{ints(src_out), ints(dst_out), ints(dst_rowptr), ints(src_rowptr),
+                           ints(by_src),  ints(order),   ints(source_order)};
+  const luna_graph_pieces pieces{ints(by_dst),  ints(tiers),      ints(seg_nodes), ints(seg_begin),
+                                 ints(seg_end), ints(seg_rowptr), ints(seg_order)};
+  int bad = 0;
+  int64_t segments = 0;
+  check(api.graph_build_all(src.data_ptr(), dst.data_ptr(), src.scalar_type() == at::kLong ? 64 : 32, nodes, source_rows,
+                            edges, &out, &pieces, &bad, &segments, scratch.data_ptr(), bytes, stream_of(src)));
+  if (bad) return {};
+  auto cut = [&](const Tensor& t) { return t.narrow(0, 0, segments); };
+  return {src_out, dst_out, dst_rowptr, src_rowptr, by_src, by_dst, order, source_order, tiers,
+          cut(seg_nodes), cut(seg_begin), cut(seg_end), seg_rowptr, cut(seg_order)};
+}
+
 // ---- spherical harmonics --------------------------------------------------------------------------------------------------
 struct Harmonics : torch::CustomClassHolder {
   luna_sh_desc desc{};
@@ -528,6 +564,7 @@ PYBIND11_MODULE(luna_torch, m) {
   py::class_<Graph, GraphPtr>(m, "Graph").def(py::init<std::array<Tensor, 5>, int64_t, int64_t>());
   py::class_<Harmonics, HarmonicsPtr>(m, "Harmonics")
       .def(py::init<const std::vector<int64_t>&, bool, int64_t, int64_t, bool>());
+  m.def("graph_tables", torch::wrap_pybind_function(graph_tables));
   m.def("conv", torch::wrap_pybind_function(conv));
   m.def("harmonics", torch::wrap_pybind_function(harmonics));
 }

@@ -3,7 +3,7 @@
 Public behaviour follows the reference's ``make_graph`` and ``LunaTPGraph`` (``src/lunatp/graph.py:17-141``) and
 ``make_source_segments`` (``src/lunatp/uvu_conv/graph.py:38-99``): same field names, same validation messages,
 inputs are copied into owned int32 tensors, ``dst`` must be ascending.  On CUDA tensors the tables are built by
-the library's ``luna_graph_build`` (radix sorts and scans on the caller's stream); CPU tensors use torch ops so
+the library's ``luna_graph_build_all`` (radix sorts and a scan on the caller's stream); CPU tensors use torch ops so
 that graphs can be prepared and inspected without a GPU.
 """
 
@@ -21,6 +21,7 @@ SOURCE_SEGMENT_EDGES = 32
 # A warp walks a node's edges one after the other, so a node with very many edges would hold one warp for the whole
 # launch.  Rows longer than this are cut into virtual rows of at most this many edges (LunaTPGraph.split_rows).
 ROW_SPLIT_EDGES = 1024
+_TABLE_LIMIT = (1 << 31) - 1024  # entries of a table with 32-bit indices
 
 
 @dataclass(frozen=True)
@@ -249,6 +250,19 @@ def make_graph(src: torch.Tensor, dst: torch.Tensor, num_nodes: int | None = Non
 
     num_edges = src.numel()
     device = src.device
+    # The usual call, sizes known and edges there: every table in one go, the indices checked on the way.  What does not
+    # pass goes through the bounds scan, which knows what to say about it.
+    source_rows = num_nodes if num_src_nodes is None else int(num_src_nodes)
+    if (device.type == "cuda" and num_edges and num_nodes is not None and 0 < num_nodes < _TABLE_LIMIT
+            and 0 < source_rows and source_rows + num_edges // SOURCE_SEGMENT_EDGES < _TABLE_LIMIT
+            and num_edges < _TABLE_LIMIT and num_nodes + num_edges // SOURCE_SEGMENT_EDGES < _TABLE_LIMIT):
+        tables = _native.binding().graph_tables(src, dst, num_nodes, source_rows)
+        if tables:
+            return LunaTPGraph(
+                src=tables[0], dst=tables[1], num_nodes=num_nodes, dst_rowptr=tables[2], src_rowptr=tables[3],
+                edge_ids_by_src=tables[4], edge_ids_by_dst=tables[5], node_order=tables[6],
+                source_node_order=tables[7], node_tiers=tables[8], source_segments=SourceSegmentTables(*tables[9:]),
+                num_src_nodes=None if num_src_nodes is None else source_rows, can_split=split)
     required = 0
     if num_edges:
         with torch.cuda.device(device) if device.type == "cuda" else _NullContext():

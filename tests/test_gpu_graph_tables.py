@@ -1,0 +1,52 @@
+"""Every table of a graph built on the GPU against the same tables from torch ops on the CPU: exactly."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+import lunaequivariance_b200 as luna
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("src", "dst", "dst_rowptr", "src_rowptr", "edge_ids_by_src", "edge_ids_by_dst", "node_order", "source_node_order",
+         "node_tiers")
+SEGMENTS = ("nodes", "begin", "end", "rowptr", "order")
+
+
+def _edges(nodes, source_rows, edges, hub, seed):
+    generator = torch.Generator().manual_seed(seed)
+    src = torch.randint(source_rows, (edges,), generator=generator)
+    if hub:  # most edges leave one node, in a number that is a multiple of a segment's length
+        src[: edges // 2 // 32 * 32] = source_rows // 2
+        src = src[torch.randperm(edges, generator=generator)]
+    return src, torch.sort(torch.randint(nodes, (edges,), generator=generator)).values
+
+
+# one edge; fewer edges than quarters; rows of exactly 31, 32, 33 rows per warp; rows without edges; more source rows than
+# destinations and fewer
+@pytest.mark.parametrize("nodes,source_rows,edges,hub", [
+    (1, 1, 1, False), (3, 3, 2, False), (30, 30, 3, False), (31, 31, 992, False), (32, 32, 1024, True),
+    (62, 62, 4_000, True), (500, 500, 300, False), (64, 900, 5_001, False), (900, 7, 5_001, True), (20_011, 20_011, 200_003, True),
+])
+@pytest.mark.parametrize("index_dtype", [torch.int32, torch.int64])
+def test_tables(nodes, source_rows, edges, hub, index_dtype):
+    src, dst = (t.to(index_dtype) for t in _edges(nodes, source_rows, edges, hub, nodes + edges))
+    other = None if source_rows == nodes else source_rows
+    want = luna.make_graph(src, dst, nodes, num_src_nodes=other)
+    got = luna.make_graph(src.cuda(), dst.cuda(), nodes, num_src_nodes=other)
+    for name in NAMES:
+        torch.testing.assert_close(getattr(got, name).cpu(), getattr(want, name), rtol=0, atol=0, msg=name)
+    for name in SEGMENTS:
+        torch.testing.assert_close(getattr(got.source_segments, name).cpu(), getattr(want.source_segments, name), rtol=0,
+                                   atol=0, msg=f"segment {name}")
+    assert got.num_src_nodes == want.num_src_nodes and got.can_split == want.can_split
+
+
+@pytest.mark.parametrize("src,dst,match", [
+    ([0, 4], [0, 1], "at least 5"), ([0, 1], [0, 4], "at least 5"), ([0, -1], [0, 1], "nonnegative"),
+    ([0, 1], [1, 0], "sorted"), ([0, 1 << 32], [0, 1], "at least 4294967297"),
+])
+def test_unfit_edge_lists_are_refused(src, dst, match):
+    with pytest.raises(ValueError, match=match):
+        luna.make_graph(torch.tensor(src, device="cuda"), torch.tensor(dst, device="cuda"), 4)
