@@ -91,7 +91,9 @@ def build_binding(nvcc: str, newest_header: float, force: bool) -> None:
     cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                cuda_include, "/usr/local/cuda/include", sysconfig.get_paths()["include"]]
-    command = [os.environ.get("CXX") or shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared",
+    # The compiler that nvcc uses for its host code, and not CXX: a compiler that links the C++ runtime statically gives
+    # the module a second copy of it beside torch's, and streams (error texts with sizes in them) then crash.
+    command = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared",
                "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=luna_torch",
                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{path}" for path in include),
                source, "-o", BINDING, f"-L{os.path.join(root, 'lib')}", "-ltorch", "-ltorch_cpu", "-ltorch_python",

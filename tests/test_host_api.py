@@ -154,3 +154,12 @@ def test_canonical_path_lists_are_detected_without_gpu():
     in1, in2, out, instructions, options = config("fixture")
     shuffled = luna.prepare_tensor_product(in1, in2, out, instructions[::-1], convolution=True)
     assert shuffled.uses_staged_kernels and shuffled.canonical_l2 == -1
+
+
+def test_launch_path_shares_the_cpp_runtime():
+    """A second, static copy of the C++ runtime beside torch's makes error texts crash."""
+    from lunaequivariance_b200 import _native
+
+    _native.binding()
+    with open(_native.BINDING_PATH, "rb") as module:
+        assert b"libstdc++.so" in module.read()
