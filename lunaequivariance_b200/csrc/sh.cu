@@ -386,11 +386,47 @@ sh_kernel(const ShParams P, const T* __restrict__ v, const T* __restrict__ g, co
   }
 }
 
+// A warp's tile of 32 rows of C values in shared memory.  Rows are moved in 16-byte pieces on both sides.  With C odd the
+// tile is the memory's own image, and scalar accesses to a column, one row per lane, meet no bank conflict.  With C even
+// (4, 16, 36: multiples of a piece) a row takes an odd number of pieces, and lanes access their rows by whole pieces, eight
+// lanes in eight different groups of banks.  Both kernels are bound by HBM.  At lmax 6, 4 M vectors, FP32 (832 MB each): 139
+// us forward and 136 us backward, 0.92 and 0.94 of a copy's bandwidth; values and gradient together 299 us as a user
+// calls them, against 344 with value-by-value copies and loads that wait for the arithmetic.
+template <typename T, int C>
+struct RowTile {
+  static constexpr int per = 16 / static_cast<int>(sizeof(T));  // values in a piece
+  static constexpr bool image = C % 2 == 1;
+  static constexpr int pitch = image ? C : ((C / per) | 1) * per;
+  static constexpr int pieces = 32 * C / per;
+  // where piece q of the tile's memory lies in shared memory
+  static __device__ __forceinline__ int piece(int q) {
+    if constexpr (image) {
+      return q * per;
+    } else {
+      return (q / (C / per)) * pitch + (q % (C / per)) * per;
+    }
+  }
+  static __device__ __forceinline__ int value(int q) { return image ? q : (q / C) * pitch + q % C; }
+};
+template <typename T>
+struct alignas(16) Piece {
+  T a[16 / sizeof(T)];
+};
+__device__ __forceinline__ void copy_piece_async(void* to, const void* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(to))), "l"(from)
+               : "memory");
+}
+__device__ __forceinline__ void commit_pieces() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void wait_pieces() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
 // Sinks of the unrolled kernels: the degree list is 0..LMAX, so degree l starts at column l * l.
 template <typename T>
 struct CanonForwardSink {
   int normalization;
-  T* row;
+  T* row;  // in shared memory, or in registers
   template <int L>
   __device__ __forceinline__ void emit(std::integral_constant<int, L>, const T* level) {
     const T scale = degree_scale<T>(L, normalization);
@@ -460,11 +496,23 @@ __device__ __forceinline__ void canon_backward(const ShParams& P, T vx, T vy, T 
     });
   });
   // seeds: the cotangent of every output component, with the degree's normalisation factor
+  if constexpr (RowTile<T, C>::image) {
+#pragma unroll
+    for (int m = 0; m < C; ++m) adj[m] = grow[m];
+  } else {
+    constexpr int per = RowTile<T, C>::per;
+#pragma unroll
+    for (int q = 0; q < C / per; ++q) {
+      const Piece<T> piece = reinterpret_cast<const Piece<T>*>(grow)[q];
+#pragma unroll
+      for (int c = 0; c < per; ++c) adj[q * per + c] = piece.a[c];
+    }
+  }
   unroll<0, LMAX + 1>([&](auto lc) {
     constexpr int l = decltype(lc)::value;
     const T scale = degree_scale<T>(l, P.normalization);
 #pragma unroll
-    for (int m = 0; m < 2 * l + 1; ++m) adj[l * l + m] = scale * grow[l * l + m];
+    for (int m = 0; m < 2 * l + 1; ++m) adj[l * l + m] *= scale;
   });
   T ax = T(0), ay = T(0), az = T(0), ar2 = T(0);
   unroll<0, LMAX - 1>([&](auto dc) {
@@ -506,10 +554,131 @@ __device__ __forceinline__ void canon_backward(const ShParams& P, T vx, T vy, T 
   }
 }
 
-// Same three modes as sh_kernel for the degree list 0..LMAX, everything about the list known at compile time.
-template <typename T, int MODE, int LMAX>
+template <typename T>
+__device__ __forceinline__ void load_vector(const T* __restrict__ v, int64_t item, int64_t n, T& x, T& y, T& z) {
+  x = T(0);
+  y = T(1);
+  z = T(0);
+  if (item < n) {
+    x = v[item * 3 + 0];
+    y = v[item * 3 + 1];
+    z = v[item * 3 + 2];
+  }
+}
+
+// The modes of sh_kernel for the degree list 0..LMAX, everything about the list known at compile time.  `aligned`: g and
+// the row output start on 16-byte boundaries, so full tiles move in pieces; other tiles move value by value.
+template <typename T, int LMAX>
 __global__ void __launch_bounds__(kBlock)
-sh_canon_kernel(const ShParams P, const T* __restrict__ v, const T* __restrict__ g, const T* __restrict__ rx,
+sh_canon_forward(const ShParams P, const T* __restrict__ v, T* __restrict__ out, int64_t n, bool aligned) {
+  constexpr int C = (LMAX + 1) * (LMAX + 1);
+  using Tile = RowTile<T, C>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T* tile = reinterpret_cast<T*>(smem_raw) + warp * 32 * Tile::pitch;
+  T* row = tile + lane * Tile::pitch;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kBlock;
+  int64_t base = static_cast<int64_t>(blockIdx.x) * kBlock + warp * 32;
+  T x, y, z, r2;
+  load_vector(v, base + lane, n, x, y, z);
+  for (; base < n; base += step) {
+    T nx, ny, nz;
+    load_vector(v, base + step + lane, n, nx, ny, nz);
+    prepare<T, T>(P, x, y, z, r2);
+    if constexpr (Tile::image) {
+      CanonForwardSink<T> sink{P.normalization, row};
+      walk_unrolled<T, T, LMAX>(T(1), x, y, z, r2, sink);
+    } else {
+      T values[C];
+      CanonForwardSink<T> sink{P.normalization, values};
+      walk_unrolled<T, T, LMAX>(T(1), x, y, z, r2, sink);
+#pragma unroll
+      for (int q = 0; q < C / Tile::per; ++q) {
+        Piece<T> piece;
+#pragma unroll
+        for (int c = 0; c < Tile::per; ++c) piece.a[c] = values[q * Tile::per + c];
+        reinterpret_cast<Piece<T>*>(row)[q] = piece;
+      }
+    }
+    __syncwarp();
+    T* to = out + base * C;
+    if (aligned && n - base >= 32) {
+#pragma unroll
+      for (int j = 0; j < (Tile::pieces + 31) / 32; ++j) {
+        const int q = j * 32 + lane;
+        if (Tile::pieces % 32 == 0 || q < Tile::pieces)
+          reinterpret_cast<Piece<T>*>(to)[q] = *reinterpret_cast<const Piece<T>*>(tile + Tile::piece(q));
+      }
+    } else {
+      const int values = static_cast<int>(n - base < 32 ? n - base : 32) * C;
+      for (int q = lane; q < values; q += 32) to[q] = tile[Tile::value(q)];
+    }
+    __syncwarp();
+    x = nx;
+    y = ny;
+    z = nz;
+  }
+}
+
+// Two tiles per warp: the next rows of g are on their way while the current ones are worked on.
+template <typename T, int LMAX>
+__global__ void __launch_bounds__(kBlock)
+sh_canon_backward(const ShParams P, const T* __restrict__ v, const T* __restrict__ g, T* __restrict__ dv, int64_t n,
+                  bool aligned) {
+  constexpr int C = (LMAX + 1) * (LMAX + 1);
+  using Tile = RowTile<T, C>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T* tiles = reinterpret_cast<T*>(smem_raw) + warp * 2 * 32 * Tile::pitch;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kBlock;
+  int64_t base = static_cast<int64_t>(blockIdx.x) * kBlock + warp * 32;
+  auto in_pieces = [&](int64_t at) { return aligned && n - at >= 32; };
+  auto fetch = [&](int64_t at, T* tile) {
+    if (in_pieces(at)) {
+      const T* from = g + at * C;
+#pragma unroll
+      for (int j = 0; j < (Tile::pieces + 31) / 32; ++j) {
+        const int q = j * 32 + lane;
+        if (Tile::pieces % 32 == 0 || q < Tile::pieces) copy_piece_async(tile + Tile::piece(q), from + q * Tile::per);
+      }
+    }
+    commit_pieces();
+  };
+  int current = 0;
+  T x, y, z;
+  fetch(base, tiles);
+  load_vector(v, base + lane, n, x, y, z);
+  for (; base < n; base += step) {
+    T* tile = tiles + current * 32 * Tile::pitch;
+    current ^= 1;
+    fetch(base + step, tiles + current * 32 * Tile::pitch);
+    T nx, ny, nz;
+    load_vector(v, base + step + lane, n, nx, ny, nz);
+    if (!in_pieces(base)) {
+      const int values = static_cast<int>(n - base < 32 ? n - base : 32) * C;
+      const T* from = g + base * C;
+      for (int q = lane; q < values; q += 32) tile[Tile::value(q)] = from[q];
+    }
+    wait_pieces<1>();
+    __syncwarp();
+    T dvx, dvy, dvz;
+    canon_backward<T, LMAX>(P, x, y, z, tile + lane * Tile::pitch, dvx, dvy, dvz);
+    const int64_t item = base + lane;
+    if (item < n) {
+      dv[item * 3 + 0] = dvx;
+      dv[item * 3 + 1] = dvy;
+      dv[item * 3 + 2] = dvz;
+    }
+    __syncwarp();
+    x = nx;
+    y = ny;
+    z = nz;
+  }
+}
+
+template <typename T, int LMAX>
+__global__ void __launch_bounds__(kBlock)
+sh_canon_double(const ShParams P, const T* __restrict__ v, const T* __restrict__ g, const T* __restrict__ rx,
                 T* __restrict__ out0, T* __restrict__ out1, int64_t n) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* smem = reinterpret_cast<T*>(smem_raw);
@@ -517,102 +686,94 @@ sh_canon_kernel(const ShParams P, const T* __restrict__ v, const T* __restrict__
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T* tile = smem + static_cast<size_t>(warp) * 32 * CP;
   T* row = tile + lane * CP;
-  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * (kBlock / 32);
-  for (int64_t base = (static_cast<int64_t>(blockIdx.x) * (kBlock / 32) + warp) * 32; base < n;
-       base += warps_total * 32) {
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kBlock;
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * kBlock + warp * 32; base < n; base += step) {
     const int rows = (n - base < 32) ? static_cast<int>(n - base) : 32;
     const int64_t item = base + lane;
     const bool active = lane < rows;
-    T vx = T(0), vy = T(1), vz = T(0);
+    T vx, vy, vz, tx = T(0), ty = T(0), tz = T(0);
+    load_vector(v, item, n, vx, vy, vz);
     if (active) {
-      vx = v[item * 3 + 0];
-      vy = v[item * 3 + 1];
-      vz = v[item * 3 + 2];
+      tx = rx[item * 3 + 0];
+      ty = rx[item * 3 + 1];
+      tz = rx[item * 3 + 2];
     }
-    if constexpr (MODE != 0) {
-      const T* gsrc = g + base * C;
-      if (rows == 32) {
-        // a full tile: the loads go out in batches of eight per lane before anything is stored, so that a warp has
-        // 1 KB (FP32) in flight instead of one row of loads waiting on the next
-        constexpr int kBatch = 8;
+    const T* gsrc = g + base * C;
+    if (rows == 32) {
+      // a full tile: the loads go out in batches of eight per lane before anything is stored, so that a warp has
+      // 1 KB (FP32) in flight instead of one row of loads waiting on the next
+      constexpr int kBatch = 8;
 #pragma unroll
-        for (int j0 = 0; j0 < C; j0 += kBatch) {
-          T batch[kBatch];
+      for (int j0 = 0; j0 < C; j0 += kBatch) {
+        T batch[kBatch];
 #pragma unroll
-          for (int j = 0; j < kBatch; ++j)
-            if (j0 + j < C) batch[j] = gsrc[(j0 + j) * 32 + lane];
+        for (int j = 0; j < kBatch; ++j)
+          if (j0 + j < C) batch[j] = gsrc[(j0 + j) * 32 + lane];
 #pragma unroll
-          for (int j = 0; j < kBatch; ++j)
-            if (j0 + j < C) {
-              const int idx = (j0 + j) * 32 + lane;
-              tile[(idx / C) * CP + (idx % C)] = batch[j];
-            }
-        }
-      } else {
-#pragma unroll 4
-        for (int idx = lane; idx < rows * C; idx += 32) tile[(idx / C) * CP + (idx % C)] = gsrc[idx];
-      }
-      __syncwarp();
-    }
-    if constexpr (MODE == 0) {
-      T x = vx, y = vy, z = vz, r2;
-      prepare<T, T>(P, x, y, z, r2);
-      CanonForwardSink<T> sink{P.normalization, row};
-      walk_unrolled<T, T, LMAX>(T(1), x, y, z, r2, sink);
-      __syncwarp();
-      T* dst = out0 + base * C;
-#pragma unroll 4
-      for (int idx = lane; idx < rows * C; idx += 32) dst[idx] = tile[(idx / C) * CP + (idx % C)];
-    } else if constexpr (MODE == 1) {
-      T dvx, dvy, dvz;
-      canon_backward<T, LMAX>(P, vx, vy, vz, row, dvx, dvy, dvz);
-      if (active) {
-        out0[item * 3 + 0] = dvx;
-        out0[item * 3 + 1] = dvy;
-        out0[item * 3 + 2] = dvz;
+        for (int j = 0; j < kBatch; ++j)
+          if (j0 + j < C) {
+            const int idx = (j0 + j) * 32 + lane;
+            tile[(idx / C) * CP + (idx % C)] = batch[j];
+          }
       }
     } else {
-      using N = Du<G3<T>>;
-      T tx = T(0), ty = T(0), tz = T(0);
-      if (active) {
-        tx = rx[item * 3 + 0];
-        ty = rx[item * 3 + 1];
-        tz = rx[item * 3 + 2];
-      }
-      const G3<T> zero{T(0), T(0), T(0), T(0)};
-      N x{{vx, T(1), T(0), T(0)}, {tx, T(0), T(0), T(0)}};
-      N y{{vy, T(0), T(1), T(0)}, {ty, T(0), T(0), T(0)}};
-      N z{{vz, T(0), T(0), T(1)}, {tz, T(0), T(0), T(0)}};
-      N r2;
-      prepare<T, N>(P, x, y, z, r2);
-      CanonDoubleSink<T> sink{P.normalization, row, out1 != nullptr};
-      walk_unrolled<T, N, LMAX>(N{{T(1), T(0), T(0), T(0)}, zero}, x, y, z, r2, sink);
-      if (active && out0 != nullptr) {
-        out0[item * 3 + 0] = sink.sx;
-        out0[item * 3 + 1] = sink.sy;
-        out0[item * 3 + 2] = sink.sz;
-      }
-      if (out1 != nullptr) {
-        __syncwarp();
-        T* dst = out1 + base * C;
 #pragma unroll 4
-        for (int idx = lane; idx < rows * C; idx += 32) dst[idx] = tile[(idx / C) * CP + (idx % C)];
-      }
+      for (int idx = lane; idx < rows * C; idx += 32) tile[(idx / C) * CP + (idx % C)] = gsrc[idx];
+    }
+    __syncwarp();
+    using N = Du<G3<T>>;
+    const G3<T> zero{T(0), T(0), T(0), T(0)};
+    N x{{vx, T(1), T(0), T(0)}, {tx, T(0), T(0), T(0)}};
+    N y{{vy, T(0), T(1), T(0)}, {ty, T(0), T(0), T(0)}};
+    N z{{vz, T(0), T(0), T(1)}, {tz, T(0), T(0), T(0)}};
+    N r2;
+    prepare<T, N>(P, x, y, z, r2);
+    CanonDoubleSink<T> sink{P.normalization, row, out1 != nullptr};
+    walk_unrolled<T, N, LMAX>(N{{T(1), T(0), T(0), T(0)}, zero}, x, y, z, r2, sink);
+    if (active && out0 != nullptr) {
+      out0[item * 3 + 0] = sink.sx;
+      out0[item * 3 + 1] = sink.sy;
+      out0[item * 3 + 2] = sink.sz;
+    }
+    if (out1 != nullptr) {
+      __syncwarp();
+      T* dst = out1 + base * C;
+#pragma unroll 4
+      for (int idx = lane; idx < rows * C; idx += 32) dst[idx] = tile[(idx / C) * CP + (idx % C)];
     }
     __syncwarp();
   }
+}
+
+template <typename K>
+int allow_smem(K kernel, size_t bytes) {
+  if (bytes > 48 * 1024)
+    LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+  return LUNA_OK;
 }
 
 template <typename T, int MODE, int LMAX>
 int launch_canon(const ShParams& P, const T* v, const T* g, const T* rx, T* out0, T* out1, int64_t n,
                  cudaStream_t stream) {
   constexpr int C = (LMAX + 1) * (LMAX + 1);
-  const size_t smem = static_cast<size_t>(kBlock / 32) * 32 * (C | 1) * sizeof(T);
-  auto kernel = sh_canon_kernel<T, MODE, LMAX>;
-  if (smem > 48 * 1024)
-    LUNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  const int64_t blocks = std::min<int64_t>(ceil_div(n, kBlock), 148 * 16);
-  kernel<<<static_cast<unsigned>(blocks), kBlock, smem, stream>>>(P, v, g, rx, out0, out1, n);
+  const bool aligned = reinterpret_cast<uintptr_t>(MODE == 0 ? static_cast<const void*>(out0) : static_cast<const void*>(g)) % 16 == 0;
+  const size_t smem = static_cast<size_t>(kBlock) * sizeof(T) *
+                      (MODE == 0 ? RowTile<T, C>::pitch : (MODE == 1 ? 2 * RowTile<T, C>::pitch : (C | 1)));
+  // the backward kernel reads ahead: no more blocks than are resident together
+  const int64_t resident = MODE == 1 ? std::min<int64_t>(16, 220 * 1024 / static_cast<int64_t>(smem + 1024)) : 16;
+  const unsigned blocks = static_cast<unsigned>(std::min<int64_t>(ceil_div(n, kBlock), 148 * resident));
+  int rc = LUNA_OK;
+  if constexpr (MODE == 0) {
+    rc = allow_smem(sh_canon_forward<T, LMAX>, smem);
+    if (rc == LUNA_OK) sh_canon_forward<T, LMAX><<<blocks, kBlock, smem, stream>>>(P, v, out0, n, aligned);
+  } else if constexpr (MODE == 1) {
+    rc = allow_smem(sh_canon_backward<T, LMAX>, smem);
+    if (rc == LUNA_OK) sh_canon_backward<T, LMAX><<<blocks, kBlock, smem, stream>>>(P, v, g, out0, n, aligned);
+  } else {
+    rc = allow_smem(sh_canon_double<T, LMAX>, smem);
+    if (rc == LUNA_OK) sh_canon_double<T, LMAX><<<blocks, kBlock, smem, stream>>>(P, v, g, rx, out0, out1, n);
+  }
+  if (rc != LUNA_OK) return rc;
   LUNA_LAUNCH_CHECK("spherical harmonics (degrees 0..lmax)");
   return LUNA_OK;
 }

@@ -100,3 +100,25 @@ def test_graph_errors_on_device():
         luna.make_graph(t([0, 0]), t([1, 0]), 2)
     graph = luna.make_graph(t([2, 0, 1]), t([0, 1, 2]))
     assert graph.num_nodes == 3 and graph.dst_rowptr.tolist() == [0, 1, 2, 3]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("lmax", [1, 2, 3, 6])
+@pytest.mark.parametrize("items,offset", [(1, 0), (31, 0), (32, 0), (33, 0), (300_001, 0), (1_001, 1)])
+def test_sh_rows_do_not_depend_on_their_tile(lmax, items, offset, dtype):
+    """Full and partial tiles, several tiles per warp, cotangents off a 16-byte boundary: every row comes out as it does
+    from a call of 77 rows at most, whose size the oracle tests above cover; bit for bit, as the arithmetic is the same."""
+    generator = torch.Generator(device=DEVICE).manual_seed(items + lmax)
+    v = torch.randn(items, 3, generator=generator, device=DEVICE, dtype=dtype).requires_grad_(True)
+    C = (lmax + 1) ** 2
+    g = torch.randn(items * C + offset, generator=generator, device=DEVICE, dtype=dtype)[offset:].view(items, C)
+    module = luna.o3.SphericalHarmonics(luna.Irreps.spherical_harmonics(lmax), normalize=True, normalization="component",
+                                        dtype=dtype)
+    out = module(v)
+    (dv,) = torch.autograd.grad(out, v, g)
+    begin = max(0, items - 77)
+    for lo, hi in ((0, min(items, 77)), (begin, items), (items // 2, min(items, items // 2 + 77))):
+        part = v.detach()[lo:hi].clone().requires_grad_(True)
+        values = module(part)
+        (grad,) = torch.autograd.grad(values, part, g[lo:hi].clone())
+        assert torch.equal(values, out[lo:hi]) and torch.equal(grad, dv[lo:hi])
