@@ -418,8 +418,12 @@ int get_device_tables(luna_uvu_plan* plan, const DeviceTables** out) {
     return append(raw.data(), raw.size());
   };
   const EdgePlan& edge = plan->edge;
-  const size_t o_epc = append_scalars(edge.prog_c), o_etc = append_scalars(edge.term_c);
-  const size_t o_epj = append(edge.prog_j.data(), edge.prog_j.size() * sizeof(unsigned short));
+  size_t o_epc[2], o_etc[2], o_epj[2];
+  for (int t = 0; t < 2; ++t) {
+    o_epc[t] = append_scalars(edge.prog_c[t]);
+    o_etc[t] = append_scalars(edge.term_c[t]);
+    o_epj[t] = append(edge.prog_j[t].data(), edge.prog_j[t].size() * sizeof(unsigned short));
+  }
 
   DeviceTables dt;
   dt.bytes = host.size();
@@ -449,9 +453,8 @@ int get_device_tables(luna_uvu_plan* plan, const DeviceTables** out) {
   dt.ell_j = base + o_mj;
   dt.ell_c = base + o_mc;
   dt.bwd_tables = base + o_blob;
-  dt.edge_prog_c = base + o_epc;
-  dt.edge_term_c = base + o_etc;
-  dt.edge_prog_j = reinterpret_cast<const unsigned short*>(base + o_epj);
+  for (int t = 0; t < 2; ++t)
+    dt.edge[t] = EdgeTables{base + o_epc[t], base + o_etc[t], reinterpret_cast<const unsigned short*>(base + o_epj[t])};
   LUNA_CUDA_CHECK(cudaDeviceGetAttribute(&dt.sm_count, cudaDevAttrMultiProcessorCount, device));
   LUNA_CUDA_CHECK(cudaDeviceGetAttribute(&dt.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   auto inserted = plan->device_tables.emplace(device, dt);

@@ -121,6 +121,11 @@ Tuning tuning_from_environment();
 
 constexpr int kTileCounterSets = 32;    // launches of one plan that may be in flight on a device at a time
 constexpr int kTileCounterWords = 64;   // per set: (next tile, warps finished) for up to 32 channel chunks
+// What an edge kernel reads of a plan: see EdgeBwdParams.
+struct EdgeTables {
+  const void *prog_c = nullptr, *term_c = nullptr;
+  const unsigned short* prog_j = nullptr;
+};
 
 struct DeviceTables {
   void* buffer = nullptr;  // one allocation holding every table
@@ -144,9 +149,7 @@ struct DeviceTables {
   // padded program; offsets in FastMeta::tb_*
   const unsigned char* bwd_tables = nullptr;
   // edge kernels (EdgePlan): the coupling-matrix program and the term list
-  const void* edge_prog_c = nullptr;
-  const unsigned short* edge_prog_j = nullptr;
-  const void* edge_term_c = nullptr;
+  EdgeTables edge[2];  // of the plan's shape, and of the shape with x and out exchanged
   int sm_count = 0;
   int max_smem_optin = 0;
 };
@@ -157,8 +160,9 @@ struct EdgePlan {
   int ch = 0;          // channels per block
   int cpl = 0;         // channels per lane
   int team_warps = 0;  // warps that share an edge
-  std::vector<double> prog_c, term_c;
-  std::vector<unsigned short> prog_j;
+  // [0] of the shape, [1] of the shape with x and out exchanged
+  std::vector<double> prog_c[2], term_c[2];
+  std::vector<unsigned short> prog_j[2];
 };
 
 }  // namespace luna

@@ -1,6 +1,8 @@
 // Which plans the edge kernels serve, the tables they read, and the choice of the compiled instance.
 #include "uvu_edge.cuh"
 
+#include <utility>
+
 namespace luna {
 namespace edgek {
 
@@ -24,33 +26,46 @@ bool choose_lanes(luna_uvu_plan* plan, int ch) {
   return best != 0;
 }
 
-template <typename S>
-bool match_shape(luna_uvu_plan* plan) {
-  const auto& paths = plan->paths;
-  const int ch = paths[0].ch;
-  if (static_cast<int>(paths.size()) != S::paths || plan->X != S::XD * ch || plan->O != S::OD * ch || plan->Y != S::YD ||
-      plan->W != S::paths * ch)
-    return false;
-  std::vector<double> term_c(S::terms, 0.0), prog_c(2 * S::m_total, 0.0);
-  std::vector<unsigned short> prog_j(S::m_total, 0);
-  std::vector<int> entry_terms(S::m_total, 0);
-  for (const PathRec& p : paths) {
-    const int l1 = (p.d1 - 1) / 2, l2 = (p.d2 - 1) / 2, l3 = (p.d3 - 1) / 2;
-    if (p.ch != ch || p.w_stride != 1 || l1 > 3 || l2 > 3 || l3 > 3 || !S::ok(l1, l2, l3)) return false;
-    if (p.x_off != ch * S::xoff(l1) || p.y_off != S::yoff(l2) || p.out_off != ch * S::ooff(l3) ||
-        p.w_off != ch * S::rank(l1, l2, l3))
-      return false;
-    // the terms: exactly the compiled-in pattern
-    const CgTerm* pattern = cg_pattern(l1, l2, l3);
-    const int n = cg_count(l1, l2, l3), toff = S::toff(l1, l2, l3), moff = S::moff(l1, l2, l3);
+// Exchanging x and out turns the pattern of a coupling into that of the exchanged degrees.
+template <int L1, int L2, int L3>
+constexpr bool pattern_transposes() {
+  using P = CgPattern<L1, L2, L3>;
+  using Q = CgPattern<L3, L2, L1>;
+  if (P::n != Q::n) return false;
+  for (int t = 0; t < P::n; ++t) {
+    bool found = false;
+    for (int u = 0; u < Q::n; ++u) found = found || (P::t[t].i == Q::t[u].k && P::t[t].j == Q::t[u].j && P::t[t].k == Q::t[u].i);
+    if (!found) return false;
+  }
+  return true;
+}
+template <int... I>
+constexpr bool patterns_transpose(std::integer_sequence<int, I...>) {
+  return (pattern_transposes<I / 16, I / 4 % 4, I % 4>() && ...);
+}
+static_assert(patterns_transpose(std::make_integer_sequence<int, 64>{}),
+              "rows by destination use the patterns of the exchanged degrees");
+
+// The tables of shape R for the plan: R is the plan's shape, or that with x and out exchanged.  False if the plan's terms
+// are not exactly the compiled-in patterns.
+template <typename R>
+bool fill_tables(luna_uvu_plan* plan, bool exchanged) {
+  std::vector<double> term_c(R::terms, 0.0), prog_c(2 * R::m_total, 0.0);
+  std::vector<unsigned short> prog_j(R::m_total, 0);
+  std::vector<int> entry_terms(R::m_total, 0);
+  for (const PathRec& p : plan->paths) {
+    const int l1 = (p.d1 - 1) / 2, l2 = (p.d2 - 1) / 2, l3 = (p.d3 - 1) / 2, a = exchanged ? l3 : l1, c = exchanged ? l1 : l3;
+    const CgTerm* pattern = cg_pattern(a, l2, c);
+    const int n = cg_count(a, l2, c), toff = R::toff(a, l2, c), moff = R::moff(a, l2, c);
     std::vector<char> seen(n, 0);
     int found = 0;
     for (int k = 0; k < p.d3; ++k)
       for (int t = plan->rowptr_k[p.byk_ptr + k]; t < plan->rowptr_k[p.byk_ptr + k + 1]; ++t) {
         const auto& term = plan->terms_k[t];  // (a, b) = (i, j)
+        const int row = exchanged ? k : term.a, column = exchanged ? term.a : k;
         int slot = -1;
         for (int u = 0; u < n; ++u)
-          if (pattern[u].i == term.a && pattern[u].j == term.b && pattern[u].k == k) slot = u;
+          if (pattern[u].i == row && pattern[u].j == term.b && pattern[u].k == column) slot = u;
         if (slot < 0 || seen[slot]) return false;
         seen[slot] = 1;
         ++found;
@@ -60,15 +75,33 @@ bool match_shape(luna_uvu_plan* plan) {
           entry += u == 0 || pattern[u].i != pattern[u - 1].i || pattern[u].k != pattern[u - 1].k;
         const int which = entry_terms[entry]++;
         if (which > 1) return false;  // degrees up to 3 have at most two terms per entry
-        prog_c[which * S::m_total + entry] = term.c;
+        prog_c[which * R::m_total + entry] = term.c;
         prog_j[entry] = static_cast<unsigned short>(prog_j[entry] | (p.y_off + term.b) << (8 * which));
       }
     if (found != n) return false;
   }
+  plan->edge.term_c[exchanged] = term_c;
+  plan->edge.prog_c[exchanged] = prog_c;
+  plan->edge.prog_j[exchanged] = prog_j;
+  return true;
+}
+
+template <typename S>
+bool match_shape(luna_uvu_plan* plan) {
+  const auto& paths = plan->paths;
+  const int ch = paths[0].ch;
+  if (static_cast<int>(paths.size()) != S::paths || plan->X != S::XD * ch || plan->O != S::OD * ch || plan->Y != S::YD ||
+      plan->W != S::paths * ch)
+    return false;
+  for (const PathRec& p : paths) {
+    const int l1 = (p.d1 - 1) / 2, l2 = (p.d2 - 1) / 2, l3 = (p.d3 - 1) / 2;
+    if (p.ch != ch || p.w_stride != 1 || l1 > 3 || l2 > 3 || l3 > 3 || !S::ok(l1, l2, l3)) return false;
+    if (p.x_off != ch * S::xoff(l1) || p.y_off != S::yoff(l2) || p.out_off != ch * S::ooff(l3) ||
+        p.w_off != ch * S::rank(l1, l2, l3))
+      return false;
+  }
+  if (!fill_tables<S>(plan, false) || !fill_tables<Transposed<S>>(plan, true)) return false;
   plan->edge.ch = ch;
-  plan->edge.term_c = term_c;
-  plan->edge.prog_c = prog_c;
-  plan->edge.prog_j = prog_j;
   return true;
 }
 

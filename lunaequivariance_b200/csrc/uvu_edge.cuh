@@ -95,6 +95,12 @@ struct Shape {
   static constexpr int LO = top(MO);
 };
 
+// The shape with the roles of x and out exchanged; the weight blocks stay where they are.
+template <typename S>
+struct Transposed : Shape<S::MO, S::MY, S::MX> {
+  static constexpr int rank(int a, int b, int c) { return S::rank(c, b, a); }
+};
+
 // The compiled shapes: network layers with edge harmonics to degree 1, 2 or 3 - first, interior, last - and the single
 // vector-vector-scalar coupling.
 constexpr int kEdgeShapes = 11;

@@ -243,8 +243,8 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.out = static_cast<T*>(a.out);
   P.src = graph->src;
   P.dst_rowptr = graph->dst_rowptr;
-  P.prog_c = static_cast<const T*>(dt.edge_prog_c);
-  P.prog_j = dt.edge_prog_j;
+  P.prog_c = static_cast<const T*>(dt.edge[0].prog_c);
+  P.prog_j = dt.edge[0].prog_j;
   P.status = dt.status;
   P.tile_counters = next_tile_counters(plan, dt);
   P.num_rows = graph->num_nodes;

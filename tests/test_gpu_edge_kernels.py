@@ -65,3 +65,32 @@ def test_channel_counts(mul, dtype):
 def test_row_splits(nodes, edges):
     for mul in (16, 128):
         check(SHAPES[3], mul, torch.float32, nodes, edges, 0.0, nodes + edges)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+def test_one_gradient_alone(shape, dtype):
+    """dL/dw alone and dL/dy alone, whose rows may be the destinations, and two tangents added into one dL/dw; rows shared
+    by teams, and tiles with rows without edges."""
+    for mul, nodes, edges, skew in ((32, 29, 400, 0.0), (48, 150, 190, 1.5), (160, 40, 130, 1.0)):
+        in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
+        instructions = all_paths(in1, in2, out)
+        module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False,
+                                        dtype=dtype)
+        meta = oracle_conv.build_specs(in1, in2, out, instructions)
+        generator = torch.Generator().manual_seed(100 + shape)
+        src, dst = skewed_graph(nodes, edges, generator, skew)
+        p = random_problem((meta["in1_dim"], meta["in2_dim"], meta["out_dim"], meta["weight_numel"]), nodes, src, dtype,
+                           generator)
+        ref = oracle_conv.conv_derivatives(meta, *(p[k].double() for k in ("x", "y", "w")), src, dst, nodes,
+                                           p["g"].double(), p["rx"].double(), p["ry"].double(), None)
+        graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+        x, y, w, g = (p[k].to(DEVICE).requires_grad_(True) for k in ("x", "y", "w", "g"))
+        result = module(x, y, w, graph=graph)
+        (gw,) = torch.autograd.grad(result, w, g, retain_graph=True)
+        (gy,) = torch.autograd.grad(result, y, g, retain_graph=True)
+        gx, gy_too = torch.autograd.grad(result, (x, y), g, create_graph=True)
+        (hw,) = torch.autograd.grad((gx, gy_too), w, (p["rx"].to(DEVICE), p["ry"].to(DEVICE)))
+        module.op.check_status()
+        for key, value in dict(gw=gw, gy=gy, hw=hw).items():
+            assert_close(value, ref[key], dtype, f"{SHAPES[shape]} x{mul} {dtype} {key} alone")
