@@ -306,6 +306,7 @@ __device__ __forceinline__ void lane_store_block(T* p, int stride, const typenam
 // y[jb].  Lane l makes entries l, l + 32, ...
 template <typename T, typename S>
 struct MatrixProgram {
+  static constexpr int elems = 0;  // of shared memory
   T a[S::m_rounds], b[S::m_rounds];
   unsigned j[(S::m_rounds + 1) / 2];  // two attribute indices of 8 bits per round
   __device__ __forceinline__ void load(const T* coefficients, const unsigned short* attributes, int lane) {
@@ -325,6 +326,36 @@ struct MatrixProgram {
       const T ya = __shfl_sync(0xffffffffu, y, static_cast<int>((j[r / 2] >> (16 * (r % 2))) & 255u));
       const T yb = __shfl_sync(0xffffffffu, y, static_cast<int>((j[r / 2] >> (16 * (r % 2) + 8)) & 255u));
       to[r * 32 + lane] = fma(b[r], yb, a[r] * ya);
+    }
+  }
+};
+
+// The same with the program in shared memory (whole rounds of 32 entries), for kernels that are short of registers.
+template <typename T, typename S>
+struct SharedMatrixProgram {
+  static constexpr int entries = S::m_rounds * 32;
+  static constexpr int elems = 2 * entries + entries * 2 / static_cast<int>(sizeof(T));
+  const T* c;
+  const unsigned short* j;
+  // by all threads of the CTA, which synchronise before the first run
+  __device__ __forceinline__ void load(T* to, const T* coefficients, const unsigned short* attributes) {
+    unsigned short* to_j = reinterpret_cast<unsigned short*>(to + 2 * entries);
+    for (int m = threadIdx.x; m < entries; m += blockDim.x) {
+      to[m] = m < S::m_total ? coefficients[m] : T(0);
+      to[entries + m] = m < S::m_total ? coefficients[S::m_total + m] : T(0);
+      to_j[m] = m < S::m_total ? attributes[m] : static_cast<unsigned short>(0);
+    }
+    c = to;
+    j = to_j;
+  }
+  __device__ __forceinline__ void run(T y, T* to, int lane) const {
+#pragma unroll
+    for (int r = 0; r < S::m_rounds; ++r) {
+      const int m = r * 32 + lane;
+      const unsigned which = j[m];
+      const T ya = __shfl_sync(0xffffffffu, y, static_cast<int>(which & 255u));
+      const T yb = __shfl_sync(0xffffffffu, y, static_cast<int>(which >> 8));
+      to[m] = fma(c[entries + m], yb, c[m] * ya);
     }
   }
 };

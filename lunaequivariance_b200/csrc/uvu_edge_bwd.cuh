@@ -52,9 +52,17 @@ template <typename T, int CPL, typename S, bool WX, bool WM, bool WY>
 struct EdgeBwd {
   static constexpr int words = sizeof(T) / 4;
   static constexpr int pair = PkT<T, CPL, UsePairs<T, CPL>::value>::W;
-  static constexpr int max_warps =
-      warps_for((S::XD * CPL * (WX ? 2 : 1) + (WY ? S::YD * pair : 0) + (2 * S::LO + 1) * CPL) * words +
-                (WM ? S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 : 0) + 48);
+  // registers for the state a lane keeps, and for its part of the matrix program
+  static constexpr int state =
+      (S::XD * CPL * (WX ? 2 : 1) + (WY ? S::YD * pair : 0) + (2 * S::LO + 1) * CPL) * words;
+  static constexpr int program_regs = WM ? S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 : 0;
+  // The program goes to shared memory where that makes room for 16 warps instead of 12 without spills: degrees (2, 2, 2)
+  // with two channels per lane, 5.2 M edges of 64 channels: 7.09 -> 6.60 ms.  Elsewhere the reads cost more than the room
+  // gives: (3, 3, 3), 12 warps for 8 with some spills, 6.38 -> 7.07 ms; dL/dw alone in FP64 5.36 -> 6.16 ms.
+  static constexpr bool shared_program =
+      WX && WM && WY && pair == 2 && warps_for(state + program_regs + 48) == 12 && warps_for(state + 48) == 16;
+  using Program = std::conditional_t<shared_program, SharedMatrixProgram<T, S>, MatrixProgram<T, S>>;
+  static constexpr int max_warps = warps_for(state + (shared_program ? 0 : program_regs) + 48);
   // slots of g: the highest degree has one, the others share one
   static constexpr int slot_of(int l3) { return l3 == S::LO && S::ooff(S::LO) > 0 ? 1 : 0; }
   static constexpr int slots = slot_of(S::LO) + 1;
@@ -71,7 +79,8 @@ struct EdgeBwd {
   static constexpr int warp_elems(int team_warps) {
     return m_elems + (WY ? red_pass * red_row + (team_warps > 1 ? 64 : 0) : 0);
   }
-  static constexpr int table_elems = (S::terms + 3) / 4 * 4;
+  static constexpr int term_elems = (S::terms + 3) / 4 * 4;
+  static constexpr int table_elems = term_elems + (WM ? Program::elems : 0);
 };
 
 // One path for a lane's packets.  xl / gxl: the lane's x and gx packets of degree l1; g2: its g packets of degree l3;
@@ -190,8 +199,11 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   if constexpr (WY)
     for (int i = threadIdx.x; i < S::terms; i += blockDim.x) ctab[i] = P.term_c[i];
 
-  MatrixProgram<T, S> program;
-  if constexpr (WM) program.load(P.prog_c, P.prog_j, lane);
+  typename K::Program program;
+  if constexpr (K::shared_program)
+    program.load(ctab + K::term_elems, P.prog_c, P.prog_j);
+  else if constexpr (WM)
+    program.load(P.prog_c, P.prog_j, lane);
   __syncthreads();
 
   const int cpw = ch / team_warps;  // channels of this warp
