@@ -128,6 +128,14 @@ Tensor prepared(const Tensor& t) {
   return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
 }
 
+// The kernels compute values only.  An operand of forward-mode AD does not have to require grad, so it can reach a launch
+// without passing an autograd function; its tangent would be dropped, which reads as a derivative of zero.
+void refuse_tangents(std::initializer_list<const Tensor*> tensors) {
+  for (const Tensor* t : tensors)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(),
+                                "forward-mode automatic differentiation is not provided");
+}
+
 void check_operand(const Op& op, const Tensor& x, const Tensor& t, const char* name, int64_t rows, int64_t columns) {
   if (!t.defined()) return;
   TORCH_CHECK_TYPE(t.scalar_type() == op.dtype, name, " must be ", op.dtype == at::kDouble ? "torch.float64" : "torch.float32",
@@ -138,6 +146,7 @@ void check_operand(const Op& op, const Tensor& x, const Tensor& t, const char* n
 }
 
 void check_operands(const Op& op, const Graph& graph, const Tensor& x, const Tensor& y, const Tensor& w, const Tensor& g) {
+  refuse_tangents({&x, &y, &w, &g});
   TORCH_CHECK(x.is_cuda(), "CUDA is required for SO3 LunaTP.");
   check_operand(op, x, x, "x", graph.native.num_src_nodes, op.X);
   check_operand(op, x, y, "edge_attr", graph.native.num_edges, op.Y);
@@ -191,6 +200,7 @@ std::array<Tensor, 4> run_double(const Op& op, const Graph& graph, const Tensor&
                                  const Tensor& g_, const Tensor& rx_, const Tensor& ry_, const Tensor& rw_, int mask) {
   std::array<Tensor, 4> out;
   if (!mask) return out;
+  refuse_tangents({&rx_, &ry_, &rw_});
   check_operands(op, graph, x_, y_, w_, g_);
   check_operand(op, x_, rx_, "rx", graph.native.num_src_nodes, op.X);
   check_operand(op, x_, ry_, "ry", graph.native.num_edges, op.Y);

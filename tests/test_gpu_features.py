@@ -176,3 +176,28 @@ def test_tensor_product_without_graph(shared, dtype):
     functional = luna.tensor_product(dev["x"], dev["y"], dev["w"], irreps_in1=in1, irreps_in2=in2,
                                      irreps_out=out_irreps, instructions=instructions, shared_weights=shared)
     assert_close(functional, ref_out.detach(), dtype, "functional tensor product")
+
+
+@pytest.mark.parametrize("requires_grad", [False, True])
+def test_forward_mode_derivatives_are_refused(requires_grad):
+    """An operand or a cotangent with a tangent raises; a result without a tangent would read as a derivative of zero."""
+    import torch.autograd.forward_ad as forward_ad
+
+    in1, in2, out, instructions, options = config("fixture")
+    module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False, **options)
+    graph = module.create_graph(torch.tensor([0, 1, 1], device=DEVICE), torch.tensor([0, 0, 1], device=DEVICE), 2)
+    shapes = ((2, module.op.in1_dim), (3, module.op.in2_dim), (3, module.op.weight_numel))
+    for dual in range(3):
+        with forward_ad.dual_level():
+            operands = [torch.ones(shape, device=DEVICE, requires_grad=requires_grad) for shape in shapes]
+            operands[dual] = forward_ad.make_dual(operands[dual], torch.ones(shapes[dual], device=DEVICE))
+            with pytest.raises(NotImplementedError):
+                module(*operands, graph=graph)
+            with torch.no_grad(), pytest.raises(NotImplementedError):
+                module(*operands, graph=graph)
+    with forward_ad.dual_level():
+        operands = [torch.ones(shape, device=DEVICE, requires_grad=True) for shape in shapes]
+        result = module(*operands, graph=graph)
+        cotangent = forward_ad.make_dual(torch.ones_like(result), torch.ones_like(result))
+        with pytest.raises(NotImplementedError):
+            torch.autograd.grad(result, operands, cotangent)

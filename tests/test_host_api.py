@@ -163,3 +163,23 @@ def test_launch_path_shares_the_cpp_runtime():
     _native.binding()
     with open(_native.BINDING_PATH, "rb") as module:
         assert b"libstdc++.so" in module.read()
+
+
+def test_forward_mode_operands_are_refused_by_the_launch_path():
+    """The kernels drop the tangent of a dual tensor, which need not require grad: it must not get as far as a launch."""
+    import torch.autograd.forward_ad as forward_ad
+
+    from lunaequivariance_b200 import _native
+    from tests.helpers import config
+
+    in1, in2, out, instructions, options = config("small")
+    op = luna.prepare_tensor_product(in1, in2, out, instructions, convolution=True, **options)
+    src, dst = torch.tensor([0, 1, 1]), torch.tensor([0, 0, 1])
+    holder = luna.make_graph(src, dst, 2).native_holder()
+    shapes = ((2, op.in1_dim), (3, op.in2_dim), (3, op.weight_numel))
+    for dual in range(3):
+        with forward_ad.dual_level():
+            operands = [torch.ones(shape) for shape in shapes]
+            operands[dual] = forward_ad.make_dual(operands[dual], torch.ones(shapes[dual]))
+            with pytest.raises(NotImplementedError, match="forward-mode"):  # asked before the device is looked at
+                _native.binding().conv(op._plan.op, holder, *operands)
