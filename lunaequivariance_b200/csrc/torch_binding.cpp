@@ -473,6 +473,7 @@ void check_vectors(const Harmonics& h, const Tensor& v) {
 }
 
 Tensor sh_forward(const Harmonics& h, const Tensor& v) {
+  if (!h.constant) refuse_tangents({&v});  // the values of degree 0 alone have no derivative
   check_vectors(h, v);
   const c10::cuda::CUDAGuard guard(v.device());
   const Tensor flat = rows_of(v);
@@ -484,6 +485,7 @@ Tensor sh_forward(const Harmonics& h, const Tensor& v) {
 }
 
 Tensor sh_backward(const Harmonics& h, const Tensor& v, const Tensor& g) {
+  refuse_tangents({&v, &g});
   check_vectors(h, v);
   const c10::cuda::CUDAGuard guard(v.device());
   const Tensor flat = rows_of(v), cotangents = rows_of(g);
@@ -493,6 +495,7 @@ Tensor sh_backward(const Harmonics& h, const Tensor& v, const Tensor& g) {
 }
 
 std::array<Tensor, 2> sh_double(const Harmonics& h, const Tensor& v, const Tensor& g, const Tensor& r, int mask) {
+  refuse_tangents({&v, &g, &r});
   check_vectors(h, v);
   const c10::cuda::CUDAGuard guard(v.device());
   const Tensor flat = rows_of(v), cotangents = rows_of(g), tangents = rows_of(r);

@@ -183,3 +183,19 @@ def test_forward_mode_operands_are_refused_by_the_launch_path():
             operands[dual] = forward_ad.make_dual(operands[dual], torch.ones(shapes[dual]))
             with pytest.raises(NotImplementedError, match="forward-mode"):  # asked before the device is looked at
                 _native.binding().conv(op._plan.op, holder, *operands)
+
+
+def test_forward_mode_vectors_are_refused_by_the_harmonics():
+    import torch.autograd.forward_ad as forward_ad
+
+    from lunaequivariance_b200 import _native
+    from lunaequivariance_b200.spherical_harmonics import SphericalHarmonicsConfig
+
+    holder = SphericalHarmonicsConfig((0, 1, 2), True, "component", torch.float32).holder(torch.float32)
+    with forward_ad.dual_level():
+        vectors = forward_ad.make_dual(torch.ones(5, 3), torch.ones(5, 3))
+        with pytest.raises(NotImplementedError, match="forward-mode"):
+            _native.binding().harmonics(holder, vectors)
+        constant = SphericalHarmonicsConfig((0,), True, "component", torch.float32).holder(torch.float32)
+        with pytest.raises(RuntimeError, match="CUDA is required"):  # not refused: its derivative is zero
+            _native.binding().harmonics(constant, vectors)
