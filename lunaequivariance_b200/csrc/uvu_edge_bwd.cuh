@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
         if (WM && pos + 2 < p_end && lane < S::YD) y_next = P.y[static_cast<int64_t>(e2) * S::YD + lane];
         if constexpr (WY) {
           // the lanes' partial gy rows through the reduction tile: entries 2r and 2r + 1 in tile row r; four lanes sum
-          // a row, a quarter each
+          // a row, a quarter each.  Idle lanes bring in zeros: what they computed is 0 times the last lane's w and g.
           constexpr int passes = (K::red_rows + K::red_pass - 1) / K::red_pass;
           static_for<0, passes>([&](auto qc) {
             constexpr int first = decltype(qc)::value * K::red_pass;
@@ -421,9 +421,9 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
             static_for<0, rows>([&](auto rc) {
               constexpr int j = 2 * (first + decltype(rc)::value);
               Vec<T, 2> pr;
-              pr.a[0] = hsum(gy2[j]);
+              pr.a[0] = active ? hsum(gy2[j]) : T(0);
               if constexpr (j + 1 < S::YD) {
-                pr.a[1] = hsum(gy2[j + 1]);
+                pr.a[1] = active ? hsum(gy2[j + 1]) : T(0);
               } else {
                 pr.a[1] = T(0);
               }

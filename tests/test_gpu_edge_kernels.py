@@ -94,3 +94,60 @@ def test_one_gradient_alone(shape, dtype):
         module.op.check_status()
         for key, value in dict(gw=gw, gy=gy, hw=hw).items():
             assert_close(value, ref[key], dtype, f"{SHAPES[shape]} x{mul} {dtype} {key} alone")
+
+
+def term_by_term(meta, x, y, w, g, src, dst):
+    """Output and first derivatives as sums over the non-zero coupling terms: a value that is not finite reaches exactly
+    the results it is a factor of (a dense contraction would multiply it by the zeros of the coupling tensors too)."""
+    out, gx, gy, gw = (torch.zeros_like(t) for t in (g, x, y, w))
+    for spec in meta["specs"]:
+        cg = torch.as_tensor(spec["cg"], dtype=torch.float64)
+        channel = torch.arange(spec["channels"])
+        for i, j, k in cg.nonzero().tolist():
+            columns = (spec["x_offset"] + channel * spec["d1"] + i, spec["y_offset"] + j,
+                       spec["weight_offset"] + channel * spec["weight_stride"],
+                       spec["out_offset"] + channel * spec["d3"] + k)
+            a, b, c, d = x[src][:, columns[0]], cg[i, j, k] * y[:, columns[1], None], w[:, columns[2]], g[dst][:, columns[3]]
+            out[:, columns[3]] = out[:, columns[3]].index_add(0, dst, a * b * c)
+            gx[:, columns[0]] = gx[:, columns[0]].index_add(0, src, b * c * d)
+            gy[:, columns[1]] += (cg[i, j, k] * a * c * d).sum(1)
+            gw[:, columns[2]] += a * b * d
+    return dict(out=out, gx=gx, gy=gy, gw=gw)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("mul", [12, 48, 64, 128, 160])
+@pytest.mark.parametrize("shape", [3, 4, 6])
+def test_values_that_are_not_finite_stay_where_they_belong(shape, mul, dtype):
+    """Infinities and NaN in the last channel, which idle lanes read too.  Finite results stay finite and right, infinite ones keep their sign; where
+    the terms disagree (infinity less infinity) any result that is not finite will do."""
+    in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
+    instructions = all_paths(in1, in2, out)
+    module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False,
+                                    dtype=dtype)
+    assert module.op.backward_variant == "row"
+    meta = oracle_conv.build_specs(in1, in2, out, instructions)
+    generator = torch.Generator().manual_seed(shape + mul)
+    nodes, edges = 9, 40
+    src, dst = skewed_graph(nodes, edges, generator, 0.0)
+    clean = random_problem((meta["in1_dim"], meta["in2_dim"], meta["out_dim"], meta["weight_numel"]), nodes, src, dtype,
+                           generator)
+    graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+    inf, nan = float("inf"), float("nan")
+    for key, row, column, value in (("x", int(src[3]), mul - 1, -inf), ("w", 5, 2 * mul - 1, inf), ("w", 5, mul - 1, nan),
+                                    ("g", int(dst[7]), mul - 1, inf)):
+        p = {k: clean[k].clone() for k in ("x", "y", "w", "g")}
+        p[key][row, column] = value
+        ref = term_by_term(meta, *(p[k].double() for k in ("x", "y", "w", "g")), src, dst)
+        x, y, w, g = (p[k].to(DEVICE).requires_grad_(True) for k in ("x", "y", "w", "g"))
+        result = module(x, y, w, graph=graph)
+        gx, gy, gw = torch.autograd.grad(result, (x, y, w), g, retain_graph=True)
+        (gy_alone,) = torch.autograd.grad(result, y, g, retain_graph=True)
+        (gw_alone,) = torch.autograd.grad(result, w, g)
+        for name, got in dict(out=result, gx=gx, gy=gy, gw=gw, gy_alone=gy_alone, gw_alone=gw_alone).items():
+            want, got = ref[name.removesuffix("_alone")], got.detach().cpu().double()
+            what = f"{SHAPES[shape]} x{mul} {dtype} {key}[{row}, {column}] = {value}: {name}"
+            finite, infinite = want.isfinite(), want.isinf()
+            assert bool((got.isfinite() == finite).all()), what
+            assert bool((got[infinite] == want[infinite]).all()), what
+            assert_close(got[finite], want[finite], dtype, what)
