@@ -51,7 +51,7 @@ static_assert(patterns_transpose(std::make_integer_sequence<int, 64>{}),
 template <typename R>
 bool fill_tables(luna_uvu_plan* plan, bool exchanged) {
   std::vector<double> term_c(R::terms, 0.0), prog_c(2 * R::m_total, 0.0);
-  std::vector<unsigned short> prog_j(R::m_total, 0);
+  std::vector<unsigned short> prog_j(R::m_total, kNoAttribute | kNoAttribute << 8);
   std::vector<int> entry_terms(R::m_total, 0);
   for (const PathRec& p : plan->paths) {
     const int l1 = (p.d1 - 1) / 2, l2 = (p.d2 - 1) / 2, l3 = (p.d3 - 1) / 2, a = exchanged ? l3 : l1, c = exchanged ? l1 : l3;
@@ -76,7 +76,7 @@ bool fill_tables(luna_uvu_plan* plan, bool exchanged) {
         const int which = entry_terms[entry]++;
         if (which > 1) return false;  // degrees up to 3 have at most two terms per entry
         prog_c[which * R::m_total + entry] = term.c;
-        prog_j[entry] = static_cast<unsigned short>(prog_j[entry] | (p.y_off + term.b) << (8 * which));
+        prog_j[entry] = static_cast<unsigned short>((prog_j[entry] & ~(255 << (8 * which))) | (p.y_off + term.b) << (8 * which));
       }
     if (found != n) return false;
   }

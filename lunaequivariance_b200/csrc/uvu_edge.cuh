@@ -303,9 +303,12 @@ __device__ __forceinline__ void lane_store_block(T* p, int stride, const typenam
 }
 
 // The program that turns an edge's attributes, one per lane, into its coupling matrices: entry m is a_m y[ja] + b_m
-// y[jb].  Lane l makes entries l, l + 32, ...
+// y[jb].  Lane l makes entries l, l + 32, ...  An entry made of one attribute only takes kNoAttribute as its second, a lane
+// that holds no attribute but zero: with any attribute in its place 0 times an infinite one would make the entry NaN.
+constexpr int kNoAttribute = 31;
 template <typename T, typename S>
 struct MatrixProgram {
+  static_assert(S::YD <= kNoAttribute, "one lane is left without an attribute");
   static constexpr int elems = 0;  // of shared memory
   T a[S::m_rounds], b[S::m_rounds];
   unsigned j[(S::m_rounds + 1) / 2];  // two attribute indices of 8 bits per round

@@ -119,7 +119,8 @@ def term_by_term(meta, x, y, w, g, src, dst):
 @pytest.mark.parametrize("mul", [12, 48, 64, 128, 160])
 @pytest.mark.parametrize("shape", [3, 4, 6])
 def test_values_that_are_not_finite_stay_where_they_belong(shape, mul, dtype):
-    """Infinities and NaN in the last channel, which idle lanes read too.  Finite results stay finite and right, infinite ones keep their sign; where
+    """Infinities and NaN in the last channel, which idle lanes read too, and in single edge attributes, which matrix
+    entries made of one attribute must not meet.  Finite results stay finite and right, infinite ones keep their sign; where
     the terms disagree (infinity less infinity) any result that is not finite will do."""
     in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
     instructions = all_paths(in1, in2, out)
@@ -135,7 +136,7 @@ def test_values_that_are_not_finite_stay_where_they_belong(shape, mul, dtype):
     graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
     inf, nan = float("inf"), float("nan")
     for key, row, column, value in (("x", int(src[3]), mul - 1, -inf), ("w", 5, 2 * mul - 1, inf), ("w", 5, mul - 1, nan),
-                                    ("g", int(dst[7]), mul - 1, inf)):
+                                    ("g", int(dst[7]), mul - 1, inf), ("y", 11, 0, inf), ("y", 11, 0, nan), ("y", 11, 2, -inf)):
         p = {k: clean[k].clone() for k in ("x", "y", "w", "g")}
         p[key][row, column] = value
         ref = term_by_term(meta, *(p[k].double() for k in ("x", "y", "w", "g")), src, dst)
