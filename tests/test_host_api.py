@@ -169,7 +169,6 @@ def test_forward_mode_operands_are_refused_by_the_launch_path():
     """The kernels drop the tangent of a dual tensor, which need not require grad: it must not get as far as a launch."""
     import torch.autograd.forward_ad as forward_ad
 
-    from lunaequivariance_b200 import _native
     from tests.helpers import config
 
     in1, in2, out, instructions, options = config("small")
@@ -188,7 +187,6 @@ def test_forward_mode_operands_are_refused_by_the_launch_path():
 def test_forward_mode_vectors_are_refused_by_the_harmonics():
     import torch.autograd.forward_ad as forward_ad
 
-    from lunaequivariance_b200 import _native
     from lunaequivariance_b200.spherical_harmonics import SphericalHarmonicsConfig
 
     holder = SphericalHarmonicsConfig((0, 1, 2), True, "component", torch.float32).holder(torch.float32)
@@ -199,3 +197,11 @@ def test_forward_mode_vectors_are_refused_by_the_harmonics():
         constant = SphericalHarmonicsConfig((0,), True, "component", torch.float32).holder(torch.float32)
         with pytest.raises(RuntimeError, match="CUDA is required"):  # not refused: its derivative is zero
             _native.binding().harmonics(constant, vectors)
+
+
+def test_default_build_leaves_line_tables_out():
+    """They made the library and its objects 360 MB, too much for a checkout that is copied about with its build."""
+    from lunaequivariance_b200 import build
+
+    assert "-lineinfo" not in build.NVCC_FLAGS
+    assert os.path.getsize(_native.LIBRARY_PATH) < 100 << 20
