@@ -160,6 +160,7 @@ struct EdgePlan {
   int ch = 0;          // channels per block
   int cpl = 0;         // channels per lane
   int team_warps = 0;  // warps that share an edge
+  int slices = 1;      // parts of a block's channels that are launched side by side
   // [0] of the shape, [1] of the shape with x and out exchanged
   std::vector<double> prog_c[2], term_c[2];
   std::vector<unsigned short> prog_j[2];
@@ -251,8 +252,8 @@ void analyse(luna_uvu_plan* plan);
 int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
             const void* w, void* out, bool accumulate, cudaStream_t stream);
 int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
-             const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w,
-             cudaStream_t stream);
+             const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w, void* scratch,
+             int64_t scratch_bytes, cudaStream_t stream);
 }  // namespace edgek
 
 // Staged kernels (bulk-copy pipeline).  fast_available() is false in a build without them.

@@ -12,6 +12,11 @@
 // One lane of the team stages an edge's rows - the whole weight row, the whole gathered node row - with one bulk copy
 // each, whatever the number of warps: DRAM sees requests of full rows.
 //
+// Slices.  Blocks too wide for a team (more than eight warps, or rows that do not fit twice in shared memory) are cut into
+// slices of 32 * CPL channels, blockIdx.y their number: a one-warp team walks the rows of its slice, whose pieces, one per
+// path and per degree, the lanes copy side by side.  Each slice has its tile counters and its part of dL/dy; the parts are
+// summed in order by a second kernel.
+//
 // Two ways of handing out rows.  Large launches: a team takes tiles of consecutive rows from a counter.  Small
 // launches, in which a row per team would leave the chip waiting for the longest rows: `group` teams of a CTA share a
 // row, each a contiguous part of its edges, and the parts are summed in a fixed order through shared memory.  A row's
@@ -29,7 +34,7 @@ namespace edgek {
 using namespace fastk;
 
 constexpr int kEdgeMaxStages = 4;
-constexpr int kEdgeMaxWarps = 32;
+constexpr int kEdgeMaxSlices = kTileCounterWords / 2;
 
 // ---- shapes ---------------------------------------------------------------------------------------------------------
 template <int MX_, int MY_, int MO_>
@@ -106,6 +111,8 @@ struct Transposed : Shape<S::MO, S::MY, S::MX> {
 constexpr int kEdgeShapes = 11;
 constexpr int kEdgeShapeMasks[kEdgeShapes][3] = {{1, 3, 3},  {1, 7, 7},   {1, 15, 15}, {3, 3, 3},   {7, 7, 7}, {15, 15, 15},
                                                  {7, 15, 15}, {3, 3, 1},  {7, 7, 1},   {15, 15, 1}, {2, 2, 1}};
+// Shapes whose kernels are compiled for slices too.  The others have no wide layers in use; theirs run the table kernels.
+constexpr bool edge_sliced(int id) { return id >= 3 && id <= 6; }
 template <int ID>
 using ShapeOf = Shape<kEdgeShapeMasks[ID][0], kEdgeShapeMasks[ID][1], kEdgeShapeMasks[ID][2]>;
 
@@ -119,6 +126,8 @@ struct EdgeBackwardArgs {
   const void *x, *y, *w, *g;
   void *gx, *gy, *gw;
   bool acc_x, acc_y, acc_w;
+  void* scratch;  // for the slices' parts of gy
+  int64_t scratch_bytes;
 };
 // The kernels of one (element type, channels per lane, shape), compiled in a file of their own.
 template <typename T, int CPL, int ID>
@@ -142,6 +151,24 @@ struct EdgeSplit {
   int64_t blocks = 1;
   int64_t tile_rows = 1;
 };
+
+// CTAs that a slice may take: as many as make whole waves of all slices' CTAs, one per SM, with at most 5 % of the SMs idle.
+// With a CTA per SM and slice, a CTA's part of a small graph is too short for what it costs to start: degrees (1, 1, 1),
+// 27 slices, 22,000 edges, forward / backward 0.37 / 0.78 ms, and 0.23 / 0.55 like this.
+inline int slice_ctas(int sm_count, int slices) {
+  int best = 1;
+  double best_use = 0.0;
+  for (int waves = 1; waves <= 4; ++waves) {
+    const int ctas = sm_count * waves / slices;
+    const double use = static_cast<double>(ctas) * slices / (static_cast<double>(sm_count) * waves);
+    if (ctas >= 1 && use > best_use) {
+      best = ctas;
+      best_use = use;
+    }
+    if (best_use >= 0.95) break;
+  }
+  return best;
+}
 
 constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
 
@@ -195,6 +222,19 @@ __host__ __device__ constexpr int edge_entry(int t) {
 }
 
 // ---- device helpers ---------------------------------------------------------------------------------------------------
+// Where element `a` of a slice's row of blocks (the degrees of `mask`, `ch` channels each) lies in the whole row, whose
+// blocks have `row_ch` channels and in which the slice begins with channel `first`.
+template <typename S>
+__device__ __forceinline__ int slice_element(int mask, int a, int ch, int row_ch, int first) {
+  int at = a;
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    if (!S::has(mask, l)) continue;
+    const int begin = S::below(mask, l), d = 2 * l + 1;
+    if (a >= ch * begin && a < ch * (begin + d)) at = a + (row_ch - ch) * begin + first * d;
+  }
+  return at;
+}
 __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }

@@ -40,7 +40,9 @@ struct EdgeBwdParams {
   unsigned* tile_counters;
   int64_t num_rows, tile_rows, tile_edges, num_tiles;  // tile_rows 0: tiles are stretches of tile_edges edges
   float rows_per_edge;
-  int ch, team_warps, teams, group;
+  int ch, row_ch;  // channels per block, or of a slice of it; channels per block
+  int64_t gy_part;  // elements between the slices' parts of gy
+  int team_warps, teams, group;
   int stages, split;
   int team_elems;  // shared memory per team
   int need_w;
@@ -160,8 +162,9 @@ __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* 
   });
 }
 
-// FULL: one warp per edge and 32 * CPL channels, known to the compiler.  DST: rows by destination (S, x and g exchanged).
-template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST>
+// FULL: one warp per edge and 32 * CPL channels, known to the compiler.  SLICED: these are a slice of wider blocks.  DST: rows
+// by destination (S, x and g exchanged).
+template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED>
 __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32, 1)
     edge_bwd_kernel(const __grid_constant__ EdgeBwdParams<T> P) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
@@ -176,6 +179,11 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   const int W = S::paths * ch, X = S::XD * ch, O = S::OD * ch;
   const bool split = P.split != 0;
   const int stage_elems = W + (split ? 0 : O);
+  static_assert(FULL || !SLICED, "a slice is one warp's full set of channels");
+  const int row_ch = SLICED ? P.row_ch : ch, first_ch = SLICED ? static_cast<int>(blockIdx.y) * ch : 0;
+  const int w_row = S::paths * row_ch, x_row = S::XD * row_ch, o_row = S::OD * row_ch;  // in memory
+  unsigned* const counters = P.tile_counters + (SLICED ? 2 * blockIdx.y : 0);
+  T* const gy_out = SLICED ? P.gy + blockIdx.y * P.gy_part : P.gy;
 
   T* const base = reinterpret_cast<T*>(smem_raw);
   T* const ring = base + static_cast<size_t>(team) * P.team_elems;
@@ -211,22 +219,51 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   const int own = FULL ? PK::W * lane : member * cpw + PK::W * min(lane, lanes - 1);  // first channel of this lane
   const bool active = FULL || lane < lanes;
   const bool leader = member == 0 && lane == 0;
+  const bool issuing = SLICED || leader;  // the pieces of a slice are copied by all lanes
   const bool want_x = WX && P.gx != nullptr, storing = WM && P.gw != nullptr;
   const uint32_t w_bytes = P.need_w ? static_cast<uint32_t>(W * sizeof(T)) : 0u;
   const uint32_t g_bytes = split ? 0u : static_cast<uint32_t>(O * sizeof(T));
   const bool staged = w_bytes + g_bytes != 0u;
 
-  auto load_stage = [&](int e, int d, int st) {  // leader only
+  // copies the degrees [from, to) of a slice of row d of g, one degree to a lane
+  auto load_pieces = [&](auto from, auto until, T* to, int d, uint64_t* bar) {
+    static_for<decltype(from)::value, decltype(until)::value>([&](auto lc) {
+      constexpr int l = decltype(lc)::value, d3 = 2 * l + 1;
+      if constexpr (S::has(S::MO, l)) {
+        if (lane == l)
+          bulk_copy_g2s(to + ch * S::ooff(l), P.g + static_cast<int64_t>(d) * o_row + row_ch * S::ooff(l) + first_ch * d3,
+                        static_cast<uint32_t>(ch * d3 * sizeof(T)), bar);
+      }
+    });
+  };
+  auto load_stage = [&](int e, int d, int st) {  // by the issuing lanes
     if (!staged) return;
     T* to = ring + static_cast<size_t>(st) * stage_elems;
+    if constexpr (SLICED) {
+      if (lane == 0) mbar_arrive_expect_tx(&full[st], w_bytes + g_bytes);
+      __syncwarp();  // also: every lane's stores have read the stage
+      if (w_bytes)
+        for (int p = lane; p < S::paths; p += 32)
+          bulk_copy_g2s_hint(to + p * ch, P.w + static_cast<int64_t>(e) * w_row + p * row_ch + first_ch,
+                             static_cast<uint32_t>(ch * sizeof(T)), &full[st], l2_policy_evict_first());
+      if (g_bytes) load_pieces(std::integral_constant<int, 0>{}, std::integral_constant<int, 4>{}, to + W, d, &full[st]);
+      return;
+    }
     mbar_arrive_expect_tx(&full[st], w_bytes + g_bytes);
     if (w_bytes)
       bulk_copy_g2s_hint(to, P.w + static_cast<int64_t>(e) * W, w_bytes, &full[st], l2_policy_evict_first());
     if (g_bytes) bulk_copy_g2s(to + W, P.g + static_cast<int64_t>(d) * O, g_bytes, &full[st]);
   };
-  auto load_slot = [&](auto slot, int d) {  // leader only
+  auto load_slot = [&](auto slot, int d) {  // by the issuing lanes
     constexpr int h = decltype(slot)::value, first = K::slot_begin(h), count = K::slot_begin(h + 1) - first;
     const uint32_t bytes = static_cast<uint32_t>(count * ch * sizeof(T));
+    if constexpr (SLICED) {
+      if (lane == 0) mbar_arrive_expect_tx(&gfull[h], bytes);
+      __syncwarp();
+      load_pieces(std::integral_constant<int, h == 0 ? 0 : S::LO>{}, std::integral_constant<int, h + 1 == K::slots ? 4 : S::LO>{},
+                  gslots, d, &gfull[h]);
+      return;
+    }
     mbar_arrive_expect_tx(&gfull[h], bytes);
     bulk_copy_g2s(gslots + first * ch, P.g + static_cast<int64_t>(d) * O + first * ch, bytes, &gfull[h]);
   };
@@ -279,9 +316,9 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     int64_t n = unit, n_hi = unit + 1;
     if (!grouped) {
       if (team_warps == 1) {
-        unit_after = take_tile(P.tile_counters, total, lane);
+        unit_after = take_tile(counters, total, lane);
       } else {
-        if (leader) tickets[team] = atomicAdd(&P.tile_counters[0], 1u);
+        if (leader) tickets[team] = atomicAdd(&counters[0], 1u);
         team_sync(team_warps, team);
         unit_after = total + static_cast<int64_t>(tickets[team]);
         team_sync(team_warps, team);
@@ -319,7 +356,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     int d0 = dst_of(e0), d1 = dst_of(e1), d2 = dst_of(e2), d3n = dst_of(e3);
     auto id_ahead = [&](int k) { return k == 1 ? e1 : (k == 2 ? e2 : e3); };
     auto dst_ahead = [&](int k) { return k == 1 ? d1 : (k == 2 ? d2 : d3n); };
-    if (leader && e0 >= 0) {
+    if (issuing && e0 >= 0) {
       load_stage(e0, d0, st);
       for (int k = 1, stage = st; k < stages; ++k) {
         if (++stage == stages) stage = 0;
@@ -347,7 +384,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           constexpr int l1 = decltype(l1c)::value;
           if constexpr (S::has(S::MX, l1)) {
             constexpr int d = 2 * l1 + 1;
-            lane_load_block<PK, T, d>(P.x + n * X + ch * S::xoff(l1) + own * d, stride, &xr[S::xoff(l1) * NP]);
+            lane_load_block<PK, T, d>(P.x + n * x_row + row_ch * S::xoff(l1) + (first_ch + own) * d, stride, &xr[S::xoff(l1) * NP]);
           }
         });
         if (!active) {
@@ -379,11 +416,11 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
             if constexpr (l3 != S::LO && S::ooff(l3) + 2 * l3 + 1 == K::slot_begin(slot + 1)) {
               if (split) {  // the slot is done with; the last one is refilled at the end of the edge
                 team_sync(team_warps, team);
-                if (leader && more) load_slot(std::integral_constant<int, slot>{}, d1);
+                if (issuing && more) load_slot(std::integral_constant<int, slot>{}, d1);
               }
             }
             if constexpr (S::ooff(l3) == 0) {  // after the first degree: the row sent back has left its stage by now
-              if (refill_stage >= 0 && leader) {
+              if (refill_stage >= 0 && issuing) {
                 bulk_wait_group_read_all();
                 if (id_ahead(stages - 1) >= 0) load_stage(id_ahead(stages - 1), dst_ahead(stages - 1), refill_stage);
               }
@@ -393,15 +430,21 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
         });
         if (storing) fence_async_shared();  // gradient writes, before the bulk store reads the stage
         team_sync(team_warps, team);      // every lane is done with the stage, the last slot and the scalars
-        if (leader) {
+        if (issuing) {
           if (split && more) load_slot(std::integral_constant<int, K::slots - 1>{}, d1);
           if (storing) {
-            T* row = P.gw + static_cast<int64_t>(e0) * W;
-            const uint32_t bytes = static_cast<uint32_t>(W * sizeof(T));
-            if (P.acc_w)
-              bulk_reduce_add_s2g(row, wrow, bytes);
-            else
-              bulk_copy_s2g_hint(row, wrow, bytes, l2_policy_evict_first());
+            T* row = P.gw + static_cast<int64_t>(e0) * w_row + first_ch;
+            auto send = [&](int at, int from, uint32_t bytes) {
+              if (P.acc_w)
+                bulk_reduce_add_s2g(row + at, wrow + from, bytes);
+              else
+                bulk_copy_s2g_hint(row + at, wrow + from, bytes, l2_policy_evict_first());
+            };
+            if constexpr (SLICED) {
+              for (int p = lane; p < S::paths; p += 32) send(p * row_ch, p * ch, static_cast<uint32_t>(ch * sizeof(T)));
+            } else {
+              send(0, 0, static_cast<uint32_t>(W * sizeof(T)));
+            }
             bulk_commit_group();
           } else if (pos + stages < p_end) {
             const int k = stages;
@@ -452,7 +495,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
               if (team_warps > 1) {
                 *reinterpret_cast<Vec<T, 2>*>(gbuf + flip * 32 + j) = Vec<T, 2>{{s0, s1}};
               } else {
-                T* to = P.gy + static_cast<int64_t>(e0) * S::YD + j;
+                T* to = gy_out + static_cast<int64_t>(e0) * S::YD + j;
                 to[0] = P.acc_y ? to[0] + s0 : s0;
                 if (j + 1 < S::YD) to[1] = P.acc_y ? to[1] + s1 : s1;
               }
@@ -464,7 +507,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
             if (member == 0 && lane < S::YD) {
               T sum = gbuf[flip * 32 + lane];
               for (int m = 1; m < team_warps; ++m) sum += gbuf[m * warp_elems + flip * 32 + lane];
-              T* to = P.gy + static_cast<int64_t>(e0) * S::YD + lane;
+              T* to = gy_out + static_cast<int64_t>(e0) * S::YD + lane;
               *to = P.acc_y ? *to + sum : sum;
             }
             flip ^= 1;
@@ -489,21 +532,22 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       }
       if constexpr (WX) {
         if (grouped) {  // the part goes to shared memory: bulk stores must have read the ring
-          if (leader) bulk_wait_group_read_all();
+          if (issuing) bulk_wait_group_read_all();
           team_sync(team_warps, team);
         }
         if (want_x && active) {
-          T* to = grouped ? ring : P.gx + n * X;
+          T* to = grouped ? ring : P.gx + n * x_row;
+          const int block = grouped ? ch : row_ch, at = grouped ? own : first_ch + own;
           static_for<0, 4>([&](auto l1c) {
             constexpr int l1 = decltype(l1c)::value, d = 2 * l1 + 1;
             if constexpr (S::has(S::MX, l1))
-              lane_store_block<PK, T, d>(to + ch * S::xoff(l1) + own * d, stride, &gxr[S::xoff(l1) * NP],
+              lane_store_block<PK, T, d>(to + block * S::xoff(l1) + at * d, stride, &gxr[S::xoff(l1) * NP],
                                          !grouped && P.acc_x);
           });
         }
       }
     }
-    if (WM && leader) bulk_wait_group_read_all();  // the next rows' copies reuse the stages
+    if (WM && issuing) bulk_wait_group_read_all();  // the next rows' copies reuse the stages
     if constexpr (WX) {
       if (grouped) {  // the parts of the row, in order
         const int barrier = 1 + (team_warps > 1 ? P.teams : 0) + group_id;
@@ -511,11 +555,12 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
         const T* parts = base + static_cast<size_t>(group_id * P.group) * P.team_elems;
         named_barrier(barrier, threads);
         if (want_x) {
-          T* to = P.gx + unit_now * X;
+          T* to = P.gx + unit_now * x_row;
           for (int a = static_cast<int>(threadIdx.x) - group_id * threads; a < X; a += threads) {
             T sum = parts[a];
             for (int q = 1; q < P.group; ++q) sum += parts[static_cast<size_t>(q) * P.team_elems + a];
-            to[a] = P.acc_x ? to[a] + sum : sum;
+            T* put = to + (SLICED ? slice_element<S>(S::MX, a, ch, row_ch, first_ch) : a);
+            *put = P.acc_x ? *put + sum : sum;
           }
         }
         fence_async_shared();  // threads have written and read the ring; its next users are bulk copies
@@ -523,19 +568,19 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       }
     }
   }
-  if (!grouped && member == 0) leave_tiles(P.tile_counters, total, lane);
-  if (WM && leader) bulk_wait_group_read_all();
+  if (!grouped && member == 0) leave_tiles(counters, total, lane);
+  if (WM && issuing) bulk_wait_group_read_all();
   if (!alive) {  // let copies that are still in flight land before the CTA's shared memory is released
     for (int d = 0; d < stages; ++d) edge_wait(&full[d], d < st ? parity : parity ^ 1u, false);
     for (int d = 0; d < K::slots; ++d) edge_wait(&gfull[d], gparity ^ 1u, false);
   }
 }
 
-template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST>
+template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED>
 int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                     const EdgeBackwardArgs& a, cudaStream_t stream) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
-  auto kernel = edge_bwd_kernel<T, CPL, S, WX, WM, WY, FULL, DST>;
+  auto kernel = edge_bwd_kernel<T, CPL, S, WX, WM, WY, FULL, DST, SLICED>;
   const EdgePlan& ep = plan->edge;
   EdgeBwdParams<T> P;
   P.x = static_cast<const T*>(DST ? a.g : a.x);
@@ -555,14 +600,24 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.status = dt.status;
   P.tile_counters = next_tile_counters(plan, dt);
   P.num_rows = !DST && graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;
-  P.ch = ep.ch;
+  P.ch = ep.ch / ep.slices;
+  P.row_ch = ep.ch;
   P.team_warps = ep.team_warps;
   P.need_w = a.gx != nullptr || a.gy != nullptr;
   P.acc_x = a.acc_x;
   P.acc_y = a.acc_y;
   P.acc_w = a.acc_w;
-  const size_t w_row = static_cast<size_t>(S::paths) * ep.ch * sizeof(T);
-  const size_t x_row = static_cast<size_t>(S::XD) * ep.ch * sizeof(T), g_row = static_cast<size_t>(S::OD) * ep.ch * sizeof(T);
+  P.gy_part = graph->num_edges * S::YD;
+  if (SLICED && WY) {
+    const int64_t need = ep.slices * P.gy_part * static_cast<int64_t>(sizeof(T));
+    if (a.scratch == nullptr || a.scratch_bytes < need)
+      return fail(LUNA_ERR_SCRATCH, "backward needs %lld bytes of scratch for the slices' parts of gy", static_cast<long long>(need));
+    if (!aligned_to(a.scratch, 16)) return fail(LUNA_ERR_MISALIGNED, "scratch must be 16-byte aligned");
+    P.gy = static_cast<T*>(a.scratch);
+    P.acc_y = 0;
+  }
+  const size_t w_row = static_cast<size_t>(S::paths) * P.ch * sizeof(T);
+  const size_t x_row = static_cast<size_t>(S::XD) * P.ch * sizeof(T), g_row = static_cast<size_t>(S::OD) * P.ch * sizeof(T);
   EdgeLaunch launch;
   const int max_teams = capped_warps(plan->tuning, K::max_warps) / ep.team_warps;
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
@@ -586,10 +641,11 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.teams = launch.warps / ep.team_warps;
   const int64_t edges = graph->num_edges;
   P.rows_per_edge = static_cast<float>(static_cast<double>(P.num_rows) / static_cast<double>(std::max<int64_t>(edges, 1)));
-  EdgeSplit cut = edge_split(P.num_rows, edges, dt.sm_count, P.teams, ep.team_warps);
+  const int ctas = SLICED ? slice_ctas(dt.sm_count, ep.slices) : dt.sm_count;
+  EdgeSplit cut = edge_split(P.num_rows, edges, ctas, P.teams, ep.team_warps);
   P.group = cut.group;
   P.tile_rows = cut.tile_rows;
-  P.tile_edges = tile_edges_for(edges, static_cast<int64_t>(dt.sm_count) * P.teams, edges_per_warp(plan->tuning, 64));
+  P.tile_edges = tile_edges_for(edges, static_cast<int64_t>(ctas) * P.teams, edges_per_warp(plan->tuning, 64));
   P.num_tiles = ceil_div(std::max<int64_t>(P.num_rows, 1), P.tile_rows);
   // A whole graph of some density, or a shard of one (its own rows plus a halo at most half as large), has hardly any
   // rows without edges, and tiles of a fixed number of rows are even without any search.  A piece of a graph (a
@@ -599,19 +655,25 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   if (P.group == 1 && !(whole && static_cast<double>(edges) >= 8.0 * static_cast<double>(P.num_rows))) {
     P.tile_rows = 0;
     P.num_tiles = ceil_div(std::max<int64_t>(edges, 1), P.tile_edges);
-    cut.blocks = std::max<int64_t>(1, std::min<int64_t>(dt.sm_count, ceil_div(P.num_tiles, P.teams)));
+    cut.blocks = std::max<int64_t>(1, std::min<int64_t>(ctas, ceil_div(P.num_tiles, P.teams)));
     if (a.gx && !a.acc_x)
       LUNA_CUDA_CHECK(cudaMemsetAsync(a.gx, 0, static_cast<size_t>(P.num_rows) * plan->X * sizeof(T), stream));
   }
   static KernelSetup setup;
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
   if (rc != LUNA_OK) return rc;
-  kernel<<<static_cast<unsigned>(cut.blocks), launch.warps * 32, launch.bytes, stream>>>(P);
+  const dim3 grid(static_cast<unsigned>(cut.blocks), static_cast<unsigned>(ep.slices));
+  kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
   LUNA_LAUNCH_CHECK("backward (edge family)");
+  if (SLICED && WY) {
+    reduce_gy_partial<T><<<static_cast<unsigned>(ceil_div(P.gy_part, 256)), 256, 0, stream>>>(
+        P.gy, static_cast<T*>(a.gy), P.gy_part, ep.slices, a.acc_y ? 1 : 0);
+    LUNA_LAUNCH_CHECK("sum of the slices' parts of gy");
+  }
   return LUNA_OK;
 }
 
-template <typename T, int CPL, typename S, bool FULL>
+template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                       const EdgeBackwardArgs& a, cudaStream_t stream) {
   const bool wx = a.gx != nullptr, ww = a.gw != nullptr, wy = a.gy != nullptr;
@@ -620,11 +682,11 @@ int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const l
   if (!wx && ww != wy) {
     constexpr bool dst = S::OD >= S::XD;
     using R = std::conditional_t<dst, Transposed<S>, S>;
-    return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst>(plan, dt, graph, a, stream)
-              : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst>(plan, dt, graph, a, stream);
+    return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED>(plan, dt, graph, a, stream)
+              : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst, SLICED>(plan, dt, graph, a, stream);
   }
-  if (wy) return launch_edge_bwd<T, CPL, S, true, true, true, FULL, false>(plan, dt, graph, a, stream);
-  if (wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false>(plan, dt, graph, a, stream);
+  if (wy) return launch_edge_bwd<T, CPL, S, true, true, true, FULL, false, SLICED>(plan, dt, graph, a, stream);
+  if (wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false, SLICED>(plan, dt, graph, a, stream);
   return LUNA_OK;
 }
 

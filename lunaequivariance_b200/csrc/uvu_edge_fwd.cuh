@@ -22,7 +22,8 @@ struct EdgeFwdParams {
   int* status;
   unsigned* tile_counters;
   int64_t num_rows, tile_rows, num_tiles;
-  int ch;          // channels per block
+  int ch;          // channels per block, or of a slice of it
+  int row_ch;      // channels per block
   int team_warps;  // warps per team
   int teams;       // per CTA
   int group;       // teams that share a row, 1: tiles
@@ -40,8 +41,8 @@ struct EdgeFwd {
   static constexpr size_t warp_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
 };
 
-// FULL: one warp per edge and 32 * CPL channels, known to the compiler.
-template <typename T, int CPL, typename S, bool FULL>
+// FULL: one warp per edge and 32 * CPL channels, known to the compiler.  SLICED: these are a slice of wider blocks.
+template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     edge_fwd_kernel(const __grid_constant__ EdgeFwdParams<T> P) {
   using K = EdgeFwd<T, CPL, S>;
@@ -55,6 +56,10 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   const int ch = FULL ? 32 * CPL : P.ch, stages = P.stages;
   const int W = S::paths * ch, X = S::XD * ch, O = S::OD * ch;
   const int stage_elems = W + X;
+  static_assert(FULL || !SLICED, "a slice is one warp's full set of channels");
+  const int row_ch = SLICED ? P.row_ch : ch, first_ch = SLICED ? static_cast<int>(blockIdx.y) * ch : 0;
+  const int w_row = S::paths * row_ch, x_row = S::XD * row_ch, o_row = S::OD * row_ch;  // in memory
+  unsigned* const counters = P.tile_counters + (SLICED ? 2 * blockIdx.y : 0);
 
   T* ring = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(team) * P.ring_elems;
   T* mbuf = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(P.teams) * P.ring_elems +
@@ -78,12 +83,29 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   const int own = FULL ? PK::W * lane : member * cpw + PK::W * min(lane, lanes - 1);  // first channel of this lane
   const bool active = FULL || lane < lanes;
   const bool leader = member == 0 && lane == 0;
+  const bool issuing = SLICED || leader;  // the pieces of a slice are copied by all lanes
   const uint32_t w_bytes = static_cast<uint32_t>(W * sizeof(T)), x_bytes = static_cast<uint32_t>(X * sizeof(T));
-  auto issue = [&](int64_t e, int s_node, int s) {  // leader only
+  auto issue = [&](int64_t e, int s_node, int s) {  // by the issuing lanes
     T* to = ring + static_cast<size_t>(s) * stage_elems;
-    mbar_arrive_expect_tx(&bars[s], w_bytes + x_bytes);
-    bulk_copy_g2s_hint(to, P.w + e * W, w_bytes, &bars[s], l2_policy_evict_first());
-    bulk_copy_g2s(to + W, P.x + static_cast<int64_t>(s_node) * X, x_bytes, &bars[s]);
+    if constexpr (SLICED) {
+      if (lane == 0) mbar_arrive_expect_tx(&bars[s], w_bytes + x_bytes);
+      __syncwarp();
+      for (int p = lane; p < S::paths; p += 32)
+        bulk_copy_g2s_hint(to + p * ch, P.w + e * w_row + p * row_ch + first_ch, static_cast<uint32_t>(ch * sizeof(T)), &bars[s],
+                           l2_policy_evict_first());
+      static_for<0, 4>([&](auto lc) {
+        constexpr int l = decltype(lc)::value, d = 2 * l + 1;
+        if constexpr (S::has(S::MX, l)) {
+          if (lane == l)
+            bulk_copy_g2s(to + W + ch * S::xoff(l), P.x + static_cast<int64_t>(s_node) * x_row + row_ch * S::xoff(l) + first_ch * d,
+                          static_cast<uint32_t>(ch * d * sizeof(T)), &bars[s]);
+        }
+      });
+    } else {
+      mbar_arrive_expect_tx(&bars[s], w_bytes + x_bytes);
+      bulk_copy_g2s_hint(to, P.w + e * W, w_bytes, &bars[s], l2_policy_evict_first());
+      bulk_copy_g2s(to + W, P.x + static_cast<int64_t>(s_node) * X, x_bytes, &bars[s]);
+    }
   };
 
   V acc[S::OD * NP];
@@ -126,9 +148,9 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     int64_t n = unit, n_hi = unit + 1;
     if (!grouped) {
       if (team_warps == 1) {
-        unit_after = take_tile(P.tile_counters, total, lane);
+        unit_after = take_tile(counters, total, lane);
       } else {
-        if (leader) tickets[team] = atomicAdd(&P.tile_counters[0], 1u);
+        if (leader) tickets[team] = atomicAdd(&counters[0], 1u);
         team_sync(team_warps, team);
         unit_after = total + static_cast<int64_t>(tickets[team]);
         team_sync(team_warps, team);
@@ -143,14 +165,14 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
       e_end = first + count * (in_group + 1) / P.group;
     }
     // all stages are empty here: fill them in ring order from the current one
-    if (leader) {
+    if (issuing) {
       for (int d = 0, stage = s; d < stages; ++d) {
         if (e + d < e_end) issue(e + d, P.src[e + d], stage);
         if (++stage == stages) stage = 0;
       }
     }
     // source node of the edge that is issued in the next iteration, attributes of the next edge
-    int src_ahead = leader && e + stages < e_end ? P.src[e + stages] : 0;
+    int src_ahead = issuing && e + stages < e_end ? P.src[e + stages] : 0;
     T y_next = lane < S::YD && e < e_end ? P.y[e * S::YD + lane] : T(0);
     program.run(y_next, mbuf + buf * K::m_elems, lane);
     if (lane < S::YD && e + 1 < e_end) y_next = P.y[(e + 1) * S::YD + lane];
@@ -190,7 +212,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         });
         buf ^= 1;
         team_sync(team_warps, team);  // every lane is done with this stage and with the matrices
-        if (leader && e + stages < e_end) {
+        if (issuing && e + stages < e_end) {
           issue(e + stages, src_ahead, s);
           if (e + stages + 1 < e_end) src_ahead = P.src[e + stages + 1];
         }
@@ -200,11 +222,12 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         }
       }
       if (active) {
-        T* to = grouped ? ring : P.out + n * O;
+        T* to = grouped ? ring : P.out + n * o_row;
+        const int block = grouped ? ch : row_ch, at = grouped ? own : first_ch + own;
         static_for<0, 4>([&](auto l3c) {
           constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
           if constexpr (S::has(S::MO, l3))
-            lane_store_block<PK, T, d3>(to + ch * S::ooff(l3) + own * d3, stride, &acc[S::ooff(l3) * NP],
+            lane_store_block<PK, T, d3>(to + block * S::ooff(l3) + at * d3, stride, &acc[S::ooff(l3) * NP],
                                         !grouped && P.accumulate);
         });
       }
@@ -214,27 +237,28 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
       const int threads = P.group * team_warps * 32;
       const T* parts = reinterpret_cast<const T*>(smem_raw) + static_cast<size_t>(group_id * P.group) * P.ring_elems;
       named_barrier(barrier, threads);
-      T* to = P.out + unit * O;
+      T* to = P.out + unit * o_row;
       for (int a = static_cast<int>(threadIdx.x) - group_id * threads; a < O; a += threads) {
         T sum = parts[a];
         for (int g = 1; g < P.group; ++g) sum += parts[static_cast<size_t>(g) * P.ring_elems + a];
-        to[a] = P.accumulate ? to[a] + sum : sum;
+        T* put = to + (SLICED ? slice_element<S>(S::MO, a, ch, row_ch, first_ch) : a);
+        *put = P.accumulate ? *put + sum : sum;
       }
       fence_async_shared();  // threads have written and read the ring; its next users are bulk copies
       named_barrier(barrier, threads);
     }
     unit = unit_after;
   }
-  if (!grouped && member == 0) leave_tiles(P.tile_counters, total, lane);
+  if (!grouped && member == 0) leave_tiles(counters, total, lane);
   if (!alive)  // let copies that are still in flight land before the CTA's shared memory is released
     for (int d = 0; d < stages; ++d) edge_wait(&bars[d], d < s ? parity : parity ^ 1u, false);
 }
 
-template <typename T, int CPL, typename S, bool FULL>
+template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                     const EdgeForwardArgs& a, cudaStream_t stream) {
   using K = EdgeFwd<T, CPL, S>;
-  auto kernel = edge_fwd_kernel<T, CPL, S, FULL>;
+  auto kernel = edge_fwd_kernel<T, CPL, S, FULL, SLICED>;
   const EdgePlan& ep = plan->edge;
   EdgeFwdParams<T> P;
   P.x = static_cast<const T*>(a.x);
@@ -248,11 +272,12 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.status = dt.status;
   P.tile_counters = next_tile_counters(plan, dt);
   P.num_rows = graph->num_nodes;
-  P.ch = ep.ch;
+  P.ch = ep.ch / ep.slices;
+  P.row_ch = ep.ch;
   P.team_warps = ep.team_warps;
   P.accumulate = a.accumulate ? 1 : 0;
-  const size_t stage = static_cast<size_t>(S::paths + S::XD) * ep.ch * sizeof(T);
-  const size_t row = static_cast<size_t>(S::OD) * ep.ch * sizeof(T);
+  const size_t stage = static_cast<size_t>(S::paths + S::XD) * P.ch * sizeof(T);
+  const size_t row = static_cast<size_t>(S::OD) * P.ch * sizeof(T);
   EdgeLaunch launch;
   const int max_teams = capped_warps(plan->tuning, K::max_warps) / ep.team_warps;
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
@@ -269,14 +294,16 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   if (launch.warps == 0) return LUNA_ERR_UNSUPPORTED;
   P.stages = launch.stages;
   P.teams = launch.warps / ep.team_warps;
-  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, dt.sm_count, P.teams, ep.team_warps);
+  const int ctas = SLICED ? slice_ctas(dt.sm_count, ep.slices) : dt.sm_count;
+  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, ep.team_warps);
   P.group = split.group;
   P.tile_rows = split.tile_rows;
   P.num_tiles = ceil_div(std::max<int64_t>(graph->num_nodes, 1), split.tile_rows);
   static KernelSetup setup;
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
   if (rc != LUNA_OK) return rc;
-  kernel<<<static_cast<unsigned>(split.blocks), launch.warps * 32, launch.bytes, stream>>>(P);
+  const dim3 grid(static_cast<unsigned>(split.blocks), static_cast<unsigned>(ep.slices));
+  kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
   LUNA_LAUNCH_CHECK("forward (edge family)");
   return LUNA_OK;
 }

@@ -11,9 +11,12 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::forward(const luna
                                                                       const luna_graph* graph, const EdgeForwardArgs& a,
                                                                       cudaStream_t stream) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
+  if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
+    if (plan->edge.slices > 1) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, a, stream);
+  }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true>(plan, dt, graph, a, stream);
-  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false>(plan, dt, graph, a, stream);
+    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, a, stream);
+  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, a, stream);
 }
 
 template <>
@@ -21,9 +24,12 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const lun
                                                                        const luna_graph* graph, const EdgeBackwardArgs& a,
                                                                        cudaStream_t stream) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
+  if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
+    if (plan->edge.slices > 1) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, a, stream);
+  }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true>(plan, dt, graph, a, stream);
-  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false>(plan, dt, graph, a, stream);
+    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, a, stream);
+  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, a, stream);
 }
 
 }  // namespace edgek

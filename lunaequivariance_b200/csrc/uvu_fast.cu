@@ -113,8 +113,10 @@ int64_t fast_smem_bytes(const luna_uvu_plan* plan, int which) {
   return static_cast<int64_t>(r.block_bytes);
 }
 
-// Per-chunk partial rows of gy when the channels of a block are split over several warps.
+// Partial rows of gy when the channels of a block are split over several launches or warps.
 int64_t fast_scratch_bytes(const luna_uvu_plan* plan, int64_t, int64_t num_edges) {
+  if (plan->edge.shape >= 0 && plan->edge.slices > 1 && !plan->force_generic)
+    return plan->edge.slices * num_edges * plan->Y * (plan->dtype == LUNA_F64 ? 8 : 4);
   if (!plan->fast_ok || plan->force_generic || plan->fast.chunks <= 1) return 0;
   const int64_t elem = plan->dtype == LUNA_F64 ? 8 : 4;
   return static_cast<int64_t>(plan->fast.chunks) * num_edges * plan->Y * elem;
@@ -172,7 +174,7 @@ int fast_backward(luna_uvu_plan* plan, const luna_graph* graph, const void* x, c
   int rc = get_device_tables(plan, &dt);
   if (rc != LUNA_OK) return rc;
   if (plan->edge.shape >= 0)
-    return edgek::backward(plan, *dt, graph, x, y, w, g, gx, acc_x, gy, acc_y, gw, acc_w, stream);
+    return edgek::backward(plan, *dt, graph, x, y, w, g, gx, acc_x, gy, acc_y, gw, acc_w, scratch, scratch_bytes, stream);
   const int cpl = plan->fast.cpl;
   if (plan->dtype == LUNA_F64) {
     auto X = static_cast<const double*>(x), Y = static_cast<const double*>(y), W = static_cast<const double*>(w);

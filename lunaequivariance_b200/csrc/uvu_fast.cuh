@@ -265,6 +265,17 @@ __device__ __forceinline__ void leave_tiles(unsigned* counters, int64_t total_wa
 }
 #endif
 
+// gy[e, j] (+)= sum over channel chunks or slices of the partial rows.
+template <typename T>
+__global__ void reduce_gy_partial(const T* __restrict__ partial, T* __restrict__ gy, int64_t count, int chunks,
+                                  int accumulate) {
+  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (idx >= count) return;
+  T acc = accumulate ? gy[idx] : T(0);
+  for (int c = 0; c < chunks; ++c) acc += partial[static_cast<int64_t>(c) * count + idx];
+  gy[idx] = acc;
+}
+
 // Edges per tile for the kernels that hand out tiles dynamically: `wanted` (64 unless overridden), but small enough
 // that every resident warp gets about eight tiles, so that a small launch (a piece of a shard, a small graph) does
 // not end with most warps idle while a few finish their last tile; never below 16 edges.

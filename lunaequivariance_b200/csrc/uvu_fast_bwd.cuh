@@ -453,18 +453,6 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) fast_bwd_kernel(const __grid_
   }
 }
 
-// gy[e, j] (+)= sum over channel chunks of the partial rows.
-template <typename T>
-__global__ void reduce_gy_partial(const T* __restrict__ partial, T* __restrict__ gy, int64_t count, int chunks,
-                                  int accumulate) {
-  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= count) return;
-  T acc = accumulate ? gy[idx] : T(0);
-  for (int c = 0; c < chunks; ++c) acc += partial[static_cast<int64_t>(c) * count + idx];
-  gy[idx] = acc;
-}
-
-
 template <typename T, int CPL, int LX, int LO>
 int launch_fast_bwd_one(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const T* x,
                         const T* y, const T* w, const T* g, T* gx, bool acc_x, T* gy, bool acc_y, T* gw, bool acc_w,

@@ -43,6 +43,7 @@ def check(shape, mul, dtype, nodes, edges, skew, seed):
     module.op.check_status()
     for key, value in dict(out=result, gx=gx, gy=gy, gw=gw, hx=hx, hy=hy, hw=hw, hg=hg).items():
         assert_close(value, ref[key], dtype, f"{shape} x{mul} {dtype} {key}")
+    return module
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
@@ -61,10 +62,47 @@ def test_channel_counts(mul, dtype):
     check(SHAPES[4], mul, dtype, 60, 90, 1.0, mul + 1)
 
 
+# one, two and four channels per lane (FP64: one and two)
+@pytest.mark.parametrize("shape,mul,dtype", [
+    (3, 352, torch.float32), (3, 576, torch.float32), (3, 864, torch.float32), (4, 544, torch.float32),
+    (4, 1024, torch.float32), (5, 640, torch.float32), (5, 704, torch.float32), (6, 352, torch.float32),
+    (6, 768, torch.float32), (3, 288, torch.float64), (4, 512, torch.float64), (5, 288, torch.float64),
+    (5, 320, torch.float64), (6, 384, torch.float64), (6, 416, torch.float64)])
+def test_wide_blocks_in_slices(shape, mul, dtype):
+    check(SHAPES[shape], mul, dtype, 7, 120, 0.0, mul)  # long rows: shared by teams
+    module = check(SHAPES[shape], mul, dtype, 40, 60, 1.0, mul + 1)  # short rows: tiles
+    assert module.op._plan.query(8) == 1  # the slices' parts of dL/dy
+    one_gradient_alone(SHAPES[shape], mul, dtype, 40, 90, 1.0, mul + 2)
+
+
 @pytest.mark.parametrize("nodes,edges", [(1, 1), (1, 2), (1, 77), (2, 9), (3, 1000), (700, 4000), (1300, 5300)])
 def test_row_splits(nodes, edges):
     for mul in (16, 128):
         check(SHAPES[3], mul, torch.float32, nodes, edges, 0.0, nodes + edges)
+
+
+def one_gradient_alone(shape, mul, dtype, nodes, edges, skew, seed):
+    in1, in2, out = irreps(mul, shape[0]), irreps(1, shape[1]), irreps(mul, shape[2])
+    instructions = all_paths(in1, in2, out)
+    module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False,
+                                    dtype=dtype)
+    meta = oracle_conv.build_specs(in1, in2, out, instructions)
+    generator = torch.Generator().manual_seed(seed)
+    src, dst = skewed_graph(nodes, edges, generator, skew)
+    p = random_problem((meta["in1_dim"], meta["in2_dim"], meta["out_dim"], meta["weight_numel"]), nodes, src, dtype,
+                       generator)
+    ref = oracle_conv.conv_derivatives(meta, *(p[k].double() for k in ("x", "y", "w")), src, dst, nodes,
+                                       p["g"].double(), p["rx"].double(), p["ry"].double(), None)
+    graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+    x, y, w, g = (p[k].to(DEVICE).requires_grad_(True) for k in ("x", "y", "w", "g"))
+    result = module(x, y, w, graph=graph)
+    (gw,) = torch.autograd.grad(result, w, g, retain_graph=True)
+    (gy,) = torch.autograd.grad(result, y, g, retain_graph=True)
+    gx, gy_too = torch.autograd.grad(result, (x, y), g, create_graph=True)
+    (hw,) = torch.autograd.grad((gx, gy_too), w, (p["rx"].to(DEVICE), p["ry"].to(DEVICE)))
+    module.op.check_status()
+    for key, value in dict(gw=gw, gy=gy, hw=hw).items():
+        assert_close(value, ref[key], dtype, f"{shape} x{mul} {dtype} {key} alone")
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
@@ -73,27 +111,7 @@ def test_one_gradient_alone(shape, dtype):
     """dL/dw alone and dL/dy alone, whose rows may be the destinations, and two tangents added into one dL/dw; rows shared
     by teams, and tiles with rows without edges."""
     for mul, nodes, edges, skew in ((32, 29, 400, 0.0), (48, 150, 190, 1.5), (160, 40, 130, 1.0)):
-        in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
-        instructions = all_paths(in1, in2, out)
-        module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False,
-                                        dtype=dtype)
-        meta = oracle_conv.build_specs(in1, in2, out, instructions)
-        generator = torch.Generator().manual_seed(100 + shape)
-        src, dst = skewed_graph(nodes, edges, generator, skew)
-        p = random_problem((meta["in1_dim"], meta["in2_dim"], meta["out_dim"], meta["weight_numel"]), nodes, src, dtype,
-                           generator)
-        ref = oracle_conv.conv_derivatives(meta, *(p[k].double() for k in ("x", "y", "w")), src, dst, nodes,
-                                           p["g"].double(), p["rx"].double(), p["ry"].double(), None)
-        graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
-        x, y, w, g = (p[k].to(DEVICE).requires_grad_(True) for k in ("x", "y", "w", "g"))
-        result = module(x, y, w, graph=graph)
-        (gw,) = torch.autograd.grad(result, w, g, retain_graph=True)
-        (gy,) = torch.autograd.grad(result, y, g, retain_graph=True)
-        gx, gy_too = torch.autograd.grad(result, (x, y), g, create_graph=True)
-        (hw,) = torch.autograd.grad((gx, gy_too), w, (p["rx"].to(DEVICE), p["ry"].to(DEVICE)))
-        module.op.check_status()
-        for key, value in dict(gw=gw, gy=gy, hw=hw).items():
-            assert_close(value, ref[key], dtype, f"{SHAPES[shape]} x{mul} {dtype} {key} alone")
+        one_gradient_alone(SHAPES[shape], mul, dtype, nodes, edges, skew, 100 + shape)
 
 
 def term_by_term(meta, x, y, w, g, src, dst):
