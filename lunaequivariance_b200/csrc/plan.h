@@ -154,13 +154,19 @@ struct DeviceTables {
   int max_smem_optin = 0;
 };
 
+// How the channels of a block are dealt out by an edge kernel.
+struct EdgeLanes {
+  int cpl = 0;         // channels per lane
+  int team_warps = 0;  // warps that share an edge
+  int slices = 1;      // parts of a block's channels that are launched side by side
+};
+
 // What the edge kernels (uvu_edge.cuh) need of a plan whose path list has one of their compiled shapes.
 struct EdgePlan {
   int shape = -1;      // index of the compiled shape, -1 if the plan has none or is kept from its kernels
   int ch = 0;          // channels per block
-  int cpl = 0;         // channels per lane
-  int team_warps = 0;  // warps that share an edge
-  int slices = 1;      // parts of a block's channels that are launched side by side
+  EdgeLanes lanes;
+  EdgeLanes lanes_all;  // of backward calls that want dL/dy and another gradient
   // [0] of the shape, [1] of the shape with x and out exchanged
   std::vector<double> prog_c[2], term_c[2];
   std::vector<unsigned short> prog_j[2];

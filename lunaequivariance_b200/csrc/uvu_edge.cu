@@ -1,5 +1,5 @@
 // Which plans the edge kernels serve, the tables they read, and the choice of the compiled instance.
-#include "uvu_edge.cuh"
+#include "uvu_edge_bwd.cuh"
 
 #include <utility>
 
@@ -8,37 +8,44 @@ namespace edgek {
 
 namespace {
 
-// Channels per lane and warps per team: a warp's pass over an edge costs about one unit of fixed work plus one per
-// channel of a lane, so 48 channels take one warp with two channels on 24 lanes, 96 one warp with four on 24 lanes.
-bool choose_lanes(luna_uvu_plan* plan, int ch) {
-  const int widest = plan->dtype == LUNA_F64 ? 2 : 4;
-  int best = 0;
-  for (int cpl = widest; cpl >= 1; cpl /= 2) {
-    if (plan->tuning.lane_channels > 0 && cpl != plan->tuning.lane_channels) continue;
-    const int team = (ch + 32 * cpl - 1) / (32 * cpl);
-    if (team > 8 || ch % (team * cpl) != 0) continue;
-    const int cost = team * (1 + cpl);
-    if (best != 0 && cost >= best) continue;
-    best = cost;
-    plan->edge.cpl = cpl;
-    plan->edge.team_warps = team;
-  }
-  return best != 0;
+// Whether the kernel of all gradients spills registers.
+template <typename T, int CPL, int... ID>
+bool spills(int shape, std::integer_sequence<int, ID...>) {
+  bool found = false;
+  ((found = found || (shape == ID && EdgeBwd<T, CPL, ShapeOf<ID>, true, true, true>::registers > 255)), ...);
+  return found;
+}
+bool spills(const luna_uvu_plan* plan, int shape, int cpl) {
+  constexpr std::make_integer_sequence<int, kEdgeShapes> all{};
+  if (plan->dtype == LUNA_F64) return cpl == 2 ? spills<double, 2>(shape, all) : spills<double, 1>(shape, all);
+  return cpl == 4 ? spills<float, 4>(shape, all) : (cpl == 2 ? spills<float, 2>(shape, all) : spills<float, 1>(shape, all));
 }
 
-// Slices for blocks that no team takes: the most channels per lane that cut a block evenly.  300 MB of weights, 20 edges per
-// node, forward / backward against the table kernels: degrees (2, 3, 3), FP32, 352 channels 0.37 / 1.41 -> 0.18 / 0.46 ms,
-// 1,024 channels 0.24 / 1.03 -> 0.12 / 0.26; (3, 3, 3), FP64, 288 channels 0.39 / 1.14 -> 0.18 / 0.47.
-bool choose_slices(luna_uvu_plan* plan, int ch) {
+// Channels per lane and warps per team, or slices for blocks that no team takes.  A warp's pass over an edge costs about one
+// unit of fixed work plus one per channel of a lane, so 48 channels take one warp with two channels on 24 lanes, 96 one warp
+// with four on 24 lanes.  A kernel that spills counts half as much again: degrees (3, 3, 3) with the most channels per lane,
+// all gradients.  300 MB of weights, FP64: 96 channels 0.64 -> 0.52 ms with one channel per lane, 224 channels 0.72 -> 0.49;
+// FP32: 128 channels 0.41 -> 0.30 with two, 256 channels 0.57 -> 0.34.
+EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, bool all_gradients, bool sliced) {
+  const int ch = plan->edge.ch, elem = plan->dtype == LUNA_F64 ? 8 : 4;
+  // one team with two stages must fit an SM's shared memory in either direction
+  const size_t room = 200 * 1024, W = static_cast<size_t>(plan->W) * elem, X = static_cast<size_t>(plan->X) * elem,
+               O = static_cast<size_t>(plan->O) * elem;
+  const size_t rows = std::max(std::max(2 * W + O, 2 * (W + X)), std::max(X, O));
+  EdgeLanes best;
+  double best_cost = 0.0;
   for (int cpl = plan->dtype == LUNA_F64 ? 2 : 4; cpl >= 1; cpl /= 2) {
     if (plan->tuning.lane_channels > 0 && cpl != plan->tuning.lane_channels) continue;
-    if (ch % (32 * cpl) != 0 || ch / (32 * cpl) > kEdgeMaxSlices) continue;
-    plan->edge.cpl = cpl;
-    plan->edge.team_warps = 1;
-    plan->edge.slices = ch / (32 * cpl);
-    return true;
+    const int parts = (ch + 32 * cpl - 1) / (32 * cpl);
+    if (sliced ? ch % (32 * cpl) != 0 || parts > kEdgeMaxSlices
+               : parts > 8 || ch % (parts * cpl) != 0 || rows + parts * 8192 > room)
+      continue;
+    const double cost = parts * (1 + cpl) * (all_gradients && spills(plan, shape, cpl) ? 1.5 : 1.0);
+    if (best.cpl != 0 && cost >= best_cost) continue;
+    best_cost = cost;
+    best = sliced ? EdgeLanes{cpl, 1, parts} : EdgeLanes{cpl, parts, 1};
   }
-  return false;
+  return best;
 }
 
 // Exchanging x and out turns the pattern of a coupling into that of the exchanged degrees.
@@ -140,43 +147,46 @@ int with_shape(int shape, F&& body) {
   }
 }
 template <typename F>
-int with_instance(const luna_uvu_plan* plan, F&& body) {
-  const EdgePlan& ep = plan->edge;
+int with_instance(const luna_uvu_plan* plan, const EdgeLanes& lanes, F&& body) {
+  const int shape = plan->edge.shape;
   if (plan->dtype == LUNA_F64)
-    return ep.cpl == 2 ? with_shape<double, 2, 0>(ep.shape, body) : with_shape<double, 1, 0>(ep.shape, body);
-  if (ep.cpl == 4) return with_shape<float, 4, 0>(ep.shape, body);
-  return ep.cpl == 2 ? with_shape<float, 2, 0>(ep.shape, body) : with_shape<float, 1, 0>(ep.shape, body);
+    return lanes.cpl == 2 ? with_shape<double, 2, 0>(shape, body) : with_shape<double, 1, 0>(shape, body);
+  if (lanes.cpl == 4) return with_shape<float, 4, 0>(shape, body);
+  return lanes.cpl == 2 ? with_shape<float, 2, 0>(shape, body) : with_shape<float, 1, 0>(shape, body);
 }
 
 }  // namespace
 
+// Slices pay against the table kernels: 300 MB of weights, 20 edges per node, forward / backward, degrees (2, 3, 3), FP32, 352
+// channels 0.37 / 1.41 -> 0.18 / 0.46 ms, 1,024 channels 0.24 / 1.03 -> 0.12 / 0.26; (3, 3, 3), FP64, 288 channels
+// 0.39 / 1.14 -> 0.18 / 0.47.
 void analyse(luna_uvu_plan* plan) {
   plan->edge = EdgePlan{};
   if (plan->paths.empty() || plan->tuning.no_canon) return;
-  const int ch = plan->paths[0].ch;
   const int elem = plan->dtype == LUNA_F64 ? 8 : 4;
-  if (ch * elem % 16 != 0) return;  // bulk copies move whole 16-byte pieces
-  // one team with two stages must fit an SM's shared memory in either direction
-  const size_t room = 200 * 1024, W = static_cast<size_t>(plan->W) * elem, X = static_cast<size_t>(plan->X) * elem,
-               O = static_cast<size_t>(plan->O) * elem;
-  const bool whole = choose_lanes(plan, ch) && std::max(std::max(2 * W + O, 2 * (W + X)), std::max(X, O)) +
-                                                       plan->edge.team_warps * 8192 <= room;
-  if (!whole && !choose_slices(plan, ch)) return;
+  if (plan->paths[0].ch * elem % 16 != 0) return;  // bulk copies move whole 16-byte pieces
   const int shape = find_shape<0>(plan);
-  if (shape >= 0 && (whole || edge_sliced(shape))) plan->edge.shape = shape;
+  if (shape < 0) return;
+  const bool sliced = choose_lanes(plan, shape, false, false).cpl == 0;
+  if (sliced && !edge_sliced(shape)) return;
+  plan->edge.lanes = choose_lanes(plan, shape, false, sliced);
+  plan->edge.lanes_all = choose_lanes(plan, shape, true, sliced);
+  if (plan->edge.lanes.cpl != 0) plan->edge.shape = shape;
 }
 
 int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
             const void* w, void* out, bool accumulate, cudaStream_t stream) {
   const EdgeForwardArgs args{x, y, w, out, accumulate};
-  return with_instance(plan, [&](auto kernels) { return kernels.forward(plan, dt, graph, args, stream); });
+  const EdgeLanes& lanes = plan->edge.lanes;
+  return with_instance(plan, lanes, [&](auto kernels) { return kernels.forward(plan, dt, graph, lanes, args, stream); });
 }
 
 int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
              const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w, void* scratch,
              int64_t scratch_bytes, cudaStream_t stream) {
   const EdgeBackwardArgs args{x, y, w, g, gx, gy, gw, acc_x, acc_y, acc_w, scratch, scratch_bytes};
-  return with_instance(plan, [&](auto kernels) { return kernels.backward(plan, dt, graph, args, stream); });
+  const EdgeLanes& lanes = gy && (gx || gw) ? plan->edge.lanes_all : plan->edge.lanes;
+  return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
 }
 
 }  // namespace edgek

@@ -133,9 +133,9 @@ struct EdgeBackwardArgs {
 template <typename T, int CPL, int ID>
 struct EdgeKernels {
   static int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
-                     const EdgeForwardArgs& a, cudaStream_t stream);
+                     const EdgeLanes& lanes, const EdgeForwardArgs& a, cudaStream_t stream);
   static int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
-                      const EdgeBackwardArgs& a, cudaStream_t stream);
+                      const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream);
 };
 
 // ---- how a launch is laid out -----------------------------------------------------------------------------------------

@@ -64,7 +64,8 @@ struct EdgeBwd {
   static constexpr bool shared_program =
       WX && WM && WY && pair == 2 && warps_for(state + program_regs + 48) == 12 && warps_for(state + 48) == 16;
   using Program = std::conditional_t<shared_program, SharedMatrixProgram<T, S>, MatrixProgram<T, S>>;
-  static constexpr int max_warps = warps_for(state + (shared_program ? 0 : program_regs) + 48);
+  static constexpr int registers = state + (shared_program ? 0 : program_regs) + 48;  // wanted; beyond 255 it spills
+  static constexpr int max_warps = warps_for(registers);
   // slots of g: the highest degree has one, the others share one
   static constexpr int slot_of(int l3) { return l3 == S::LO && S::ooff(S::LO) > 0 ? 1 : 0; }
   static constexpr int slots = slot_of(S::LO) + 1;
@@ -578,10 +579,9 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
 
 template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED>
 int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
-                    const EdgeBackwardArgs& a, cudaStream_t stream) {
+                    const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
   auto kernel = edge_bwd_kernel<T, CPL, S, WX, WM, WY, FULL, DST, SLICED>;
-  const EdgePlan& ep = plan->edge;
   EdgeBwdParams<T> P;
   P.x = static_cast<const T*>(DST ? a.g : a.x);
   P.y = static_cast<const T*>(a.y);
@@ -600,16 +600,16 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.status = dt.status;
   P.tile_counters = next_tile_counters(plan, dt);
   P.num_rows = !DST && graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;
-  P.ch = ep.ch / ep.slices;
-  P.row_ch = ep.ch;
-  P.team_warps = ep.team_warps;
+  P.ch = plan->edge.ch / lanes.slices;
+  P.row_ch = plan->edge.ch;
+  P.team_warps = lanes.team_warps;
   P.need_w = a.gx != nullptr || a.gy != nullptr;
   P.acc_x = a.acc_x;
   P.acc_y = a.acc_y;
   P.acc_w = a.acc_w;
   P.gy_part = graph->num_edges * S::YD;
   if (SLICED && WY) {
-    const int64_t need = ep.slices * P.gy_part * static_cast<int64_t>(sizeof(T));
+    const int64_t need = lanes.slices * P.gy_part * static_cast<int64_t>(sizeof(T));
     if (a.scratch == nullptr || a.scratch_bytes < need)
       return fail(LUNA_ERR_SCRATCH, "backward needs %lld bytes of scratch for the slices' parts of gy", static_cast<long long>(need));
     if (!aligned_to(a.scratch, 16)) return fail(LUNA_ERR_MISALIGNED, "scratch must be 16-byte aligned");
@@ -619,16 +619,16 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   const size_t w_row = static_cast<size_t>(S::paths) * P.ch * sizeof(T);
   const size_t x_row = static_cast<size_t>(S::XD) * P.ch * sizeof(T), g_row = static_cast<size_t>(S::OD) * P.ch * sizeof(T);
   EdgeLaunch launch;
-  const int max_teams = capped_warps(plan->tuning, K::max_warps) / ep.team_warps;
+  const int max_teams = capped_warps(plan->tuning, K::max_warps) / lanes.team_warps;
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
     for (int option = 0; option < 3; ++option) {  // three or two stages with g in them, or two and g by degree
       const int stages = option == 0 ? 3 : 2, split = option == 2;
       size_t team = split ? stages * w_row + g_row : stages * (w_row + g_row);
       team = (std::max(team, x_row) + 127) / 128 * 128;
       const size_t bytes = teams * (team + (kEdgeMaxStages + kEdgeMaxSlots) * sizeof(uint64_t) + sizeof(unsigned)) +
-                           (static_cast<size_t>(teams) * ep.team_warps * K::warp_elems(ep.team_warps) + K::table_elems) * sizeof(T);
+                           (static_cast<size_t>(teams) * lanes.team_warps * K::warp_elems(lanes.team_warps) + K::table_elems) * sizeof(T);
       if (bytes > static_cast<size_t>(dt.max_smem_optin)) continue;
-      launch.warps = teams * ep.team_warps;
+      launch.warps = teams * lanes.team_warps;
       launch.stages = stages;
       launch.split = split;
       launch.bytes = bytes;
@@ -638,11 +638,11 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   if (launch.warps == 0) return LUNA_ERR_UNSUPPORTED;
   P.stages = launch.stages;
   P.split = launch.split;
-  P.teams = launch.warps / ep.team_warps;
+  P.teams = launch.warps / lanes.team_warps;
   const int64_t edges = graph->num_edges;
   P.rows_per_edge = static_cast<float>(static_cast<double>(P.num_rows) / static_cast<double>(std::max<int64_t>(edges, 1)));
-  const int ctas = SLICED ? slice_ctas(dt.sm_count, ep.slices) : dt.sm_count;
-  EdgeSplit cut = edge_split(P.num_rows, edges, ctas, P.teams, ep.team_warps);
+  const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
+  EdgeSplit cut = edge_split(P.num_rows, edges, ctas, P.teams, lanes.team_warps);
   P.group = cut.group;
   P.tile_rows = cut.tile_rows;
   P.tile_edges = tile_edges_for(edges, static_cast<int64_t>(ctas) * P.teams, edges_per_warp(plan->tuning, 64));
@@ -662,12 +662,12 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   static KernelSetup setup;
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
   if (rc != LUNA_OK) return rc;
-  const dim3 grid(static_cast<unsigned>(cut.blocks), static_cast<unsigned>(ep.slices));
+  const dim3 grid(static_cast<unsigned>(cut.blocks), static_cast<unsigned>(lanes.slices));
   kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
   LUNA_LAUNCH_CHECK("backward (edge family)");
   if (SLICED && WY) {
     reduce_gy_partial<T><<<static_cast<unsigned>(ceil_div(P.gy_part, 256)), 256, 0, stream>>>(
-        P.gy, static_cast<T*>(a.gy), P.gy_part, ep.slices, a.acc_y ? 1 : 0);
+        P.gy, static_cast<T*>(a.gy), P.gy_part, lanes.slices, a.acc_y ? 1 : 0);
     LUNA_LAUNCH_CHECK("sum of the slices' parts of gy");
   }
   return LUNA_OK;
@@ -675,18 +675,18 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
 
 template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
-                      const EdgeBackwardArgs& a, cudaStream_t stream) {
+                      const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
   const bool wx = a.gx != nullptr, ww = a.gw != nullptr, wy = a.gy != nullptr;
   // One gradient per edge and none per row.  FP64, degrees (2, 3, 3), 128 channels, 1.05 M edges: rows by source 5.91 ms
   // (gw) and 6.44 ms (gy), by destination 5.36 and 5.95 ms.
   if (!wx && ww != wy) {
     constexpr bool dst = S::OD >= S::XD;
     using R = std::conditional_t<dst, Transposed<S>, S>;
-    return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED>(plan, dt, graph, a, stream)
-              : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst, SLICED>(plan, dt, graph, a, stream);
+    return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED>(plan, dt, graph, lanes, a, stream)
+              : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst, SLICED>(plan, dt, graph, lanes, a, stream);
   }
-  if (wy) return launch_edge_bwd<T, CPL, S, true, true, true, FULL, false, SLICED>(plan, dt, graph, a, stream);
-  if (wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false, SLICED>(plan, dt, graph, a, stream);
+  if (wy) return launch_edge_bwd<T, CPL, S, true, true, true, FULL, false, SLICED>(plan, dt, graph, lanes, a, stream);
+  if (wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false, SLICED>(plan, dt, graph, lanes, a, stream);
   return LUNA_OK;
 }
 

@@ -256,10 +256,9 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
 
 template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
-                    const EdgeForwardArgs& a, cudaStream_t stream) {
+                    const EdgeLanes& lanes, const EdgeForwardArgs& a, cudaStream_t stream) {
   using K = EdgeFwd<T, CPL, S>;
   auto kernel = edge_fwd_kernel<T, CPL, S, FULL, SLICED>;
-  const EdgePlan& ep = plan->edge;
   EdgeFwdParams<T> P;
   P.x = static_cast<const T*>(a.x);
   P.y = static_cast<const T*>(a.y);
@@ -272,20 +271,20 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.status = dt.status;
   P.tile_counters = next_tile_counters(plan, dt);
   P.num_rows = graph->num_nodes;
-  P.ch = ep.ch / ep.slices;
-  P.row_ch = ep.ch;
-  P.team_warps = ep.team_warps;
+  P.ch = plan->edge.ch / lanes.slices;
+  P.row_ch = plan->edge.ch;
+  P.team_warps = lanes.team_warps;
   P.accumulate = a.accumulate ? 1 : 0;
   const size_t stage = static_cast<size_t>(S::paths + S::XD) * P.ch * sizeof(T);
   const size_t row = static_cast<size_t>(S::OD) * P.ch * sizeof(T);
   EdgeLaunch launch;
-  const int max_teams = capped_warps(plan->tuning, K::max_warps) / ep.team_warps;
+  const int max_teams = capped_warps(plan->tuning, K::max_warps) / lanes.team_warps;
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
     for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
       const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
-      const size_t bytes = teams * (ring + ep.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned));
+      const size_t bytes = teams * (ring + lanes.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned));
       if (bytes > static_cast<size_t>(dt.max_smem_optin)) continue;
-      launch.warps = teams * ep.team_warps;
+      launch.warps = teams * lanes.team_warps;
       launch.stages = stages;
       launch.bytes = bytes;
       P.ring_elems = static_cast<int>(ring / sizeof(T));
@@ -293,16 +292,16 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
     }
   if (launch.warps == 0) return LUNA_ERR_UNSUPPORTED;
   P.stages = launch.stages;
-  P.teams = launch.warps / ep.team_warps;
-  const int ctas = SLICED ? slice_ctas(dt.sm_count, ep.slices) : dt.sm_count;
-  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, ep.team_warps);
+  P.teams = launch.warps / lanes.team_warps;
+  const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
+  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps);
   P.group = split.group;
   P.tile_rows = split.tile_rows;
   P.num_tiles = ceil_div(std::max<int64_t>(graph->num_nodes, 1), split.tile_rows);
   static KernelSetup setup;
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
   if (rc != LUNA_OK) return rc;
-  const dim3 grid(static_cast<unsigned>(split.blocks), static_cast<unsigned>(ep.slices));
+  const dim3 grid(static_cast<unsigned>(split.blocks), static_cast<unsigned>(lanes.slices));
   kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
   LUNA_LAUNCH_CHECK("forward (edge family)");
   return LUNA_OK;

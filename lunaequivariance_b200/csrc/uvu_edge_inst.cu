@@ -8,28 +8,28 @@ namespace edgek {
 
 template <>
 int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::forward(const luna_uvu_plan* plan, const DeviceTables& dt,
-                                                                      const luna_graph* graph, const EdgeForwardArgs& a,
+                                                                      const luna_graph* graph, const EdgeLanes& lanes, const EdgeForwardArgs& a,
                                                                       cudaStream_t stream) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
   if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
-    if (plan->edge.slices > 1) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, a, stream);
+    if (lanes.slices > 1) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, lanes, a, stream);
   }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, a, stream);
-  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, a, stream);
+    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, lanes, a, stream);
+  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, lanes, a, stream);
 }
 
 template <>
 int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const luna_uvu_plan* plan, const DeviceTables& dt,
-                                                                       const luna_graph* graph, const EdgeBackwardArgs& a,
+                                                                       const luna_graph* graph, const EdgeLanes& lanes, const EdgeBackwardArgs& a,
                                                                        cudaStream_t stream) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
   if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
-    if (plan->edge.slices > 1) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, a, stream);
+    if (lanes.slices > 1) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, lanes, a, stream);
   }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, a, stream);
-  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, a, stream);
+    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, lanes, a, stream);
+  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, lanes, a, stream);
 }
 
 }  // namespace edgek

@@ -115,8 +115,8 @@ int64_t fast_smem_bytes(const luna_uvu_plan* plan, int which) {
 
 // Partial rows of gy when the channels of a block are split over several launches or warps.
 int64_t fast_scratch_bytes(const luna_uvu_plan* plan, int64_t, int64_t num_edges) {
-  if (plan->edge.shape >= 0 && plan->edge.slices > 1 && !plan->force_generic)
-    return plan->edge.slices * num_edges * plan->Y * (plan->dtype == LUNA_F64 ? 8 : 4);
+  if (plan->edge.shape >= 0 && plan->edge.lanes.slices > 1 && !plan->force_generic)
+    return std::max(plan->edge.lanes.slices, plan->edge.lanes_all.slices) * num_edges * plan->Y * (plan->dtype == LUNA_F64 ? 8 : 4);
   if (!plan->fast_ok || plan->force_generic || plan->fast.chunks <= 1) return 0;
   const int64_t elem = plan->dtype == LUNA_F64 ? 8 : 4;
   return static_cast<int64_t>(plan->fast.chunks) * num_edges * plan->Y * elem;
