@@ -122,7 +122,8 @@ typedef struct {
   const int32_t* edge_ids_by_src; /* [E] */
 } luna_graph;
 
-/* Bytes of scratch the backward / double-backward entry points need for this plan and graph size (may be 0). */
+/* Bytes of scratch the backward / double-backward entry points need for this plan and graph size when they produce gy.
+ * 0 unless the plan's blocks are so wide that their channels are split over several launches' or warps' partial rows. */
 LUNA_API int64_t luna_uvu_conv_scratch_bytes(const luna_uvu_plan* plan, int64_t num_nodes, int64_t num_edges);
 
 /* out[N, out_dim] = sum over incoming edges of the weighted coupled product.  Replaces forward.run

@@ -67,7 +67,7 @@ extern "C" int64_t luna_uvu_plan_query(const luna_uvu_plan* plan, int what) {
     case LUNA_PLAN_CANONICAL_L2: return plan->fast_ok ? plan->fast.canon_l2 : -1;
     case LUNA_PLAN_SPARSE_TERMS: return plan->fast_ok ? plan->fast.sparse_terms : 0;
     case LUNA_PLAN_BWD_VARIANT: return fast_bwd_variant(plan);
-    case LUNA_PLAN_NEEDS_SCRATCH: return (plan->edge.shape < 0 || plan->edge.lanes.slices > 1) && fast_scratch_bytes(plan, 1, 1) > 0;
+    case LUNA_PLAN_NEEDS_SCRATCH: return fast_scratch_bytes(plan, 1, 1) > 0;
     default: return -1;
   }
 }

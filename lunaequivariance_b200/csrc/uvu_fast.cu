@@ -113,13 +113,16 @@ int64_t fast_smem_bytes(const luna_uvu_plan* plan, int which) {
   return static_cast<int64_t>(r.block_bytes);
 }
 
-// Partial rows of gy when the channels of a block are split over several launches or warps.
+// Partial rows of gy when the channels of a block are split over several launches or warps: edge kernels in slices, or table
+// kernels in channel chunks, whichever serve the plan.
 int64_t fast_scratch_bytes(const luna_uvu_plan* plan, int64_t, int64_t num_edges) {
-  if (plan->edge.shape >= 0 && plan->edge.lanes.slices > 1 && !plan->force_generic)
-    return std::max(plan->edge.lanes.slices, plan->edge.lanes_all.slices) * num_edges * plan->Y * (plan->dtype == LUNA_F64 ? 8 : 4);
-  if (!plan->fast_ok || plan->force_generic || plan->fast.chunks <= 1) return 0;
-  const int64_t elem = plan->dtype == LUNA_F64 ? 8 : 4;
-  return static_cast<int64_t>(plan->fast.chunks) * num_edges * plan->Y * elem;
+  if (plan->force_generic) return 0;
+  int64_t parts = 1;
+  if (plan->edge.shape >= 0)
+    parts = std::max(plan->edge.lanes.slices, plan->edge.lanes_all.slices);
+  else if (plan->fast_ok)
+    parts = plan->fast.chunks;
+  return parts > 1 ? parts * num_edges * plan->Y * (plan->dtype == LUNA_F64 ? 8 : 4) : 0;
 }
 
 int fast_forward(luna_uvu_plan* plan, const luna_graph* graph, const void* x, const void* y, const void* w,

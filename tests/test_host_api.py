@@ -205,3 +205,21 @@ def test_default_build_leaves_line_tables_out():
 
     assert "-lineinfo" not in build.NVCC_FLAGS
     assert os.path.getsize(_native.LIBRARY_PATH) < 100 << 20
+
+
+def test_scratch_is_asked_for_only_where_it_is_used(monkeypatch):
+    from tests.helpers import all_paths, config
+
+    def plan(in1, in2, out, instructions, dtype):
+        op = luna.prepare_tensor_product(in1, in2, out, instructions, convolution=True, dtype=dtype)
+        return op, _native.library().luna_uvu_conv_scratch_bytes(op._plan.handle, 100, 1000), op._plan.query(8)
+
+    cfg2 = config("cfg2")[:4]
+    wide = ("352x0e+352x1o", "1x0e+1x1o", "352x0e+352x1o")
+    op, size, needs = plan(*cfg2, torch.float64)  # one team of warps takes the 128 channels
+    assert (op.backward_variant, size, needs) == ("row", 0, 0)
+    op, size, needs = plan(*wide, all_paths(*wide), torch.float32)  # eleven slices
+    assert (op.backward_variant, size, needs) == ("row", 11 * 1000 * 4 * 4, 1)
+    monkeypatch.setenv("LUNA_B200_NO_CANON", "1")
+    op, size, needs = plan(*cfg2, torch.float64)  # two channel chunks of the table kernels
+    assert (op.backward_variant, size, needs) == ("tables", 2 * 1000 * 16 * 8, 1)

@@ -3,10 +3,11 @@
 Some embedders of the library cannot give the backward pass a scratch buffer because they cannot allocate device
 memory at the point where they call it (a plugin inside another program's step, a loop that must avoid
 ``cudaMalloc``'s device-wide synchronisation, a process with a closed memory pool).  For them the library carries
-an 8 MiB array of its own.  These tests call that entry point through the C-ABI on a configuration whose backward
-pass really uses scratch (128 channels in FP64 are split over two warps), twice in a row because the array is
-shared between calls and keeps the previous call's contents, and compare with ``luna_uvu_conv_bwd``.  This file
-is collected last so that a run that stops at the first failure has already run everything else.
+an 8 MiB array of its own.  These tests call that entry point through the C-ABI on configurations whose backward
+pass really uses scratch (the kernels that read the path list from tables split 128 channels in FP64 over two warps;
+the edge kernels, which would serve these lists otherwise, need none), twice in a row because the array is shared
+between calls and keeps the previous call's contents, and compare with ``luna_uvu_conv_bwd``.  This file is collected
+last so that a run that stops at the first failure has already run everything else.
 """
 
 import ctypes
@@ -47,7 +48,12 @@ def call_noalloc(op, graph, x, y, w, g):
     return status, (gx, gy, gw)
 
 
-def test_noalloc_backward_matches_regular_entry_point_twice():
+@pytest.fixture()
+def table_kernels(monkeypatch):
+    monkeypatch.setenv("LUNA_B200_NO_CANON", "1")  # read when a plan is created
+
+
+def test_noalloc_backward_matches_regular_entry_point_twice(table_kernels):
     dtype = torch.float64
     conv = make_conv("cfg2", dtype)
     op = conv.op
@@ -79,7 +85,7 @@ def test_noalloc_backward_matches_regular_entry_point_twice():
     _native.check(lib.luna_uvu_check_status(op._plan.handle, None))
 
 
-def test_noalloc_refuses_instead_of_allocating():
+def test_noalloc_refuses_instead_of_allocating(table_kernels):
     dtype = torch.float32
     conv = make_conv("wide", dtype)  # 256 channels in FP32: two chunks, 32 bytes of scratch per edge
     op = conv.op
@@ -121,3 +127,20 @@ def test_noalloc_refuses_instead_of_allocating():
     torch.cuda.synchronize()
     for name, a, b in zip(("gx", "gy", "gw"), got, want):
         assert_close(a, b.detach().cpu(), dtype, f"noalloc wide {name}")
+
+
+@pytest.mark.parametrize("name,dtype,nodes,edges", [("wide", torch.float32, 4096, 270_000), ("cfg2", torch.float64, 900, 33_000)])
+def test_noalloc_takes_any_graph_where_no_scratch_is_used(name, dtype, nodes, edges):
+    """The edge kernels sum dL/dy within a team of warps: graphs that are beyond the array in the table kernels."""
+    conv = make_conv(name, dtype)
+    lib = _native.library()
+    assert conv.op.backward_variant == "row"
+    assert lib.luna_uvu_conv_scratch_bytes(conv.op._plan.handle, nodes, edges) == 0
+    graph, (x, y, w, g) = problem(conv, nodes, edges, dtype, 9)
+    with torch.cuda.device(DEVICE):
+        _native.check(lib.luna_uvu_conv_noalloc_prepare(conv.op._plan.handle))
+    status, got = call_noalloc(conv.op, graph, x, y, w, g)
+    _native.check(status)
+    want = conv_mod.run_backward(conv.op, x, y, w, g, graph)
+    for key, a, b in zip(("gx", "gy", "gw"), got, want):
+        assert_close(a, b.detach().cpu(), dtype, f"noalloc {name} {key}")
