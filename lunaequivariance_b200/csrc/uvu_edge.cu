@@ -38,7 +38,7 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, bool all_gradients,
     if (plan->tuning.lane_channels > 0 && cpl != plan->tuning.lane_channels) continue;
     const int parts = (ch + 32 * cpl - 1) / (32 * cpl);
     if (sliced ? ch % (32 * cpl) != 0 || parts > kEdgeMaxSlices
-               : parts > 8 || ch % (parts * cpl) != 0 || rows + parts * 8192 > room)
+               : parts > capped_warps(plan->tuning, 8) || ch % (parts * cpl) != 0 || rows + parts * 8192 > room)
       continue;
     const double cost = parts * (1 + cpl) * (all_gradients && spills(plan, shape, cpl) ? 1.5 : 1.0);
     if (best.cpl != 0 && cost >= best_cost) continue;

@@ -175,7 +175,7 @@ constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
 // Small launches.  With R rows of d edges and T teams on the chip, a row per team takes d * ceil(R / T) edge steps of
 // the last team; parts of a row per team take about d * R / T.  Sharing costs two barriers and a pass through shared
 // memory per row, so it stops where the tiles of the large launches are even enough.
-inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps) {
+inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps, int64_t wanted_tile) {
   EdgeSplit s;
   const int64_t all = static_cast<int64_t>(sm_count) * teams;
   const double degree = static_cast<double>(edges) / static_cast<double>(std::max<int64_t>(rows, 1));
@@ -190,7 +190,7 @@ inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams
     s.blocks = std::max<int64_t>(1, std::min<int64_t>(sm_count, rows));
     return s;
   }
-  const int64_t tile_edges = tile_edges_for(edges, all, 64);
+  const int64_t tile_edges = tile_edges_for(edges, all, wanted_tile);
   s.tile_rows = std::min<int64_t>(1 << 20, std::max<int64_t>(1, static_cast<int64_t>(tile_edges / std::max(degree, 1e-3) + 0.5)));
   const int64_t tiles = ceil_div(std::max<int64_t>(rows, 1), s.tile_rows);
   s.blocks = std::max<int64_t>(1, std::min<int64_t>(sm_count, ceil_div(tiles, teams)));

@@ -635,17 +635,18 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
       P.team_elems = static_cast<int>(team / sizeof(T));
       break;
     }
-  if (launch.warps == 0) return LUNA_ERR_UNSUPPORTED;
+  if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
   P.split = launch.split;
   P.teams = launch.warps / lanes.team_warps;
   const int64_t edges = graph->num_edges;
   P.rows_per_edge = static_cast<float>(static_cast<double>(P.num_rows) / static_cast<double>(std::max<int64_t>(edges, 1)));
   const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
-  EdgeSplit cut = edge_split(P.num_rows, edges, ctas, P.teams, lanes.team_warps);
+  const int64_t tile = edges_per_warp(plan->tuning, 64);
+  EdgeSplit cut = edge_split(P.num_rows, edges, ctas, P.teams, lanes.team_warps, tile);
   P.group = cut.group;
   P.tile_rows = cut.tile_rows;
-  P.tile_edges = tile_edges_for(edges, static_cast<int64_t>(ctas) * P.teams, edges_per_warp(plan->tuning, 64));
+  P.tile_edges = tile_edges_for(edges, static_cast<int64_t>(ctas) * P.teams, tile);
   P.num_tiles = ceil_div(std::max<int64_t>(P.num_rows, 1), P.tile_rows);
   // A whole graph of some density, or a shard of one (its own rows plus a halo at most half as large), has hardly any
   // rows without edges, and tiles of a fixed number of rows are even without any search.  A piece of a graph (a

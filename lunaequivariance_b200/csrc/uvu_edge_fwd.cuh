@@ -290,11 +290,11 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
       P.ring_elems = static_cast<int>(ring / sizeof(T));
       break;
     }
-  if (launch.warps == 0) return LUNA_ERR_UNSUPPORTED;
+  if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
   P.teams = launch.warps / lanes.team_warps;
   const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
-  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps);
+  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps, 64);
   P.group = split.group;
   P.tile_rows = split.tile_rows;
   P.num_tiles = ceil_div(std::max<int64_t>(graph->num_nodes, 1), split.tile_rows);

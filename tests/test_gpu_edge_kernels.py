@@ -75,6 +75,16 @@ def test_wide_blocks_in_slices(shape, mul, dtype):
     one_gradient_alone(SHAPES[shape], mul, dtype, 40, 90, 1.0, mul + 2)
 
 
+@pytest.mark.parametrize("knob,shape,mul,dtype", [
+    ("LUNA_B200_MAXW=1", 3, 160, torch.float32), ("LUNA_B200_MAXW=1", 6, 128, torch.float64),
+    ("LUNA_B200_MAXW=3", 4, 256, torch.float32), ("LUNA_B200_EPW=1", 4, 64, torch.float32)])
+def test_tuning_settings(knob, shape, mul, dtype, monkeypatch):
+    """Fewer warps than a team would have, and tiles of other sizes, on the same kernels."""
+    monkeypatch.setenv(*knob.split("="))
+    check(SHAPES[shape], mul, dtype, 23, 260, 0.0, mul)
+    check(SHAPES[shape], mul, dtype, 3000, 26000 if mul == 64 else 3100, 0.0, mul + 1)
+
+
 @pytest.mark.parametrize("nodes,edges", [(1, 1), (1, 2), (1, 77), (2, 9), (3, 1000), (700, 4000), (1300, 5300)])
 def test_row_splits(nodes, edges):
     for mul in (16, 128):
