@@ -240,29 +240,22 @@ std::array<Tensor, N> spread(const variable_list& list, int mask) {
 }
 Tensor contiguous(const Tensor& t) { return t.defined() ? t.contiguous() : t; }
 
-// dF/d(operand `slot`), slots 0..3 = x, y, w, g; a, b, c: the other three operands in that order.
+// dF/d(operand `slot`), slots 0..3 = x, y, w, g; a, b, c: the other three operands in that order.  The kernels take all four
+// operands and look at the shape of the free slot's only: `free` lends it (none for g).
 struct ConvPartial : Function<ConvPartial> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& a, const Tensor& b, const Tensor& c, int64_t slot, const OpPtr& op,
-                        const GraphPtr& graph) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& a, const Tensor& b, const Tensor& c,
+                        const std::optional<Tensor>& free, int64_t slot, const OpPtr& op, const GraphPtr& graph) {
     ctx->set_materialize_grads(false);
     ctx->save_for_backward({a, b, c});
     ctx->saved_data["slot"] = slot;
     keep(ctx, "op", op);
     keep(ctx, "graph", graph);
-    const auto full = operands({a, b, c}, slot, Tensor());
-    if (slot == 3) return run_forward(*op, *graph, full[0], full[1], full[2]);
-    // the kernels take all four operands; the one in the free slot is only looked at for its shape
-    const at::TensorOptions options = a.options();
-    const luna_graph& n = graph->native;
-    Tensor stand_in;
-    if (slot == 0) stand_in = at::empty({n.num_src_nodes, op->X}, options);
-    if (slot == 1) stand_in = at::empty({n.num_edges, op->Y}, options);
-    if (slot == 2) stand_in = at::empty({n.num_edges, op->W}, options);
-    const auto all = operands({a, b, c}, slot, stand_in);
+    const auto all = operands({a, b, c}, slot, free ? *free : Tensor());
+    if (slot == 3) return run_forward(*op, *graph, all[0], all[1], all[2]);
     return run_backward(*op, *graph, all[0], all[1], all[2], all[3], 1 << slot)[slot];
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
-    variable_list out(6);
+    variable_list out(7);
     if (!grads[0].defined()) return out;
     const auto saved = ctx->get_saved_variables();
     const int64_t slot = ctx->saved_data["slot"].toInt();
@@ -286,7 +279,9 @@ struct ConvPartial : Function<ConvPartial> {
     std::array<Tensor, 3> others;
     for (int64_t s = 0, next = 0; s < 4; ++s)
       if (s != slot) others[next++] = full[s];
-    return apply(others[0], others[1], others[2], slot, op, graph);
+    // without history: nothing depends on its values
+    const std::optional<Tensor> free = slot == 3 ? std::nullopt : std::optional<Tensor>(full[slot].detach());
+    return apply(others[0], others[1], others[2], free, slot, op, graph);
   }
 };
 

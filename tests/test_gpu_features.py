@@ -201,3 +201,24 @@ def test_forward_mode_derivatives_are_refused(requires_grad):
         cotangent = forward_ad.make_dual(torch.ones_like(result), torch.ones_like(result))
         with pytest.raises(NotImplementedError):
             torch.autograd.grad(result, operands, cotangent)
+
+
+def test_third_order_allocates_its_results_only():
+    """The kernels look at the shape of the operand they differentiate by; no stand-in of its size is made for it."""
+    in1, in2, out, instructions, options = config("cfg5")
+    module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False, **options)
+    generator = torch.Generator().manual_seed(3)
+    nodes, edges = 500, 9000
+    src, dst = random_graph(nodes, edges, generator)
+    graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+    rand = lambda *shape: torch.randn(*shape, device=DEVICE, requires_grad=True)
+    x, y, w = rand(nodes, module.op.in1_dim), rand(edges, module.op.in2_dim), rand(edges, module.op.weight_numel)
+    result = module(x, y, w, graph=graph)
+    (gy,) = torch.autograd.grad(result, y, rand(*result.shape), create_graph=True)
+    (hx,) = torch.autograd.grad(gy, x, rand(*gy.shape), create_graph=True)
+    bx = torch.randn_like(hx)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    (dw,) = torch.autograd.grad(hx, w, bx)  # one partial derivative
+    assert torch.cuda.max_memory_allocated() - before < 1.25 * dw.numel() * dw.element_size()
