@@ -82,25 +82,26 @@ typedef struct luna_uvu_plan luna_uvu_plan;
 LUNA_API int luna_uvu_plan_create(const luna_uvu_desc* desc, luna_uvu_plan** plan);
 LUNA_API void luna_uvu_plan_destroy(luna_uvu_plan* plan);
 
-/* Plan queries. */
+/* Plan queries.  They describe the kernels that aligned operands get: the edge kernels, for the path lists and channel
+ * counts that these are compiled for, or the staged kernels that read the path list from tables. */
 typedef enum {
-  LUNA_PLAN_FAST_PATH = 0,      /* 1 if the staged (bulk-copy) kernels apply to this configuration */
-  LUNA_PLAN_CHANNELS_PER_LANE = 1,
-  LUNA_PLAN_CHANNEL_CHUNKS = 2,
-  LUNA_PLAN_FWD_SMEM_BYTES = 3,
-  LUNA_PLAN_BWD_SMEM_BYTES = 4,
-  LUNA_PLAN_CANONICAL_L2 = 5,   /* highest edge-attribute degree if the path list is the full list of allowed
-                                   (l1, l2, l3) couplings in standard order (kernels unrolled at compile time), else -1 */
-  LUNA_PLAN_SPARSE_TERMS = 6,   /* > 0 if the plan's coupling terms have the compiled-in non-zero patterns, so the
-                                   backward kernel with per-lane contraction of the edge-attribute gradient applies */
+  LUNA_PLAN_FAST_PATH = 0,      /* 1 if staged (bulk-copy) kernels apply to this configuration */
+  LUNA_PLAN_CHANNELS_PER_LANE = 1, /* of the forward kernel; 0 without staged kernels */
+  LUNA_PLAN_CHANNEL_CHUNKS = 2, /* parts of a block's channels that are launched side by side; 0 without staged kernels */
+  LUNA_PLAN_FWD_SMEM_BYTES = 3, /* shared memory of a block, at most */
+  LUNA_PLAN_BWD_SMEM_BYTES = 4, /* the same for all gradients */
+  LUNA_PLAN_CANONICAL_L2 = 5,   /* highest edge-attribute degree if the path list is every allowed (l1, l2, l3) coupling
+                                   of the degrees 0..LX, 0..L2 and 0..LO, in this order, else -1 */
+  LUNA_PLAN_SPARSE_TERMS = 6,   /* > 0 if the path list is such a list and has its coupling patterns compiled in */
   LUNA_PLAN_BWD_VARIANT = 7,    /* which first-order backward kernel aligned inputs get: a luna_bwd_variant */
   LUNA_PLAN_NEEDS_SCRATCH = 8   /* 1 if backward calls that produce gy use the scratch buffer, 0 if they take none */
 } luna_plan_query;
 typedef enum {
   LUNA_BWD_TABLE_DRIVEN = 0, /* one thread per output element, any configuration */
   LUNA_BWD_STAGED_TABLES = 1, /* staged kernel that reads the path list from tables */
-  LUNA_BWD_ROW_STAGES = 2,    /* compiled-in coupling patterns, one warp per edge, whole weight rows staged */
-  LUNA_BWD_UNIT_RING = 3      /* compiled-in coupling patterns, one warp per edge, (edge, degree) units in a ring */
+  LUNA_BWD_ROW_STAGES = 2     /* edge kernels: path list and coupling patterns compiled in, a team of warps per edge, whole
+                                 weight rows (or a slice's part of them) staged */
+  LUNA_BWD_UNIT_RING = 3      /* of earlier builds; does not occur */
 } luna_bwd_variant;
 LUNA_API int64_t luna_uvu_plan_query(const luna_uvu_plan* plan, int what);
 

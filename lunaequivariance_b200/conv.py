@@ -162,14 +162,14 @@ class LunaTPUVUConv:
 
     @property
     def uses_compiled_patterns(self) -> bool:
-        """Whether the backward kernel with compiled-in coupling patterns applies."""
+        """Whether the path list is the full list of allowed couplings and runs kernels that have it compiled in."""
         return self._plan.query(6) > 0
 
     @property
     def backward_variant(self) -> str:
         """Which first-order backward kernel aligned inputs get: ``generic`` (table-driven), ``tables`` (staged,
-        path list read from tables), ``row`` or ``units`` (compiled-in coupling patterns)."""
-        return ("generic", "tables", "row", "units")[self._plan.query(7)]
+        path list read from tables) or ``row`` (edge kernels: path list and coupling patterns compiled in)."""
+        return ("generic", "tables", "row")[self._plan.query(7)]
 
     def check_status(self, device=None) -> None:
         """Raise ``RuntimeError`` if a kernel of this operator gave up a bounded wait since the last check.

@@ -58,14 +58,16 @@ int zero_fill(void* p, int64_t numel, size_t elem, cudaStream_t stream) {
 
 extern "C" int64_t luna_uvu_plan_query(const luna_uvu_plan* plan, int what) {
   if (!plan) return -1;
+  const bool edge = plan->edge.shape >= 0;  // else the table kernels, if any staged ones
   switch (what) {
-    case LUNA_PLAN_FAST_PATH: return (plan->fast_ok || plan->edge.shape >= 0) && !plan->force_generic;
-    case LUNA_PLAN_CHANNELS_PER_LANE: return plan->fast_ok ? plan->fast.cpl : 0;
-    case LUNA_PLAN_CHANNEL_CHUNKS: return plan->fast_ok ? plan->fast.chunks : 0;
+    case LUNA_PLAN_FAST_PATH: return (plan->fast_ok || edge) && !plan->force_generic;
+    case LUNA_PLAN_CHANNELS_PER_LANE: return edge ? plan->edge.lanes.cpl : (plan->fast_ok ? plan->fast.cpl : 0);
+    case LUNA_PLAN_CHANNEL_CHUNKS: return edge ? plan->edge.lanes.slices : (plan->fast_ok ? plan->fast.chunks : 0);
     case LUNA_PLAN_FWD_SMEM_BYTES: return fast_smem_bytes(plan, 0);
     case LUNA_PLAN_BWD_SMEM_BYTES: return fast_smem_bytes(plan, 1);
-    case LUNA_PLAN_CANONICAL_L2: return plan->fast_ok ? plan->fast.canon_l2 : -1;
-    case LUNA_PLAN_SPARSE_TERMS: return plan->fast_ok ? plan->fast.sparse_terms : 0;
+    case LUNA_PLAN_CANONICAL_L2: return edge ? edgek::canonical_l2(plan) : (plan->fast_ok ? plan->fast.canon_l2 : -1);
+    case LUNA_PLAN_SPARSE_TERMS:
+      return edge && edgek::canonical_l2(plan) >= 0 ? static_cast<int64_t>(plan->edge.term_c[0].size()) : 0;
     case LUNA_PLAN_BWD_VARIANT: return fast_bwd_variant(plan);
     case LUNA_PLAN_NEEDS_SCRATCH: return fast_scratch_bytes(plan, 1, 1) > 0;
     default: return -1;

@@ -197,37 +197,6 @@ bool fill_layout(luna_uvu_plan* plan, FastMeta& f, int cpl) {
               f.m_off[q] == fastk::canon_moff(f.LX, L2, f.LO, l1, l2, l3);
     }
     if (canon) f.canon_l2 = L2;
-    // sparse term list: every path's terms must have exactly the compiled-in pattern
-    f.sparse_terms = 0;
-    if (canon && L2 <= 3 && f.LX <= 3 && f.LO <= 3) {
-      const int total_terms = fastk::canon_toff(f.LX, L2, f.LO, -1, -1, -1);
-      std::vector<char> seen(static_cast<size_t>(total_terms), 0);
-      bool match = true;
-      for (size_t q = 0; q < order.size() && match; ++q) {
-        const PathRec& p = paths[order[q]];
-        const int l1 = (p.d1 - 1) / 2, l2 = (p.d2 - 1) / 2, l3 = (p.d3 - 1) / 2;
-        const fastk::CgTerm* pattern = fastk::cg_pattern(l1, l2, l3);
-        const int n = fastk::cg_count(l1, l2, l3);
-        const int toff = fastk::canon_toff(f.LX, L2, f.LO, l1, l2, l3);
-        match = pattern != nullptr && p.y_off == l2 * l2;
-        int found = 0;
-        for (int k = 0; k < p.d3 && match; ++k)
-          for (int t = plan->rowptr_k[p.byk_ptr + k]; t < plan->rowptr_k[p.byk_ptr + k + 1] && match; ++t) {
-            const auto& term = plan->terms_k[t];  // (a, b) = (i, j)
-            int slot = -1;
-            for (int u = 0; u < n; ++u)
-              if (pattern[u].i == term.a && pattern[u].j == term.b && pattern[u].k == k) slot = u;
-            if (slot < 0 || seen[toff + slot]) {
-              match = false;
-            } else {
-              seen[toff + slot] = 1;
-              ++found;
-            }
-          }
-        if (found != n) match = false;  // a pattern entry the plan does not have would be a wasted (zero) term
-      }
-      if (match) f.sparse_terms = total_terms;
-    }
   }
 
   // the program in padded (ELL) form for the kernels: term t of entry m at [t * m_total + m], exactly two

@@ -66,8 +66,6 @@ struct CopyPiece {
 struct FastMeta {
   int LX, LO;                 // highest degree present in x / out
   int canon_l2;               // highest edge-harmonic degree if the path list is the canonical full list, else -1
-  int sparse_terms;           // length of the term list (canon_toff total) if the plan's coupling terms have the
-                              // patterns of cg_patterns.h and y is laid out as degrees 0..L2 in order, else 0
   int cpl;                    // channels per lane
   int chunks;                 // channel chunks per feature block (a warp handles 32 * cpl channels)
   int ch;                     // channels per block (uniform)
@@ -260,6 +258,9 @@ int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph*
 int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
              const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w, void* scratch,
              int64_t scratch_bytes, cudaStream_t stream);
+// Of a plan with a shape: the highest edge-attribute degree if its degrees are all of 0..l, else -1; shared memory of a block.
+int canonical_l2(const luna_uvu_plan* plan);
+size_t smem_bytes(const luna_uvu_plan* plan, bool backward, int max_smem);
 }  // namespace edgek
 
 // Staged kernels (bulk-copy pipeline).  fast_available() is false in a build without them.

@@ -189,5 +189,23 @@ int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
 }
 
+int canonical_l2(const luna_uvu_plan* plan) {
+  int top = -1;
+  for (int mask : kEdgeShapeMasks[plan->edge.shape])
+    if ((mask & (mask + 1)) != 0) return -1;
+  for (int mask = kEdgeShapeMasks[plan->edge.shape][1]; mask != 0; mask >>= 1) ++top;
+  return top;
+}
+
+size_t smem_bytes(const luna_uvu_plan* plan, bool backward, int max_smem) {
+  const EdgeLanes& lanes = backward ? plan->edge.lanes_all : plan->edge.lanes;
+  size_t bytes = 0;
+  with_instance(plan, lanes, [&](auto kernels) {
+    bytes = kernels.smem_bytes(plan, lanes, backward, max_smem);
+    return LUNA_OK;
+  });
+  return bytes;
+}
+
 }  // namespace edgek
 }  // namespace luna

@@ -136,6 +136,8 @@ struct EdgeKernels {
                      const EdgeLanes& lanes, const EdgeForwardArgs& a, cudaStream_t stream);
   static int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                       const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream);
+  // shared memory of a block of the forward kernel, or of the backward kernel of all gradients
+  static size_t smem_bytes(const luna_uvu_plan* plan, const EdgeLanes& lanes, bool backward, int max_smem);
 };
 
 // ---- how a launch is laid out -----------------------------------------------------------------------------------------
@@ -144,6 +146,7 @@ struct EdgeLaunch {
   int stages = 0;  // per team
   int split = 0;   // backward: g in one slot per degree instead of in the stages
   size_t bytes = 0;
+  int team_elems = 0;  // of shared memory
 };
 // Rows shared by `group` teams, or 1: rows are handed out in tiles.
 struct EdgeSplit {

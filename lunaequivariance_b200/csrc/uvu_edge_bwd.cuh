@@ -577,6 +577,31 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   }
 }
 
+// K: the EdgeBwd of the kernel.
+template <typename T, typename S, typename K>
+EdgeLaunch edge_bwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch, int max_smem) {
+  const size_t w_row = static_cast<size_t>(S::paths) * ch * sizeof(T);
+  const size_t x_row = static_cast<size_t>(S::XD) * ch * sizeof(T), g_row = static_cast<size_t>(S::OD) * ch * sizeof(T);
+  EdgeLaunch launch;
+  const int max_teams = capped_warps(tuning, K::max_warps) / lanes.team_warps;
+  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
+    for (int option = 0; option < 3; ++option) {  // three or two stages with g in them, or two and g by degree
+      const int stages = option == 0 ? 3 : 2, split = option == 2;
+      size_t team = split ? stages * w_row + g_row : stages * (w_row + g_row);
+      team = (std::max(team, x_row) + 127) / 128 * 128;
+      const size_t bytes = teams * (team + (kEdgeMaxStages + kEdgeMaxSlots) * sizeof(uint64_t) + sizeof(unsigned)) +
+                           (static_cast<size_t>(teams) * lanes.team_warps * K::warp_elems(lanes.team_warps) + K::table_elems) * sizeof(T);
+      if (bytes > static_cast<size_t>(max_smem)) continue;
+      launch.warps = teams * lanes.team_warps;
+      launch.stages = stages;
+      launch.split = split;
+      launch.bytes = bytes;
+      launch.team_elems = static_cast<int>(team / sizeof(T));
+      break;
+    }
+  return launch;
+}
+
 template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED>
 int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                     const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
@@ -616,27 +641,10 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
     P.gy = static_cast<T*>(a.scratch);
     P.acc_y = 0;
   }
-  const size_t w_row = static_cast<size_t>(S::paths) * P.ch * sizeof(T);
-  const size_t x_row = static_cast<size_t>(S::XD) * P.ch * sizeof(T), g_row = static_cast<size_t>(S::OD) * P.ch * sizeof(T);
-  EdgeLaunch launch;
-  const int max_teams = capped_warps(plan->tuning, K::max_warps) / lanes.team_warps;
-  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
-    for (int option = 0; option < 3; ++option) {  // three or two stages with g in them, or two and g by degree
-      const int stages = option == 0 ? 3 : 2, split = option == 2;
-      size_t team = split ? stages * w_row + g_row : stages * (w_row + g_row);
-      team = (std::max(team, x_row) + 127) / 128 * 128;
-      const size_t bytes = teams * (team + (kEdgeMaxStages + kEdgeMaxSlots) * sizeof(uint64_t) + sizeof(unsigned)) +
-                           (static_cast<size_t>(teams) * lanes.team_warps * K::warp_elems(lanes.team_warps) + K::table_elems) * sizeof(T);
-      if (bytes > static_cast<size_t>(dt.max_smem_optin)) continue;
-      launch.warps = teams * lanes.team_warps;
-      launch.stages = stages;
-      launch.split = split;
-      launch.bytes = bytes;
-      P.team_elems = static_cast<int>(team / sizeof(T));
-      break;
-    }
+  const EdgeLaunch launch = edge_bwd_launch<T, S, K>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
   if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
+  P.team_elems = launch.team_elems;
   P.split = launch.split;
   P.teams = launch.warps / lanes.team_warps;
   const int64_t edges = graph->num_edges;

@@ -254,10 +254,31 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     for (int d = 0; d < stages; ++d) edge_wait(&bars[d], d < s ? parity : parity ^ 1u, false);
 }
 
+// As many teams as fit the shared memory with three stages each (two, if they are then more).
+template <typename T, int CPL, typename S>
+EdgeLaunch edge_fwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch, int max_smem) {
+  using K = EdgeFwd<T, CPL, S>;
+  const size_t stage = static_cast<size_t>(S::paths + S::XD) * ch * sizeof(T);
+  const size_t row = static_cast<size_t>(S::OD) * ch * sizeof(T);
+  EdgeLaunch launch;
+  const int max_teams = capped_warps(tuning, K::max_warps) / lanes.team_warps;
+  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
+    for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
+      const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
+      const size_t bytes = teams * (ring + lanes.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned));
+      if (bytes > static_cast<size_t>(max_smem)) continue;
+      launch.warps = teams * lanes.team_warps;
+      launch.stages = stages;
+      launch.bytes = bytes;
+      launch.team_elems = static_cast<int>(ring / sizeof(T));
+      break;
+    }
+  return launch;
+}
+
 template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                     const EdgeLanes& lanes, const EdgeForwardArgs& a, cudaStream_t stream) {
-  using K = EdgeFwd<T, CPL, S>;
   auto kernel = edge_fwd_kernel<T, CPL, S, FULL, SLICED>;
   EdgeFwdParams<T> P;
   P.x = static_cast<const T*>(a.x);
@@ -275,23 +296,10 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.row_ch = plan->edge.ch;
   P.team_warps = lanes.team_warps;
   P.accumulate = a.accumulate ? 1 : 0;
-  const size_t stage = static_cast<size_t>(S::paths + S::XD) * P.ch * sizeof(T);
-  const size_t row = static_cast<size_t>(S::OD) * P.ch * sizeof(T);
-  EdgeLaunch launch;
-  const int max_teams = capped_warps(plan->tuning, K::max_warps) / lanes.team_warps;
-  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
-    for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
-      const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
-      const size_t bytes = teams * (ring + lanes.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned));
-      if (bytes > static_cast<size_t>(dt.max_smem_optin)) continue;
-      launch.warps = teams * lanes.team_warps;
-      launch.stages = stages;
-      launch.bytes = bytes;
-      P.ring_elems = static_cast<int>(ring / sizeof(T));
-      break;
-    }
+  const EdgeLaunch launch = edge_fwd_launch<T, CPL, S>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
   if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
+  P.ring_elems = launch.team_elems;
   P.teams = launch.warps / lanes.team_warps;
   const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
   const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps, 64);

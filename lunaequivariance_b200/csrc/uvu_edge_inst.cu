@@ -32,5 +32,15 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const lun
   return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, lanes, a, stream);
 }
 
+template <>
+size_t EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::smem_bytes(const luna_uvu_plan* plan, const EdgeLanes& lanes,
+                                                                            bool backward, int max_smem) {
+  using S = ShapeOf<LUNA_EDGE_SHAPE>;
+  const int ch = plan->edge.ch / lanes.slices;
+  if (!backward) return edge_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, lanes, ch, max_smem).bytes;
+  using K = EdgeBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>;
+  return edge_bwd_launch<LUNA_EDGE_T, S, K>(plan->tuning, lanes, ch, max_smem).bytes;
+}
+
 }  // namespace edgek
 }  // namespace luna

@@ -85,6 +85,7 @@ constexpr int kSmemLimit = 227 * 1024;
 }
 
 int64_t fast_smem_bytes(const luna_uvu_plan* plan, int which) {
+  if (plan->edge.shape >= 0) return static_cast<int64_t>(edgek::smem_bytes(plan, which != 0, kSmemLimit));
   if (!plan->fast_ok) return 0;
   const FastMeta& f = plan->fast;
   const size_t elem = plan->dtype == LUNA_F64 ? 8 : 4;

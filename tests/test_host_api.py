@@ -223,3 +223,22 @@ def test_scratch_is_asked_for_only_where_it_is_used(monkeypatch):
     monkeypatch.setenv("LUNA_B200_NO_CANON", "1")
     op, size, needs = plan(*cfg2, torch.float64)  # two channel chunks of the table kernels
     assert (op.backward_variant, size, needs) == ("tables", 2 * 1000 * 16 * 8, 1)
+
+
+@pytest.mark.parametrize("mul,lmax,dtype,lanes,chunks", [
+    (48, 2, torch.float32, 2, 1), (64, 2, torch.float32, 2, 1), (128, 3, torch.float64, 2, 1), (352, 1, torch.float32, 1, 11)])
+def test_plan_queries_describe_the_kernels_that_run(mul, lmax, dtype, lanes, chunks):
+    from tests.helpers import all_paths
+
+    block = lambda m, top: "+".join(f"{m}x{l}{'eo'[l % 2]}" for l in range(top + 1))
+    irreps = (block(mul, lmax), block(1, lmax), block(mul, lmax))
+    op = luna.prepare_tensor_product(*irreps, all_paths(*irreps), convolution=True, dtype=dtype)
+    assert op.backward_variant == "row" and op.uses_staged_kernels and op.uses_compiled_patterns
+    assert (op.canonical_l2, op._plan.query(1), op._plan.query(2)) == (lmax, lanes, chunks)
+    row = op.weight_numel // chunks * (8 if dtype == torch.float64 else 4)
+    for smem in (op._plan.query(3), op._plan.query(4)):
+        assert 2 * row < smem <= 227 * 1024
+    # a full list that no kernel has compiled in
+    irreps = (block(64, 1), block(1, 2), block(64, 2))
+    op = luna.prepare_tensor_product(*irreps, all_paths(*irreps), convolution=True, dtype=dtype)
+    assert op.backward_variant == "tables" and op.canonical_l2 == 2 and not op.uses_compiled_patterns
