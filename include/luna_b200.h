@@ -99,7 +99,7 @@ typedef enum {
 typedef enum {
   LUNA_BWD_TABLE_DRIVEN = 0, /* one thread per output element, any configuration */
   LUNA_BWD_STAGED_TABLES = 1, /* staged kernel that reads the path list from tables */
-  LUNA_BWD_ROW_STAGES = 2     /* edge kernels: path list and coupling patterns compiled in, a team of warps per edge, whole
+  LUNA_BWD_ROW_STAGES = 2,    /* edge kernels: path list and coupling patterns compiled in, a team of warps per edge, whole
                                  weight rows (or a slice's part of them) staged */
   LUNA_BWD_UNIT_RING = 3      /* of earlier builds; does not occur */
 } luna_bwd_variant;
