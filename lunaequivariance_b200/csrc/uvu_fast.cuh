@@ -26,7 +26,6 @@
 namespace luna {
 namespace fastk {
 
-constexpr int kWarps = 4;           // default warps per CTA; each warp streams its own edge range
 constexpr int kMaxWarps = 16;       // upper bound on warps per CTA
 constexpr int kFwdMaxWarps = 8;     // forward kernel: its launch bounds leave it 255 registers
 constexpr int kMaxStages = 4;
@@ -78,11 +77,6 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
   uint64_t policy;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-  return policy;
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-  uint64_t policy;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
   return policy;
 }
 __device__ __forceinline__ void bulk_copy_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
@@ -151,22 +145,6 @@ __device__ __forceinline__ void store_vectors_streaming(T* p, const T* flat) {
     } else {
       __stcs(reinterpret_cast<float*>(v + n), *reinterpret_cast<const float*>(&t));
     }
-  }
-}
-
-// Reads a d1 x d3 matrix (row-major, 16-byte aligned, padded to a multiple of 16 bytes) from shared memory with
-// 128-bit loads; every lane reads the same address, so each load is one broadcast.
-template <typename T, int COUNT>
-__device__ __forceinline__ void load_matrix(const T* m, T* regs) {
-  constexpr int per = 16 / sizeof(T);
-  constexpr int nv = (COUNT + per - 1) / per;
-  const Vec<T, per>* v = reinterpret_cast<const Vec<T, per>*>(m);
-#pragma unroll
-  for (int n = 0; n < nv; ++n) {
-    const Vec<T, per> t = v[n];
-#pragma unroll
-    for (int c = 0; c < per; ++c)
-      if (n * per + c < COUNT) regs[n * per + c] = t.a[c];
   }
 }
 
@@ -327,20 +305,6 @@ __host__ __device__ constexpr int canon_moff(int LX, int L2, int LO, int a, int 
   return m;
 }
 
-// first coupling term of the path in the sparse term list: paths in (l3, l1, l2) order, every path's terms (in the
-// (i, k, j) order of CgPattern) padded to a multiple of four; past-the-end arguments give the total
-__host__ __device__ constexpr int canon_toff(int LX, int L2, int LO, int a, int b, int c) {
-  int t = 0;
-  for (int l3 = 0; l3 <= LO; ++l3)
-    for (int l1 = 0; l1 <= LX; ++l1)
-      for (int l2 = 0; l2 <= L2; ++l2) {
-        if (!canon_ok(LX, L2, LO, l1, l2, l3)) continue;
-        if (l1 == a && l2 == b && l3 == c) return t;
-        t += (cg_count(l1, l2, l3) + 3) / 4 * 4;
-      }
-  return t;
-}
-
 // ---- per-edge coupling matrices -------------------------------------------------------------------------------------
 // The program that turns an edge's y row into the M matrices lives in shared memory in padded form: term t of
 // entry m is (ell_c[t * m_total + m], ell_j[t * m_total + m]); padding terms have coefficient 0.
@@ -367,25 +331,11 @@ __device__ __forceinline__ void load_ell(unsigned char* smem, const T* __restric
   __syncthreads();
 }
 
-// mbuf[m] = sum_t c[t][m] * ybuf[j[t][m]]; lanes stride over the entries, conflict-free shared loads.
-template <typename T>
-__device__ __forceinline__ void compute_m(const T* ell_c, const unsigned char* ell_j, int m_terms, const T* ybuf,
-                                          T* mbuf, int m_total, int lane) {
-#pragma unroll 2
-  for (int m = lane; m < m_total; m += 32) {
-    T a = ell_c[m] * ybuf[ell_j[m]];
-    for (int t = 1; t < m_terms; ++t) a = fma(ell_c[t * m_total + m], ybuf[ell_j[t * m_total + m]], a);
-    mbuf[m] = a;
-  }
-}
-
 // FP32 with an even number of channels per lane uses packed two-wide arithmetic; everything else the scalar path.
 template <typename T, int CPL>
 struct UsePairs {
   static constexpr bool value = sizeof(T) == 4 && (CPL % 2 == 0);
 };
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 
 // One warp's share of the coupling-matrix computation when `parts` warps split the entries: warp `part` handles
 // entries (r * parts + part) * 32 + lane.  Two entries per trip with all loads issued before the arithmetic;

@@ -8,8 +8,7 @@ namespace fastk {
 
 // ---- arithmetic packets ---------------------------------------------------------------------------------------------
 // A lane's CPL channels are processed as NP packets of W channels: FP32 pairs with packed two-wide FMAs when CPL is
-// even, scalars otherwise.  Coupling-matrix entries are stored W times in shared memory so that one load fills a
-// packet.  A pair lives in one 64-bit register from the load to the last use (the packed instructions take 64-bit
+// even, scalars otherwise.  A pair lives in one 64-bit register from the load to the last use (the packed instructions take 64-bit
 // operands; keeping the halves as separate floats costs a register move per operand).
 struct Pair {
   unsigned long long v;
@@ -78,23 +77,7 @@ __device__ __forceinline__ V zero_packet() {
   }
 }
 
-// Memory row [channel][component] (CPL x D, this lane's channels) -> packets [component][packet].
-template <typename PK, typename T, int CPL, int D>
-__device__ __forceinline__ void load_packets(const T* p, typename PK::V* out) {
-  using V = typename PK::V;
-  constexpr int W = PK::W, NP = PK::NP;
-  T row[CPL * D];
-  load_vectors<T, CPL, D>(p, row);
-#pragma unroll
-  for (int i = 0; i < D; ++i)
-#pragma unroll
-    for (int q = 0; q < NP; ++q) {
-      T vals[W];
-#pragma unroll
-      for (int c = 0; c < W; ++c) vals[c] = row[(q * W + c) * D + i];
-      out[i * NP + q] = make_packet(vals, V{});
-    }
-}
+// Packets [component][packet] -> memory row [channel][component] (CPL x D, this lane's channels).
 template <typename PK, typename T, int CPL, int D>
 __device__ __forceinline__ void unpack_packets(const typename PK::V* in, T* row) {
   constexpr int W = PK::W, NP = PK::NP;
@@ -124,33 +107,6 @@ __device__ __forceinline__ void load_lane_packets(const T* p, typename PK::V* ou
     load_vectors<T, CPL, 1>(p, out);
   }
 }
-
-// One row of a coupling matrix (D3P entries, each stored W times) from shared memory; every lane reads the same
-// address, so each load is one broadcast.  Rows start on 16-byte boundaries except in FP32 without duplication (8).
-template <typename T, int W, int D3P, typename V>
-__device__ __forceinline__ void load_matrix_row(const T* p, V* row) {
-  if constexpr (W == 2) {  // two packets per 128-bit load
-    static_assert(D3P % 2 == 0, "row length must be even");
-    const ulonglong2* v = reinterpret_cast<const ulonglong2*>(p);
-#pragma unroll
-    for (int n = 0; n < D3P / 2; ++n) {
-      const ulonglong2 t = v[n];
-      row[2 * n].v = t.x;
-      row[2 * n + 1].v = t.y;
-    }
-  } else {
-    constexpr int per = (sizeof(T) == 4 ? 8 : 16) / sizeof(T);
-    static_assert(D3P % per == 0, "row length must be a whole number of vectors");
-    const Vec<T, per>* v = reinterpret_cast<const Vec<T, per>*>(p);
-#pragma unroll
-    for (int n = 0; n < D3P / per; ++n) {
-      const Vec<T, per> t = v[n];
-#pragma unroll
-      for (int c = 0; c < per; ++c) row[n * per + c] = t.a[c];
-    }
-  }
-}
-
 
 // ---- helpers of the kernels that keep the coupling matrices unduplicated -----------------------------------------
 // A scalar as a packet with both halves equal.  The assembler folds this move into the broadcast operand form of
