@@ -219,15 +219,15 @@ def test_input_validation_errors():
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 @pytest.mark.parametrize("name", ["cfg2", "cfg5", "cfg4"])
-@pytest.mark.parametrize("knob", ["LUNA_B200_NO_CANON=1", "LUNA_B200_NO_SPARSE=1", "LUNA_B200_BWD_KERNEL=row",
-                                  "LUNA_B200_BWD_KERNEL=units", "LUNA_B200_NO_PLAIN=1"])
-def test_staged_kernel_variants_match_oracle(name, dtype, knob, monkeypatch):
-    """The canonical configurations through the kernels they do not all take by default: loops over run-time path
-    tables (NO_CANON), the unrolled kernel with dense coupling matrices (NO_SPARSE), and the two data-movement
-    variants of the backward kernel with compiled-in coupling patterns (row stages / unit ring)."""
+@pytest.mark.parametrize("knob,variant", [("LUNA_B200_NO_CANON=1", "tables"), ("LUNA_B200_LANE_CHANNELS=1", "row"),
+                                          ("LUNA_B200_LANE_CHANNELS=2", "row"), ("LUNA_B200_MAXW=2", "row")])
+def test_staged_kernel_variants_match_oracle(name, dtype, knob, variant, monkeypatch):
+    """The canonical configurations through the kernels and layouts they do not all take by default: the staged kernels
+    that loop over run-time path tables (NO_CANON), and the edge kernels with other channels per lane and fewer warps."""
     monkeypatch.setenv(*knob.split("="))
     conv = run_case(name, dtype, nodes=37, edges=301, seed=3)
     assert conv.op.uses_staged_kernels and conv.op.canonical_l2 >= 0
+    assert conv.op.backward_variant == variant
 
 
 def test_backward_skips_source_rows_without_edges():
