@@ -41,7 +41,7 @@ from bench_workloads import CUTOFF, DENSITY, WORKLOADS, build_graph_edges, build
 # atoms); a run on another atom count scales them by its edges, which is what the traffic grows with.  A run whose plan
 # picks another variant reports null.
 NCU_TRAFFIC_BYTES_PER_EDGE = {
-    ("cfg2", "forward", "staged"): 9.48e3,
+    ("cfg2", "forward", "row"): 9.08e3,
     ("cfg2", "backward", "row"): 18.31e3,
 }
 SH6_ITEMS = 4_000_000
@@ -442,8 +442,8 @@ class ConvWorkload:
         dom_bytes, dom_ms = (bwd_bytes, bwd_ms) if dominant == "backward" else (fwd_bytes, fwd_ms)
         achieved = dom_bytes / (dom_ms * 1e-3) / 1e9
         step_gbs = (fwd_bytes + bwd_bytes) / ((fwd_ms + bwd_ms) * 1e-3) / 1e9
-        variant = "staged" if dominant == "forward" else op.backward_variant
-        per_edge = NCU_TRAFFIC_BYTES_PER_EDGE.get((self.name, dominant, variant)) if op.uses_staged_kernels else None
+        per_edge = (NCU_TRAFFIC_BYTES_PER_EDGE.get((self.name, dominant, op.backward_variant))
+                    if op.uses_staged_kernels else None)
         result.update(
             ms_per_step=ms, value=edges_total.item() / (ms * 1e-3), collective_ms=gather_ms + return_ms,
             roofline={

@@ -389,9 +389,9 @@ sh_kernel(const ShParams P, const T* __restrict__ v, const T* __restrict__ g, co
 // A warp's tile of 32 rows of C values in shared memory.  Rows are moved in 16-byte pieces on both sides.  With C odd the
 // tile is the memory's own image, and scalar accesses to a column, one row per lane, meet no bank conflict.  With C even
 // (4, 16, 36: multiples of a piece) a row takes an odd number of pieces, and lanes access their rows by whole pieces, eight
-// lanes in eight different groups of banks.  Both kernels are bound by HBM.  At lmax 6, 4 M vectors, FP32 (832 MB each): 139
-// us forward and 136 us backward, 0.92 and 0.94 of a copy's bandwidth; values and gradient together 299 us as a user
-// calls them, against 344 with value-by-value copies and loads that wait for the arithmetic.
+// lanes in eight different groups of banks.  Both kernels are bound by HBM.  At lmax 6, 4 M vectors, FP32 (832
+// and 880 MB): 144 us forward and 139 us backward, 0.88 and 0.97 of a copy's bandwidth; values and gradient together 299 us as
+// a user calls them, against 344 with value-by-value copies and loads that wait for the arithmetic.
 template <typename T, int C>
 struct RowTile {
   static constexpr int per = 16 / static_cast<int>(sizeof(T));  // values in a piece

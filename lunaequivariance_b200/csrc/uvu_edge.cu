@@ -8,7 +8,7 @@ namespace edgek {
 
 namespace {
 
-// Whether the kernel of all gradients spills registers.
+// Whether the kernel of all gradients spills registers by hundreds of bytes (a few bytes are common, and harmless).
 template <typename T, int CPL, int... ID>
 bool spills(int shape, std::integer_sequence<int, ID...>) {
   bool found = false;

@@ -58,13 +58,15 @@ struct EdgeBwd {
   static constexpr int state =
       (S::XD * CPL * (WX ? 2 : 1) + (WY ? S::YD * pair : 0) + (2 * S::LO + 1) * CPL) * words;
   static constexpr int program_regs = WM ? S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 : 0;
-  // The program goes to shared memory where that makes room for 16 warps instead of 12 without spills: degrees (2, 2, 2)
-  // with two channels per lane, 5.2 M edges of 64 channels: 7.09 -> 6.60 ms.  Elsewhere the reads cost more than the room
-  // gives: (3, 3, 3), 12 warps for 8 with some spills, 6.38 -> 7.07 ms; dL/dw alone in FP64 5.36 -> 6.16 ms.
+  // The program goes to shared memory where the registers that it frees make room for 16 warps instead of 12.  One instance
+  // is like that: degrees (2, 2, 2) with two FP32 channels per lane.  52 edges per node, best of nine: 5.2 M edges of 64
+  // channels 6.90 -> 6.44 ms, 0.11 M edges 0.188 -> 0.180; 2.1 M edges of 48 channels, where the kernel spills 20 bytes, 3.03
+  // -> 2.89.  Elsewhere the reads cost more than the room gives: (3, 3, 3), 12 warps for 8, 6.38 -> 7.07 ms; dL/dw alone in
+  // FP64 5.36 -> 6.16 ms.
   static constexpr bool shared_program =
       WX && WM && WY && pair == 2 && warps_for(state + program_regs + 48) == 12 && warps_for(state + 48) == 16;
   using Program = std::conditional_t<shared_program, SharedMatrixProgram<T, S>, MatrixProgram<T, S>>;
-  static constexpr int registers = state + (shared_program ? 0 : program_regs) + 48;  // wanted; beyond 255 it spills
+  static constexpr int registers = state + (shared_program ? 0 : program_regs) + 48;  // an estimate; beyond 255 it spills hundreds of bytes
   static constexpr int max_warps = warps_for(registers);
   // slots of g: the highest degree has one, the others share one
   static constexpr int slot_of(int l3) { return l3 == S::LO && S::ooff(S::LO) > 0 ? 1 : 0; }
