@@ -19,7 +19,7 @@ this recipe
    64-bit variant, ``src/lunatp/utils/layout.py:441-517``).
 
 No reference source is copied into this repository; the generated ``.cu`` text stays in the build folder under
-``oracle/_ref/build`` (ignored by git and not shipped to the GPU box).  ``oracle/ref_kernels.py`` loads the libraries
+``oracle/_ref/build`` (ignored by git).  ``oracle/ref_kernels.py`` loads the libraries
 on a machine with a GPU and calls their entry points.
 
     python oracle/build_ref.py /path/to/LunaEquivariance [config ...]
