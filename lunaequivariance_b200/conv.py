@@ -745,7 +745,9 @@ def _conv(op: LunaTPUVUConv, x, edge_attr, weight, graph: LunaTPGraph):
             x.contiguous(), edge_attr.contiguous(), weight.contiguous(), None, graph.table_list(),
             graph.num_nodes, False, op.torch_config)
         return out
-    if x.is_cuda and graph.src.is_cuda and graph.split_rows() is None:
+    if x.is_cuda and graph.src.device != x.device and graph.num_edges:  # kernels would follow tables of another memory
+        raise ValueError("features, weights and graph must share one CUDA device")
+    if x.is_cuda and graph.split_rows() is None:
         return _native.binding().conv(op._plan.op, graph.native_holder(), x, edge_attr, weight)
     return UVUConvForward.apply(op, _through_view(x), _through_view(edge_attr), _through_view(weight), graph)
 

@@ -215,6 +215,11 @@ def test_input_validation_errors():
         conv(x, y, w, graph=graph, env=torch.ones(2, device=DEVICE, dtype=torch.float64))
     with pytest.raises(RuntimeError, match="CUDA is required"):
         conv(x.cpu(), y.cpu(), w.cpu(), graph=graph)
+    on_host = conv.create_graph(torch.tensor([0, 1]), torch.tensor([0, 1]), 2)
+    with pytest.raises(ValueError, match="share one CUDA device"):
+        conv(x, y, w, graph=on_host)
+    empty = conv.create_graph(torch.tensor([], dtype=torch.int64), torch.tensor([], dtype=torch.int64), 2)  # nothing to read
+    assert conv(x, y[:0], w[:0], graph=empty).abs().max().item() == 0.0
 
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
