@@ -140,7 +140,7 @@ def test_custom_op_fake_shapes():
 
 
 def test_canonical_path_lists_are_detected_without_gpu():
-    """Full lists of allowed couplings select the kernels unrolled at compile time; anything else does not."""
+    """Full lists of allowed couplings of degrees from 0 on are recognised; lists with gaps or in another order are not."""
     from tests.helpers import config
 
     expected = {"cfg2": 3, "cfg4": 3, "cfg5": 2, "fixture": 1, "wide": 1, "cfg1": -1, "partial": -1}
