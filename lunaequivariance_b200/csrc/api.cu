@@ -67,7 +67,7 @@ extern "C" int64_t luna_uvu_plan_query(const luna_uvu_plan* plan, int what) {
     case LUNA_PLAN_BWD_SMEM_BYTES: return fast_smem_bytes(plan, 1);
     case LUNA_PLAN_CANONICAL_L2: return edge ? edgek::canonical_l2(plan) : (plan->fast_ok ? plan->fast.canon_l2 : -1);
     case LUNA_PLAN_SPARSE_TERMS:
-      return edge && edgek::canonical_l2(plan) >= 0 ? static_cast<int64_t>(plan->edge.term_c[0].size()) : 0;
+      return edge && edgek::canonical_l2(plan) >= 0 ? static_cast<int64_t>(plan->edge.term_c[0].size() + plan->edge.coef[0].size()) : 0;
     case LUNA_PLAN_BWD_VARIANT: return fast_bwd_variant(plan);
     case LUNA_PLAN_NEEDS_SCRATCH: return fast_scratch_bytes(plan, 1, 1) > 0;
     default: return -1;

@@ -166,7 +166,7 @@ struct EdgePlan {
   EdgeLanes lanes;
   EdgeLanes lanes_all;  // of backward calls that want dL/dy and another gradient
   // [0] of the shape, [1] of the shape with x and out exchanged
-  std::vector<double> prog_c[2], term_c[2];
+  std::vector<double> prog_c[2], term_c[2], coef[2];
   std::vector<unsigned short> prog_j[2];
 };
 

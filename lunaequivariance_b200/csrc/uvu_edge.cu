@@ -1,6 +1,7 @@
 // Which plans the edge kernels serve, the tables they read, and the choice of the compiled instance.
 #include "uvu_edge_bwd.cuh"
 
+#include <cmath>
 #include <utility>
 
 namespace luna {
@@ -75,9 +76,12 @@ bool fill_tables(luna_uvu_plan* plan, bool exchanged) {
   std::vector<double> term_c(R::terms, 0.0), prog_c(2 * R::m_total, 0.0);
   std::vector<unsigned short> prog_j(R::m_total, kNoAttribute | kNoAttribute << 8);
   std::vector<int> entry_terms(R::m_total, 0);
+  std::vector<double> coef(R::coff(-1, -1, -1), 0.0);
   for (const PathRec& p : plan->paths) {
     const int l1 = (p.d1 - 1) / 2, l2 = (p.d2 - 1) / 2, l3 = (p.d3 - 1) / 2, a = exchanged ? l3 : l1, c = exchanged ? l1 : l3;
     const CgTerm* pattern = cg_pattern(a, l2, c);
+    const bool diagonal = R::diagonal(a, l2, c);
+    double* const one = &coef[diagonal ? R::coff(a, l2, c) : 0];
     const int n = cg_count(a, l2, c), toff = R::toff(a, l2, c), moff = R::moff(a, l2, c);
     std::vector<char> seen(n, 0);
     int found = 0;
@@ -91,6 +95,11 @@ bool fill_tables(luna_uvu_plan* plan, bool exchanged) {
         if (slot < 0 || seen[slot]) return false;
         seen[slot] = 1;
         ++found;
+        if (diagonal) {  // one coefficient, up to the rounding of the tensor
+          if (found == 1) *one = term.c;
+          if (std::abs(term.c - *one) > std::abs(*one) * (plan->dtype == LUNA_F64 ? 4e-15 : 5e-7)) return false;
+          continue;
+        }
         term_c[toff + slot] = term.c;
         int entry = moff - 1;  // the term's (i, k) among the pattern's distinct ones
         for (int u = 0; u <= slot; ++u)
@@ -105,6 +114,7 @@ bool fill_tables(luna_uvu_plan* plan, bool exchanged) {
   plan->edge.term_c[exchanged] = term_c;
   plan->edge.prog_c[exchanged] = prog_c;
   plan->edge.prog_j[exchanged] = prog_j;
+  plan->edge.coef[exchanged] = coef;
   return true;
 }
 

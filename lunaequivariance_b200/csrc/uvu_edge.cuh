@@ -34,8 +34,10 @@ using namespace fastk;
 
 constexpr int kEdgeMaxStages = 4;
 constexpr int kEdgeMaxSlices = kTileCounterWords / 2;
+constexpr int kEdgeMaxCoefs = 10;  // paths with a degree of zero
 
 // ---- shapes ---------------------------------------------------------------------------------------------------------
+constexpr int top_degree(int mask) { return mask >= 8 ? 3 : (mask >= 4 ? 2 : (mask >= 2 ? 1 : 0)); }
 template <int MX_, int MY_, int MO_>
 struct Shape {
   static constexpr int MX = MX_, MY = MY_, MO = MO_;
@@ -67,6 +69,22 @@ struct Shape {
     return r;
   }
   static constexpr int paths = rank(-1, -1, -1);
+  // A path with a degree of zero couples component by component with one coefficient (edge_diagonal): it has no matrix and
+  // no terms.  Position of its coefficient; past-the-end arguments give their number.
+  static constexpr bool diagonal(int l1, int l2, int l3) { return l1 == 0 || l2 == 0 || l3 == 0; }
+  static constexpr int coff(int a, int b, int c) {
+    int n = 0;
+    for (int l3 = 0; l3 < 4; ++l3)
+      for (int l1 = 0; l1 < 4; ++l1)
+        for (int l2 = 0; l2 < 4; ++l2) {
+          if (l1 == a && l2 == b && l3 == c) return n;
+          if (ok(l1, l2, l3) && diagonal(l1, l2, l3)) ++n;
+        }
+    return n;
+  }
+  // the edge's attributes as they are, behind the matrices: every degree at a multiple of four
+  static constexpr int ypos(int l) { return l == 3 ? 16 : 4 * l; }
+  static constexpr int y_elems = ypos(top_degree(MY)) + 4 * ((2 * top_degree(MY) + 4) / 4);
   // first entry of a path in an edge's coupling-matrix buffer: the entries that some edge attribute reaches, in (i, k)
   // order, paths in (l3, l1, l2) order, every path padded to a multiple of four
   static constexpr int moff(int a, int b, int c) {
@@ -76,12 +94,13 @@ struct Shape {
         for (int l2 = 0; l2 < 4; ++l2) {
           if (!ok(l1, l2, l3)) continue;
           if (l1 == a && l2 == b && l3 == c) return m;
-          m += (cg_pair_count(l1, l2, l3) + 3) / 4 * 4;
+          m += diagonal(l1, l2, l3) ? 0 : (cg_pair_count(l1, l2, l3) + 3) / 4 * 4;
         }
     return m;
   }
   static constexpr int m_total = moff(-1, -1, -1);
   static constexpr int m_rounds = (m_total + 31) / 32;
+  static constexpr int m_elems = m_rounds * 32 + y_elems;
   // first coupling term of a path in the term list: (l3, l1, l2) order, every path's terms padded to a multiple of four
   static constexpr int toff(int a, int b, int c) {
     int t = 0;
@@ -90,13 +109,12 @@ struct Shape {
         for (int l2 = 0; l2 < 4; ++l2) {
           if (!ok(l1, l2, l3)) continue;
           if (l1 == a && l2 == b && l3 == c) return t;
-          t += (cg_count(l1, l2, l3) + 3) / 4 * 4;
+          t += diagonal(l1, l2, l3) ? 0 : (cg_count(l1, l2, l3) + 3) / 4 * 4;
         }
     return t;
   }
   static constexpr int terms = toff(-1, -1, -1);
-  static constexpr int top(int mask) { return mask >= 8 ? 3 : (mask >= 4 ? 2 : (mask >= 2 ? 1 : 0)); }
-  static constexpr int LO = top(MO);
+  static constexpr int LO = top_degree(MO);
 };
 
 // The shape with the roles of x and out exchanged; the weight blocks stay where they are.
@@ -283,6 +301,13 @@ __device__ __forceinline__ void edge_load_four(const T* p, T* out) {
   }
 }
 
+// The 2l + 1 attributes of degree l out of an edge's matrix buffer.
+template <typename S, int l, typename T>
+__device__ __forceinline__ void edge_attributes(const T* buffer, T* y) {
+#pragma unroll
+  for (int q = 0; q < (2 * l + 4) / 4; ++q) edge_load_four<T>(buffer + S::m_rounds * 32 + S::ypos(l) + 4 * q, y + 4 * q);
+}
+
 // A lane's channels.  Packet q of a lane holds PK::W consecutive channels, and the packets of the warp's lanes lie side
 // by side: packet q of lane l starts at channel  own + q * stride  with  own = first + W * l  and  stride = W * lanes.
 // Weights then arrive as ready-made packets, and the scalar loads that assemble the packets of a node row (channel-
@@ -352,13 +377,24 @@ __device__ __forceinline__ void lane_store_block(T* p, int stride, const typenam
 // y[jb].  Lane l makes entries l, l + 32, ...  An entry made of one attribute only takes kNoAttribute as its second, a lane
 // that holds no attribute but zero: with any attribute in its place 0 times an infinite one would make the entry NaN.
 constexpr int kNoAttribute = 31;
+// Where lane j stores attribute j of the edge, behind the matrices.
+template <typename S>
+__device__ __forceinline__ int attribute_position(int j) {
+  int at = 0;
+#pragma unroll
+  for (int l = 0; l < 4; ++l)
+    if (S::has(S::MY, l) && j >= S::yoff(l)) at = S::m_rounds * 32 + S::ypos(l) + j - S::yoff(l);
+  return at;
+}
 template <typename T, typename S>
 struct MatrixProgram {
   static_assert(S::YD <= kNoAttribute, "one lane is left without an attribute");
   static constexpr int elems = 0;  // of shared memory
-  T a[S::m_rounds], b[S::m_rounds];
-  unsigned j[(S::m_rounds + 1) / 2];  // two attribute indices of 8 bits per round
+  T a[S::m_rounds + 1], b[S::m_rounds + 1];
+  unsigned j[(S::m_rounds + 2) / 2];  // two attribute indices of 8 bits per round
+  int own;                            // where this lane's attribute goes
   __device__ __forceinline__ void load(const T* coefficients, const unsigned short* attributes, int lane) {
+    own = attribute_position<S>(lane);
 #pragma unroll
     for (int r = 0; r < (S::m_rounds + 1) / 2; ++r) j[r] = 0u;
 #pragma unroll
@@ -376,6 +412,7 @@ struct MatrixProgram {
       const T yb = __shfl_sync(0xffffffffu, y, static_cast<int>((j[r / 2] >> (16 * (r % 2) + 8)) & 255u));
       to[r * 32 + lane] = fma(b[r], yb, a[r] * ya);
     }
+    if (lane < S::YD) to[own] = y;
   }
 };
 
@@ -386,6 +423,7 @@ struct SharedMatrixProgram {
   static constexpr int elems = 2 * entries + entries * 2 / static_cast<int>(sizeof(T));
   const T* c;
   const unsigned short* j;
+  int own;
   // by all threads of the CTA, which synchronise before the first run
   __device__ __forceinline__ void load(T* to, const T* coefficients, const unsigned short* attributes) {
     unsigned short* to_j = reinterpret_cast<unsigned short*>(to + 2 * entries);
@@ -396,6 +434,7 @@ struct SharedMatrixProgram {
     }
     c = to;
     j = to_j;
+    own = attribute_position<S>(static_cast<int>(threadIdx.x & 31));
   }
   __device__ __forceinline__ void run(T y, T* to, int lane) const {
 #pragma unroll
@@ -406,6 +445,7 @@ struct SharedMatrixProgram {
       const T yb = __shfl_sync(0xffffffffu, y, static_cast<int>(which >> 8));
       to[m] = fma(c[entries + m], yb, c[m] * ya);
     }
+    if (lane < S::YD) to[own] = y;
   }
 };
 

@@ -19,6 +19,7 @@ struct EdgeFwdParams {
   const int *src, *dst_rowptr;
   const T* prog_c;               // [2][m_total] coefficients of the two attributes an entry depends on
   const unsigned short* prog_j;  // [m_total] the two attributes, 8 bits each
+  T coef[kEdgeMaxCoefs];         // of the paths with a degree of zero
   int* status;
   unsigned* tile_counters;
   int64_t num_rows, tile_rows, num_tiles;
@@ -35,7 +36,7 @@ struct EdgeFwdParams {
 template <typename T, int CPL, typename S>
 struct EdgeFwd {
   static constexpr int words = sizeof(T) / 4;
-  static constexpr int m_elems = S::m_rounds * 32;
+  static constexpr int m_elems = S::m_elems;
   static constexpr int max_warps =
       warps_for((S::OD + S::XD) * CPL * words + S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 + 44);
   static constexpr size_t warp_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
@@ -114,6 +115,33 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   bool alive = true;
   int buf = 0;          // matrix buffer of the current edge
 
+  // The paths with a degree of zero, c their coefficient: out_k += (c y w) x_k, (c w x) y_k or (c w) sum_i y_i x_i.
+  auto diagonal_body = [&](auto l1c, auto l2c, auto l3c, const T* wq, const T* buffer, const V* xl, V* al) {
+    constexpr int l1 = decltype(l1c)::value, l2 = decltype(l2c)::value, l3 = decltype(l3c)::value;
+    const T c = P.coef[S::coff(l1, l2, l3)];
+    T y[8];
+    edge_attributes<S, l2>(buffer, y);
+    V w2[NP];
+    lane_load<PK, T>(wq, stride, w2);
+    const V scale = bcast_packet(l2 == 0 ? c * y[0] : c, V{});
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      V cw = vmul(scale, w2[p]);
+      if constexpr (l2 == 0) {
+#pragma unroll
+        for (int k = 0; k < 2 * l3 + 1; ++k) al[k * NP + p] = vfma(cw, xl[k * NP + p], al[k * NP + p]);
+      } else if constexpr (l1 == 0) {
+        cw = vmul(cw, xl[p]);
+#pragma unroll
+        for (int k = 0; k < 2 * l3 + 1; ++k) al[k * NP + p] = vfma(bcast_packet(y[k], V{}), cw, al[k * NP + p]);
+      } else {
+        V sum = vmul(bcast_packet(y[0], V{}), xl[p]);
+#pragma unroll
+        for (int i = 1; i < 2 * l1 + 1; ++i) sum = vfma(bcast_packet(y[i], V{}), xl[i * NP + p], sum);
+        al[p] = vfma(cw, sum, al[p]);
+      }
+    }
+  };
   // out_k += sum_i M[i][k] * (x_i * w) for one path, over the entries of M that the pattern has
   auto path_body = [&](auto l1c, auto l2c, auto l3c, const T* wq, const T* matrix, const V* xl, V* al) {
     constexpr int l1 = decltype(l1c)::value, l2 = decltype(l2c)::value, l3 = decltype(l3c)::value;
@@ -203,9 +231,13 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
               constexpr int l3 = decltype(l3c)::value;
               static_for<0, 4>([&](auto l2c) {
                 constexpr int l2 = decltype(l2c)::value;
-                if constexpr (S::ok(l1, l2, l3))
-                  path_body(l1c, l2c, l3c, ws + S::rank(l1, l2, l3) * ch, m_now + S::moff(l1, l2, l3), xl,
-                            &acc[S::ooff(l3) * NP]);
+                if constexpr (S::ok(l1, l2, l3)) {
+                  const T* wq = ws + S::rank(l1, l2, l3) * ch;
+                  if constexpr (S::diagonal(l1, l2, l3))
+                    diagonal_body(l1c, l2c, l3c, wq, m_now, xl, &acc[S::ooff(l3) * NP]);
+                  else
+                    path_body(l1c, l2c, l3c, wq, m_now + S::moff(l1, l2, l3), xl, &acc[S::ooff(l3) * NP]);
+                }
               });
             });
           }
@@ -289,6 +321,7 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.dst_rowptr = graph->dst_rowptr;
   P.prog_c = static_cast<const T*>(dt.edge[0].prog_c);
   P.prog_j = dt.edge[0].prog_j;
+  for (int c = 0; c < S::coff(-1, -1, -1); ++c) P.coef[c] = static_cast<T>(plan->edge.coef[0][c]);
   P.status = dt.status;
   P.tile_counters = next_tile_counters(plan, dt);
   P.num_rows = graph->num_nodes;

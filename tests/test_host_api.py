@@ -242,3 +242,22 @@ def test_plan_queries_describe_the_kernels_that_run(mul, lmax, dtype, lanes, chu
     irreps = (block(64, 1), block(1, 2), block(64, 2))
     op = luna.prepare_tensor_product(*irreps, all_paths(*irreps), convolution=True, dtype=dtype)
     assert op.backward_variant == "tables" and op.canonical_l2 == 2 and not op.uses_compiled_patterns
+
+
+@pytest.mark.parametrize("dtype,rounding", [(torch.float32, 1e-7), (torch.float64, 1e-15)])
+def test_compiled_patterns_need_one_coefficient_where_a_degree_is_zero(dtype, rounding):
+    """The edge kernels take the coupling of a path with a degree of zero as one number: terms that differ by rounding are
+    that, terms that differ by more go to the kernels that read every term."""
+    from tests.helpers import all_paths
+
+    irreps = ("64x0e+64x1o", "1x0e+1x1o", "64x0e+64x1o")
+    meta = luna.prepare_tensor_product(*irreps, all_paths(*irreps), convolution=True, dtype=dtype).meta
+    for factor, variant in ((1 + rounding, "row"), (1.001, "tables")):
+        for spec in meta["generated_specs"]:
+            if len(spec["terms"]) != 3:
+                continue
+            i, j, k, c = spec["terms"][1]
+            terms = [spec["terms"][0], (i, j, k, c * factor), spec["terms"][2]]
+            changed = [dict(s, terms=terms) if s is spec else s for s in meta["generated_specs"]]
+            op = luna.create_uvu_conv_operator(dict(meta, generated_specs=changed), dtype=dtype)
+            assert op.backward_variant == variant, (spec["l1"], spec["l2"], spec["l3"], factor)
