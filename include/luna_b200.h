@@ -149,6 +149,12 @@ LUNA_API int luna_uvu_conv_bwd_add_gx(luna_uvu_plan* plan, const luna_graph* gra
                              const void* w, const void* g, void* gx, void* gy, void* gw, void* scratch,
                              int64_t scratch_bytes, void* stream);
 
+/* As luna_uvu_conv_bwd, except that gw is added to instead of written: for callers that hold another contribution to the
+ * weights' gradient, as both orders of a force training step make one. */
+LUNA_API int luna_uvu_conv_bwd_add_gw(luna_uvu_plan* plan, const luna_graph* graph, const void* x, const void* y,
+                             const void* w, const void* g, void* gx, void* gy, void* gw, void* scratch,
+                             int64_t scratch_bytes, void* stream);
+
 /* Same result as luna_uvu_conv_bwd, for callers that cannot allocate device memory and so have no scratch
  * buffer to pass: code running inside another program's step without an allocator of its own, loops that must
  * not hit cudaMalloc's device-wide synchronisation, processes whose memory pool is fixed at start-up.  No

@@ -18,6 +18,9 @@
 // the other in memory, g stays in registers for the row and x is gathered.  Taken where a row of x is no longer than a row
 // of g, which is then the smaller gather (layers that widen their degrees, first layers most of all).
 //
+// gw alone, added to what is there: the rows that are added to arrive in the stages in the weights' place, and the sums
+// begin with them.
+//
 // Every wait is bounded; a wait that runs out sets the plan's status word.
 #pragma once
 
@@ -90,9 +93,9 @@ struct EdgeBwd {
 };
 
 // One path for a lane's packets.  xl / gxl: the lane's x and gx packets of degree l1; g2: its g packets of degree l3;
-// w2: its weights; dot receives sum_i x_i s_i; gyl: the accumulators of degree l2.  The arithmetic of a row i is issued
+// w2: its weights; dot receives (ADD: is added) sum_i x_i s_i; gyl: the accumulators of degree l2.  The arithmetic of a row i is issued
 // in batches of independent instructions, so that the latency of one is covered by the others with few warps resident.
-template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, typename V>
+template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
 __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* g2, const V* w2, V* dot, const T* mbuf,
                                           const T* ctab) {
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
@@ -159,7 +162,7 @@ __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* 
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
           if constexpr (WX) gxl[i * NP + p] = vfma(w2[p], sa[p], gxl[i * NP + p]);
-          dot[p] = t0 == 0 ? vmul(xl[i * NP + p], sa[p]) : vfma(xl[i * NP + p], sa[p], dot[p]);
+          dot[p] = t0 == 0 && !ADD ? vmul(xl[i * NP + p], sa[p]) : vfma(xl[i * NP + p], sa[p], dot[p]);
         }
       }
     }
@@ -174,7 +177,7 @@ __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* 
 // eleven paths of degrees (2, 2, 2) are like that, eight of the seventeen of (2, 3, 3).  Forward and backward with all paths in
 // edge_path, and like this: (2, 3, 3), 128 channels, 2.6 M edges 15.88 -> 15.33 ms; (3, 3, 3), 64 channels, 1.6 M edges 8.99
 // -> 8.54; (2, 2, 2), 64 channels, 5.2 M edges 10.23 -> 9.98; FP64 force step, 1.05 M edges 34.8 -> 33.9.
-template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, typename V>
+template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
 __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const V* g2, const V* w2, V* dot, const T* mbuf, T c) {
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP, d = 2 * (l1 > l3 ? l1 : l3) + 1;
@@ -198,7 +201,7 @@ __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const
       const V cy = bcast_packet(c * y[0], V{});
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        dot[p] = vmul(cy, sum[p]);
+        dot[p] = ADD ? vfma(cy, sum[p], dot[p]) : vmul(cy, sum[p]);
         if constexpr (WX) {
           const V wy = vmul(cy, w2[p]);
 #pragma unroll
@@ -227,7 +230,7 @@ __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         const V s = vmul(cc, sum[p]);
-        dot[p] = vmul(xl[p], s);
+        dot[p] = ADD ? vfma(xl[p], s, dot[p]) : vmul(xl[p], s);
         if constexpr (WX) gxl[p] = vfma(w2[p], s, gxl[p]);
       }
     }
@@ -250,7 +253,7 @@ __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const
         V sum = vmul(bcast_packet(y[0], V{}), xl[p]);
 #pragma unroll
         for (int i = 1; i < d; ++i) sum = vfma(bcast_packet(y[i], V{}), xl[i * NP + p], sum);
-        dot[p] = vmul(cg[p], sum);
+        dot[p] = ADD ? vfma(cg[p], sum, dot[p]) : vmul(cg[p], sum);
         if constexpr (WX) {
 #pragma unroll
           for (int i = 0; i < d; ++i) gxl[i * NP + p] = vfma(bcast_packet(y[i], V{}), cgw[p], gxl[i * NP + p]);
@@ -261,8 +264,8 @@ __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const
 }
 
 // FULL: one warp per edge and 32 * CPL channels, known to the compiler.  SLICED: these are a slice of wider blocks.  DST: rows
-// by destination (S, x and g exchanged).
-template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED>
+// by destination (S, x and g exchanged).  ADD: gw alone, added to; w names gw.
+template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED, bool ADD>
 __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32, 1)
     edge_bwd_kernel(const __grid_constant__ EdgeBwdParams<T> P) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
@@ -278,6 +281,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   const bool split = P.split != 0;
   const int stage_elems = W + (split ? 0 : O);
   static_assert(FULL || !SLICED, "a slice is one warp's full set of channels");
+  static_assert(!ADD || (WM && !WX && !WY), "the weights' place in a stage must be free");
   const int row_ch = SLICED ? P.row_ch : ch, first_ch = SLICED ? static_cast<int>(blockIdx.y) * ch : 0;
   const int w_row = S::paths * row_ch, x_row = S::XD * row_ch, o_row = S::OD * row_ch;  // in memory
   unsigned* const counters = P.tile_counters + (SLICED ? 2 * blockIdx.y : 0);
@@ -391,12 +395,16 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           T* wq = wrow + S::rank(l1, l2, l3) * ch + own;
           V w2[NP], dot[NP];
           lane_load<PK, T>(wq, stride, w2);
+          if constexpr (ADD) {
+#pragma unroll
+            for (int p = 0; p < NP; ++p) dot[p] = w2[p];
+          }
           const V* xl = &xr[S::xoff(l1) * NP];
           V *gxl = &gxr[WX ? S::xoff(l1) * NP : 0], *gyl = &gy2[WY ? S::yoff(l2) : 0];
           if constexpr (S::diagonal(l1, l2, l3))
-            edge_diagonal<T, CPL, S, l1, l2, l3, WX, WM, WY, V>(xl, gxl, gyl, g2, w2, dot, mbuf, P.coef[S::coff(l1, l2, l3)]);
+            edge_diagonal<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, P.coef[S::coff(l1, l2, l3)]);
           else
-            edge_path<T, CPL, S, l1, l2, l3, WX, WM, WY, V>(xl, gxl, gyl, g2, w2, dot, mbuf, ctab);
+            edge_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, ctab);
           if (storing && active) lane_store<PK, T>(wq, stride, dot);  // the gradients leave with the row
         }
       });
@@ -701,15 +709,15 @@ EdgeLaunch edge_bwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
   return launch;
 }
 
-template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED>
+template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED, bool ADD = false>
 int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                     const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
-  auto kernel = edge_bwd_kernel<T, CPL, S, WX, WM, WY, FULL, DST, SLICED>;
+  auto kernel = edge_bwd_kernel<T, CPL, S, WX, WM, WY, FULL, DST, SLICED, ADD>;
   EdgeBwdParams<T> P;
   P.x = static_cast<const T*>(DST ? a.g : a.x);
   P.y = static_cast<const T*>(a.y);
-  P.w = static_cast<const T*>(a.w);
+  P.w = static_cast<const T*>(ADD ? a.gw : a.w);
   P.g = static_cast<const T*>(DST ? a.x : a.g);
   P.gx = static_cast<T*>(a.gx);
   P.gy = static_cast<T*>(a.gy);
@@ -728,10 +736,10 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.ch = plan->edge.ch / lanes.slices;
   P.row_ch = plan->edge.ch;
   P.team_warps = lanes.team_warps;
-  P.need_w = a.gx != nullptr || a.gy != nullptr;
+  P.need_w = ADD || a.gx != nullptr || a.gy != nullptr;
   P.acc_x = a.acc_x;
   P.acc_y = a.acc_y;
-  P.acc_w = a.acc_w;
+  P.acc_w = !ADD && a.acc_w;
   P.gy_part = graph->num_edges * S::YD;
   if (SLICED && WY) {
     const int64_t need = lanes.slices * P.gy_part * static_cast<int64_t>(sizeof(T));
@@ -791,6 +799,8 @@ int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const l
   if (!wx && ww != wy) {
     constexpr bool dst = S::OD >= S::XD;
     using R = std::conditional_t<dst, Transposed<S>, S>;
+    if (ww && a.acc_w)
+      return launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED, true>(plan, dt, graph, lanes, a, stream);
     return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED>(plan, dt, graph, lanes, a, stream)
               : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst, SLICED>(plan, dt, graph, lanes, a, stream);
   }
