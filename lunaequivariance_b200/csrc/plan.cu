@@ -387,10 +387,9 @@ int get_device_tables(luna_uvu_plan* plan, const DeviceTables** out) {
     return append(raw.data(), raw.size());
   };
   const EdgePlan& edge = plan->edge;
-  size_t o_epc[2], o_etc[2], o_epj[2];
+  size_t o_epc[2], o_epj[2];
   for (int t = 0; t < 2; ++t) {
     o_epc[t] = append_scalars(edge.prog_c[t]);
-    o_etc[t] = append_scalars(edge.term_c[t]);
     o_epj[t] = append(edge.prog_j[t].data(), edge.prog_j[t].size() * sizeof(unsigned short));
   }
 
@@ -423,7 +422,7 @@ int get_device_tables(luna_uvu_plan* plan, const DeviceTables** out) {
   dt.ell_c = base + o_mc;
   dt.bwd_tables = base + o_blob;
   for (int t = 0; t < 2; ++t)
-    dt.edge[t] = EdgeTables{base + o_epc[t], base + o_etc[t], reinterpret_cast<const unsigned short*>(base + o_epj[t])};
+    dt.edge[t] = EdgeTables{base + o_epc[t], reinterpret_cast<const unsigned short*>(base + o_epj[t])};
   LUNA_CUDA_CHECK(cudaDeviceGetAttribute(&dt.sm_count, cudaDevAttrMultiProcessorCount, device));
   LUNA_CUDA_CHECK(cudaDeviceGetAttribute(&dt.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   auto inserted = plan->device_tables.emplace(device, dt);

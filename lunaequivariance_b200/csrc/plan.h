@@ -121,7 +121,7 @@ constexpr int kTileCounterSets = 32;    // launches of one plan that may be in f
 constexpr int kTileCounterWords = 64;   // per set: (next tile, warps finished) for up to 32 channel chunks
 // What an edge kernel reads of a plan: see EdgeBwdParams.
 struct EdgeTables {
-  const void *prog_c = nullptr, *term_c = nullptr;
+  const void* prog_c = nullptr;
   const unsigned short* prog_j = nullptr;
 };
 
@@ -146,7 +146,7 @@ struct DeviceTables {
   // entry indices of the edge-attribute gradient's program (gy[j] = sum_t c[t] * G[m[t]]), y indices of the
   // padded program; offsets in FastMeta::tb_*
   const unsigned char* bwd_tables = nullptr;
-  // edge kernels (EdgePlan): the coupling-matrix program and the term list
+  // edge kernels (EdgePlan): the coupling-matrix program
   EdgeTables edge[2];  // of the plan's shape, and of the shape with x and out exchanged
   int sm_count = 0;
   int max_smem_optin = 0;

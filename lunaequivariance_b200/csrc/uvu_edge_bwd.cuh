@@ -21,6 +21,11 @@
 // gw alone, added to what is there: the rows that are added to arrive in the stages in the weights' place, and the sums
 // begin with them.
 //
+// The coefficients of the coupling terms are kernel parameters: an operand of the FMA that uses them, instead of a load from a
+// table in shared memory, whose pipe is the busiest one at (2, 2, 2) with 64 channels (61 % of its wavefronts).  All gradients,
+// table and parameters: (2, 2, 2), 64 channels, 5.2 M edges 6.95 -> 6.43 ms; (3, 3, 3), 64 channels, 0.8 M edges 3.27 -> 3.01;
+// (2, 3, 3), 128 channels, FP64, 0.4 M edges 5.33 -> 4.36, dL/dy alone in FP32, 1.05 M edges 2.34 -> 2.13.
+//
 // Every wait is bounded; a wait that runs out sets the plan's status word.
 #pragma once
 
@@ -31,14 +36,15 @@ namespace edgek {
 
 constexpr int kEdgeMaxSlots = 2;
 
-template <typename T>
+// N: coupling terms that the kernel reads.
+template <typename T, int N>
 struct EdgeBwdParams {
   const T *x, *y, *w, *g;
   T *gx, *gy, *gw;
   const int *dst, *src_rowptr, *edge_ids;
   const T* prog_c;               // [2][m_total] coefficients of the two attributes a matrix entry depends on
   const unsigned short* prog_j;  // [m_total] the two attributes, 8 bits each
-  const T* term_c;               // [terms] coefficients of the coupling terms
+  T term[N];                     // coefficients of the coupling terms
   T coef[kEdgeMaxCoefs];         // of the paths with a degree of zero
   int* status;
   unsigned* tile_counters;
@@ -88,8 +94,8 @@ struct EdgeBwd {
   static constexpr int warp_elems(int team_warps) {
     return m_elems + (WY ? red_pass * red_row + (team_warps > 1 ? 64 : 0) : 0);
   }
-  static constexpr int term_elems = (S::terms + 3) / 4 * 4;
-  static constexpr int table_elems = term_elems + (WM ? Program::elems : 0);
+  static constexpr int terms = WY && S::terms > 0 ? S::terms : 1;
+  static constexpr int table_elems = WM ? Program::elems : 0;
 };
 
 // One path for a lane's packets.  xl / gxl: the lane's x and gx packets of degree l1; g2: its g packets of degree l3;
@@ -97,7 +103,7 @@ struct EdgeBwd {
 // in batches of independent instructions, so that the latency of one is covered by the others with few warps resident.
 template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
 __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* g2, const V* w2, V* dot, const T* mbuf,
-                                          const T* ctab) {
+                                          const T* term) {
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   using PT = CgPattern<l1, l2, l3>;
@@ -110,17 +116,12 @@ __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* 
       constexpr int t1 = edge_row_end<PT>(t0);
       // groups of four table entries that cover the row
       constexpr int e0 = edge_entry<PT>(t0), e1 = edge_entry<PT>(t1 - 1);
-      constexpr int m_lo = e0 / 4, m_hi = e1 / 4, c_lo = t0 / 4, c_hi = (t1 - 1) / 4;
-      T mm[WM ? 4 * (m_hi - m_lo + 1) : 1], cc[WY ? 4 * (c_hi - c_lo + 1) : 1];
+      constexpr int m_lo = e0 / 4, m_hi = e1 / 4;
+      T mm[WM ? 4 * (m_hi - m_lo + 1) : 1];
       if constexpr (WM)
         static_for<m_lo, m_hi + 1>([&](auto qc) {
           constexpr int q = decltype(qc)::value;
           edge_load_four<T>(mbuf + moff + 4 * q, mm + 4 * (q - m_lo));
-        });
-      if constexpr (WY)
-        static_for<c_lo, c_hi + 1>([&](auto qc) {
-          constexpr int q = decltype(qc)::value;
-          edge_load_four<T>(ctab + toff + 4 * q, cc + 4 * (q - c_lo));
         });
       if constexpr (WY) {
         V xw[NP];
@@ -139,7 +140,7 @@ __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* 
         static_for<t0, t1>([&](auto uc) {
           constexpr int t = decltype(uc)::value;
           constexpr int j = PT::t[t].j, slot = edge_entry<PT>(t) - e0;
-          gyl[j] = vfma(bcast_packet(cc[t - 4 * c_lo], V{}), pik[slot], gyl[j]);
+          gyl[j] = vfma(bcast_packet(term[toff + t], V{}), pik[slot], gyl[j]);
         });
       }
       if constexpr (WM) {
@@ -267,7 +268,7 @@ __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const
 // by destination (S, x and g exchanged).  ADD: gw alone, added to; w names gw.
 template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED, bool ADD>
 __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32, 1)
-    edge_bwd_kernel(const __grid_constant__ EdgeBwdParams<T> P) {
+    edge_bwd_kernel(const __grid_constant__ EdgeBwdParams<T, EdgeBwd<T, CPL, S, WX, WM, WY>::terms> P) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   using V = typename PK::V;
@@ -295,8 +296,8 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   T* const mbuf = warp_mem + static_cast<size_t>(warp) * warp_elems;
   T* const red = mbuf + K::m_elems;
   T* const gbuf = red + K::red_pass * K::red_row;
-  T* const ctab = warp_mem + static_cast<size_t>(blockDim.x >> 5) * warp_elems;
-  uint64_t* const all_bars = reinterpret_cast<uint64_t*>(ctab + K::table_elems);
+  T* const tables = warp_mem + static_cast<size_t>(blockDim.x >> 5) * warp_elems;
+  uint64_t* const all_bars = reinterpret_cast<uint64_t*>(tables + K::table_elems);
   uint64_t* const full = all_bars + team * (kEdgeMaxStages + kEdgeMaxSlots);
   uint64_t* const gfull = full + kEdgeMaxStages;
   unsigned* const tickets = reinterpret_cast<unsigned*>(all_bars + P.teams * (kEdgeMaxStages + kEdgeMaxSlots));
@@ -306,12 +307,9 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     for (int s = 0; s < K::slots; ++s) mbar_init(&gfull[s], 1);
     fence_barrier_init();
   }
-  if constexpr (WY)
-    for (int i = threadIdx.x; i < S::terms; i += blockDim.x) ctab[i] = P.term_c[i];
-
   typename K::Program program;
   if constexpr (K::shared_program)
-    program.load(ctab + K::term_elems, P.prog_c, P.prog_j);
+    program.load(tables, P.prog_c, P.prog_j);
   else if constexpr (WM)
     program.load(P.prog_c, P.prog_j, lane);
   __syncthreads();
@@ -404,7 +402,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           if constexpr (S::diagonal(l1, l2, l3))
             edge_diagonal<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, P.coef[S::coff(l1, l2, l3)]);
           else
-            edge_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, ctab);
+            edge_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, P.term);
           if (storing && active) lane_store<PK, T>(wq, stride, dot);  // the gradients leave with the row
         }
       });
@@ -413,52 +411,55 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
 
   const bool grouped = P.group > 1;
   const int in_group = team % P.group, group_id = team / P.group, groups = P.teams / P.group;
-  const int64_t total = static_cast<int64_t>(gridDim.x) * (grouped ? groups : P.teams);
-  int64_t unit = grouped ? blockIdx.x + static_cast<int64_t>(gridDim.x) * group_id
-                         : static_cast<int64_t>(blockIdx.x) * P.teams + team;
-  const int64_t units = grouped ? P.num_rows : P.num_tiles;
-  int64_t seen_row = 0, seen_pos = 0;  // a row boundary this warp has seen, and where its edges begin
+  // edges and rows fit 31 bits, and every register counts
+  const unsigned total = gridDim.x * static_cast<unsigned>(grouped ? groups : P.teams);
+  unsigned unit = grouped ? blockIdx.x + gridDim.x * group_id : blockIdx.x * P.teams + team;
+  const unsigned units = static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
+  int seen_row = 0, seen_pos = 0;  // a row boundary this warp has seen, and where its edges begin
 #pragma unroll 1
   while (unit < units) {
-    int64_t unit_after = unit + total;
-    int64_t n = unit, n_hi = unit + 1;
+    unsigned unit_after = unit + total;
+    int n = static_cast<int>(unit), n_hi = n + 1;
     if (!grouped) {
       if (team_warps == 1) {
-        unit_after = take_tile(counters, total, lane);
+        unit_after = static_cast<unsigned>(take_tile(counters, total, lane));
       } else {
         if (leader) tickets[team] = atomicAdd(&counters[0], 1u);
         team_sync(team_warps, team);
-        unit_after = total + static_cast<int64_t>(tickets[team]);
+        unit_after = total + tickets[team];
         team_sync(team_warps, team);
       }
       if (P.tile_rows > 0) {
-        n = unit * P.tile_rows;
-        n_hi = n + P.tile_rows < P.num_rows ? n + P.tile_rows : P.num_rows;
+        const int64_t first = unit * P.tile_rows, end = first + P.tile_rows;
+        n = static_cast<int>(first);
+        n_hi = static_cast<int>(end < P.num_rows ? end : P.num_rows);
       } else {
         // tile t: the rows whose edges begin in [t, t + 1) * tile_edges of the source-sorted edge order (guessed from
         // where the warp's previous tile ended, assuming rows of average length in between)
         const int64_t guess =
             seen_row + static_cast<int64_t>(static_cast<float>(unit * P.tile_edges - seen_pos) * P.rows_per_edge);
-        n = unit == 0 ? 0 : warp_lower_bound_guess(P.src_rowptr, P.num_rows, unit * P.tile_edges, guess, lane);
-        n_hi = unit + 1 == P.num_tiles
-                   ? P.num_rows
-                   : warp_lower_bound_near(P.src_rowptr, P.num_rows, (unit + 1) * P.tile_edges, n, lane);
+        n = unit == 0 ? 0
+                      : static_cast<int>(warp_lower_bound_guess(P.src_rowptr, P.num_rows, unit * P.tile_edges, guess, lane));
+        n_hi = static_cast<int>(unit + 1 == units ? P.num_rows
+                                                  : warp_lower_bound_near(P.src_rowptr, P.num_rows, (unit + int64_t(1)) * P.tile_edges,
+                                                                          n, lane));
       }
     }
     const int64_t unit_now = unit;
     unit = unit_after;
     if (n >= n_hi) continue;  // a row with more edges than a tile spans several tile numbers
-    int64_t pos = P.src_rowptr[n], p_end = P.src_rowptr[n_hi];
+    int pos = P.src_rowptr[n], p_end = P.src_rowptr[n_hi];
     seen_row = n_hi;
     seen_pos = p_end;
     if (grouped) {
-      const int64_t first = pos, count = p_end - pos;
-      pos = first + count * in_group / P.group;
-      p_end = first + count * (in_group + 1) / P.group;
+      const int first = pos;
+      const int64_t count = p_end - pos;
+      pos = first + static_cast<int>(count * in_group / P.group);
+      p_end = first + static_cast<int>(count * (in_group + 1) / P.group);
     }
     // ids of the current and the next four edges, destinations of the first four of them
-    auto edge_at = [&](int64_t p) { return DST ? static_cast<int>(p) : P.edge_ids[p]; };
-    auto id_at = [&](int64_t p) { return p < p_end ? edge_at(p) : -1; };
+    auto edge_at = [&](int p) { return DST ? p : P.edge_ids[p]; };
+    auto id_at = [&](int p) { return p < p_end ? edge_at(p) : -1; };
     auto dst_of = [&](int e) { return e >= 0 ? P.dst[e] : 0; };
     int e0 = id_at(pos), e1 = id_at(pos + 1), e2 = id_at(pos + 2), e3 = id_at(pos + 3), e4 = id_at(pos + 4);
     int d0 = dst_of(e0), d1 = dst_of(e1), d2 = dst_of(e2), d3n = dst_of(e3);
@@ -479,12 +480,12 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     int refill_stage = -1;  // a stage whose row is on its way back, to be refilled with the edge `stages` after it
 #pragma unroll 1
     for (; n < n_hi; ++n) {
-      const int64_t pe = min(static_cast<int64_t>(P.src_rowptr[n + 1]), p_end);
+      const int pe = min(P.src_rowptr[n + 1], p_end);
       if (!grouped && P.tile_rows == 0 && pos >= pe) {
         // A row without edges in a piece of a graph, which has long runs of them (their gx is cleared beforehand): jump
         // to the row that holds the next edge instead of walking the run one dependent load at a time.
         if (pos >= p_end) break;
-        n = warp_lower_bound(P.src_rowptr, P.num_rows, pos + 1, lane) - 2;
+        n = static_cast<int>(warp_lower_bound(P.src_rowptr, P.num_rows, pos + 1, lane)) - 2;
         continue;
       }
       if (pos < pe) {
@@ -492,7 +493,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           constexpr int l1 = decltype(l1c)::value;
           if constexpr (S::has(S::MX, l1)) {
             constexpr int d = 2 * l1 + 1;
-            lane_load_block<PK, T, d>(P.x + n * x_row + row_ch * S::xoff(l1) + (first_ch + own) * d, stride, &xr[S::xoff(l1) * NP]);
+            lane_load_block<PK, T, d>(P.x + static_cast<int64_t>(n) * x_row + row_ch * S::xoff(l1) + (first_ch + own) * d, stride, &xr[S::xoff(l1) * NP]);
           }
         });
         if (!active) {
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           team_sync(team_warps, team);
         }
         if (want_x && active) {
-          T* to = grouped ? ring : P.gx + n * x_row;
+          T* to = grouped ? ring : P.gx + static_cast<int64_t>(n) * x_row;
           const int block = grouped ? ch : row_ch, at = grouped ? own : first_ch + own;
           static_for<0, 4>([&](auto l1c) {
             constexpr int l1 = decltype(l1c)::value, d = 2 * l1 + 1;
@@ -714,7 +715,7 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
                     const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
   auto kernel = edge_bwd_kernel<T, CPL, S, WX, WM, WY, FULL, DST, SLICED, ADD>;
-  EdgeBwdParams<T> P;
+  EdgeBwdParams<T, K::terms> P;
   P.x = static_cast<const T*>(DST ? a.g : a.x);
   P.y = static_cast<const T*>(a.y);
   P.w = static_cast<const T*>(ADD ? a.gw : a.w);
@@ -726,7 +727,8 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.src_rowptr = DST ? graph->dst_rowptr : graph->src_rowptr;
   P.edge_ids = DST ? nullptr : graph->edge_ids_by_src;
   const EdgeTables& tables = dt.edge[DST ? 1 : 0];
-  P.term_c = static_cast<const T*>(tables.term_c);
+  if constexpr (WY)
+    for (int t = 0; t < S::terms; ++t) P.term[t] = static_cast<T>(plan->edge.term_c[DST ? 1 : 0][t]);
   P.prog_c = static_cast<const T*>(tables.prog_c);
   P.prog_j = tables.prog_j;
   for (int c = 0; c < S::coff(-1, -1, -1); ++c) P.coef[c] = static_cast<T>(plan->edge.coef[DST ? 1 : 0][c]);

@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   const bool leader = member == 0 && lane == 0;
   const bool issuing = SLICED || leader;  // the pieces of a slice are copied by all lanes
   const uint32_t w_bytes = static_cast<uint32_t>(W * sizeof(T)), x_bytes = static_cast<uint32_t>(X * sizeof(T));
-  auto issue = [&](int64_t e, int s_node, int s) {  // by the issuing lanes
+  auto issue = [&](int edge, int s_node, int s) {  // by the issuing lanes
+    const int64_t e = edge;
     T* to = ring + static_cast<size_t>(s) * stage_elems;
     if constexpr (SLICED) {
       if (lane == 0) mbar_arrive_expect_tx(&bars[s], w_bytes + x_bytes);
@@ -164,33 +165,35 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   };
   const bool grouped = P.group > 1;
   const int in_group = team % P.group, group_id = team / P.group, groups = P.teams / P.group;
-  const int64_t total = static_cast<int64_t>(gridDim.x) * (grouped ? groups : P.teams);
+  // edges and rows fit 31 bits, and every register counts
+  const unsigned total = gridDim.x * static_cast<unsigned>(grouped ? groups : P.teams);
   // a group takes every total-th row; a team's first tile is its own number, and further ones come from a counter, one
   // ahead of need, so that a team that started late or met long rows simply takes fewer
-  int64_t unit = grouped ? blockIdx.x + static_cast<int64_t>(gridDim.x) * group_id
-                         : static_cast<int64_t>(blockIdx.x) * P.teams + team;
-  const int64_t units = grouped ? P.num_rows : P.num_tiles;
+  unsigned unit = grouped ? blockIdx.x + gridDim.x * group_id : blockIdx.x * P.teams + team;
+  const unsigned units = static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
 #pragma unroll 1
   while (unit < units) {
-    int64_t unit_after = unit + total;
-    int64_t n = unit, n_hi = unit + 1;
+    unsigned unit_after = unit + total;
+    int n = static_cast<int>(unit), n_hi = n + 1;
     if (!grouped) {
       if (team_warps == 1) {
-        unit_after = take_tile(counters, total, lane);
+        unit_after = static_cast<unsigned>(take_tile(counters, total, lane));
       } else {
         if (leader) tickets[team] = atomicAdd(&counters[0], 1u);
         team_sync(team_warps, team);
-        unit_after = total + static_cast<int64_t>(tickets[team]);
+        unit_after = total + tickets[team];
         team_sync(team_warps, team);
       }
-      n = unit * P.tile_rows;
-      n_hi = n + P.tile_rows < P.num_rows ? n + P.tile_rows : P.num_rows;
+      const int64_t first = unit * P.tile_rows, end = first + P.tile_rows;
+      n = static_cast<int>(first);
+      n_hi = static_cast<int>(end < P.num_rows ? end : P.num_rows);
     }
-    int64_t e = P.dst_rowptr[n], e_end = P.dst_rowptr[n_hi];
+    int e = P.dst_rowptr[n], e_end = P.dst_rowptr[n_hi];
     if (grouped) {
-      const int64_t first = e, count = e_end - e;
-      e = first + count * in_group / P.group;
-      e_end = first + count * (in_group + 1) / P.group;
+      const int first = e;
+      const int64_t count = e_end - e;
+      e = first + static_cast<int>(count * in_group / P.group);
+      e_end = first + static_cast<int>(count * (in_group + 1) / P.group);
     }
     // all stages are empty here: fill them in ring order from the current one
     if (issuing) {
@@ -201,13 +204,13 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     }
     // source node of the edge that is issued in the next iteration, attributes of the next edge
     int src_ahead = issuing && e + stages < e_end ? P.src[e + stages] : 0;
-    T y_next = lane < S::YD && e < e_end ? P.y[e * S::YD + lane] : T(0);
+    T y_next = lane < S::YD && e < e_end ? P.y[static_cast<int64_t>(e) * S::YD + lane] : T(0);
     program.run(y_next, mbuf + buf * K::m_elems, lane);
-    if (lane < S::YD && e + 1 < e_end) y_next = P.y[(e + 1) * S::YD + lane];
+    if (lane < S::YD && e + 1 < e_end) y_next = P.y[static_cast<int64_t>(e + 1) * S::YD + lane];
     __syncwarp();
 #pragma unroll 1
     for (; n < n_hi; ++n) {
-      const int64_t row_end = min(static_cast<int64_t>(P.dst_rowptr[n + 1]), e_end);
+      const int row_end = min(P.dst_rowptr[n + 1], e_end);
 #pragma unroll
       for (int a = 0; a < S::OD * NP; ++a) acc[a] = zero_packet<V>();
 #pragma unroll 1
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         const T* ws = ring + static_cast<size_t>(s) * stage_elems + own;
         const T* xs = ring + static_cast<size_t>(s) * stage_elems + W;
         program.run(y_next, mbuf + (buf ^ 1) * K::m_elems, lane);  // of the next edge; of no use after the last one
-        if (lane < S::YD && e + 2 < e_end) y_next = P.y[(e + 2) * S::YD + lane];
+        if (lane < S::YD && e + 2 < e_end) y_next = P.y[static_cast<int64_t>(e + 2) * S::YD + lane];
         const T* m_now = mbuf + buf * K::m_elems;
         static_for<0, 4>([&](auto l1c) {
           constexpr int l1 = decltype(l1c)::value;
@@ -254,7 +257,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         }
       }
       if (active) {
-        T* to = grouped ? ring : P.out + n * o_row;
+        T* to = grouped ? ring : P.out + static_cast<int64_t>(n) * o_row;
         const int block = grouped ? ch : row_ch, at = grouped ? own : first_ch + own;
         static_for<0, 4>([&](auto l3c) {
           constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
       const int threads = P.group * team_warps * 32;
       const T* parts = reinterpret_cast<const T*>(smem_raw) + static_cast<size_t>(group_id * P.group) * P.ring_elems;
       named_barrier(barrier, threads);
-      T* to = P.out + unit * o_row;
+      T* to = P.out + static_cast<int64_t>(unit) * o_row;
       for (int a = static_cast<int>(threadIdx.x) - group_id * threads; a < O; a += threads) {
         T sum = parts[a];
         for (int g = 1; g < P.group; ++g) sum += parts[static_cast<size_t>(g) * P.ring_elems + a];
