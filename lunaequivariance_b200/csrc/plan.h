@@ -157,6 +157,7 @@ struct EdgeLanes {
   int cpl = 0;         // channels per lane
   int team_warps = 0;  // warps that share an edge
   int slices = 1;      // parts of a block's channels that are launched side by side
+  int edges = 1;       // that a warp walks at a time (2: one on each half)
 };
 
 // What the edge kernels (uvu_edge.cuh) need of a plan whose path list has one of their compiled shapes.

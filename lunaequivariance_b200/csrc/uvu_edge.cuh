@@ -134,6 +134,8 @@ constexpr int kEdgeShapeMasks[kEdgeShapes][3] = {{1, 3, 3},  {1, 7, 7},   {1, 15
                                                  {7, 15, 15}, {3, 3, 1},  {7, 7, 1},   {15, 15, 1}, {2, 2, 1}};
 // Shapes whose kernels are compiled for slices too.  The others have no wide layers in use; theirs run the table kernels.
 constexpr bool edge_sliced(int id) { return id >= 3 && id <= 6; }
+// Channels per lane of the kernels that walk two edges at a time.
+constexpr bool edge_paired(int cpl) { return cpl <= 2; }
 template <int ID>
 using ShapeOf = Shape<kEdgeShapeMasks[ID][0], kEdgeShapeMasks[ID][1], kEdgeShapeMasks[ID][2]>;
 
@@ -199,14 +201,15 @@ constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
 // Small launches.  With R rows of d edges and T teams on the chip, a row per team takes d * ceil(R / T) edge steps of
 // the last team; parts of a row per team take about d * R / T.  Sharing costs two barriers and a pass through shared
 // memory per row, so it stops where the tiles of the large launches are even enough.
-inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps, int64_t wanted_tile) {
+inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps, int64_t wanted_tile,
+                            int at_once) {
   EdgeSplit s;
   const int64_t all = static_cast<int64_t>(sm_count) * teams;
   const double degree = static_cast<double>(edges) / static_cast<double>(std::max<int64_t>(rows, 1));
   if (rows <= 4 * all && degree >= 4.0) {
-    // enough parts that every SM has work, and at least two edges in a part
+    // enough parts that every SM has work, and at least two steps of a team in a part
     int want = rows * 2 <= all ? 8 : (rows <= 2 * all ? 4 : 2);
-    while (want > 1 && (want > teams || teams % want != 0 || degree < 2.0 * want)) want /= 2;
+    while (want > 1 && (want > teams || teams % want != 0 || degree < 2.0 * at_once * want)) want /= 2;
     if (want > 1 && team_warps > 1 && teams + teams / want > kNamedBarriers) want = 1;
     s.group = want;
   }
@@ -413,6 +416,39 @@ struct MatrixProgram {
       to[r * 32 + lane] = fma(b[r], yb, a[r] * ya);
     }
     if (lane < S::YD) to[own] = y;
+  }
+};
+
+// The same for two edges at a time, one to each half of the warp: place is the lane's in its half, y and the buffer are the
+// half's.
+template <typename T, typename S>
+struct HalfMatrixProgram {
+  static constexpr int rounds = 2 * S::m_rounds;
+  T a[rounds + 1], b[rounds + 1];
+  unsigned j[(rounds + 2) / 2];
+  int own;
+  __device__ __forceinline__ void load(const T* coefficients, const unsigned short* attributes, int place) {
+    own = attribute_position<S>(place);
+#pragma unroll
+    for (int r = 0; r < (rounds + 1) / 2; ++r) j[r] = 0u;
+#pragma unroll
+    for (int r = 0; r < rounds; ++r) {
+      const int m = r * 16 + place;
+      a[r] = m < S::m_total ? coefficients[m] : T(0);
+      b[r] = m < S::m_total ? coefficients[S::m_total + m] : T(0);
+      j[r / 2] |= (m < S::m_total ? static_cast<unsigned>(attributes[m]) : 0u) << (16 * (r % 2));
+    }
+  }
+  __device__ __forceinline__ void run(T y, T* to, int place) const {
+#pragma unroll
+    for (int r = 0; r < rounds; ++r) {
+      const unsigned ja = (j[r / 2] >> (16 * (r % 2))) & 255u, jb = (j[r / 2] >> (16 * (r % 2) + 8)) & 255u;
+      const T ya = __shfl_sync(0xffffffffu, y, static_cast<int>(ja & 15u), 16);
+      T yb = __shfl_sync(0xffffffffu, y, static_cast<int>(jb & 15u), 16);
+      if (S::YD == 16 && jb == kNoAttribute) yb = T(0);  // else the half's last lane holds no attribute
+      to[r * 16 + place] = fma(b[r], yb, a[r] * ya);
+    }
+    if (place < S::YD) to[own] = y;
   }
 };
 

@@ -42,6 +42,88 @@ struct EdgeFwd {
   static constexpr size_t warp_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
 };
 
+// out_k += sum_i M[i][k] * (x_i * w) for one path, over the entries of M that the pattern has.  xl / al: a lane's packets of
+// x and of the sums, of degrees l1 and l3; wq: its first weight; buffer: the edge's matrices.
+template <typename T, int CPL, typename S, int l1, int l2, int l3, typename V>
+__device__ __forceinline__ void forward_path(const T* wq, int stride, const T* buffer, const V* xl, V* al) {
+  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  constexpr int NP = PK::NP;
+  using PT = CgPattern<l1, l2, l3>;
+  const T* matrix = buffer + S::moff(l1, l2, l3);
+  V w2[NP], xw[NP];
+  T m[4];
+  lane_load<PK, T>(wq, stride, w2);
+  static_for<0, PT::n>([&](auto tc) {
+    constexpr int t = decltype(tc)::value;
+    if constexpr (edge_new_entry<PT>(t)) {
+      constexpr int i = PT::t[t].i, k = PT::t[t].k, entry = edge_entry<PT>(t);
+      if constexpr (entry % 4 == 0) edge_load_four<T>(matrix + entry, m);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        if constexpr (edge_new_row<PT>(t)) xw[p] = vmul(xl[i * NP + p], w2[p]);
+        al[k * NP + p] = vfma(bcast_packet(m[entry % 4], V{}), xw[p], al[k * NP + p]);
+      }
+    }
+  });
+}
+// The paths with a degree of zero, c their coefficient: out_k += (c y w) x_k, (c w x) y_k or (c w) sum_i y_i x_i.
+template <typename T, int CPL, typename S, int l1, int l2, int l3, typename V>
+__device__ __forceinline__ void forward_diagonal(const T* wq, int stride, const T* buffer, T c, const V* xl, V* al) {
+  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  constexpr int NP = PK::NP;
+  T y[8];
+  edge_attributes<S, l2>(buffer, y);
+  V w2[NP];
+  lane_load<PK, T>(wq, stride, w2);
+  const V scale = bcast_packet(l2 == 0 ? c * y[0] : c, V{});
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    V cw = vmul(scale, w2[p]);
+    if constexpr (l2 == 0) {
+#pragma unroll
+      for (int k = 0; k < 2 * l3 + 1; ++k) al[k * NP + p] = vfma(cw, xl[k * NP + p], al[k * NP + p]);
+    } else if constexpr (l1 == 0) {
+      cw = vmul(cw, xl[p]);
+#pragma unroll
+      for (int k = 0; k < 2 * l3 + 1; ++k) al[k * NP + p] = vfma(bcast_packet(y[k], V{}), cw, al[k * NP + p]);
+    } else {
+      V sum = vmul(bcast_packet(y[0], V{}), xl[p]);
+#pragma unroll
+      for (int i = 1; i < 2 * l1 + 1; ++i) sum = vfma(bcast_packet(y[i], V{}), xl[i * NP + p], sum);
+      al[p] = vfma(cw, sum, al[p]);
+    }
+  }
+}
+// All paths of an edge, for a lane's channels.  ws: its first weight; xs: the edge's row of x.
+template <typename T, int CPL, typename S, typename V>
+__device__ __forceinline__ void forward_edge(const T* ws, const T* xs, int ch, int own, int stride, const T* buffer,
+                                             const T* coef, V* acc) {
+  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  constexpr int NP = PK::NP;
+  static_for<0, 4>([&](auto l1c) {
+    constexpr int l1 = decltype(l1c)::value;
+    if constexpr (S::has(S::MX, l1)) {
+      constexpr int d1 = 2 * l1 + 1;
+      V xl[d1 * NP];
+      lane_load_block<PK, T, d1>(xs + ch * S::xoff(l1) + own * d1, stride, xl);
+      static_for<0, 4>([&](auto l3c) {
+        constexpr int l3 = decltype(l3c)::value;
+        static_for<0, 4>([&](auto l2c) {
+          constexpr int l2 = decltype(l2c)::value;
+          if constexpr (S::ok(l1, l2, l3)) {
+            const T* wq = ws + S::rank(l1, l2, l3) * ch;
+            V* al = &acc[S::ooff(l3) * NP];
+            if constexpr (S::diagonal(l1, l2, l3))
+              forward_diagonal<T, CPL, S, l1, l2, l3>(wq, stride, buffer, coef[S::coff(l1, l2, l3)], xl, al);
+            else
+              forward_path<T, CPL, S, l1, l2, l3>(wq, stride, buffer, xl, al);
+          }
+        });
+      });
+    }
+  });
+}
+
 // FULL: one warp per edge and 32 * CPL channels, known to the compiler.  SLICED: these are a slice of wider blocks.
 template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
@@ -116,53 +198,6 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   bool alive = true;
   int buf = 0;          // matrix buffer of the current edge
 
-  // The paths with a degree of zero, c their coefficient: out_k += (c y w) x_k, (c w x) y_k or (c w) sum_i y_i x_i.
-  auto diagonal_body = [&](auto l1c, auto l2c, auto l3c, const T* wq, const T* buffer, const V* xl, V* al) {
-    constexpr int l1 = decltype(l1c)::value, l2 = decltype(l2c)::value, l3 = decltype(l3c)::value;
-    const T c = P.coef[S::coff(l1, l2, l3)];
-    T y[8];
-    edge_attributes<S, l2>(buffer, y);
-    V w2[NP];
-    lane_load<PK, T>(wq, stride, w2);
-    const V scale = bcast_packet(l2 == 0 ? c * y[0] : c, V{});
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      V cw = vmul(scale, w2[p]);
-      if constexpr (l2 == 0) {
-#pragma unroll
-        for (int k = 0; k < 2 * l3 + 1; ++k) al[k * NP + p] = vfma(cw, xl[k * NP + p], al[k * NP + p]);
-      } else if constexpr (l1 == 0) {
-        cw = vmul(cw, xl[p]);
-#pragma unroll
-        for (int k = 0; k < 2 * l3 + 1; ++k) al[k * NP + p] = vfma(bcast_packet(y[k], V{}), cw, al[k * NP + p]);
-      } else {
-        V sum = vmul(bcast_packet(y[0], V{}), xl[p]);
-#pragma unroll
-        for (int i = 1; i < 2 * l1 + 1; ++i) sum = vfma(bcast_packet(y[i], V{}), xl[i * NP + p], sum);
-        al[p] = vfma(cw, sum, al[p]);
-      }
-    }
-  };
-  // out_k += sum_i M[i][k] * (x_i * w) for one path, over the entries of M that the pattern has
-  auto path_body = [&](auto l1c, auto l2c, auto l3c, const T* wq, const T* matrix, const V* xl, V* al) {
-    constexpr int l1 = decltype(l1c)::value, l2 = decltype(l2c)::value, l3 = decltype(l3c)::value;
-    using PT = CgPattern<l1, l2, l3>;
-    V w2[NP], xw[NP];
-    T m[4];
-    lane_load<PK, T>(wq, stride, w2);
-    static_for<0, PT::n>([&](auto tc) {
-      constexpr int t = decltype(tc)::value;
-      if constexpr (edge_new_entry<PT>(t)) {
-        constexpr int i = PT::t[t].i, k = PT::t[t].k, entry = edge_entry<PT>(t);
-        if constexpr (entry % 4 == 0) edge_load_four<T>(matrix + entry, m);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          if constexpr (edge_new_row<PT>(t)) xw[p] = vmul(xl[i * NP + p], w2[p]);
-          al[k * NP + p] = vfma(bcast_packet(m[entry % 4], V{}), xw[p], al[k * NP + p]);
-        }
-      }
-    });
-  };
   const bool grouped = P.group > 1;
   const int in_group = team % P.group, group_id = team / P.group, groups = P.teams / P.group;
   // edges and rows fit 31 bits, and every register counts
@@ -224,27 +259,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         program.run(y_next, mbuf + (buf ^ 1) * K::m_elems, lane);  // of the next edge; of no use after the last one
         if (lane < S::YD && e + 2 < e_end) y_next = P.y[static_cast<int64_t>(e + 2) * S::YD + lane];
         const T* m_now = mbuf + buf * K::m_elems;
-        static_for<0, 4>([&](auto l1c) {
-          constexpr int l1 = decltype(l1c)::value;
-          if constexpr (S::has(S::MX, l1)) {
-            constexpr int d1 = 2 * l1 + 1;
-            V xl[d1 * NP];
-            lane_load_block<PK, T, d1>(xs + ch * S::xoff(l1) + own * d1, stride, xl);
-            static_for<0, 4>([&](auto l3c) {
-              constexpr int l3 = decltype(l3c)::value;
-              static_for<0, 4>([&](auto l2c) {
-                constexpr int l2 = decltype(l2c)::value;
-                if constexpr (S::ok(l1, l2, l3)) {
-                  const T* wq = ws + S::rank(l1, l2, l3) * ch;
-                  if constexpr (S::diagonal(l1, l2, l3))
-                    diagonal_body(l1c, l2c, l3c, wq, m_now, xl, &acc[S::ooff(l3) * NP]);
-                  else
-                    path_body(l1c, l2c, l3c, wq, m_now + S::moff(l1, l2, l3), xl, &acc[S::ooff(l3) * NP]);
-                }
-              });
-            });
-          }
-        });
+        forward_edge<T, CPL, S>(ws, xs, ch, own, stride, m_now, P.coef, acc);
         buf ^= 1;
         team_sync(team_warps, team);  // every lane is done with this stage and with the matrices
         if (issuing && e + stages < e_end) {
@@ -309,46 +324,6 @@ EdgeLaunch edge_fwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
       break;
     }
   return launch;
-}
-
-template <typename T, int CPL, typename S, bool FULL, bool SLICED>
-int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
-                    const EdgeLanes& lanes, const EdgeForwardArgs& a, cudaStream_t stream) {
-  auto kernel = edge_fwd_kernel<T, CPL, S, FULL, SLICED>;
-  EdgeFwdParams<T> P;
-  P.x = static_cast<const T*>(a.x);
-  P.y = static_cast<const T*>(a.y);
-  P.w = static_cast<const T*>(a.w);
-  P.out = static_cast<T*>(a.out);
-  P.src = graph->src;
-  P.dst_rowptr = graph->dst_rowptr;
-  P.prog_c = static_cast<const T*>(dt.edge[0].prog_c);
-  P.prog_j = dt.edge[0].prog_j;
-  for (int c = 0; c < S::coff(-1, -1, -1); ++c) P.coef[c] = static_cast<T>(plan->edge.coef[0][c]);
-  P.status = dt.status;
-  P.tile_counters = next_tile_counters(plan, dt);
-  P.num_rows = graph->num_nodes;
-  P.ch = plan->edge.ch / lanes.slices;
-  P.row_ch = plan->edge.ch;
-  P.team_warps = lanes.team_warps;
-  P.accumulate = a.accumulate ? 1 : 0;
-  const EdgeLaunch launch = edge_fwd_launch<T, CPL, S>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
-  if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
-  P.stages = launch.stages;
-  P.ring_elems = launch.team_elems;
-  P.teams = launch.warps / lanes.team_warps;
-  const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
-  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps, 64);
-  P.group = split.group;
-  P.tile_rows = split.tile_rows;
-  P.num_tiles = ceil_div(std::max<int64_t>(graph->num_nodes, 1), split.tile_rows);
-  static KernelSetup setup;
-  const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
-  if (rc != LUNA_OK) return rc;
-  const dim3 grid(static_cast<unsigned>(split.blocks), static_cast<unsigned>(lanes.slices));
-  kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
-  LUNA_LAUNCH_CHECK("forward (edge family)");
-  return LUNA_OK;
 }
 
 }  // namespace edgek

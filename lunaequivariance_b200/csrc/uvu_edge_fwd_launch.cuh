@@ -1,0 +1,57 @@
+// Launches of the forward kernels of the edge family.
+#pragma once
+
+#include "uvu_edge_fwd.cuh"
+#include "uvu_pair_fwd.cuh"
+
+namespace luna {
+namespace edgek {
+
+template <typename T, int CPL, typename S, bool FULL, bool SLICED, bool PAIR>
+int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
+                    const EdgeLanes& lanes, const EdgeForwardArgs& a, cudaStream_t stream) {
+  static_assert(!PAIR || (FULL && !SLICED), "two edges at a time: a half warp's full set of channels");
+  void (*kernel)(EdgeFwdParams<T>);
+  if constexpr (PAIR)
+    kernel = pair_fwd_kernel<T, CPL, S>;
+  else
+    kernel = edge_fwd_kernel<T, CPL, S, FULL, SLICED>;
+  EdgeFwdParams<T> P;
+  P.x = static_cast<const T*>(a.x);
+  P.y = static_cast<const T*>(a.y);
+  P.w = static_cast<const T*>(a.w);
+  P.out = static_cast<T*>(a.out);
+  P.src = graph->src;
+  P.dst_rowptr = graph->dst_rowptr;
+  P.prog_c = static_cast<const T*>(dt.edge[0].prog_c);
+  P.prog_j = dt.edge[0].prog_j;
+  for (int c = 0; c < S::coff(-1, -1, -1); ++c) P.coef[c] = static_cast<T>(plan->edge.coef[0][c]);
+  P.status = dt.status;
+  P.tile_counters = next_tile_counters(plan, dt);
+  P.num_rows = graph->num_nodes;
+  P.ch = plan->edge.ch / lanes.slices;
+  P.row_ch = plan->edge.ch;
+  P.team_warps = lanes.team_warps;
+  P.accumulate = a.accumulate ? 1 : 0;
+  const EdgeLaunch launch = PAIR ? pair_fwd_launch<T, CPL, S>(plan->tuning, P.ch, dt.max_smem_optin)
+                                 : edge_fwd_launch<T, CPL, S>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
+  if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
+  P.stages = launch.stages;
+  P.ring_elems = launch.team_elems;
+  P.teams = launch.warps / lanes.team_warps;
+  const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
+  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps, 64, lanes.edges);
+  P.group = split.group;
+  P.tile_rows = split.tile_rows;
+  P.num_tiles = ceil_div(std::max<int64_t>(graph->num_nodes, 1), split.tile_rows);
+  static KernelSetup setup;
+  const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
+  if (rc != LUNA_OK) return rc;
+  const dim3 grid(static_cast<unsigned>(split.blocks), static_cast<unsigned>(lanes.slices));
+  kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
+  LUNA_LAUNCH_CHECK("forward (edge family)");
+  return LUNA_OK;
+}
+
+}  // namespace edgek
+}  // namespace luna

@@ -1,7 +1,7 @@
 // The edge kernels of one element type, channels per lane and shape.  The build compiles this file once for each
 // combination (LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE), so that they compile in parallel.
-#include "uvu_edge_bwd.cuh"
-#include "uvu_edge_fwd.cuh"
+#include "uvu_edge_bwd_launch.cuh"
+#include "uvu_edge_fwd_launch.cuh"
 
 namespace luna {
 namespace edgek {
@@ -12,11 +12,14 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::forward(const luna
                                                                       cudaStream_t stream) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
   if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
-    if (lanes.slices > 1) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, lanes, a, stream);
+    if (lanes.slices > 1) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, false>(plan, dt, graph, lanes, a, stream);
+  }
+  if constexpr (edge_paired(LUNA_EDGE_CPL)) {
+    if (lanes.edges == 2) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, true>(plan, dt, graph, lanes, a, stream);
   }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, lanes, a, stream);
-  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, lanes, a, stream);
+    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, false>(plan, dt, graph, lanes, a, stream);
+  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false, false>(plan, dt, graph, lanes, a, stream);
 }
 
 template <>
@@ -25,11 +28,14 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const lun
                                                                        cudaStream_t stream) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
   if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
-    if (lanes.slices > 1) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true>(plan, dt, graph, lanes, a, stream);
+    if (lanes.slices > 1) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, false>(plan, dt, graph, lanes, a, stream);
+  }
+  if constexpr (edge_paired(LUNA_EDGE_CPL)) {
+    if (lanes.edges == 2) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, true>(plan, dt, graph, lanes, a, stream);
   }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false>(plan, dt, graph, lanes, a, stream);
-  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false>(plan, dt, graph, lanes, a, stream);
+    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, false>(plan, dt, graph, lanes, a, stream);
+  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false, false>(plan, dt, graph, lanes, a, stream);
 }
 
 template <>
@@ -37,6 +43,11 @@ size_t EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::smem_bytes(cons
                                                                             bool backward, int max_smem) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
   const int ch = plan->edge.ch / lanes.slices;
+  if constexpr (edge_paired(LUNA_EDGE_CPL)) {
+    if (lanes.edges == 2)
+      return backward ? pair_bwd_launch<LUNA_EDGE_T, S, PairBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>>(plan->tuning, ch, max_smem).bytes
+                      : pair_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, ch, max_smem).bytes;
+  }
   if (!backward) return edge_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, lanes, ch, max_smem).bytes;
   using K = EdgeBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>;
   return edge_bwd_launch<LUNA_EDGE_T, S, K>(plan->tuning, lanes, ch, max_smem).bytes;

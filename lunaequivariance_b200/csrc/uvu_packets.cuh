@@ -68,6 +68,9 @@ __device__ __forceinline__ float make_packet(const float* vals, float) { return 
 __device__ __forceinline__ double make_packet(const double* vals, double) { return vals[0]; }
 __device__ __forceinline__ void split_packet(float a, float* vals) { vals[0] = a; }
 __device__ __forceinline__ void split_packet(double a, double* vals) { vals[0] = a; }
+__device__ __forceinline__ Pair shfl_xor_packet(Pair a, int mask) { return Pair{__shfl_xor_sync(0xffffffffu, a.v, mask)}; }
+__device__ __forceinline__ float shfl_xor_packet(float a, int mask) { return __shfl_xor_sync(0xffffffffu, a, mask); }
+__device__ __forceinline__ double shfl_xor_packet(double a, int mask) { return __shfl_xor_sync(0xffffffffu, a, mask); }
 template <typename V>
 __device__ __forceinline__ V zero_packet() {
   if constexpr (sizeof(V) == sizeof(Pair) && !std::is_floating_point<V>::value) {

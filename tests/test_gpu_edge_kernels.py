@@ -180,3 +180,18 @@ def test_values_that_are_not_finite_stay_where_they_belong(shape, mul, dtype):
             assert bool((got.isfinite() == finite).all()), what
             assert bool((got[infinite] == want[infinite]).all()), what
             assert_close(got[finite], want[finite], dtype, what)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+def test_two_edges_at_a_time(shape, dtype):
+    """16 and 32 channels, a half warp per edge: rows of odd and even lengths, one edge, rows without edges between the two
+    edges of a pair, and one gradient alone."""
+    for mul in (16, 32):
+        module = check(SHAPES[shape], mul, dtype, 31, 403, 0.0, mul + shape)
+        if mul == 16 or dtype == torch.float32:
+            assert module.op._plan.query(1) == mul // 16  # channels per lane
+        check(SHAPES[shape], mul, dtype, 150, 191, 1.5, mul + shape + 50)
+        one_gradient_alone(SHAPES[shape], mul, dtype, 150, 191, 1.5, mul + shape + 90)
+    for nodes, edges in ((1, 1), (1, 2), (2, 3), (900, 7201), (2500, 2501)):
+        check(SHAPES[shape], 16, dtype, nodes, edges, 0.5, nodes + edges)
