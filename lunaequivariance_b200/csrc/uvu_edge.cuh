@@ -16,10 +16,12 @@
 // path and per degree, the lanes copy side by side.  Each slice has its tile counters and its part of dL/dy; the parts are
 // summed in order by a second kernel.
 //
-// Two ways of handing out rows.  Large launches: a team takes tiles of consecutive rows from a counter.  Small
-// launches, in which a row per team would leave the chip waiting for the longest rows: `group` teams of a CTA share a
-// row, each a contiguous part of its edges, and the parts are summed in a fixed order through shared memory.  A row's
-// sum depends on its own edges and on `group`, not on which team got it.
+// Three ways of handing out rows.  Large launches: a team takes tiles of consecutive rows from a counter.  Small launches, in
+// which a few tiles per team would leave the chip waiting for the last ones: every CTA has an equal stretch of the edges, up
+// to whole rows, and every team of it an equal part of that, whatever the rows; a row that several teams share is summed
+// at the end, in the teams' order, through shared memory.  The forward of very few rows: `group` teams of a CTA share a row, each
+// a contiguous part of its edges, and the parts are summed in a fixed order through shared memory.  A row's sum depends on
+// its own edges and on the launch's sizes (in a group: on `group` alone), not on which team got it.
 #pragma once
 
 #include <atomic>
@@ -34,6 +36,8 @@ using namespace fastk;
 
 constexpr int kEdgeMaxStages = 4;
 constexpr int kEdgeMaxSlices = kTileCounterWords / 2;
+constexpr int64_t kPartEdges = 256;          // of a team, at most
+constexpr int64_t kPartGathered = 24 << 20;  // bytes
 constexpr int kEdgeMaxCoefs = 10;  // paths with a degree of zero
 
 // ---- shapes ---------------------------------------------------------------------------------------------------------
@@ -171,9 +175,10 @@ struct EdgeLaunch {
   size_t bytes = 0;
   int team_elems = 0;  // of shared memory
 };
-// Rows shared by `group` teams, or 1: rows are handed out in tiles.
+// Rows shared by `group` teams, or else equal parts of the edges, or else tiles of rows.
 struct EdgeSplit {
   int group = 1;
+  bool parts = false;
   int64_t blocks = 1;
   int64_t tile_rows = 1;
 };
@@ -198,22 +203,28 @@ inline int slice_ctas(int sm_count, int slices) {
 
 constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
 
-// Small launches.  With R rows of d edges and T teams on the chip, a row per team takes d * ceil(R / T) edge steps of
-// the last team; parts of a row per team take about d * R / T.  Sharing costs two barriers and a pass through shared
-// memory per row, so it stops where the tiles of the large launches are even enough.
+// Parts of the edges are even to about a row per CTA; what they lose is order: a CTA's rows are its own, so the rows that all
+// CTAs gather at a time are spread over the whole graph.  So: as long as a team's part is short, and while the node rows that
+// are gathered (`gathered` bytes) stay in L2 whoever reads them.  Groups (`may_group`): while a CTA has three rows
+// or fewer, too few for even parts; a row's sum is then the same in any piece of the graph that is as small.  Rows and edges
+// shared as before (groups of up to eight teams, then tiles) and in parts, forward / all gradients: (2, 2, 2), 64 channels,
+// 2,083 nodes of 41 edges 80 / 160 -> 78 / 148 us, 4,000 of 30 98 / 201 -> 90 / 180; 48 channels, 10,001 of 52 290 / 777 -> 258 /
+// 711; 32 channels, 4,003 of 52 100 / 202 -> 88 / 176.  With 442 edges a team (64 channels, 20,000 nodes) the two are even, and
+// with 64 MB of gathered rows ((3, 3, 3), 128 channels, 8,000 nodes) parts lose: forward 0.98 -> 1.27 ms.
 inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps, int64_t wanted_tile,
-                            int at_once) {
+                            int at_once, int64_t gathered, bool may_group) {
   EdgeSplit s;
   const int64_t all = static_cast<int64_t>(sm_count) * teams;
   const double degree = static_cast<double>(edges) / static_cast<double>(std::max<int64_t>(rows, 1));
-  if (rows <= 4 * all && degree >= 4.0) {
-    // enough parts that every SM has work, and at least two steps of a team in a part
-    int want = rows * 2 <= all ? 8 : (rows <= 2 * all ? 4 : 2);
+  const bool few = may_group && rows <= 3 * static_cast<int64_t>(sm_count);
+  if (few && degree >= 4.0) {
+    int want = 8;  // and at least two steps of a team in a part
     while (want > 1 && (want > teams || teams % want != 0 || degree < 2.0 * at_once * want)) want /= 2;
     if (want > 1 && team_warps > 1 && teams + teams / want > kNamedBarriers) want = 1;
     s.group = want;
   }
-  if (s.group > 1) {
+  if (s.group > 1 || (!few && edges <= kPartEdges * all && gathered <= kPartGathered && degree >= 4.0)) {
+    s.parts = s.group == 1;
     s.blocks = std::max<int64_t>(1, std::min<int64_t>(sm_count, rows));
     return s;
   }
@@ -271,6 +282,106 @@ __device__ __forceinline__ void team_sync(int team_warps, int team_id) {
     __syncwarp();
   else
     named_barrier(1 + team_id, team_warps * 32);
+}
+// A team's part of a launch: its edges [pos, end), the rows [n, n_hi) that they are of, and whether the first of these rows began
+// in an earlier team's part (joined) and the last one goes on in the next team's (open).
+struct TeamPart {
+  int n, n_hi, pos, end;
+  int cta_pos, cta_edges;  // the CTA's edges
+  int joined, open;
+  // the row that the next team goes on with, or -1
+  __device__ __forceinline__ int open_row() const { return open ? n_hi - 1 : -1; }
+  // whether the first row began earlier and ends here
+  __device__ __forceinline__ bool closes() const { return joined && n != open_row(); }
+};
+__device__ __forceinline__ int part_begin(int cta_pos, int cta_edges, int team, int teams) {
+  return cta_pos + static_cast<int>(static_cast<unsigned>(cta_edges) * static_cast<unsigned>(team) / static_cast<unsigned>(teams));
+}
+// The first rows that begin at `bound` or after it, one search in each half of the warp, and where they begin.  A guess is
+// looked up with its neighbours, 16 entries at a time, and mended by what they say; after three of those the interval is halved
+// (rows of very uneven length).  Not inlined: the searches of all kernels would be a sixth of the library.
+struct FoundRow {
+  int row, begin;
+};
+static __device__ __noinline__ FoundRow part_rows(const int* rowptr, int rows, int bound, float guess, float rows_per_edge, int lane) {
+  const int place = lane & 15, shift = lane & 16;
+  int lo = 0, hi = rows;  // of the answer
+  FoundRow found{rows, 0};
+  bool done = false;
+#pragma unroll 1
+  for (int step = 0; __any_sync(0xffffffffu, !done); ++step) {
+    const int wanted = step < 3 ? static_cast<int>(fminf(fmaxf(guess, 0.0f), static_cast<float>(rows))) : lo + (hi - lo) / 2;
+    const int base = max(lo, min(wanted - 8, hi - 15));
+    const int at = base + place, value = at <= hi ? rowptr[at] : 0x7fffffff;
+    const int below = __popc((__ballot_sync(0xffffffffu, value < bound) >> shift) & 0xffffu);
+    const int first = __shfl_sync(0xffffffffu, value, shift), last = __shfl_sync(0xffffffffu, value, shift + 15);
+    const int here = __shfl_sync(0xffffffffu, value, shift + min(below, 15));
+    if (done) continue;
+    if (below < 16 && (below > 0 || base == lo)) {
+      found = FoundRow{base + below, here};
+      done = true;
+    } else if (below == 16) {
+      lo = base + 16;
+      guess = static_cast<float>(lo) + static_cast<float>(bound - last) * rows_per_edge;
+    } else {
+      hi = base;
+      guess = static_cast<float>(hi) + static_cast<float>(bound - first) * rows_per_edge;
+    }
+  }
+  return found;
+}
+__device__ __forceinline__ TeamPart team_part(const int* __restrict__ rowptr, int64_t rows, int64_t edges, float rows_per_edge,
+                                              int team, int teams, int lane) {
+  TeamPart p;
+  const int all = static_cast<int>(rows), first_half = lane < 16;
+  // the CTA: the rows that begin in its stretch of the edges
+  const int from = static_cast<int>(edges * blockIdx.x / gridDim.x), to = static_cast<int>(edges * (blockIdx.x + 1) / gridDim.x);
+  const int bound = first_half ? from : to;
+  FoundRow f = part_rows(rowptr, all, bound, static_cast<float>(bound) * rows_per_edge, rows_per_edge, lane);
+  const int r0 = __shfl_sync(0xffffffffu, f.row, 0), p0 = __shfl_sync(0xffffffffu, f.begin, 0);
+  int r1 = __shfl_sync(0xffffffffu, f.row, 16), p1 = __shfl_sync(0xffffffffu, f.begin, 16);
+  if (blockIdx.x + 1 == gridDim.x) {  // rows without edges at the end
+    r1 = all;
+    p1 = static_cast<int>(edges);
+  }
+  p.cta_pos = p0;
+  p.cta_edges = p1 - p0;
+  p.pos = part_begin(p0, p.cta_edges, team, teams);
+  p.end = part_begin(p0, p.cta_edges, team + 1, teams);
+  const int mine = first_half ? p.pos : p.end;
+  const float per_edge = static_cast<float>(r1 - r0) / static_cast<float>(max(p.cta_edges, 1));
+  f = part_rows(rowptr, all, mine, static_cast<float>(r0) + static_cast<float>(mine - p0) * per_edge, per_edge, lane);
+  p.n = __shfl_sync(0xffffffffu, f.row, 0);
+  p.n_hi = __shfl_sync(0xffffffffu, f.row, 16);
+  p.joined = p.pos < p.end && __shfl_sync(0xffffffffu, f.begin, 0) > p.pos;
+  p.open = p.pos < p.end && __shfl_sync(0xffffffffu, f.begin, 16) > p.end;
+  if (team + 1 == teams) {
+    p.n_hi = r1;
+    p.open = 0;
+  }
+  if (p.joined) --p.n;
+  return p;
+}
+// The row that a team's part joined and ended gets the earlier teams' sums, which lie `stride` elements apart in shared memory, in
+// their order: by the team's threads, `elements` of the row at row(a).  After a barrier of the CTA.
+template <typename T, typename F>
+__device__ __forceinline__ void add_earlier_parts(const TeamPart& p, int row_begin, const T* parts, size_t stride, int team, int teams,
+                                                  int thread, int threads, int elements, F&& row) {
+  unsigned with_edges = 0u;  // the teams before this one, back to where the row begins, that have any of its edges
+  for (int q = team - 1, end = p.pos; q >= 0; --q) {
+    const int begin = part_begin(p.cta_pos, p.cta_edges, q, teams);
+    if (begin < end) with_edges |= 1u << q;
+    if (begin <= row_begin) break;
+    end = begin;
+  }
+#pragma unroll 1
+  for (int a = thread; a < elements; a += threads) {
+    T* to = row(a);
+    T sum = *to;
+#pragma unroll 1
+    for (unsigned left = with_edges; left != 0u; left &= left - 1u) sum += parts[(__ffs(static_cast<int>(left)) - 1) * stride + a];
+    *to = sum;
+  }
 }
 // After one wait has run out the kernel keeps its control flow (other warps may be waiting for it at a barrier), writes
 // nothing more to rely on, and stops spending time on waits.

@@ -48,11 +48,13 @@ struct EdgeBwdParams {
   T coef[kEdgeMaxCoefs];         // of the paths with a degree of zero
   int* status;
   unsigned* tile_counters;
-  int64_t num_rows, tile_rows, tile_edges, num_tiles;  // tile_rows 0: tiles are stretches of tile_edges edges
+  int64_t num_rows, num_edges, tile_rows, tile_edges, num_tiles;  // tile_rows 0: tiles are stretches of tile_edges edges
   float rows_per_edge;
   int ch, row_ch;  // channels per block, or of a slice of it; channels per block
   int64_t gy_part;  // elements between the slices' parts of gy
-  int team_warps, teams, group;
+  int team_warps, teams;
+  int parts;      // equal parts of the edges instead of tiles
+  int every_row;  // rows without edges are written too, and not cleared beforehand
   int stages, split;
   int team_elems;  // shared memory per team
   int need_w;
@@ -322,6 +324,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   uint64_t* const full = all_bars + team * (kEdgeMaxStages + kEdgeMaxSlots);
   uint64_t* const gfull = full + kEdgeMaxStages;
   unsigned* const tickets = reinterpret_cast<unsigned*>(all_bars + P.teams * (kEdgeMaxStages + kEdgeMaxSlots));
+  TeamPart* const kept = reinterpret_cast<TeamPart*>(tickets + P.teams);
 
   if (member == 0 && lane == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
@@ -418,18 +421,26 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     });
   };
 
-  const bool grouped = P.group > 1;
-  const int in_group = team % P.group, group_id = team / P.group, groups = P.teams / P.group;
+  const bool parts = P.parts != 0, every_row = P.every_row != 0;
+  int open_row = -1;  // whose sum goes to shared memory, to be added to what the next team has of it
   // edges and rows fit 31 bits, and every register counts
-  const unsigned total = gridDim.x * static_cast<unsigned>(grouped ? groups : P.teams);
-  unsigned unit = grouped ? blockIdx.x + gridDim.x * group_id : blockIdx.x * P.teams + team;
-  const unsigned units = static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
+  const unsigned total = gridDim.x * static_cast<unsigned>(P.teams);
+  unsigned unit = blockIdx.x * P.teams + team;
+  const unsigned units = parts ? total : static_cast<unsigned>(P.num_tiles);
   int seen_row = 0, seen_pos = 0;  // a row boundary this warp has seen, and where its edges begin
 #pragma unroll 1
   while (unit < units) {
     unsigned unit_after = unit + total;
-    int n = static_cast<int>(unit), n_hi = n + 1;
-    if (!grouped) {
+    int n, n_hi, pos, p_end;
+    if (parts) {
+      const TeamPart part = team_part(P.src_rowptr, P.num_rows, P.num_edges, P.rows_per_edge, team, P.teams, lane);
+      n = part.n;
+      n_hi = part.n_hi;
+      pos = part.pos;
+      p_end = part.end;
+      open_row = part.open_row();
+      if (leader) kept[team] = part;  // for the end of the launch
+    } else {
       if (team_warps == 1) {
         unit_after = static_cast<unsigned>(take_tile(counters, total, lane));
       } else {
@@ -454,17 +465,13 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
                                                                           n, lane));
       }
     }
-    const int64_t unit_now = unit;
     unit = unit_after;
     if (n >= n_hi) continue;  // a row with more edges than a tile spans several tile numbers
-    int pos = P.src_rowptr[n], p_end = P.src_rowptr[n_hi];
-    seen_row = n_hi;
-    seen_pos = p_end;
-    if (grouped) {
-      const int first = pos;
-      const int64_t count = p_end - pos;
-      pos = first + static_cast<int>(count * in_group / P.group);
-      p_end = first + static_cast<int>(count * (in_group + 1) / P.group);
+    if (!parts) {
+      pos = P.src_rowptr[n];
+      p_end = P.src_rowptr[n_hi];
+      seen_row = n_hi;
+      seen_pos = p_end;
     }
     // ids of the current and the next four edges, destinations of the first four of them
     auto edge_at = [&](int p) { return DST ? p : P.edge_ids[p]; };
@@ -490,7 +497,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
 #pragma unroll 1
     for (; n < n_hi; ++n) {
       const int pe = min(P.src_rowptr[n + 1], p_end);
-      if (!grouped && P.tile_rows == 0 && pos >= pe) {
+      if (!every_row && pos >= pe) {
         // A row without edges in a piece of a graph, which has long runs of them (their gx is cleared beforehand): jump
         // to the row that holds the next edge instead of walking the run one dependent load at a time.
         if (pos >= p_end) break;
@@ -649,44 +656,36 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
         }
       }
       if constexpr (WX) {
-        if (grouped) {  // the part goes to shared memory: bulk stores must have read the ring
+        const bool rest = n == open_row;
+        if (rest) {  // goes to shared memory: bulk stores must have read the ring
           if (issuing) bulk_wait_group_read_all();
           team_sync(team_warps, team);
         }
         if (want_x && active) {
-          T* to = grouped ? ring : P.gx + static_cast<int64_t>(n) * x_row;
-          const int block = grouped ? ch : row_ch, at = grouped ? own : first_ch + own;
+          T* to = rest ? ring : P.gx + static_cast<int64_t>(n) * x_row;
+          const int block = rest ? ch : row_ch, at = rest ? own : first_ch + own;
           static_for<0, 4>([&](auto l1c) {
             constexpr int l1 = decltype(l1c)::value, d = 2 * l1 + 1;
             if constexpr (S::has(S::MX, l1))
               lane_store_block<PK, T, d>(to + block * S::xoff(l1) + at * d, stride, &gxr[S::xoff(l1) * NP],
-                                         !grouped && P.acc_x);
+                                         !rest && P.acc_x);
           });
         }
       }
     }
     if (WM && issuing) bulk_wait_group_read_all();  // the next rows' copies reuse the stages
-    if constexpr (WX) {
-      if (grouped) {  // the parts of the row, in order
-        const int barrier = 1 + (team_warps > 1 ? P.teams : 0) + group_id;
-        const int threads = P.group * team_warps * 32;
-        const T* parts = base + static_cast<size_t>(group_id * P.group) * P.team_elems;
-        named_barrier(barrier, threads);
-        if (want_x) {
-          T* to = P.gx + unit_now * x_row;
-          for (int a = static_cast<int>(threadIdx.x) - group_id * threads; a < X; a += threads) {
-            T sum = parts[a];
-            for (int q = 1; q < P.group; ++q) sum += parts[static_cast<size_t>(q) * P.team_elems + a];
-            T* put = to + (SLICED ? slice_element<S>(S::MX, a, ch, row_ch, first_ch) : a);
-            *put = P.acc_x ? *put + sum : sum;
-          }
-        }
-        fence_async_shared();  // threads have written and read the ring; its next users are bulk copies
-        named_barrier(barrier, threads);
-      }
+  }
+  if (!parts) {
+    if (member == 0) leave_tiles(counters, total, lane);
+  } else if constexpr (WX) {
+    __syncthreads();
+    const TeamPart part = kept[team];
+    if (want_x && part.closes()) {
+      T* const row = P.gx + static_cast<int64_t>(part.n) * x_row;
+      add_earlier_parts(part, P.src_rowptr[part.n], base, P.team_elems, team, P.teams, member * 32 + lane, team_warps * 32, X,
+                        [&](int a) { return row + (SLICED ? slice_element<S>(S::MX, a, ch, row_ch, first_ch) : a); });
     }
   }
-  if (!grouped && member == 0) leave_tiles(counters, total, lane);
   if (WM && issuing) bulk_wait_group_read_all();
   if (!alive) {  // let copies that are still in flight land before the CTA's shared memory is released
     for (int d = 0; d < stages; ++d) edge_wait(&full[d], d < st ? parity : parity ^ 1u, false);

@@ -19,7 +19,7 @@ EdgeLaunch edge_bwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
       const int stages = option == 0 ? 3 : 2, split = option == 2;
       size_t team = split ? stages * w_row + g_row : stages * (w_row + g_row);
       team = (std::max(team, x_row) + 127) / 128 * 128;
-      const size_t bytes = teams * (team + (kEdgeMaxStages + kEdgeMaxSlots) * sizeof(uint64_t) + sizeof(unsigned)) +
+      const size_t bytes = teams * (team + (kEdgeMaxStages + kEdgeMaxSlots) * sizeof(uint64_t) + sizeof(unsigned) + sizeof(TeamPart)) +
                            (static_cast<size_t>(teams) * lanes.team_warps * K::warp_elems(lanes.team_warps) + K::table_elems) * sizeof(T);
       if (bytes > static_cast<size_t>(max_smem)) continue;
       launch.warps = teams * lanes.team_warps;
@@ -92,8 +92,12 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.rows_per_edge = static_cast<float>(static_cast<double>(P.num_rows) / static_cast<double>(std::max<int64_t>(edges, 1)));
   const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
   const int64_t tile = edges_per_warp(plan->tuning, 64);
-  EdgeSplit cut = edge_split(P.num_rows, edges, ctas, P.teams, lanes.team_warps, tile, lanes.edges);
-  P.group = cut.group;
+  const int64_t sources = graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;
+  EdgeSplit cut = edge_split(P.num_rows, edges, ctas, P.teams, lanes.team_warps, tile, lanes.edges,
+                             (DST ? sources : graph->num_nodes) * S::OD * plan->edge.ch * static_cast<int64_t>(sizeof(T)), false);
+  P.num_edges = edges;
+  P.parts = cut.parts;
+  P.every_row = 1;
   P.tile_rows = cut.tile_rows;
   P.tile_edges = tile_edges_for(edges, static_cast<int64_t>(ctas) * P.teams, tile);
   P.num_tiles = ceil_div(std::max<int64_t>(P.num_rows, 1), P.tile_rows);
@@ -102,10 +106,13 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   // destination range against all source rows) has long runs of rows without edges: its tiles are cut by edge count,
   // and the rows that are jumped over are cleared here.
   const bool whole = DST || graph->num_src_nodes <= 0 || graph->num_src_nodes <= graph->num_nodes + graph->num_nodes / 2;
-  if (P.group == 1 && !(whole && static_cast<double>(edges) >= 8.0 * static_cast<double>(P.num_rows))) {
-    P.tile_rows = 0;
-    P.num_tiles = ceil_div(std::max<int64_t>(edges, 1), P.tile_edges);
-    cut.blocks = std::max<int64_t>(1, std::min<int64_t>(ctas, ceil_div(P.num_tiles, P.teams)));
+  if (!(whole && (cut.parts || static_cast<double>(edges) >= 8.0 * static_cast<double>(P.num_rows)))) {
+    P.every_row = 0;
+    if (!cut.parts) {
+      P.tile_rows = 0;
+      P.num_tiles = ceil_div(std::max<int64_t>(edges, 1), P.tile_edges);
+      cut.blocks = std::max<int64_t>(1, std::min<int64_t>(ctas, ceil_div(P.num_tiles, P.teams)));
+    }
     if (a.gx && !a.acc_x)
       LUNA_CUDA_CHECK(cudaMemsetAsync(a.gx, 0, static_cast<size_t>(P.num_rows) * plan->X * sizeof(T), stream));
   }

@@ -22,12 +22,14 @@ struct EdgeFwdParams {
   T coef[kEdgeMaxCoefs];         // of the paths with a degree of zero
   int* status;
   unsigned* tile_counters;
-  int64_t num_rows, tile_rows, num_tiles;
+  int64_t num_rows, num_edges, tile_rows, num_tiles;
+  float rows_per_edge;
   int ch;          // channels per block, or of a slice of it
   int row_ch;      // channels per block
   int team_warps;  // warps per team
   int teams;       // per CTA
-  int group;       // teams that share a row, 1: tiles
+  int group;       // teams that share a row, or 1
+  int parts;       // equal parts of the edges
   int stages;
   int ring_elems;  // per team
   int accumulate;
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
                                                static_cast<size_t>(blockDim.x >> 5) * (2 * K::m_elems)) +
                    team * kEdgeMaxStages;
   unsigned* tickets = reinterpret_cast<unsigned*>(bars + (P.teams - team) * kEdgeMaxStages);
+  TeamPart* const kept = reinterpret_cast<TeamPart*>(tickets + P.teams);
   if (member == 0 && lane == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&bars[s], 1);
     fence_barrier_init();
@@ -198,19 +201,28 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   bool alive = true;
   int buf = 0;          // matrix buffer of the current edge
 
-  const bool grouped = P.group > 1;
+  const bool grouped = P.group > 1, parts = P.parts != 0;
+  int open_row = -1;  // whose sum goes to shared memory, to be added to what the next team has of it
   const int in_group = team % P.group, group_id = team / P.group, groups = P.teams / P.group;
   // edges and rows fit 31 bits, and every register counts
   const unsigned total = gridDim.x * static_cast<unsigned>(grouped ? groups : P.teams);
   // a group takes every total-th row; a team's first tile is its own number, and further ones come from a counter, one
   // ahead of need, so that a team that started late or met long rows simply takes fewer
   unsigned unit = grouped ? blockIdx.x + gridDim.x * group_id : blockIdx.x * P.teams + team;
-  const unsigned units = static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
+  const unsigned units = parts ? total : static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
 #pragma unroll 1
   while (unit < units) {
     unsigned unit_after = unit + total;
-    int n = static_cast<int>(unit), n_hi = n + 1;
-    if (!grouped) {
+    int n = static_cast<int>(unit), n_hi = n + 1, e, e_end;
+    if (parts) {
+      const TeamPart part = team_part(P.dst_rowptr, P.num_rows, P.num_edges, P.rows_per_edge, team, P.teams, lane);
+      n = part.n;
+      n_hi = part.n_hi;
+      e = part.pos;
+      e_end = part.end;
+      open_row = part.open_row();
+      if (leader) kept[team] = part;  // for the end of the launch
+    } else if (!grouped) {
       if (team_warps == 1) {
         unit_after = static_cast<unsigned>(take_tile(counters, total, lane));
       } else {
@@ -223,7 +235,10 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
       n = static_cast<int>(first);
       n_hi = static_cast<int>(end < P.num_rows ? end : P.num_rows);
     }
-    int e = P.dst_rowptr[n], e_end = P.dst_rowptr[n_hi];
+    if (!parts) {
+      e = P.dst_rowptr[n];
+      e_end = P.dst_rowptr[n_hi];
+    }
     if (grouped) {
       const int first = e;
       const int64_t count = e_end - e;
@@ -272,13 +287,14 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         }
       }
       if (active) {
-        T* to = grouped ? ring : P.out + static_cast<int64_t>(n) * o_row;
-        const int block = grouped ? ch : row_ch, at = grouped ? own : first_ch + own;
+        const bool rest = grouped || n == open_row;
+        T* to = rest ? ring : P.out + static_cast<int64_t>(n) * o_row;
+        const int block = rest ? ch : row_ch, at = rest ? own : first_ch + own;
         static_for<0, 4>([&](auto l3c) {
           constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
           if constexpr (S::has(S::MO, l3))
             lane_store_block<PK, T, d3>(to + block * S::ooff(l3) + at * d3, stride, &acc[S::ooff(l3) * NP],
-                                        !grouped && P.accumulate);
+                                        !rest && P.accumulate);
         });
       }
     }
@@ -299,7 +315,17 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     }
     unit = unit_after;
   }
-  if (!grouped && member == 0) leave_tiles(counters, total, lane);
+  if (parts) {
+    __syncthreads();
+    const TeamPart part = kept[team];
+    if (part.closes()) {
+      T* const row = P.out + static_cast<int64_t>(part.n) * o_row;
+      add_earlier_parts(part, P.dst_rowptr[part.n], reinterpret_cast<const T*>(smem_raw), P.ring_elems, team, P.teams,
+                        member * 32 + lane, team_warps * 32, O, [&](int a) { return row + (SLICED ? slice_element<S>(S::MO, a, ch, row_ch, first_ch) : a); });
+    }
+  } else if (!grouped && member == 0) {
+    leave_tiles(counters, total, lane);
+  }
   if (!alive)  // let copies that are still in flight land before the CTA's shared memory is released
     for (int d = 0; d < stages; ++d) edge_wait(&bars[d], d < s ? parity : parity ^ 1u, false);
 }
@@ -315,7 +341,7 @@ EdgeLaunch edge_fwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
     for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
       const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
-      const size_t bytes = teams * (ring + lanes.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned));
+      const size_t bytes = teams * (ring + lanes.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned) + sizeof(TeamPart));
       if (bytes > static_cast<size_t>(max_smem)) continue;
       launch.warps = teams * lanes.team_warps;
       launch.stages = stages;

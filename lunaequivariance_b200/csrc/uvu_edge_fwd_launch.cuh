@@ -40,8 +40,14 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.ring_elems = launch.team_elems;
   P.teams = launch.warps / lanes.team_warps;
   const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
-  const EdgeSplit split = edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps, 64, lanes.edges);
+  const int64_t sources = graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;
+  const EdgeSplit split =
+      edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps, 64, lanes.edges,
+                 sources * plan->X * static_cast<int64_t>(sizeof(T)), true);
   P.group = split.group;
+  P.num_edges = graph->num_edges;
+  P.rows_per_edge = static_cast<float>(static_cast<double>(P.num_rows) / static_cast<double>(std::max<int64_t>(P.num_edges, 1)));
+  P.parts = split.parts;
   P.tile_rows = split.tile_rows;
   P.num_tiles = ceil_div(std::max<int64_t>(graph->num_nodes, 1), split.tile_rows);
   static KernelSetup setup;

@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   T* const red = warp_mem + 2 * K::m_elems;
   uint64_t* const full =
       reinterpret_cast<uint64_t*>(base + static_cast<size_t>(P.teams) * (P.team_elems + K::warp_elems)) + warp * kEdgeMaxStages;
+  TeamPart* const kept = reinterpret_cast<TeamPart*>(full + (P.teams - warp) * kEdgeMaxStages);
 
   if (lane == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&full[s], 2);  // both halves' copies
@@ -83,18 +84,20 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       });
     });
   };
-  const bool grouped = P.group > 1;
+  const bool parts = P.parts != 0, every_row = P.every_row != 0;
+  int open_row = -1;  // whose sum goes to shared memory, to be added to what the next team has of it
   const bool acc_x = P.acc_x != 0;
   // gxr of one half to row n, added to what is there if `add`, and zero again
   auto store = [&](int n, int by, bool add) {
     if constexpr (WX) {
       if (half == by) {
         if (want_x) {
-          T* to = grouped ? ring : P.gx + static_cast<int64_t>(n) * X;
+          const bool rest = n == open_row;
+          T* to = rest ? ring : P.gx + static_cast<int64_t>(n) * X;
           static_for<0, 4>([&](auto l1c) {
             constexpr int l1 = decltype(l1c)::value, d = 2 * l1 + 1;
             if constexpr (S::has(S::MX, l1))
-              lane_store_block<PK, T, d>(to + ch * S::xoff(l1) + own * d, stride, &gxr[S::xoff(l1) * NP], !grouped && add);
+              lane_store_block<PK, T, d>(to + ch * S::xoff(l1) + own * d, stride, &gxr[S::xoff(l1) * NP], !rest && add);
           });
         }
 #pragma unroll
@@ -112,17 +115,23 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     }
   };
 
-  const int in_group = warp % P.group, group_id = warp / P.group, groups = P.teams / P.group;
-  const unsigned total = gridDim.x * static_cast<unsigned>(grouped ? groups : P.teams);
-  unsigned unit = grouped ? blockIdx.x + gridDim.x * group_id : blockIdx.x * P.teams + warp;
-  const unsigned units = static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
-  const bool every_row = grouped || P.tile_rows > 0;  // rows without edges are written too
+  const unsigned total = gridDim.x * static_cast<unsigned>(P.teams);
+  unsigned unit = blockIdx.x * P.teams + warp;
+  const unsigned units = parts ? total : static_cast<unsigned>(P.num_tiles);
   int seen_row = 0, seen_pos = 0;  // a row boundary this warp has seen, and where its edges begin
 #pragma unroll 1
   while (unit < units) {
     unsigned unit_after = unit + total;
-    int n = static_cast<int>(unit), n_hi = n + 1;
-    if (!grouped) {
+    int n, n_hi, pos, p_end;
+    if (parts) {
+      const TeamPart part = team_part(P.src_rowptr, P.num_rows, P.num_edges, P.rows_per_edge, warp, P.teams, lane);
+      n = part.n;
+      n_hi = part.n_hi;
+      pos = part.pos;
+      p_end = part.end;
+      open_row = part.open_row();
+      if (lane == 0) kept[warp] = part;  // for the end of the launch
+    } else {
       unit_after = static_cast<unsigned>(take_tile(P.tile_counters, total, lane));
       if (P.tile_rows > 0) {
         const int64_t first = unit * P.tile_rows, end = first + P.tile_rows;
@@ -138,17 +147,13 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
                                                                           n, lane));
       }
     }
-    const int64_t unit_now = unit;
     unit = unit_after;
     if (n >= n_hi) continue;  // a row with more edges than a tile spans several tile numbers
-    int pos = P.src_rowptr[n], p_end = P.src_rowptr[n_hi];
-    seen_row = n_hi;
-    seen_pos = p_end;
-    if (grouped) {
-      const int first = pos;
-      const int64_t count = p_end - pos;
-      pos = first + static_cast<int>(count * in_group / P.group);
-      p_end = first + static_cast<int>(count * (in_group + 1) / P.group);
+    if (!parts) {
+      pos = P.src_rowptr[n];
+      p_end = P.src_rowptr[n_hi];
+      seen_row = n_hi;
+      seen_pos = p_end;
     }
     // of this half: ids of the edges of the current and the next four pairs (-1: none), destinations of the first four
     auto id_at = [&](int p) { return p < p_end ? (DST ? p : P.edge_ids[p]) : -1; };
@@ -321,7 +326,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       }
     }
     if constexpr (WX) {
-      if (grouped) {  // the part goes to shared memory: bulk stores must have read the ring
+      if (open_row >= 0) {  // the last row's sum goes to shared memory: bulk stores must have read the ring
         if (issuing) bulk_wait_group_read_all();
         __syncwarp();
       }
@@ -334,25 +339,17 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       }
     }
     if (WM && issuing) bulk_wait_group_read_all();  // the next rows' copies reuse the stages
-    if constexpr (WX) {
-      if (grouped) {  // the parts of the row, in order
-        const int threads = P.group * 32;
-        const T* parts = base + static_cast<size_t>(group_id * P.group) * P.team_elems;
-        named_barrier(1 + group_id, threads);
-        if (want_x) {
-          T* to = P.gx + unit_now * X;
-          for (int a = static_cast<int>(threadIdx.x) - group_id * threads; a < X; a += threads) {
-            T sum = parts[a];
-            for (int q = 1; q < P.group; ++q) sum += parts[static_cast<size_t>(q) * P.team_elems + a];
-            to[a] = P.acc_x ? to[a] + sum : sum;
-          }
-        }
-        fence_async_shared();  // threads have written and read the ring; its next users are bulk copies
-        named_barrier(1 + group_id, threads);
-      }
+  }
+  if (!parts) {
+    leave_tiles(P.tile_counters, total, lane);
+  } else if constexpr (WX) {
+    __syncthreads();
+    const TeamPart part = kept[warp];
+    if (want_x && part.closes()) {
+      T* const row = P.gx + static_cast<int64_t>(part.n) * X;
+      add_earlier_parts(part, P.src_rowptr[part.n], base, P.team_elems, warp, P.teams, lane, 32, X, [&](int a) { return row + a; });
     }
   }
-  if (!grouped) leave_tiles(P.tile_counters, total, lane);
   if (WM && issuing) bulk_wait_group_read_all();
   if (!alive)  // let copies that are still in flight land before the CTA's shared memory is released
     for (int d = 0; d < stages; ++d) edge_wait(&full[d], d < st ? parity : parity ^ 1u, false);
@@ -366,7 +363,7 @@ EdgeLaunch pair_bwd_launch(const Tuning& tuning, int ch, int max_smem) {
   for (int warps = capped_warps(tuning, K::max_warps); warps >= 1 && launch.warps == 0; --warps)
     for (int stages = 3; stages >= 2; --stages) {
       const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
-      const size_t bytes = warps * (ring + K::warp_elems * sizeof(T) + kEdgeMaxStages * sizeof(uint64_t));
+      const size_t bytes = warps * (ring + K::warp_elems * sizeof(T) + kEdgeMaxStages * sizeof(uint64_t) + sizeof(TeamPart));
       if (bytes > static_cast<size_t>(max_smem)) continue;
       launch.warps = warps;
       launch.stages = stages;

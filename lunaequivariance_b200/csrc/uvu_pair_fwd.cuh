@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
   uint64_t* const bars = reinterpret_cast<uint64_t*>(reinterpret_cast<T*>(smem_raw) +
                                                      static_cast<size_t>(P.teams) * (P.ring_elems + 4 * S::m_elems)) +
                          warp * kEdgeMaxStages;
+  TeamPart* const kept = reinterpret_cast<TeamPart*>(bars + (P.teams - warp) * kEdgeMaxStages);
   if (lane == 0) {
     for (int s = 0; s < stages; ++s) mbar_init(&bars[s], 2);  // both halves' copies
     fence_barrier_init();
@@ -67,20 +68,22 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
   uint32_t parity = 0;
   bool alive = true;
   int buf = 0;
-  const bool grouped = P.group > 1;
+  const bool grouped = P.group > 1, parts = P.parts != 0;
+  int open_row = -1;  // whose sum goes to shared memory, to be added to what the next team has of it
   const int in_group = warp % P.group, group_id = warp / P.group, groups = P.teams / P.group;
   const unsigned total = gridDim.x * static_cast<unsigned>(grouped ? groups : P.teams);
   unsigned unit = grouped ? blockIdx.x + gridDim.x * group_id : blockIdx.x * P.teams + warp;
-  const unsigned units = static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
+  const unsigned units = parts ? total : static_cast<unsigned>(grouped ? P.num_rows : P.num_tiles);
 
   // acc of one half to row n, added to what is there if `add`, and zero again
   auto store = [&](int n, int by, bool add) {
     if (half == by) {
-      T* to = grouped ? ring : P.out + static_cast<int64_t>(n) * O;
+      const bool rest = grouped || n == open_row;
+      T* to = rest ? ring : P.out + static_cast<int64_t>(n) * O;
       static_for<0, 4>([&](auto l3c) {
         constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
         if constexpr (S::has(S::MO, l3))
-          lane_store_block<PK, T, d3>(to + ch * S::ooff(l3) + own * d3, stride, &acc[S::ooff(l3) * NP], !grouped && add);
+          lane_store_block<PK, T, d3>(to + ch * S::ooff(l3) + own * d3, stride, &acc[S::ooff(l3) * NP], !rest && add);
       });
 #pragma unroll
       for (int a = 0; a < S::OD * NP; ++a) acc[a] = zero_packet<V>();
@@ -99,14 +102,25 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
 #pragma unroll 1
   while (unit < units) {
     unsigned unit_after = unit + total;
-    int n = static_cast<int>(unit), n_hi = n + 1;
-    if (!grouped) {
+    int n = static_cast<int>(unit), n_hi = n + 1, e, e_end;
+    if (parts) {
+      const TeamPart part = team_part(P.dst_rowptr, P.num_rows, P.num_edges, P.rows_per_edge, warp, P.teams, lane);
+      n = part.n;
+      n_hi = part.n_hi;
+      e = part.pos;
+      e_end = part.end;
+      open_row = part.open_row();
+      if (lane == 0) kept[warp] = part;  // for the end of the launch
+    } else if (!grouped) {
       unit_after = static_cast<unsigned>(take_tile(P.tile_counters, total, lane));
       const int64_t first = unit * P.tile_rows, end = first + P.tile_rows;
       n = static_cast<int>(first);
       n_hi = static_cast<int>(end < P.num_rows ? end : P.num_rows);
     }
-    int e = P.dst_rowptr[n], e_end = P.dst_rowptr[n_hi];
+    if (!parts) {
+      e = P.dst_rowptr[n];
+      e_end = P.dst_rowptr[n_hi];
+    }
     if (grouped) {
       const int first = e;
       const int64_t count = e_end - e;
@@ -185,7 +199,17 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
     }
     unit = unit_after;
   }
-  if (!grouped) leave_tiles(P.tile_counters, total, lane);
+  if (parts) {
+    __syncthreads();
+    const TeamPart part = kept[warp];
+    if (part.closes()) {
+      T* const row = P.out + static_cast<int64_t>(part.n) * O;
+      add_earlier_parts(part, P.dst_rowptr[part.n], reinterpret_cast<const T*>(smem_raw), P.ring_elems, warp, P.teams,
+                        lane, 32, O, [&](int a) { return row + a; });
+    }
+  } else if (!grouped) {
+    leave_tiles(P.tile_counters, total, lane);
+  }
   if (!alive)  // let copies that are still in flight land before the CTA's shared memory is released
     for (int d = 0; d < stages; ++d) edge_wait(&bars[d], d < s ? parity : parity ^ 1u, false);
 }
@@ -198,7 +222,7 @@ EdgeLaunch pair_fwd_launch(const Tuning& tuning, int ch, int max_smem) {
   for (int warps = max_warps; warps >= 1 && launch.warps == 0; --warps)
     for (int stages = warps * 2 > max_warps ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
       const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
-      const size_t bytes = warps * (ring + 4 * S::m_elems * sizeof(T) + kEdgeMaxStages * sizeof(uint64_t));
+      const size_t bytes = warps * (ring + 4 * S::m_elems * sizeof(T) + kEdgeMaxStages * sizeof(uint64_t) + sizeof(TeamPart));
       if (bytes > static_cast<size_t>(max_smem)) continue;
       launch.warps = warps;
       launch.stages = stages;

@@ -195,3 +195,14 @@ def test_two_edges_at_a_time(shape, dtype):
         one_gradient_alone(SHAPES[shape], mul, dtype, 150, 191, 1.5, mul + shape + 90)
     for nodes, edges in ((1, 1), (1, 2), (2, 3), (900, 7201), (2500, 2501)):
         check(SHAPES[shape], 16, dtype, nodes, edges, 0.5, nodes + edges)
+
+
+# one warp per edge, two edges per warp, two warps per edge, slices
+@pytest.mark.parametrize("mul,dtype", [(48, torch.float32), (16, torch.float32), (160, torch.float32), (352, torch.float32),
+                                       (64, torch.float64), (32, torch.float64)])
+def test_equal_parts_of_the_edges(mul, dtype):
+    """Rows that many teams share, parts within one row, more CTAs than rows, rows without edges at either end of a part."""
+    for nodes, edges, skew in ((1, 500, 0.0), (3, 41, 0.0), (149, 1500, 0.0), (149, 1500, 2.0), (600, 9001, 3.0), (2900, 29007, 0.3)):
+        check(SHAPES[3], mul, dtype, nodes, edges, skew, nodes + mul)
+    check(SHAPES[4], mul, dtype, 300, 5003, 2.5, mul)
+    one_gradient_alone(SHAPES[4], mul, dtype, 300, 5003, 2.5, mul)
