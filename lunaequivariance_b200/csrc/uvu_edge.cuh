@@ -503,7 +503,6 @@ __device__ __forceinline__ int attribute_position(int j) {
 template <typename T, typename S>
 struct MatrixProgram {
   static_assert(S::YD <= kNoAttribute, "one lane is left without an attribute");
-  static constexpr int elems = 0;  // of shared memory
   T a[S::m_rounds + 1], b[S::m_rounds + 1];
   unsigned j[(S::m_rounds + 2) / 2];  // two attribute indices of 8 bits per round
   int own;                            // where this lane's attribute goes
@@ -560,39 +559,6 @@ struct HalfMatrixProgram {
       to[r * 16 + place] = fma(b[r], yb, a[r] * ya);
     }
     if (place < S::YD) to[own] = y;
-  }
-};
-
-// The same with the program in shared memory (whole rounds of 32 entries), for kernels that are short of registers.
-template <typename T, typename S>
-struct SharedMatrixProgram {
-  static constexpr int entries = S::m_rounds * 32;
-  static constexpr int elems = 2 * entries + entries * 2 / static_cast<int>(sizeof(T));
-  const T* c;
-  const unsigned short* j;
-  int own;
-  // by all threads of the CTA, which synchronise before the first run
-  __device__ __forceinline__ void load(T* to, const T* coefficients, const unsigned short* attributes) {
-    unsigned short* to_j = reinterpret_cast<unsigned short*>(to + 2 * entries);
-    for (int m = threadIdx.x; m < entries; m += blockDim.x) {
-      to[m] = m < S::m_total ? coefficients[m] : T(0);
-      to[entries + m] = m < S::m_total ? coefficients[S::m_total + m] : T(0);
-      to_j[m] = m < S::m_total ? attributes[m] : static_cast<unsigned short>(0);
-    }
-    c = to;
-    j = to_j;
-    own = attribute_position<S>(static_cast<int>(threadIdx.x & 31));
-  }
-  __device__ __forceinline__ void run(T y, T* to, int lane) const {
-#pragma unroll
-    for (int r = 0; r < S::m_rounds; ++r) {
-      const int m = r * 32 + lane;
-      const unsigned which = j[m];
-      const T ya = __shfl_sync(0xffffffffu, y, static_cast<int>(which & 255u));
-      const T yb = __shfl_sync(0xffffffffu, y, static_cast<int>(which >> 8));
-      to[m] = fma(c[entries + m], yb, c[m] * ya);
-    }
-    if (lane < S::YD) to[own] = y;
   }
 };
 

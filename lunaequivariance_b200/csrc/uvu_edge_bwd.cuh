@@ -70,15 +70,7 @@ struct EdgeBwd {
   static constexpr int state =
       (S::XD * CPL * (WX ? 2 : 1) + (WY ? S::YD * pair : 0) + (2 * S::LO + 1) * CPL) * words;
   static constexpr int program_regs = WM ? S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 : 0;
-  // The program goes to shared memory where the registers that it frees make room for 16 warps instead of 12.  One instance
-  // is like that: degrees (2, 2, 2) with two FP32 channels per lane.  52 edges per node, best of nine: 5.2 M edges of 64
-  // channels 6.90 -> 6.44 ms, 0.11 M edges 0.188 -> 0.180; 2.1 M edges of 48 channels, where the kernel spills 20 bytes, 3.03
-  // -> 2.89.  Elsewhere the reads cost more than the room gives: (3, 3, 3), 12 warps for 8, 6.38 -> 7.07 ms; dL/dw alone in
-  // FP64 5.36 -> 6.16 ms.
-  static constexpr bool shared_program =
-      WX && WM && WY && pair == 2 && warps_for(state + program_regs + 48) == 12 && warps_for(state + 48) == 16;
-  using Program = std::conditional_t<shared_program, SharedMatrixProgram<T, S>, MatrixProgram<T, S>>;
-  static constexpr int registers = state + (shared_program ? 0 : program_regs) + 48;  // an estimate; beyond 255 it spills hundreds of bytes
+  static constexpr int registers = state + program_regs + 48;  // an estimate; beyond 255 it spills hundreds of bytes
   static constexpr int max_warps = warps_for(registers);
   // slots of g: the highest degree has one, the others share one
   static constexpr int slot_of(int l3) { return l3 == S::LO && S::ooff(S::LO) > 0 ? 1 : 0; }
@@ -97,7 +89,6 @@ struct EdgeBwd {
     return m_elems + (WY ? red_pass * red_row + (team_warps > 1 ? 64 : 0) : 0);
   }
   static constexpr int terms = WY && S::terms > 0 ? S::terms : 1;
-  static constexpr int table_elems = WM ? Program::elems : 0;
 };
 
 // One path for a lane's packets.  xl / gxl: the lane's x and gx packets of degree l1; g2: its g packets of degree l3;
@@ -319,8 +310,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   T* const mbuf = warp_mem + static_cast<size_t>(warp) * warp_elems;
   T* const red = mbuf + K::m_elems;
   T* const gbuf = red + K::red_pass * K::red_row;
-  T* const tables = warp_mem + static_cast<size_t>(blockDim.x >> 5) * warp_elems;
-  uint64_t* const all_bars = reinterpret_cast<uint64_t*>(tables + K::table_elems);
+  uint64_t* const all_bars = reinterpret_cast<uint64_t*>(warp_mem + static_cast<size_t>(blockDim.x >> 5) * warp_elems);
   uint64_t* const full = all_bars + team * (kEdgeMaxStages + kEdgeMaxSlots);
   uint64_t* const gfull = full + kEdgeMaxStages;
   unsigned* const tickets = reinterpret_cast<unsigned*>(all_bars + P.teams * (kEdgeMaxStages + kEdgeMaxSlots));
@@ -331,11 +321,8 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     for (int s = 0; s < K::slots; ++s) mbar_init(&gfull[s], 1);
     fence_barrier_init();
   }
-  typename K::Program program;
-  if constexpr (K::shared_program)
-    program.load(tables, P.prog_c, P.prog_j);
-  else if constexpr (WM)
-    program.load(P.prog_c, P.prog_j, lane);
+  MatrixProgram<T, S> program;
+  if constexpr (WM) program.load(P.prog_c, P.prog_j, lane);
   __syncthreads();
 
   const int cpw = ch / team_warps;  // channels of this warp

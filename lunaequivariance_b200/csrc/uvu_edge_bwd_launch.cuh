@@ -20,7 +20,7 @@ EdgeLaunch edge_bwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
       size_t team = split ? stages * w_row + g_row : stages * (w_row + g_row);
       team = (std::max(team, x_row) + 127) / 128 * 128;
       const size_t bytes = teams * (team + (kEdgeMaxStages + kEdgeMaxSlots) * sizeof(uint64_t) + sizeof(unsigned) + sizeof(TeamPart)) +
-                           (static_cast<size_t>(teams) * lanes.team_warps * K::warp_elems(lanes.team_warps) + K::table_elems) * sizeof(T);
+                           (static_cast<size_t>(teams) * lanes.team_warps * K::warp_elems(lanes.team_warps)) * sizeof(T);
       if (bytes > static_cast<size_t>(max_smem)) continue;
       launch.warps = teams * lanes.team_warps;
       launch.stages = stages;
