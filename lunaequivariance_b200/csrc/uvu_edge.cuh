@@ -488,7 +488,10 @@ __device__ __forceinline__ void lane_store_block(T* p, int stride, const typenam
 }
 
 // The program that turns an edge's attributes, one per lane, into its coupling matrices: entry m is a_m y[ja] + b_m
-// y[jb].  Lane l makes entries l, l + 32, ...  An entry made of one attribute only takes kNoAttribute as its second, a lane
+// y[jb].  Entries are made in rounds of 32, one to a lane; `team_warps` warps that share the
+// matrices take turns.  The forward's teams do, which leaves FP64, degrees (2, 3, 3), 128 channels room for four teams instead of
+// three: 0.4 M edges 1.55 -> 1.40 ms.  The backward's warps have matrices of their own: shared ones cost it a barrier an edge, or
+// the order of events (all gradients of the same case 4.31 -> 4.57).  An entry made of one attribute only takes kNoAttribute as its second, a lane
 // that holds no attribute but zero: with any attribute in its place 0 times an infinite one would make the entry NaN.
 constexpr int kNoAttribute = 31;
 // Where lane j stores attribute j of the edge, behind the matrices.
@@ -506,26 +509,28 @@ struct MatrixProgram {
   T a[S::m_rounds + 1], b[S::m_rounds + 1];
   unsigned j[(S::m_rounds + 2) / 2];  // two attribute indices of 8 bits per round
   int own;                            // where this lane's attribute goes
-  __device__ __forceinline__ void load(const T* coefficients, const unsigned short* attributes, int lane) {
+  __device__ __forceinline__ void load(const T* coefficients, const unsigned short* attributes, int lane, int member, int team_warps) {
     own = attribute_position<S>(lane);
 #pragma unroll
     for (int r = 0; r < (S::m_rounds + 1) / 2; ++r) j[r] = 0u;
 #pragma unroll
     for (int r = 0; r < S::m_rounds; ++r) {
-      const int m = r * 32 + lane;
+      const int m = (r * team_warps + member) * 32 + lane;
       a[r] = m < S::m_total ? coefficients[m] : T(0);
       b[r] = m < S::m_total ? coefficients[S::m_total + m] : T(0);
       j[r / 2] |= (m < S::m_total ? static_cast<unsigned>(attributes[m]) : 0u) << (16 * (r % 2));
     }
   }
-  __device__ __forceinline__ void run(T y, T* to, int lane) const {
+  __device__ __forceinline__ void run(T y, T* to, int lane, int member, int team_warps) const {
 #pragma unroll
     for (int r = 0; r < S::m_rounds; ++r) {
+      const int round = r * team_warps + member;
+      if (round >= S::m_rounds) break;  // never with one warp
       const T ya = __shfl_sync(0xffffffffu, y, static_cast<int>((j[r / 2] >> (16 * (r % 2))) & 255u));
       const T yb = __shfl_sync(0xffffffffu, y, static_cast<int>((j[r / 2] >> (16 * (r % 2) + 8)) & 255u));
-      to[r * 32 + lane] = fma(b[r], yb, a[r] * ya);
+      to[round * 32 + lane] = fma(b[r], yb, a[r] * ya);
     }
-    if (lane < S::YD) to[own] = y;
+    if (member == 0 && lane < S::YD) to[own] = y;
   }
 };
 

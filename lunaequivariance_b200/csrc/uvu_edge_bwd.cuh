@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     fence_barrier_init();
   }
   MatrixProgram<T, S> program;
-  if constexpr (WM) program.load(P.prog_c, P.prog_j, lane);
+  if constexpr (WM) program.load(P.prog_c, P.prog_j, lane, 0, 1);
   __syncthreads();
 
   const int cpw = ch / team_warps;  // channels of this warp
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       if (split) static_for<0, K::slots>([&](auto h) { load_slot(h, d0); });
     }
     T y_next = lane < S::YD && e0 >= 0 ? P.y[static_cast<int64_t>(e0) * S::YD + lane] : T(0);
-    if constexpr (WM) program.run(y_next, mbuf, lane);
+    if constexpr (WM) program.run(y_next, mbuf, lane, 0, 1);
     if (WM && e1 >= 0 && lane < S::YD) y_next = P.y[static_cast<int64_t>(e1) * S::YD + lane];
     __syncwarp();
     int refill_stage = -1;  // a stage whose row is on its way back, to be refilled with the edge `stages` after it
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           }
         }
         if (storing) refill_stage = st;
-        if constexpr (WM) program.run(y_next, mbuf, lane);
+        if constexpr (WM) program.run(y_next, mbuf, lane, 0, 1);
         if (WM && pos + 2 < p_end && lane < S::YD) y_next = P.y[static_cast<int64_t>(e2) * S::YD + lane];
         if constexpr (WY) {
           // the lanes' partial gy rows through the reduction tile: entries 2r and 2r + 1 in tile row r; four lanes sum

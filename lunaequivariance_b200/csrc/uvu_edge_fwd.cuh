@@ -41,7 +41,7 @@ struct EdgeFwd {
   static constexpr int m_elems = S::m_elems;
   static constexpr int max_warps =
       warps_for((S::OD + S::XD) * CPL * words + S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 + 44);
-  static constexpr size_t warp_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
+  static constexpr size_t team_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
 };
 
 // out_k += sum_i M[i][k] * (x_i * w) for one path, over the entries of M that the pattern has.  xl / al: a lane's packets of
@@ -148,10 +148,10 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
 
   T* ring = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(team) * P.ring_elems;
   T* mbuf = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(P.teams) * P.ring_elems +
-            static_cast<size_t>(warp) * (2 * K::m_elems);
+            static_cast<size_t>(team) * (2 * K::m_elems);
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<T*>(smem_raw) +
                                                static_cast<size_t>(P.teams) * P.ring_elems +
-                                               static_cast<size_t>(blockDim.x >> 5) * (2 * K::m_elems)) +
+                                               static_cast<size_t>(P.teams) * (2 * K::m_elems)) +
                    team * kEdgeMaxStages;
   unsigned* tickets = reinterpret_cast<unsigned*>(bars + (P.teams - team) * kEdgeMaxStages);
   TeamPart* const kept = reinterpret_cast<TeamPart*>(tickets + P.teams);
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   }
 
   MatrixProgram<T, S> program;
-  program.load(P.prog_c, P.prog_j, lane);
+  program.load(P.prog_c, P.prog_j, lane, member, team_warps);
   __syncthreads();
 
   const int cpw = ch / team_warps;  // channels of this warp
@@ -255,9 +255,9 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     // source node of the edge that is issued in the next iteration, attributes of the next edge
     int src_ahead = issuing && e + stages < e_end ? P.src[e + stages] : 0;
     T y_next = lane < S::YD && e < e_end ? P.y[static_cast<int64_t>(e) * S::YD + lane] : T(0);
-    program.run(y_next, mbuf + buf * K::m_elems, lane);
+    program.run(y_next, mbuf + buf * K::m_elems, lane, member, team_warps);
     if (lane < S::YD && e + 1 < e_end) y_next = P.y[static_cast<int64_t>(e + 1) * S::YD + lane];
-    __syncwarp();
+    team_sync(team_warps, team);
 #pragma unroll 1
     for (; n < n_hi; ++n) {
       const int row_end = min(P.dst_rowptr[n + 1], e_end);
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         }
         const T* ws = ring + static_cast<size_t>(s) * stage_elems + own;
         const T* xs = ring + static_cast<size_t>(s) * stage_elems + W;
-        program.run(y_next, mbuf + (buf ^ 1) * K::m_elems, lane);  // of the next edge; of no use after the last one
+        program.run(y_next, mbuf + (buf ^ 1) * K::m_elems, lane, member, team_warps);  // of the next edge; of no use after the last one
         if (lane < S::YD && e + 2 < e_end) y_next = P.y[static_cast<int64_t>(e + 2) * S::YD + lane];
         const T* m_now = mbuf + buf * K::m_elems;
         forward_edge<T, CPL, S>(ws, xs, ch, own, stride, m_now, P.coef, acc);
@@ -341,7 +341,7 @@ EdgeLaunch edge_fwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
     for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
       const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
-      const size_t bytes = teams * (ring + lanes.team_warps * K::warp_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned) + sizeof(TeamPart));
+      const size_t bytes = teams * (ring + K::team_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned) + sizeof(TeamPart));
       if (bytes > static_cast<size_t>(max_smem)) continue;
       launch.warps = teams * lanes.team_warps;
       launch.stages = stages;
