@@ -159,6 +159,15 @@ extern "C" int luna_uvu_conv_dbl_bwd(luna_uvu_plan* plan, const luna_graph* grap
     return zero_fill(hg, N * plan->O, es, stream);
   }
   const bool fast = use_fast(plan, {x, w, g, rx, rw, hx, hw, hg});
+  // Force training without a gradient of the features: only ry is there, and hg = F_g(x, ry, w) and hw = F_w(x, ry, g) share
+  // their operands.
+  const bool together = fast && plan->edge.shape >= 0 && ry && !rx && !rw && hg && hw && !hx && edgek::joins_output(plan);
+  if (together) {
+    const DeviceTables* dt = nullptr;
+    LUNA_TRY(get_device_tables(plan, &dt));
+    LUNA_TRY(edgek::output_and_weights(plan, *dt, graph, x, ry, w, g, hg, hw, stream));
+    return hy ? zero_fill(hy, E * plan->Y, es, stream) : LUNA_OK;
+  }
 
   // hg = F_g(rx, y, w) + F_g(x, ry, w) + F_g(x, y, rw): a forward pass on the tangents.
   if (hg) {

@@ -259,6 +259,10 @@ int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph*
 int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
              const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w, void* scratch,
              int64_t scratch_bytes, cudaStream_t stream);
+// The output F_g(x, y, w) and gw = F_w(x, y, g) in one launch.
+int output_and_weights(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
+                       const void* w, const void* g, void* out, void* gw, cudaStream_t stream);
+bool joins_output(const luna_uvu_plan* plan);  // whether that launch pays
 // Of a plan with a shape: the highest edge-attribute degree if its degrees are all of 0..l, else -1; shared memory of a block.
 int canonical_l2(const luna_uvu_plan* plan);
 size_t smem_bytes(const luna_uvu_plan* plan, bool backward, int max_smem);

@@ -199,9 +199,25 @@ int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph*
 int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
              const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w, void* scratch,
              int64_t scratch_bytes, cudaStream_t stream) {
-  const EdgeBackwardArgs args{x, y, w, g, gx, gy, gw, acc_x, acc_y, acc_w, scratch, scratch_bytes};
+  const EdgeBackwardArgs args{x, y, w, g, gx, gy, gw, acc_x, acc_y, acc_w, scratch, scratch_bytes, nullptr};
   const EdgeLanes& lanes = gy && (gx || gw) ? plan->edge.lanes_all : plan->edge.lanes;
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
+}
+
+int output_and_weights(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
+                       const void* w, const void* g, void* out, void* gw, cudaStream_t stream) {
+  const EdgeBackwardArgs args{x, y, w, g, nullptr, nullptr, gw, false, false, false, nullptr, 0, out};
+  const EdgeLanes& lanes = plan->edge.lanes;
+  return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
+}
+
+bool joins_output(const luna_uvu_plan* plan) {
+  bool joins = false;
+  with_instance(plan, plan->edge.lanes, [&](auto kernels) {
+    joins = kernels.joins_output();
+    return LUNA_OK;
+  });
+  return joins;
 }
 
 int canonical_l2(const luna_uvu_plan* plan) {

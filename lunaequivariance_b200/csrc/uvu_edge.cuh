@@ -155,6 +155,7 @@ struct EdgeBackwardArgs {
   bool acc_x, acc_y, acc_w;
   void* scratch;  // for the slices' parts of gy
   int64_t scratch_bytes;
+  void* out;  // with gw alone: the output as well, if not null
 };
 // The kernels of one (element type, channels per lane, shape), compiled in a file of their own.
 template <typename T, int CPL, int ID>
@@ -163,6 +164,7 @@ struct EdgeKernels {
                      const EdgeLanes& lanes, const EdgeForwardArgs& a, cudaStream_t stream);
   static int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                       const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream);
+  static bool joins_output();  // whether output and gw come in one launch
   // shared memory of a block of the forward kernel, or of the backward kernel of all gradients
   static size_t smem_bytes(const luna_uvu_plan* plan, const EdgeLanes& lanes, bool backward, int max_smem);
 };

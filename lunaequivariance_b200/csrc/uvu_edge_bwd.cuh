@@ -18,6 +18,10 @@
 // the other in memory, g stays in registers for the row and x is gathered.  Taken where a row of x is no longer than a row
 // of g, which is then the smaller gather (layers that widen their degrees, first layers most of all).
 //
+// Output and gw in one pass.  With the roles exchanged a row's sum is the output, so the kernel of gx and gw, by destination,
+// makes the output and gw together: the second order of force training wants both for the same operands, and they share the
+// weights' and the features' way from memory and the products of the coupling matrices with x.
+//
 // gw alone, added to what is there: the rows that are added to arrive in the stages in the weights' place, and the sums
 // begin with them.
 //

@@ -47,7 +47,7 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.y = static_cast<const T*>(a.y);
   P.w = static_cast<const T*>(ADD ? a.gw : a.w);
   P.g = static_cast<const T*>(DST ? a.x : a.g);
-  P.gx = static_cast<T*>(a.gx);
+  P.gx = static_cast<T*>(DST ? a.out : a.gx);
   P.gy = static_cast<T*>(a.gy);
   P.gw = static_cast<T*>(a.gw);
   P.dst = DST ? graph->src : graph->dst;
@@ -65,7 +65,7 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.ch = plan->edge.ch / lanes.slices;
   P.row_ch = plan->edge.ch;
   P.team_warps = lanes.team_warps;
-  P.need_w = ADD || a.gx != nullptr || a.gy != nullptr;
+  P.need_w = ADD || WX || a.gx != nullptr || a.gy != nullptr;
   P.acc_x = a.acc_x;
   P.acc_y = a.acc_y;
   P.acc_w = !ADD && a.acc_w;
@@ -113,8 +113,8 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
       P.num_tiles = ceil_div(std::max<int64_t>(edges, 1), P.tile_edges);
       cut.blocks = std::max<int64_t>(1, std::min<int64_t>(ctas, ceil_div(P.num_tiles, P.teams)));
     }
-    if (a.gx && !a.acc_x)
-      LUNA_CUDA_CHECK(cudaMemsetAsync(a.gx, 0, static_cast<size_t>(P.num_rows) * plan->X * sizeof(T), stream));
+    if (WX && P.gx && !a.acc_x)
+      LUNA_CUDA_CHECK(cudaMemsetAsync(P.gx, 0, static_cast<size_t>(P.num_rows) * S::XD * plan->edge.ch * sizeof(T), stream));
   }
   static KernelSetup setup;
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
@@ -130,10 +130,23 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   return LUNA_OK;
 }
 
+// Whether output and gw come in one launch: unless the sums cost half the warps that gw alone has (128 channels of a first layer).
+// Forward and gw in turn, and together: FP64, (2, 3, 3), 128 channels, 0.4 M edges 3.83 -> 2.75 ms; FP32, the same, 1.05 M edges
+// 3.95 -> 3.13; (2, 2, 2), 64 channels, 5.2 M edges 6.72 -> 5.09; (0, 3, 3), 128 channels, 1.05 M edges 1.06 -> 1.20.
+template <typename T, int CPL, typename S>
+constexpr bool edge_joins_output() {
+  using R = Transposed<S>;
+  return 2 * EdgeBwd<T, CPL, R, true, true, false>::max_warps > EdgeBwd<T, CPL, R, false, true, false>::max_warps;
+}
+
 template <typename T, int CPL, typename S, bool FULL, bool SLICED, bool PAIR>
 int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                       const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
   const bool wx = a.gx != nullptr, ww = a.gw != nullptr, wy = a.gy != nullptr;
+  if constexpr (edge_joins_output<T, CPL, S>()) {
+    if (a.out)
+      return launch_edge_bwd<T, CPL, Transposed<S>, true, true, false, FULL, true, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
+  }
   // One gradient per edge and none per row.  FP64, degrees (2, 3, 3), 128 channels, 1.05 M edges: rows by source 5.91 ms
   // (gw) and 6.44 ms (gy), by destination 5.36 and 5.95 ms.
   if (!wx && ww != wy) {

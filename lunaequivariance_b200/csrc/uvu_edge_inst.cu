@@ -39,6 +39,11 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const lun
 }
 
 template <>
+bool EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::joins_output() {
+  return edge_joins_output<LUNA_EDGE_T, LUNA_EDGE_CPL, ShapeOf<LUNA_EDGE_SHAPE>>();
+}
+
+template <>
 size_t EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::smem_bytes(const luna_uvu_plan* plan, const EdgeLanes& lanes,
                                                                             bool backward, int max_smem) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
