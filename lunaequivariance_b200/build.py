@@ -28,6 +28,8 @@ NVCC_FLAGS = [
     "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "--expt-relaxed-constexpr",
+    # 2.2 MB of device code a unit become 0.4; a module is unpacked when its first kernel is loaded
+    "--compress-mode=size",
 ]
 
 
