@@ -206,3 +206,29 @@ def test_equal_parts_of_the_edges(mul, dtype):
         check(SHAPES[3], mul, dtype, nodes, edges, skew, nodes + mul)
     check(SHAPES[4], mul, dtype, 300, 5003, 2.5, mul)
     one_gradient_alone(SHAPES[4], mul, dtype, 300, 5003, 2.5, mul)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+def test_output_and_weight_gradient_of_the_second_order(shape, dtype):
+    """The two in one call, as force training asks for them: one launch, or two where that is faster."""
+    from lunaequivariance_b200 import conv as conv_mod
+
+    for mul, nodes, edges, skew in ((16, 150, 191, 1.5), (48, 31, 403, 0.0), (128, 60, 90, 1.0), (352, 7, 120, 0.0)):
+        in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
+        instructions = all_paths(in1, in2, out)
+        module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False, dtype=dtype)
+        meta = oracle_conv.build_specs(in1, in2, out, instructions)
+        generator = torch.Generator().manual_seed(shape + mul)
+        src, dst = skewed_graph(nodes, edges, generator, skew)
+        p = random_problem((meta["in1_dim"], meta["in2_dim"], meta["out_dim"], meta["weight_numel"]), nodes, src, dtype,
+                           generator)
+        ref = oracle_conv.conv_derivatives(meta, *(p[k].double() for k in ("x", "y", "w")), src, dst, nodes, p["g"].double(),
+                                           None, p["ry"].double(), None)
+        graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+        x, y, w, g, ry = (p[k].to(DEVICE) for k in ("x", "y", "w", "g", "ry"))
+        hx, hy, hw, hg = conv_mod.run_double_backward(module.op, x, y, w, g, None, ry, None, graph, needs=(False, False, True, True))
+        module.op.check_status()
+        assert hx is None and hy is None
+        assert_close(hw, ref["hw"], dtype, f"{SHAPES[shape]} x{mul} {dtype} hw")
+        assert_close(hg, ref["hg"], dtype, f"{SHAPES[shape]} x{mul} {dtype} hg")
