@@ -164,7 +164,8 @@ struct EdgeLanes {
 struct EdgePlan {
   int shape = -1;      // index of the compiled shape, -1 if the plan has none or is kept from its kernels
   int ch = 0;          // channels per block
-  EdgeLanes lanes;
+  EdgeLanes lanes;      // of the forward
+  EdgeLanes lanes_one;  // of backward calls that want one gradient, or dL/dx and dL/dw
   EdgeLanes lanes_all;  // of backward calls that want dL/dy and another gradient
   // [0] of the shape, [1] of the shape with x and out exchanged
   std::vector<double> prog_c[2], term_c[2], coef[2];

@@ -9,6 +9,8 @@ namespace edgek {
 
 namespace {
 
+enum class EdgeUse { kForward, kOneGradient, kAllGradients };
+
 // Whether the kernel of all gradients spills registers by hundreds of bytes (a few bytes are common, and harmless).
 template <typename T, int CPL, int... ID>
 bool spills(int shape, std::integer_sequence<int, ID...>) {
@@ -22,12 +24,26 @@ bool spills(const luna_uvu_plan* plan, int shape, int cpl) {
   return cpl == 4 ? spills<float, 4>(shape, all) : (cpl == 2 ? spills<float, 2>(shape, all) : spills<float, 1>(shape, all));
 }
 
+template <int... ID>
+bool paired(int shape, int cpl, std::integer_sequence<int, ID...>) {
+  bool found = false;
+  ((found = found || (shape == ID && edge_paired<ID>(cpl))), ...);
+  return found;
+}
+bool paired(int shape, int cpl) { return paired(shape, cpl, std::make_integer_sequence<int, kEdgeShapes>{}); }
+
 // Channels per lane and warps per team, or slices for blocks that no team takes.  A warp's pass over an edge costs about one
 // unit of fixed work plus one per channel of a lane, so 48 channels take one warp with two channels on 24 lanes, 96 one warp
 // with four on 24 lanes.  A kernel that spills counts half as much again: degrees (3, 3, 3) with the most channels per lane,
 // all gradients.  300 MB of weights, FP64: 96 channels 0.64 -> 0.52 ms with one channel per lane, 224 channels 0.72 -> 0.49;
 // FP32: 128 channels 0.41 -> 0.30 with two, 256 channels 0.57 -> 0.34.
-EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, bool all_gradients, bool sliced) {
+//
+// 16 channels per lane of half a warp: two edges at a time, if the rows of two pairs leave room for eight warps.  With fewer it
+// loses: FP64, 32 channels, degrees (2, 3, 3), six warps, all gradients of 0.4 M edges 1.30 -> 1.75 ms.  64 channels, one edge and
+// two, forward / all gradients / dL/dy / dL/dw, 0.8 M edges: (1, 1, 1) 165 / 555 / 322 / 416 -> 174 / 380 / 194 / 260 us; (1, 1, 0)
+// 143 / 476 / 330 / 250 -> 156 / 310 / 188 / 231; (0, 2, 2), 1.05 M edges, 282 / 710 / 422 / 518 -> 215 / 478 / 250 / 332; (2, 2, 0)
+// 233 / 545 / 370 / 424 -> 176 / 439 / 215 / 268.  So the forward has it at degree 2 only.
+EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool sliced) {
   const int ch = plan->edge.ch, elem = plan->dtype == LUNA_F64 ? 8 : 4;
   // one team with two stages must fit an SM's shared memory in either direction
   const size_t room = 200 * 1024, W = static_cast<size_t>(plan->W) * elem, X = static_cast<size_t>(plan->X) * elem,
@@ -41,16 +57,17 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, bool all_gradients,
     if (sliced ? ch % (32 * cpl) != 0 || parts > kEdgeMaxSlices
                : parts > capped_warps(plan->tuning, 8) || ch % (parts * cpl) != 0 || rows + parts * 8192 > room)
       continue;
-    const double cost = parts * (1 + cpl) * (all_gradients && spills(plan, shape, cpl) ? 1.5 : 1.0);
+    const double cost = parts * (1 + cpl) * (use == EdgeUse::kAllGradients && spills(plan, shape, cpl) ? 1.5 : 1.0);
     if (best.cpl != 0 && cost >= best_cost) continue;
     best_cost = cost;
     best = sliced ? EdgeLanes{cpl, 1, parts} : EdgeLanes{cpl, parts, 1};
   }
-  // 16 or 32 channels: two edges at a time, if the rows of two pairs leave room for eight warps.  (With fewer it loses: FP64, 32
-  // channels, degrees (2, 3, 3), six warps, all gradients of 0.4 M edges 1.30 -> 1.75 ms.)
-  if (!sliced && ch % 16 == 0 && ch / 16 <= 2 && (plan->tuning.lane_channels == 0 || plan->tuning.lane_channels == ch / 16) &&
+  const int half = ch / 16, *masks = kEdgeShapeMasks[shape];
+  const bool lanes_exist = ch % 16 == 0 && (half == 1 || half == 2 || (half == 4 && elem == 4 &&
+                                                                       (use != EdgeUse::kForward || (masks[0] | masks[2]) >= 4)));
+  if (!sliced && lanes_exist && paired(shape, half) && (plan->tuning.lane_channels == 0 || plan->tuning.lane_channels == half) &&
       4 * (W + std::max(X, O)) <= 24 * 1024)
-    return EdgeLanes{ch / 16, 1, 1, 2};
+    return EdgeLanes{half, 1, 1, 2};
   return best;
 }
 
@@ -182,10 +199,11 @@ void analyse(luna_uvu_plan* plan) {
   if (plan->paths[0].ch * elem % 16 != 0) return;  // bulk copies move whole 16-byte pieces
   const int shape = find_shape<0>(plan);
   if (shape < 0) return;
-  const bool sliced = choose_lanes(plan, shape, false, false).cpl == 0;
+  const bool sliced = choose_lanes(plan, shape, EdgeUse::kForward, false).cpl == 0;
   if (sliced && !edge_sliced(shape)) return;
-  plan->edge.lanes = choose_lanes(plan, shape, false, sliced);
-  plan->edge.lanes_all = choose_lanes(plan, shape, true, sliced);
+  plan->edge.lanes = choose_lanes(plan, shape, EdgeUse::kForward, sliced);
+  plan->edge.lanes_one = choose_lanes(plan, shape, EdgeUse::kOneGradient, sliced);
+  plan->edge.lanes_all = choose_lanes(plan, shape, EdgeUse::kAllGradients, sliced);
   if (plan->edge.lanes.cpl != 0) plan->edge.shape = shape;
 }
 
@@ -200,20 +218,20 @@ int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph
              const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w, void* scratch,
              int64_t scratch_bytes, cudaStream_t stream) {
   const EdgeBackwardArgs args{x, y, w, g, gx, gy, gw, acc_x, acc_y, acc_w, scratch, scratch_bytes, nullptr};
-  const EdgeLanes& lanes = gy && (gx || gw) ? plan->edge.lanes_all : plan->edge.lanes;
+  const EdgeLanes& lanes = gy && (gx || gw) ? plan->edge.lanes_all : plan->edge.lanes_one;
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
 }
 
 int output_and_weights(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
                        const void* w, const void* g, void* out, void* gw, cudaStream_t stream) {
   const EdgeBackwardArgs args{x, y, w, g, nullptr, nullptr, gw, false, false, false, nullptr, 0, out};
-  const EdgeLanes& lanes = plan->edge.lanes;
+  const EdgeLanes& lanes = plan->edge.lanes_one;
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
 }
 
 bool joins_output(const luna_uvu_plan* plan) {
   bool joins = false;
-  with_instance(plan, plan->edge.lanes, [&](auto kernels) {
+  with_instance(plan, plan->edge.lanes_one, [&](auto kernels) {
     joins = kernels.joins_output();
     return LUNA_OK;
   });

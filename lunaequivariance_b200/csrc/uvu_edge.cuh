@@ -138,10 +138,17 @@ constexpr int kEdgeShapeMasks[kEdgeShapes][3] = {{1, 3, 3},  {1, 7, 7},   {1, 15
                                                  {7, 15, 15}, {3, 3, 1},  {7, 7, 1},   {15, 15, 1}, {2, 2, 1}};
 // Shapes whose kernels are compiled for slices too.  The others have no wide layers in use; theirs run the table kernels.
 constexpr bool edge_sliced(int id) { return id >= 3 && id <= 6; }
-// Channels per lane of the kernels that walk two edges at a time.
-constexpr bool edge_paired(int cpl) { return cpl <= 2; }
 template <int ID>
 using ShapeOf = Shape<kEdgeShapeMasks[ID][0], kEdgeShapeMasks[ID][1], kEdgeShapeMasks[ID][2]>;
+// Shapes and channels per lane whose kernels walk two edges at a time: one and two, and with four those whose paths all have a
+// degree of zero and whose degrees end at 2.  The others have more arithmetic in an edge than beside it, or too many registers:
+// (2, 2, 2), 64 channels, all gradients of 0.24 M edges 0.345 -> 0.391 ms with two at a time; (0, 3, 3), forward of 0.8 M edges
+// 0.249 -> 0.475.
+template <int ID>
+constexpr bool edge_paired(int cpl) {
+  using S = ShapeOf<ID>;
+  return cpl <= 2 || (S::m_total == 0 && top_degree(S::MX) <= 2 && top_degree(S::MO) <= 2);
+}
 
 // ---- launch arguments, type-erased ------------------------------------------------------------------------------------
 struct EdgeForwardArgs {

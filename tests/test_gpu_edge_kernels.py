@@ -232,3 +232,13 @@ def test_output_and_weight_gradient_of_the_second_order(shape, dtype):
         assert hx is None and hy is None
         assert_close(hw, ref["hw"], dtype, f"{SHAPES[shape]} x{mul} {dtype} hw")
         assert_close(hg, ref["hg"], dtype, f"{SHAPES[shape]} x{mul} {dtype} hg")
+
+
+@pytest.mark.parametrize("shape", [0, 1, 3, 7, 8, 10])
+def test_two_edges_at_a_time_with_four_channels_per_lane(shape):
+    """64 channels of the shapes whose paths all have a degree of zero; the forward at degree 2 only."""
+    module = check(SHAPES[shape], 64, torch.float32, 31, 403, 0.0, shape)
+    assert module.op._plan.query(1) == (4 if shape in (1, 8) else 2)
+    check(SHAPES[shape], 64, torch.float32, 150, 191, 1.5, shape + 50)
+    check(SHAPES[shape], 64, torch.float32, 900, 7201, 0.5, shape + 70)
+    one_gradient_alone(SHAPES[shape], 64, torch.float32, 150, 191, 1.5, shape + 90)
