@@ -28,6 +28,7 @@
 
 #include "uvu_fast.cuh"
 #include "uvu_packets.cuh"
+#include "uvu_parts.cuh"
 
 namespace luna {
 namespace edgek {
@@ -291,20 +292,6 @@ __device__ __forceinline__ void team_sync(int team_warps, int team_id) {
     __syncwarp();
   else
     named_barrier(1 + team_id, team_warps * 32);
-}
-// A team's part of a launch: its edges [pos, end), the rows [n, n_hi) that they are of, and whether the first of these rows began
-// in an earlier team's part (joined) and the last one goes on in the next team's (open).
-struct TeamPart {
-  int n, n_hi, pos, end;
-  int cta_pos, cta_edges;  // the CTA's edges
-  int joined, open;
-  // the row that the next team goes on with, or -1
-  __device__ __forceinline__ int open_row() const { return open ? n_hi - 1 : -1; }
-  // whether the first row began earlier and ends here
-  __device__ __forceinline__ bool closes() const { return joined && n != open_row(); }
-};
-__device__ __forceinline__ int part_begin(int cta_pos, int cta_edges, int team, int teams) {
-  return cta_pos + static_cast<int>(static_cast<unsigned>(cta_edges) * static_cast<unsigned>(team) / static_cast<unsigned>(teams));
 }
 // The first rows that begin at `bound` or after it, one search in each half of the warp, and where they begin.  A guess is
 // looked up with its neighbours, 16 entries at a time, and mended by what they say; after three of those the interval is halved

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
     program.run(y_next, mbuf + buf * S::m_elems, place);
     y_next = place < S::YD && mine + 2 < e_end ? P.y[static_cast<int64_t>(mine + 2) * S::YD + place] : T(0);
     __syncwarp();
-    int row_end = min(P.dst_rowptr[n + 1], e_end);
+    int row_end = first_row_end(P.dst_rowptr, n, n_hi, e_end);
 #pragma unroll 1
     for (; e < e_end; e += 2, mine += 2) {
 #pragma unroll 1

@@ -1,10 +1,13 @@
 """The edge kernels at the sizes where they can go wrong, against the CPU oracle: every compiled shape, channel counts
 that leave lanes idle or need several warps per edge, rows shared by several teams and rows handed out in tiles."""
 
+import dataclasses
+
 import pytest
 import torch
 
 import lunaequivariance_b200 as luna
+from lunaequivariance_b200 import conv as conv_mod
 from oracle import uvu_conv as oracle_conv
 from tests.helpers import all_paths, assert_close, random_problem
 from tests.test_gpu_random_shapes import skewed_graph
@@ -242,3 +245,31 @@ def test_two_edges_at_a_time_with_four_channels_per_lane(shape):
     check(SHAPES[shape], 64, torch.float32, 150, 191, 1.5, shape + 50)
     check(SHAPES[shape], 64, torch.float32, 900, 7201, 0.5, shape + 70)
     one_gradient_alone(SHAPES[shape], 64, torch.float32, 150, 191, 1.5, shape + 90)
+
+
+@pytest.mark.parametrize("shape,mul", [(3, 32), (3, 16), (8, 64), (10, 16)])
+def test_parts_without_edges_behind_the_last_row(shape, mul):
+    """Teams without an edge where the last row has begun already, which find no row there; the row tables are views that end
+    inside a larger tensor, as a caller's may."""
+    in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
+    instructions = all_paths(in1, in2, out)
+    module = luna.TensorProductConv(in1, in2, out, instructions, internal_weights=False, shared_weights=False)
+    meta = oracle_conv.build_specs(in1, in2, out, instructions)
+    generator = torch.Generator().manual_seed(shape + mul)
+    for degrees in ([4] * 500, [5] * 450, [16] * 1000 + [200]):
+        nodes, dst = len(degrees), torch.arange(len(degrees)).repeat_interleave(torch.tensor(degrees))
+        src = torch.randint(nodes, dst.shape, generator=generator)
+        p = random_problem((meta["in1_dim"], meta["in2_dim"], meta["out_dim"], meta["weight_numel"]), nodes, src, torch.float32,
+                           generator)
+        ref = oracle_conv.conv_derivatives(meta, *(p[k].double() for k in ("x", "y", "w")), src, dst, nodes, p["g"].double(),
+                                           None, None, None)
+        graph = module.create_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+        behind = torch.full((5,), 2**31 - 1, dtype=torch.int32, device=DEVICE)
+        graph = dataclasses.replace(graph, dst_rowptr=torch.cat([graph.dst_rowptr, behind])[:nodes + 1],
+                                    src_rowptr=torch.cat([graph.src_rowptr, behind])[:nodes + 1])
+        x, y, w, g = (p[k].to(DEVICE) for k in ("x", "y", "w", "g"))
+        result = conv_mod.run_forward(module.op, x, y, w, graph)
+        gx, gy, gw = conv_mod.run_backward(module.op, x, y, w, g, graph)
+        module.op.check_status()
+        for key, value in dict(out=result, gx=gx, gy=gy, gw=gw).items():
+            assert_close(value, ref[key], torch.float32, f"{SHAPES[shape]} x{mul} {nodes} nodes {key}")
