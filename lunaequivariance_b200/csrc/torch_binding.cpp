@@ -15,9 +15,12 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <array>
+#include <memory>
 #include <mutex>
 #include <optional>
+#include <utility>
 
 #include "../../include/luna_b200.h"
 
@@ -242,20 +245,69 @@ std::array<Tensor, N> spread(const variable_list& list, int mask) {
 }
 Tensor contiguous(const Tensor& t) { return t.defined() ? t.contiguous() : t; }
 
-// The weights' second name.  Energy training differentiates the weights once, force training twice: the gradients of both
-// orders meet at the weights, and the engine adds two tensors of the weights' size, three more passes over memory beside the
-// two that wrote them.  So ConvForward has the weights as a second output that nobody sees, and what comes after saves
-// that one: the second order's gradient then arrives at ConvForward's own backward, whose kernel adds to it in place.
+// Energy training differentiates the weights once, force training twice: the gradients of both orders meet at the weights, and
+// the engine adds two tensors of the weights' size, three more passes over memory beside the two that wrote them.  So the second
+// order's graph names the weights through a node of its own (SecondOrderWeights), which leaves its gradient here if the first
+// order's node, ConvForward, is going to run in the same task; that one's kernel adds to it in place.  Neither node sees
+// anything of the other's: ConvForward has one output, and runs when something reaches that.  What a task that failed has left
+// stays until the graph goes, and later tasks leave nothing.
 // FP64 force step, degrees (2, 3, 3), 128 channels, 1.05 M edges (18 GB of weights): 33.6 -> 27.4 ms; FP32, (2, 2, 2),
 // 32 channels, 0.2 M edges (295 MB): 936 -> 818 us.
-struct ConvForward;
-constexpr uint32_t kWeightsOutput = 1;
-bool second_name(const Tensor& w);
-// Whether the running task wants the gradient of input `edge`, saved as `t`.  Behind a second name the question is about the
-// weights, not about the ConvForward in between, which may run for another input.
-bool wanted(AutogradContext* ctx, size_t edge, const Tensor& t) {
-  return ctx->needs_input_grad(edge) && (!second_name(t) || t.grad_fn()->task_should_compute_output(2));
-}
+//
+// Not where the first order has run by then (an energy that is linear in the output, next to the forces in one loss: nothing
+// orders the two nodes), where a hook sees what ConvForward returns, or where a graph of the gradient is wanted: there the
+// engine adds them.
+struct WeightGradient : torch::CustomClassHolder {
+  explicit WeightGradient(const std::shared_ptr<torch::autograd::Node>& node) : first_order(node) {}
+
+  // Whether `gradient` was left for the first order.
+  bool leave(const Tensor& gradient) {
+    const auto node = first_order.lock();
+    const auto* reached = torch::autograd::get_current_graph_task_nodes_in_graph();
+    const auto* wanted = torch::autograd::get_current_graph_task_exec_info();
+    const int64_t running = torch::autograd::get_current_graph_task_id();
+    if (!node || !reached || !wanted || running < 0 || !node->post_hooks().empty() || reached->count(node.get()) == 0) return false;
+    if (!wanted->empty()) {
+      const auto info = wanted->find(node.get());
+      if (info == wanted->end() || !info->second.should_execute()) return false;
+    }
+    const std::lock_guard<std::mutex> lock(mutex);
+    if (left.defined() || running <= forgotten || std::find(done.begin(), done.end(), running) != done.end()) return false;
+    left = gradient;
+    task = running;
+    return true;
+  }
+  // The first order runs: what was left for it in this task, if anything.
+  Tensor take() {
+    const int64_t running = torch::autograd::get_current_graph_task_id();
+    const std::lock_guard<std::mutex> lock(mutex);
+    forgotten = std::max(forgotten, done[next]);
+    done[next] = running;
+    next = (next + 1) % done.size();
+    return task == running ? std::exchange(left, Tensor()) : Tensor();
+  }
+
+ private:
+  const std::weak_ptr<torch::autograd::Node> first_order;
+  std::mutex mutex;  // tasks of several threads may run through one graph
+  Tensor left;
+  int64_t task = -1;                                   // that it was left in
+  std::array<int64_t, 8> done{-1, -1, -1, -1, -1, -1, -1, -1};  // the last tasks in which the first order ran; their numbers rise
+  size_t next = 0;
+  int64_t forgotten = -1;  // no task up to this one is looked up any more
+};
+
+struct SecondOrderWeights : Function<SecondOrderWeights> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& w, const c10::intrusive_ptr<WeightGradient>& sum) {
+    ctx->set_materialize_grads(false);
+    keep(ctx, "sum", sum);
+    return w.detach();
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    if (grads[0].defined() && !at::GradMode::is_enabled() && kept<WeightGradient>(ctx, "sum")->leave(grads[0])) return {Tensor(), Tensor()};
+    return {grads[0], Tensor()};
+  }
+};
 
 // dF/d(operand `slot`), slots 0..3 = x, y, w, g; a, b, c: the other three operands in that order.  The kernels take all four
 // operands and look at the shape of the free slot's only: `free` lends it (none for g).
@@ -282,7 +334,7 @@ struct ConvPartial : Function<ConvPartial> {
     const auto full = operands({saved[0], saved[1], saved[2]}, slot, grads[0].contiguous());
     for (int64_t other = 0, position = 0; other < 4; ++other) {
       if (other == slot) continue;
-      if (wanted(ctx, position, saved[position])) out[position] = of(full, other, op, graph);
+      if (ctx->needs_input_grad(position)) out[position] = of(full, other, op, graph);
       ++position;
     }
     return out;
@@ -331,7 +383,7 @@ struct ConvDouble : Function<ConvDouble> {
                                         {0, 5, 9, 3}, {4, 1, 2, 10}, {0, 5, 2, 10}, {0, 1, 6, 10}};
     for (int v = 0, edge = 0; v < 7; ++v) {
       if (!t[v].defined()) continue;  // a missing tangent has no edge
-      if (!wanted(ctx, edge++, t[v])) continue;
+      if (!ctx->needs_input_grad(edge++)) continue;
       Tensor sum;
       for (const auto& term : terms) {
         bool whole = true;
@@ -364,10 +416,10 @@ struct ConvBackward : Function<ConvBackward> {
     variable_list out(7);
     const auto r = spread<3>(grads, static_cast<int>(ctx->saved_data["mask"].toInt()));
     if (!r[0].defined() && !r[1].defined() && !r[2].defined()) return out;
-    const auto saved = ctx->get_saved_variables();
     int mask = 0;
-    for (int s = 0; s < 4; ++s) mask |= wanted(ctx, s, saved[s]) ? 1 << s : 0;
+    for (int s = 0; s < 4; ++s) mask |= ctx->needs_input_grad(s) ? 1 << s : 0;
     if (!mask) return out;
+    const auto saved = ctx->get_saved_variables();
     const auto op = kept<Op>(ctx, "op");
     const auto graph = kept<Graph>(ctx, "graph");
     std::array<Tensor, 4> h;
@@ -384,52 +436,52 @@ struct ConvBackward : Function<ConvBackward> {
   }
 };
 
-// Below this size of the weights their second name is not worth the host time of an output (some 1.5 us in every tracked
-// call): the engine's sum of 32 MiB takes 15 us.
-constexpr int64_t kSecondNameBytes = 32 << 20;
+// Below this size of the weights the engine's sum, 15 us for 32 MiB, is not worth a node.
+constexpr int64_t kSecondOrderBytes = 32 << 20;
 
 struct ConvForward : Function<ConvForward> {
-  // out and, if they are large enough and want a gradient, the weights under their second name
-  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& y, const Tensor& w, const OpPtr& op,
-                               const GraphPtr& graph) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& y, const Tensor& w, const OpPtr& op,
+                        const GraphPtr& graph) {
     ctx->set_materialize_grads(false);
-    variable_list out{run_forward(*op, *graph, x, y, w)};
-    if (w.requires_grad() && static_cast<int64_t>(w.nbytes()) >= kSecondNameBytes) out.push_back(w.detach());
-    ctx->save_for_backward({x, y, out.size() > 1 ? out[kWeightsOutput] : w});
+    ctx->save_for_backward({x, y, w});
     keep(ctx, "op", op);
     keep(ctx, "graph", graph);
-    return out;
+    return run_forward(*op, *graph, x, y, w);
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     variable_list out(5);
+    const auto sum = ctx->saved_data.count("sum") ? kept<WeightGradient>(ctx, "sum") : c10::intrusive_ptr<WeightGradient>();
+    const Tensor later = sum ? sum->take() : Tensor();
     int mask = 0;
     for (int s = 0; s < 3; ++s) mask |= ctx->needs_input_grad(s) ? 1 << s : 0;
-    const Tensor none;
-    const Tensor& later = grads.size() > kWeightsOutput && mask & kW ? grads[kWeightsOutput] : none;
     if (!grads[0].defined() || !mask) {
       out[2] = later;
       return out;
     }
-    // in place only where nobody else can see the tensor
-    const bool ours = later.defined() && !at::GradMode::is_enabled() && later.use_count() == 1 && later.has_storage() &&
-                      later.storage().use_count() == 1 && !later.requires_grad() && later.layout() == at::kStrided &&
-                      later.is_contiguous() && reinterpret_cast<uintptr_t>(later.data_ptr()) % 16 == 0;
     const auto saved = ctx->get_saved_variables();
     const auto op = kept<Op>(ctx, "op");
     const auto graph = kept<Graph>(ctx, "graph");
     const Tensor g = grads[0].contiguous();
-    const auto d = at::GradMode::is_enabled()
-                       ? spread<3>(ConvBackward::apply(saved[0], saved[1], saved[2], g, static_cast<int64_t>(mask), op, graph), mask)
-                       : run_backward(*op, *graph, saved[0], saved[1], saved[2], g, mask, ours ? later : none);
+    // in place only where nobody else can see the tensor
+    const bool ours = later.defined() && mask & kW && !at::GradMode::is_enabled() && later.use_count() == 1 && later.has_storage() &&
+                      later.storage().use_count() == 1 && !later.requires_grad() && later.layout() == at::kStrided &&
+                      later.is_contiguous() && reinterpret_cast<uintptr_t>(later.data_ptr()) % 16 == 0;
+    std::array<Tensor, 3> d;
+    if (at::GradMode::is_enabled()) {
+      Tensor w = saved[2];
+      if (w.requires_grad() && static_cast<int64_t>(w.nbytes()) >= kSecondOrderBytes) {
+        if (!sum) keep(ctx, "sum", c10::make_intrusive<WeightGradient>(torch::autograd::get_current_node()));
+        w = SecondOrderWeights::apply(w, kept<WeightGradient>(ctx, "sum"));
+      }
+      d = spread<3>(ConvBackward::apply(saved[0], saved[1], w, g, static_cast<int64_t>(mask), op, graph), mask);
+    } else {
+      d = run_backward(*op, *graph, saved[0], saved[1], saved[2], g, mask, ours ? later : Tensor());
+    }
+    if (later.defined() && !ours) d[2] = d[2].defined() ? d[2] + later : later;
     for (int s = 0; s < 3; ++s) out[s] = d[s];
-    if (later.defined() && !ours) out[2] = d[2] + later;
     return out;
   }
 };
-bool second_name(const Tensor& w) {
-  return w.defined() && w.output_nr() == kWeightsOutput &&
-         dynamic_cast<torch::autograd::CppNode<ConvForward>*>(w.grad_fn().get()) != nullptr;
-}
 
 bool tracked(std::initializer_list<const Tensor*> tensors) {
   if (!at::GradMode::is_enabled()) return false;
@@ -440,7 +492,7 @@ bool tracked(std::initializer_list<const Tensor*> tensors) {
 
 Tensor conv(const OpPtr& op, const GraphPtr& graph, const Tensor& x, const Tensor& y, const Tensor& w) {
   pybind11::gil_scoped_release release;
-  return tracked({&x, &y, &w}) ? ConvForward::apply(x, y, w, op, graph)[0] : run_forward(*op, *graph, x, y, w);
+  return tracked({&x, &y, &w}) ? ConvForward::apply(x, y, w, op, graph) : run_forward(*op, *graph, x, y, w);
 }
 
 // ---- graph tables ---------------------------------------------------------------------------------------------------------
