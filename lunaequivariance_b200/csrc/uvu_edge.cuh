@@ -20,8 +20,10 @@
 // which a few tiles per team would leave the chip waiting for the last ones: every CTA has an equal stretch of the edges, up
 // to whole rows, and every team of it an equal part of that, whatever the rows; a row that several teams share is summed
 // at the end, in the teams' order, through shared memory.  The forward of very few rows: `group` teams of a CTA share a row, each
-// a contiguous part of its edges, and the parts are summed in a fixed order through shared memory.  A row's sum depends on
-// its own edges and on the launch's sizes (in a group: on `group` alone), not on which team got it.
+// a contiguous part of its edges, and the parts are summed in a fixed order through shared memory.  No sum depends
+// on which team was first.  A row's sum is one over its own edges, in their order, where tiles are handed out; in a group it is
+// cut by the row's length and `group`; in equal parts it is cut where a team's part ends, so by the lengths of other rows too.
+// So a piece of a graph gives the same rows to the bit where both launches hand out tiles, and else to rounding.
 #pragma once
 
 #include <atomic>
@@ -216,7 +218,7 @@ constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
 // Parts of the edges are even to about a row per CTA; what they lose is order: a CTA's rows are its own, so the rows that all
 // CTAs gather at a time are spread over the whole graph.  So: as long as a team's part is short, and while the node rows that
 // are gathered (`gathered` bytes) stay in L2 whoever reads them.  Groups (`may_group`): while a CTA has three rows
-// or fewer, too few for even parts; a row's sum is then the same in any piece of the graph that is as small.  Rows and edges
+// or fewer, too few for even parts; pieces of such a graph that have the same group give the same sums.  Rows and edges
 // shared as before (groups of up to eight teams, then tiles) and in parts, forward / all gradients: (2, 2, 2), 64 channels,
 // 2,083 nodes of 41 edges 80 / 160 -> 78 / 148 us, 4,000 of 30 98 / 201 -> 90 / 180; 48 channels, 10,001 of 52 290 / 777 -> 258 /
 // 711; 32 channels, 4,003 of 52 100 / 202 -> 88 / 176.  With 442 edges a team (64 channels, 20,000 nodes) the two are even, and

@@ -9,8 +9,9 @@
 //
 // The edges of a tile are taken in pairs from its first one, whatever the rows.  Where a row ends between the two edges of
 // a pair, the second half leaves its sum of that row in memory, begins the next row with that pair, and the first half adds
-// what it has when it is done.  Either way a row's sum is that of its first, third, ... edges plus that of the others, wherever
-// its tile begins.
+// what it has when it is done.  Either way the sum of a row that lies in one tile is that of its first, third, ... edges plus that
+// of the others, wherever the tile begins.  Where the call adds to its output, a row that ends inside a pair is (what is there +
+// the second half's) + the first half's, any other what is there + both; a row cut by equal parts is paired anew in each part.
 #pragma once
 
 #include "uvu_edge_fwd.cuh"

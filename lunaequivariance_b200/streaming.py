@@ -14,7 +14,10 @@ directions for the whole step.  Node features and their gradients stay on the de
 source-row gradient is accumulated across chunks by the kernels (``luna_uvu_conv_bwd_add_gx``).
 
 The reference has no counterpart (its operators take device tensors only); results are those of one call on the
-whole graph, bit for bit in ``out``, ``gy`` and ``gw`` and up to the order of the per-chunk additions in ``gx``.
+whole graph: bit for bit in ``gy`` and ``gw``, up to the order of the per-chunk additions in ``gx``, and up to the order
+of a row's sum in ``out``.  That order depends on the size of a launch (``edge_split`` in ``csrc/uvu_edge.cuh``): it is the
+same, and ``out`` equal bit for bit, where the whole graph and every chunk have more than 256 edges per team of warps (some 0.3
+to 0.9 million) and more than three rows per SM.
 """
 
 from __future__ import annotations

@@ -64,6 +64,27 @@ def test_destination_ranges_add_up(name, dtype):
     assert graph.destination_range(17, 150)[0] is graph.destination_range(17, 150)[0]  # cached
 
 
+@pytest.mark.parametrize("cuts,same", [((0, 1600, 3200), True), ((0, 800, 1600, 2400, 3200), False)])
+def test_pieces_of_a_graph_that_hands_out_tiles(cuts, same, monkeypatch):
+    """With two warps per CTA a whole graph of 165,000 edges hands out tiles; so do its halves, and then every row of ``out`` is
+    the same to the bit.  Its quarters are cut into equal parts of their edges, and sum rows in another order."""
+    monkeypatch.setenv("LUNA_B200_MAXW", "2")
+    module, op, graph, t, _ = problem("cfg5", torch.float32, atoms=3200)
+    teams = 2 * torch.cuda.get_device_properties(DEVICE).multi_processor_count
+    assert graph.num_edges > 256 * teams
+    ref = whole(op, graph, t)
+    for begin, end in zip(cuts[:-1], cuts[1:]):
+        piece, e0, e1 = graph.destination_range(begin, end)
+        assert (e1 - e0 > 256 * teams) == same
+        out = conv_mod.run_forward(op, t["x"], t["y"][e0:e1], t["w"][e0:e1], piece)
+        _, gy, gw = conv_mod.run_backward(op, t["x"], t["y"][e0:e1], t["w"][e0:e1], t["g"][begin:end], piece,
+                                          (False, True, True))
+        assert torch.equal(gy, ref["gy"][e0:e1]) and torch.equal(gw, ref["gw"][e0:e1])
+        assert_close(out, ref["out"][begin:end].cpu(), torch.float32, f"rows {begin} to {end}")
+        assert not same or torch.equal(out, ref["out"][begin:end])
+    op.check_status()
+
+
 def test_add_gx_needs_a_tensor_and_out_shapes_are_checked():
     module, op, graph, t, _ = problem("cfg5", torch.float32, atoms=60)
     with pytest.raises(ValueError, match="add_gx"):
