@@ -147,7 +147,7 @@ def term_by_term(meta, x, y, w, g, src, dst):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("mul", [12, 48, 64, 128, 160])
+@pytest.mark.parametrize("mul", [12, 16, 32, 48, 64, 128, 160])
 @pytest.mark.parametrize("shape", [3, 4, 6])
 def test_values_that_are_not_finite_stay_where_they_belong(shape, mul, dtype):
     """Infinities and NaN in the last channel, which idle lanes read too, and in single edge attributes, which matrix
