@@ -24,25 +24,26 @@ bool spills(const luna_uvu_plan* plan, int shape, int cpl) {
   return cpl == 4 ? spills<float, 4>(shape, all) : (cpl == 2 ? spills<float, 2>(shape, all) : spills<float, 1>(shape, all));
 }
 
-template <int... ID>
-bool paired(int shape, int cpl, std::integer_sequence<int, ID...>) {
+template <typename T, int CPL, int... ID>
+bool paired(int shape, bool forward, std::integer_sequence<int, ID...>) {
   bool found = false;
-  ((found = found || (shape == ID && edge_paired<ID>(cpl))), ...);
+  ((found = found || (shape == ID && edge_paired<T, CPL, ID>(forward))), ...);
   return found;
 }
-bool paired(int shape, int cpl) { return paired(shape, cpl, std::make_integer_sequence<int, kEdgeShapes>{}); }
+bool paired(const luna_uvu_plan* plan, int shape, int cpl, bool forward) {
+  constexpr std::make_integer_sequence<int, kEdgeShapes> all{};
+  if (plan->dtype == LUNA_F64)
+    return cpl == 1 ? paired<double, 1>(shape, forward, all) : cpl == 2 && paired<double, 2>(shape, forward, all);
+  return cpl == 1 ? paired<float, 1>(shape, forward, all)
+                  : (cpl == 2 ? paired<float, 2>(shape, forward, all) : cpl == 4 && paired<float, 4>(shape, forward, all));
+}
 
 // Channels per lane and warps per team, or slices for blocks that no team takes.  A warp's pass over an edge costs about one
 // unit of fixed work plus one per channel of a lane, so 48 channels take one warp with two channels on 24 lanes, 96 one warp
 // with four on 24 lanes.  A kernel that spills counts half as much again: degrees (3, 3, 3) with the most channels per lane,
 // all gradients.  300 MB of weights, FP64: 96 channels 0.64 -> 0.52 ms with one channel per lane, 224 channels 0.72 -> 0.49;
 // FP32: 128 channels 0.41 -> 0.30 with two, 256 channels 0.57 -> 0.34.
-//
-// 16 channels per lane of half a warp: two edges at a time, if the rows of two pairs leave room for eight warps.  With fewer it
-// loses: FP64, 32 channels, degrees (2, 3, 3), six warps, all gradients of 0.4 M edges 1.30 -> 1.75 ms.  64 channels, one edge and
-// two, forward / all gradients / dL/dy / dL/dw, 0.8 M edges: (1, 1, 1) 165 / 555 / 322 / 416 -> 174 / 380 / 194 / 260 us; (1, 1, 0)
-// 143 / 476 / 330 / 250 -> 156 / 310 / 188 / 231; (0, 2, 2), 1.05 M edges, 282 / 710 / 422 / 518 -> 215 / 478 / 250 / 332; (2, 2, 0)
-// 233 / 545 / 370 / 424 -> 176 / 439 / 215 / 268.  So the forward has it at degree 2 only.
+// ch / 16 channels on each of a half warp's 16 lanes, two edges at a time, where that is compiled (edge_paired).
 EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool sliced) {
   const int ch = plan->edge.ch, elem = plan->dtype == LUNA_F64 ? 8 : 4;
   // one team with two stages must fit an SM's shared memory in either direction
@@ -62,11 +63,9 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool s
     best_cost = cost;
     best = sliced ? EdgeLanes{cpl, 1, parts} : EdgeLanes{cpl, parts, 1};
   }
-  const int half = ch / 16, *masks = kEdgeShapeMasks[shape];
-  const bool lanes_exist = ch % 16 == 0 && (half == 1 || half == 2 || (half == 4 && elem == 4 &&
-                                                                       (use != EdgeUse::kForward || (masks[0] | masks[2]) >= 4)));
-  if (!sliced && lanes_exist && paired(shape, half) && (plan->tuning.lane_channels == 0 || plan->tuning.lane_channels == half) &&
-      4 * (W + std::max(X, O)) <= 24 * 1024)
+  const int half = ch / 16;
+  if (!sliced && ch % 16 == 0 && (plan->tuning.lane_channels == 0 || plan->tuning.lane_channels == half) &&
+      paired(plan, shape, half, use == EdgeUse::kForward))
     return EdgeLanes{half, 1, 1, 2};
   return best;
 }

@@ -143,14 +143,20 @@ constexpr int kEdgeShapeMasks[kEdgeShapes][3] = {{1, 3, 3},  {1, 7, 7},   {1, 15
 constexpr bool edge_sliced(int id) { return id >= 3 && id <= 6; }
 template <int ID>
 using ShapeOf = Shape<kEdgeShapeMasks[ID][0], kEdgeShapeMasks[ID][1], kEdgeShapeMasks[ID][2]>;
-// Shapes and channels per lane whose kernels walk two edges at a time: one and two, and with four those whose paths all have a
-// degree of zero and whose degrees end at 2.  The others have more arithmetic in an edge than beside it, or too many registers:
-// (2, 2, 2), 64 channels, all gradients of 0.24 M edges 0.345 -> 0.391 ms with two at a time; (0, 3, 3), forward of 0.8 M edges
-// 0.249 -> 0.475.
-template <int ID>
-constexpr bool edge_paired(int cpl) {
+// Whether the kernels of 16 * CPL channels walk two edges at a time, with CPL channels on each lane of a half warp: what is
+// compiled and what is chosen.  One and two channels per lane, if the rows of two pairs leave room for eight warps.  With fewer it
+// loses: FP64, 32 channels, degrees (2, 3, 3), six warps, all gradients of 0.4 M edges 1.30 -> 1.75 ms.  Four FP32 channels for shapes
+// whose paths all have a degree of zero and whose degrees end at 2.  The others have more arithmetic in an edge than beside it, or
+// too many registers: (2, 2, 2), 64 channels, all gradients of 0.24 M edges 0.345 -> 0.391 ms with two at a time; (0, 3, 3), forward of
+// 0.8 M edges 0.249 -> 0.475.  Of these the forward at degree 2 only: one edge and two, forward / all gradients / dL/dy / dL/dw, 0.8 M
+// edges: (1, 1, 1) 165 / 555 / 322 / 416 -> 174 / 380 / 194 / 260 us; (1, 1, 0) 143 / 476 / 330 / 250 -> 156 / 310 / 188 / 231; (0, 2, 2),
+// 1.05 M edges, 282 / 710 / 422 / 518 -> 215 / 478 / 250 / 332; (2, 2, 0) 233 / 545 / 370 / 424 -> 176 / 439 / 215 / 268.
+template <typename T, int CPL, int ID>
+constexpr bool edge_paired(bool forward) {
   using S = ShapeOf<ID>;
-  return cpl <= 2 || (S::m_total == 0 && top_degree(S::MX) <= 2 && top_degree(S::MO) <= 2);
+  constexpr int top = top_degree(S::MX | S::MO), row = S::paths + (S::XD > S::OD ? S::XD : S::OD);
+  const bool four = sizeof(T) == 4 && S::m_total == 0 && (top == 2 || (top == 1 && !forward));
+  return (CPL <= 2 || four) && 4 * row * 16 * CPL * static_cast<int>(sizeof(T)) <= 24 * 1024;
 }
 
 // ---- launch arguments, type-erased ------------------------------------------------------------------------------------

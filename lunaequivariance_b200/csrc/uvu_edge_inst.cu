@@ -14,7 +14,7 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::forward(const luna
   if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
     if (lanes.slices > 1) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, false>(plan, dt, graph, lanes, a, stream);
   }
-  if constexpr (edge_paired<LUNA_EDGE_SHAPE>(LUNA_EDGE_CPL)) {
+  if constexpr (edge_paired<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>(true)) {
     if (lanes.edges == 2) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, true>(plan, dt, graph, lanes, a, stream);
   }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
@@ -30,7 +30,7 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const lun
   if constexpr (edge_sliced(LUNA_EDGE_SHAPE)) {
     if (lanes.slices > 1) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, false>(plan, dt, graph, lanes, a, stream);
   }
-  if constexpr (edge_paired<LUNA_EDGE_SHAPE>(LUNA_EDGE_CPL)) {
+  if constexpr (edge_paired<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>(false)) {
     if (lanes.edges == 2) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, true>(plan, dt, graph, lanes, a, stream);
   }
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
@@ -48,11 +48,9 @@ size_t EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::smem_bytes(cons
                                                                             bool backward, int max_smem) {
   using S = ShapeOf<LUNA_EDGE_SHAPE>;
   const int ch = plan->edge.ch / lanes.slices;
-  if constexpr (edge_paired<LUNA_EDGE_SHAPE>(LUNA_EDGE_CPL)) {
-    if (lanes.edges == 2)
-      return backward ? pair_bwd_launch<LUNA_EDGE_T, S, PairBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>>(plan->tuning, ch, max_smem).bytes
-                      : pair_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, ch, max_smem).bytes;
-  }
+  if (lanes.edges == 2)
+    return backward ? pair_bwd_launch<LUNA_EDGE_T, S, PairBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>>(plan->tuning, ch, max_smem).bytes
+                    : pair_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, ch, max_smem).bytes;
   if (!backward) return edge_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, lanes, ch, max_smem).bytes;
   using K = EdgeBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>;
   return edge_bwd_launch<LUNA_EDGE_T, S, K>(plan->tuning, lanes, ch, max_smem).bytes;

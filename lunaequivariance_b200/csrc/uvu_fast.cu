@@ -120,7 +120,7 @@ int64_t fast_scratch_bytes(const luna_uvu_plan* plan, int64_t, int64_t num_edges
   if (plan->force_generic) return 0;
   int64_t parts = 1;
   if (plan->edge.shape >= 0)
-    parts = std::max(plan->edge.lanes.slices, plan->edge.lanes_all.slices);
+    parts = std::max(std::max(plan->edge.lanes.slices, plan->edge.lanes_one.slices), plan->edge.lanes_all.slices);
   else if (plan->fast_ok)
     parts = plan->fast.chunks;
   return parts > 1 ? parts * num_edges * plan->Y * (plan->dtype == LUNA_F64 ? 8 : 4) : 0;
