@@ -247,55 +247,123 @@ Tensor contiguous(const Tensor& t) { return t.defined() ? t.contiguous() : t; }
 
 // Energy training differentiates the weights once, force training twice: the gradients of both orders meet at the weights, and
 // the engine adds two tensors of the weights' size, three more passes over memory beside the two that wrote them.  So the second
-// order's graph names the weights through a node of its own (SecondOrderWeights), which leaves its gradient here if the first
-// order's node, ConvForward, is going to run in the same task; that one's kernel adds to it in place.  Neither node sees
-// anything of the other's: ConvForward has one output, and runs when something reaches that.  What a task that failed has left
-// stays until the graph goes, and later tasks leave nothing.
+// order's graph names the weights through a node of its own (SecondOrderWeights), and if both that one and the first order's node,
+// ConvForward, run in a task, the first order's kernel adds to the second order's gradient in place.  Which of the two comes first is
+// the engine's choice unless the energy is nonlinear in the output: the second order leaves its gradient for the first, or the first
+// leaves its operands for the second.  Neither node sees anything else of the other: ConvForward has one output, and runs when
+// something reaches that.
 // FP64 force step, degrees (2, 3, 3), 128 channels, 1.05 M edges (18 GB of weights): 33.6 -> 27.4 ms; FP32, (2, 2, 2),
-// 32 channels, 0.2 M edges (295 MB): 936 -> 818 us.
+// 32 channels, 0.2 M edges (295 MB): 936 -> 818 us.  Energy and forces in one loss, the energy linear in the output: FP64, 0.4 M edges
+// 11.5 -> 8.9 ms; FP32, 0.2 M edges 610 -> 514 us.
 //
-// Not where the first order has run by then (an energy that is linear in the output, next to the forces in one loss: nothing
-// orders the two nodes), where a hook sees what ConvForward returns, or where a graph of the gradient is wanted: there the
-// engine adds them.
-struct WeightGradient : torch::CustomClassHolder {
-  explicit WeightGradient(const std::shared_ptr<torch::autograd::Node>& node) : first_order(node) {}
+// Not where a hook sees what one of the nodes returns, or where a graph of the gradient is wanted: there the engine adds them.
+using NodePtr = std::shared_ptr<torch::autograd::Node>;
 
-  // Whether `gradient` was left for the first order.
-  bool leave(const Tensor& gradient) {
-    const auto node = first_order.lock();
-    const auto* reached = torch::autograd::get_current_graph_task_nodes_in_graph();
-    const auto* wanted = torch::autograd::get_current_graph_task_exec_info();
-    const int64_t running = torch::autograd::get_current_graph_task_id();
-    if (!node || !reached || !wanted || running < 0 || !node->post_hooks().empty() || reached->count(node.get()) == 0) return false;
-    if (!wanted->empty()) {
-      const auto info = wanted->find(node.get());
-      if (info == wanted->end() || !info->second.should_execute()) return false;
-    }
+// Whether the running task runs a node, or has.
+bool in_running_task(const NodePtr& node) {
+  const auto* reached = torch::autograd::get_current_graph_task_nodes_in_graph();
+  const auto* wanted = torch::autograd::get_current_graph_task_exec_info();
+  if (!node || !reached || !wanted || reached->count(node.get()) == 0) return false;
+  if (wanted->empty()) return true;
+  const auto info = wanted->find(node.get());
+  return info != wanted->end() && info->second.should_execute();
+}
+
+// The last tasks that something was done in.  Their numbers rise; of those before the ones kept anything may be true.
+struct RecentTasks {
+  std::array<int64_t, 8> tasks{-1, -1, -1, -1, -1, -1, -1, -1};
+  size_t next = 0;
+  int64_t forgotten = -1;
+  void add(int64_t task) {
+    forgotten = std::max(forgotten, tasks[next]);
+    tasks[next] = task;
+    next = (next + 1) % tasks.size();
+  }
+  bool may_have(int64_t task) const {
+    return task <= forgotten || std::find(tasks.begin(), tasks.end(), task) != tasks.end();
+  }
+};
+
+// Where the two nodes leave things for each other.  What a task that failed has left stays until the graph goes, and later tasks
+// leave nothing.
+struct WeightGradient : torch::CustomClassHolder {
+  struct Operands {
+    Tensor x, y, w, g;
+    OpPtr op;
+    GraphPtr graph;
+  };
+
+  explicit WeightGradient(const NodePtr& node) : first(node) {}
+  void second_order_is(const NodePtr& node) {
     const std::lock_guard<std::mutex> lock(mutex);
-    if (left.defined() || running <= forgotten || std::find(done.begin(), done.end(), running) != done.end()) return false;
-    left = gradient;
-    task = running;
+    second = node;
+  }
+
+  // By the first order's node when it runs: what the second order has left for it in this task, if anything.
+  Tensor first_runs() {
+    const int64_t running = torch::autograd::get_current_graph_task_id();
+    const std::lock_guard<std::mutex> lock(mutex);
+    first_ran.add(running);
+    return gradient_task == running ? std::exchange(gradient, Tensor()) : Tensor();
+  }
+  // Whether its operands were left for the second order's node, which runs later in this task.
+  bool leave_operands(const Operands& all) {
+    const std::lock_guard<std::mutex> lock(mutex);
+    const NodePtr node = second.lock();
+    const int64_t running = torch::autograd::get_current_graph_task_id();
+    if (running < 0 || operands || second_ran.may_have(running) || !quiet(node) || !in_running_task(node)) return false;
+    operands = all;
+    operands_task = running;
+    operands_for = node;
     return true;
   }
-  // The first order runs: what was left for it in this task, if anything.
-  Tensor take() {
+  // By a second order's node when it runs.
+  std::optional<Operands> second_runs() {
     const int64_t running = torch::autograd::get_current_graph_task_id();
     const std::lock_guard<std::mutex> lock(mutex);
-    forgotten = std::max(forgotten, done[next]);
-    done[next] = running;
-    next = (next + 1) % done.size();
-    return task == running ? std::exchange(left, Tensor()) : Tensor();
+    second_ran.add(running);
+    if (!operands || operands_task != running || operands_for.lock() != torch::autograd::get_current_node()) return std::nullopt;
+    return std::exchange(operands, std::nullopt);
+  }
+  bool leave_gradient(const Tensor& w_gradient) {
+    const std::lock_guard<std::mutex> lock(mutex);
+    const int64_t running = torch::autograd::get_current_graph_task_id();
+    const NodePtr node = first.lock();
+    if (running < 0 || gradient.defined() || first_ran.may_have(running) || !quiet(node) || !in_running_task(node)) return false;
+    gradient = w_gradient;
+    gradient_task = running;
+    return true;
   }
 
  private:
-  const std::weak_ptr<torch::autograd::Node> first_order;
+  // Whether no hook sees what the running node returns, nor what the other one does.
+  static bool quiet(const NodePtr& other) {
+    const NodePtr running = torch::autograd::get_current_node();
+    return running && other && running->post_hooks().empty() && other->post_hooks().empty();
+  }
+
   std::mutex mutex;  // tasks of several threads may run through one graph
-  Tensor left;
-  int64_t task = -1;                                   // that it was left in
-  std::array<int64_t, 8> done{-1, -1, -1, -1, -1, -1, -1, -1};  // the last tasks in which the first order ran; their numbers rise
-  size_t next = 0;
-  int64_t forgotten = -1;  // no task up to this one is looked up any more
+  const std::weak_ptr<torch::autograd::Node> first;
+  std::weak_ptr<torch::autograd::Node> second;  // the last one made
+  std::weak_ptr<torch::autograd::Node> operands_for;
+  RecentTasks first_ran, second_ran;
+  Tensor gradient;
+  std::optional<Operands> operands;
+  int64_t gradient_task = -1, operands_task = -1;
 };
+
+// Whether nobody else can see the second order's gradient, so that a kernel may add to it.
+bool only_ours(const Tensor& t) {
+  return t.defined() && t.use_count() == 1 && t.has_storage() && t.storage().use_count() == 1 && !t.requires_grad() &&
+         t.layout() == at::kStrided && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+}
+// The first order's gradients, that of the weights added to the second order's if there is one.
+std::array<Tensor, 3> first_on_second(const WeightGradient::Operands& all, int mask, const Tensor& second) {
+  const bool ours = mask & kW && only_ours(second);
+  auto d = run_backward(*all.op, *all.graph, all.x, all.y, all.w, all.g, mask, ours ? second : Tensor());
+  if (second.defined() && !ours) d[2] = d[2].defined() ? d[2] + second : second;
+  return d;
+}
 
 struct SecondOrderWeights : Function<SecondOrderWeights> {
   static Tensor forward(AutogradContext* ctx, const Tensor& w, const c10::intrusive_ptr<WeightGradient>& sum) {
@@ -304,7 +372,10 @@ struct SecondOrderWeights : Function<SecondOrderWeights> {
     return w.detach();
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
-    if (grads[0].defined() && !at::GradMode::is_enabled() && kept<WeightGradient>(ctx, "sum")->leave(grads[0])) return {Tensor(), Tensor()};
+    if (at::GradMode::is_enabled()) return {grads[0], Tensor()};
+    const auto sum = kept<WeightGradient>(ctx, "sum");
+    if (const auto operands = sum->second_runs()) return {first_on_second(*operands, kW, grads[0])[2], Tensor()};
+    if (grads[0].defined() && sum->leave_gradient(grads[0])) return {Tensor(), Tensor()};
     return {grads[0], Tensor()};
   }
 };
@@ -450,34 +521,35 @@ struct ConvForward : Function<ConvForward> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     variable_list out(5);
-    const auto sum = ctx->saved_data.count("sum") ? kept<WeightGradient>(ctx, "sum") : c10::intrusive_ptr<WeightGradient>();
-    const Tensor later = sum ? sum->take() : Tensor();
+    auto sum = ctx->saved_data.count("sum") ? kept<WeightGradient>(ctx, "sum") : c10::intrusive_ptr<WeightGradient>();
+    const Tensor second = sum ? sum->first_runs() : Tensor();
     int mask = 0;
     for (int s = 0; s < 3; ++s) mask |= ctx->needs_input_grad(s) ? 1 << s : 0;
     if (!grads[0].defined() || !mask) {
-      out[2] = later;
+      out[2] = second;
       return out;
     }
     const auto saved = ctx->get_saved_variables();
     const auto op = kept<Op>(ctx, "op");
     const auto graph = kept<Graph>(ctx, "graph");
     const Tensor g = grads[0].contiguous();
-    // in place only where nobody else can see the tensor
-    const bool ours = later.defined() && mask & kW && !at::GradMode::is_enabled() && later.use_count() == 1 && later.has_storage() &&
-                      later.storage().use_count() == 1 && !later.requires_grad() && later.layout() == at::kStrided &&
-                      later.is_contiguous() && reinterpret_cast<uintptr_t>(later.data_ptr()) % 16 == 0;
     std::array<Tensor, 3> d;
     if (at::GradMode::is_enabled()) {
       Tensor w = saved[2];
       if (w.requires_grad() && static_cast<int64_t>(w.nbytes()) >= kSecondOrderBytes) {
-        if (!sum) keep(ctx, "sum", c10::make_intrusive<WeightGradient>(torch::autograd::get_current_node()));
-        w = SecondOrderWeights::apply(w, kept<WeightGradient>(ctx, "sum"));
+        if (!sum) {
+          sum = c10::make_intrusive<WeightGradient>(torch::autograd::get_current_node());
+          keep(ctx, "sum", sum);
+        }
+        w = SecondOrderWeights::apply(w, sum);
+        sum->second_order_is(w.grad_fn());
       }
       d = spread<3>(ConvBackward::apply(saved[0], saved[1], w, g, static_cast<int64_t>(mask), op, graph), mask);
     } else {
-      d = run_backward(*op, *graph, saved[0], saved[1], saved[2], g, mask, ours ? later : Tensor());
+      const WeightGradient::Operands all{saved[0], saved[1], saved[2], g, op, graph};
+      if (sum && mask & kW && !second.defined() && sum->leave_operands(all)) mask &= ~kW;
+      d = first_on_second(all, mask, second);
     }
-    if (later.defined() && !ours) d[2] = d[2].defined() ? d[2] + later : later;
     for (int s = 0; s < 3; ++s) out[s] = d[s];
     return out;
   }

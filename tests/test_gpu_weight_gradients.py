@@ -197,6 +197,52 @@ def test_one_loss_of_an_energy_that_is_linear_and_of_its_forces(edges):
         assert_close(gw, want, p.dtype, f"create_graph={create_graph}")
 
 
+@pytest.mark.parametrize("wanted", [(2,), (0, 1, 2)], ids=["weights", "all"])
+@pytest.mark.parametrize("name", CASES)
+@pytest.mark.parametrize("linear,energy_too", [(False, False), (False, True), (True, True)])
+def test_the_sum_is_made_in_place(name, linear, energy_too, wanted):
+    """Whichever order comes first, a second tensor of the weights' size is never there."""
+    p = Problem(name)
+
+    def step(conv, x, y, w, scale):
+        energy = energy_of(conv(x, y, w), linear, scale)
+        (gy,) = torch.autograd.grad(energy, y, create_graph=True)
+        return gy.square().sum() + (energy if energy_too else 0.0)
+
+    tensors = p.device()
+    loss = step(p.conv, *tensors)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got = torch.autograd.grad(loss, [tensors[i] for i in wanted])
+    assert torch.cuda.max_memory_allocated() - before < 1.5 * tensors[2].nbytes
+    cpu = [t.double().requires_grad_(True) for t in p.cpu]
+    conv = lambda x, y, w: oracle_conv.conv_forward(p.meta, x, y, w, p.src, p.dst, NODES)
+    want = torch.autograd.grad(step(conv, *cpu, p.scale.double()), [cpu[i] for i in wanted])
+    for value, ref, i in zip(got, want, wanted):
+        assert_close(value, ref, p.dtype, f"{name} {linear} {energy_too} {i}")
+
+
+@pytest.mark.parametrize("energy_first", [True, False])
+def test_two_force_losses_through_one_graph(energy_first):
+    """Two second orders, of which one at most meets the first order; alone, and in one loss."""
+    p = Problem("vector")
+    cpu = [t.double().requires_grad_(True) for t in p.cpu]
+    reference = lambda x, y, w: oracle_conv.conv_forward(p.meta, x, y, w, p.src, p.dst, NODES)
+
+    def losses(conv, x, y, w, scale):
+        energy = (conv(x, y, w) * scale).sum()
+        (gy,) = torch.autograd.grad(energy, y, create_graph=True)
+        (gx,) = torch.autograd.grad(energy, x, create_graph=True)
+        a, b = gy.square().sum(), gx.square().sum()
+        return (energy + a, energy + b, energy + a + b) if energy_first else (a + energy, b + energy, a + b + energy)
+
+    tensors = p.device()
+    for got, want in zip(losses(p.conv, *tensors), losses(reference, *cpu, p.scale.double())):
+        (value,) = torch.autograd.grad(got, tensors[2], retain_graph=True)
+        assert_close(value, torch.autograd.grad(want, cpu[2], retain_graph=True)[0], p.dtype, "two losses")
+
+
 def test_passes_after_one_that_failed():
     """The second order's gradient has been set aside when a pass ends with an error; the next ones have their own."""
     p = Problem("vector")
