@@ -41,8 +41,8 @@ bool paired(const luna_uvu_plan* plan, int shape, int cpl, bool forward) {
 // Channels per lane and warps per team, or slices for blocks that no team takes.  A warp's pass over an edge costs about one
 // unit of fixed work plus one per channel of a lane, so 48 channels take one warp with two channels on 24 lanes, 96 one warp
 // with four on 24 lanes.  A kernel that spills counts half as much again: degrees (3, 3, 3) with the most channels per lane,
-// all gradients.  300 MB of weights, FP64: 96 channels 0.64 -> 0.52 ms with one channel per lane, 224 channels 0.72 -> 0.49;
-// FP32: 128 channels 0.41 -> 0.30 with two, 256 channels 0.57 -> 0.34.
+// all gradients, which then spills 176 (FP32) or 276 bytes and more.  300 MB of weights, FP64: 96 channels 0.44 -> 0.41 ms with one
+// channel per lane, 224 channels 0.83 -> 0.54; FP32: 128 channels 0.33 -> 0.27 with two (2.6 GB: 2.03 -> 1.54), 256 channels 0.39 -> 0.30.
 // ch / 16 channels on each of a half warp's 16 lanes, two edges at a time, where that is compiled (edge_paired).
 EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool sliced) {
   const int ch = plan->edge.ch, elem = plan->dtype == LUNA_F64 ? 8 : 4;
