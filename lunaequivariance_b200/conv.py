@@ -567,8 +567,9 @@ def run_triple_backward(op, x, y, w, g, rx, ry, rw, bx, by, bw, bg, graph, needs
             if seed is None:
                 continue
             parts = [partial(slot, *operands) for operands in terms if all(o is not None for o in operands)]
-            if parts:
-                outputs.append(sum(parts[1:], parts[0]))
+            output = sum(parts[1:], parts[0]) if parts else None
+            if output is not None and output.requires_grad:  # else it depends on none of the wanted operands
+                outputs.append(output)
                 seeds.append(seed.contiguous())
         wanted = [leaf for leaf, need in zip(leaves, needs) if leaf is not None and need]
         found = iter(torch.autograd.grad(outputs, wanted, seeds, allow_unused=True)) if outputs and wanted else iter(())

@@ -68,6 +68,26 @@ def _third_order(function, x, y, w, seeds):
     return out, first, second, third
 
 
+@pytest.mark.parametrize("slot", range(7))
+def test_third_order_of_one_operand(slot, oracle_kernels):
+    """Some of the second-order outputs do not depend on the one operand whose gradient is asked for."""
+    module, meta, graph, src, dst, t, rand = _problem("small")
+    like = [t["x"], t["y"], t["w"], rand(graph.num_nodes, meta["out_dim"])]
+    operands = [*like, *(rand(*v.shape) for v in like[:3])]
+    seeds = [rand(*v.shape) for v in like]
+    needs = tuple(i == slot for i in range(7))
+    found = conv_mod.run_triple_backward(module.op, *operands, *seeds, graph, needs=needs)
+    leaves = [v.clone().requires_grad_(True) for v in operands]
+    x, y, w, g, rx, ry, rw = leaves
+    out = oracle_conv.conv_forward(meta, x, y, w, src, dst, graph.num_nodes)
+    first = torch.autograd.grad(out, (x, y, w), g, create_graph=True)
+    second = torch.autograd.grad(first, (x, y, w, g), (rx, ry, rw), create_graph=True)
+    want = torch.autograd.grad(second, leaves, seeds)
+    for i, value in enumerate(found):
+        assert (value is not None) == needs[i]
+    torch.testing.assert_close(found[slot], want[slot], rtol=1e-12, atol=1e-12)
+
+
 @pytest.mark.parametrize("name", ["small", "mul2"])
 def test_third_order_chain_matches_dense_autograd(name, oracle_kernels):
     module, meta, graph, src, dst, t, rand = _problem(name)
