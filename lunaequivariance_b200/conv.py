@@ -566,11 +566,12 @@ def run_triple_backward(op, x, y, w, g, rx, ry, rw, bx, by, bw, bg, graph, needs
         for seed, slot, terms in programs:
             if seed is None:
                 continue
+            # Every partial is an output of its own: their sum would have no history inside a registered op, where only
+            # autograd functions record one.  A partial of none of the wanted operands has none either.
             parts = [partial(slot, *operands) for operands in terms if all(o is not None for o in operands)]
-            output = sum(parts[1:], parts[0]) if parts else None
-            if output is not None and output.requires_grad:  # else it depends on none of the wanted operands
-                outputs.append(output)
-                seeds.append(seed.contiguous())
+            parts = [part for part in parts if part.requires_grad]
+            outputs += parts
+            seeds += [seed.contiguous()] * len(parts)
         wanted = [leaf for leaf, need in zip(leaves, needs) if leaf is not None and need]
         found = iter(torch.autograd.grad(outputs, wanted, seeds, allow_unused=True)) if outputs and wanted else iter(())
     result = []

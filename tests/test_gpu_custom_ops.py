@@ -51,6 +51,31 @@ def test_custom_ops_differentiate_twice(name, dtype):
         assert_close(value, ref[key], dtype, f"{name} op {key}")
 
 
+@pytest.mark.parametrize("slots", [range(7), *([i] for i in range(7))])
+def test_custom_ops_differentiate_three_times(slots):
+    """All operands of the second order, and each alone, of which some of the outputs are independent."""
+    module, graph, p, _ = _problem("fixture", torch.float64)
+    meta = oracle_conv.build_specs(*config("fixture")[:4])
+    generator = torch.Generator().manual_seed(9)
+    seeds = [torch.randn(p[k].shape, generator=generator, dtype=torch.float64) for k in ("x", "y", "w", "g")]
+
+    def third(conv, device):
+        leaves = [p[k].detach().to(device).requires_grad_(i in slots) for i, k in enumerate(("x", "y", "w", "g", "rx", "ry", "rw"))]
+        x, y, w, g, rx, ry, rw = leaves
+        for t in (x, y, w, g):  # the second order is there whatever the third one asks for
+            t.requires_grad_(True)
+        first = torch.autograd.grad(conv(x, y, w), (x, y, w), g, create_graph=True)
+        second = torch.autograd.grad(first, (x, y, w, g), (rx, ry, rw), create_graph=True)
+        return torch.autograd.grad(second, [leaves[i] for i in slots], [s.to(device) for s in seeds])
+
+    got = third(lambda x, y, w: torch.ops.lunatp.uvu_conv_forward(x, y, w, None, graph.table_list(), graph.num_nodes, False,
+                                                                  module.op.torch_config)[0], DEVICE)
+    src, dst = graph.src.cpu(), graph.dst.cpu()
+    want = third(lambda x, y, w: oracle_conv.conv_forward(meta, x, y, w, src, dst, graph.num_nodes), "cpu")
+    for i, a, b in zip(slots, got, want):
+        assert_close(a, b, torch.float64, f"third order, operand {i}")
+
+
 def test_opcheck_forward_op():
     module, graph, p, _ = _problem("one", torch.float64, nodes=5, edges=9)
     args = (p["x"].requires_grad_(True), p["y"].requires_grad_(True), p["w"].requires_grad_(True), None,
