@@ -7,7 +7,7 @@
 #include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
 
-#include "common.h"
+#include "graph_short.cuh"
 
 namespace luna {
 namespace {
@@ -66,8 +66,8 @@ __global__ void init_bounds(Bounds* result) {
 // (where a row's full pieces stand in the order of pieces) and the numbers of pieces by node (the pieces' row
 // pointers).  Sums are taken modulo 2^32: only differences within a set, which are smaller, are used.
 // What bounds it is the number of dependent launches, 3 to 17 us each: 16 of them, 135 us on the device for 1.05 M edges
-// and 20,000 nodes.  The whole call takes 202 us; with a sort for each order, two more of 64-bit keys for the pieces and
-// some forty tensor operations it took 755.
+// and 20,000 nodes, 201 us for the whole call.  Graphs whose rows all have at most 255 edges are built by counting
+// (graph_short.cuh) in 105; this is the way for longer rows, for luna_graph_build, and for graphs of over a million nodes.
 struct TableSizes {
   int64_t nodes, src_nodes, edges;
   bool segments;
@@ -245,7 +245,12 @@ ScratchLayout layout(TableSizes z) {
   l.full_at = take(static_cast<size_t>(z.src_nodes) * 4 + 4);
   l.part_at = take(static_cast<size_t>(z.src_nodes) * 4 + 4);
   l.cub_temp = take(l.cub_bytes);
-  l.total = cursor;
+  ShortTables t{};
+  t.nodes = z.nodes;
+  t.src_nodes = z.src_nodes;
+  t.edges = z.edges;
+  size_t zeroed = 0;
+  l.total = short_rows_likely(z.nodes, z.src_nodes, z.edges) ? std::max(cursor, short_layout(&t, nullptr, &zeroed)) : cursor;
   return l;
 }
 
@@ -400,6 +405,37 @@ extern "C" int luna_graph_build_all(const void* src, const void* dst, int index_
     return fail(LUNA_ERR_INVALID_ARGUMENT, "segment tables missing");
   auto stream = static_cast<cudaStream_t>(stream_);
   auto* base = static_cast<unsigned char*>(scratch);
+  if (short_rows_likely(num_nodes, num_src_nodes, num_edges)) {
+    ShortTables t{};
+    t.nodes = num_nodes;
+    t.src_nodes = num_src_nodes;
+    t.edges = num_edges;
+    t.src = out->src;
+    t.dst = out->dst;
+    t.iota = pieces->edge_ids_by_dst;
+    t.dst_rowptr = out->dst_rowptr;
+    t.src_rowptr = out->src_rowptr;
+    t.edge_ids = out->edge_ids_by_src;
+    t.node_order = out->node_order;
+    t.source_node_order = out->source_node_order;
+    t.tiers = pieces->node_tiers;
+    t.segment_nodes = pieces->segment_nodes;
+    t.segment_begin = pieces->segment_begin;
+    t.segment_end = pieces->segment_end;
+    t.segment_rowptr = pieces->segment_rowptr;
+    t.segment_order = pieces->segment_order;
+    size_t zeroed = 0;
+    short_layout(&t, base, &zeroed);
+    const int launched = index_bits == 64 ? short_tables<int64_t>(src, dst, t, zeroed, stream)
+                                          : short_tables<int32_t>(src, dst, t, zeroed, stream);
+    if (launched != LUNA_OK) return launched;
+    int head[2] = {0, 0};  // flag and number of pieces
+    LUNA_CUDA_CHECK(cudaMemcpyAsync(head, t.head, sizeof(head), cudaMemcpyDeviceToHost, stream));
+    LUNA_CUDA_CHECK(cudaStreamSynchronize(stream));
+    *bad = head[0] == kUnfit;
+    *num_segments = head[0] == 0 ? head[1] : 0;
+    if (head[0] != kLongRow) return LUNA_OK;
+  }
   const int built = wide_keys(z) ? build_tables<uint64_t>(src, dst, index_bits, z, *out, pieces, base, l, stream)
                                  : build_tables<uint32_t>(src, dst, index_bits, z, *out, pieces, base, l, stream);
   if (built != LUNA_OK) return built;

@@ -23,15 +23,7 @@ def _edges(nodes, source_rows, edges, hub, seed):
     return src, torch.sort(torch.randint(nodes, (edges,), generator=generator)).values
 
 
-# one edge; fewer edges than quarters; rows of exactly 31, 32, 33 rows per warp; rows without edges; more source rows than
-# destinations and fewer
-@pytest.mark.parametrize("nodes,source_rows,edges,hub", [
-    (1, 1, 1, False), (3, 3, 2, False), (30, 30, 3, False), (31, 31, 992, False), (32, 32, 1024, True),
-    (62, 62, 4_000, True), (500, 500, 300, False), (64, 900, 5_001, False), (900, 7, 5_001, True), (20_011, 20_011, 200_003, True),
-])
-@pytest.mark.parametrize("index_dtype", [torch.int32, torch.int64])
-def test_tables(nodes, source_rows, edges, hub, index_dtype):
-    src, dst = (t.to(index_dtype) for t in _edges(nodes, source_rows, edges, hub, nodes + edges))
+def _compare(src, dst, nodes, source_rows):
     other = None if source_rows == nodes else source_rows
     want = luna.make_graph(src, dst, nodes, num_src_nodes=other)
     got = luna.make_graph(src.cuda(), dst.cuda(), nodes, num_src_nodes=other)
@@ -41,6 +33,34 @@ def test_tables(nodes, source_rows, edges, hub, index_dtype):
         torch.testing.assert_close(getattr(got.source_segments, name).cpu(), getattr(want.source_segments, name), rtol=0,
                                    atol=0, msg=f"segment {name}")
     assert got.num_src_nodes == want.num_src_nodes and got.can_split == want.can_split
+
+
+# one edge; fewer edges than quarters; rows of exactly 31, 32, 33 rows per warp; rows without edges; more source rows than
+# destinations and fewer
+@pytest.mark.parametrize("nodes,source_rows,edges,hub", [
+    (1, 1, 1, False), (3, 3, 2, False), (30, 30, 3, False), (31, 31, 992, False), (32, 32, 1024, True),
+    (62, 62, 4_000, True), (500, 500, 300, False), (64, 900, 5_001, False), (900, 7, 5_001, True), (20_011, 20_011, 200_003, True),
+])
+@pytest.mark.parametrize("index_dtype", [torch.int32, torch.int64])
+def test_tables(nodes, source_rows, edges, hub, index_dtype):
+    src, dst = (t.to(index_dtype) for t in _edges(nodes, source_rows, edges, hub, nodes + edges))
+    _compare(src, dst, nodes, source_rows)
+
+
+# Rows of up to 255 edges are counted into place, a longer one anywhere sends the graph to the general sorts: both sides of the
+# line, whole blocks of 512 nodes and one more, every length of a row that is sorted in another number of registers, and rows
+# without edges.
+@pytest.mark.parametrize("longest", [32, 33, 64, 65, 128, 129, 254, 255, 256])
+@pytest.mark.parametrize("nodes,source_rows", [(512, 512), (1_025, 1_025), (513, 700), (1_024, 511)])
+def test_longest_row(longest, nodes, source_rows):
+    generator = torch.Generator().manual_seed(longest + nodes)
+    edges = 12 * nodes
+    for hub_side in (0, 1):
+        rows = (source_rows, nodes)
+        ends = [torch.randint(n - 1, (edges,), generator=generator) for n in rows]  # the last row is the long one
+        ends[hub_side][torch.randperm(edges, generator=generator)[:longest]] = rows[hub_side] - 1
+        order = torch.argsort(ends[1], stable=True)
+        _compare(ends[0][order], ends[1][order], nodes, source_rows)
 
 
 @pytest.mark.parametrize("src,dst,match", [
