@@ -28,7 +28,7 @@ NVCC_FLAGS = [
     "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "--expt-relaxed-constexpr",
-    # 101 MB of library become 20.  A module is unpacked when its first kernel is loaded: the first call of a layer takes 3.2 ms
+    # 136 MB of library become 27.  A module is unpacked when its first kernel is loaded: the first call of a layer takes 3.2 ms
     # instead of 1.4, once for each kind of layer.
     "--compress-mode=size",
 ]
@@ -43,7 +43,7 @@ def find_nvcc() -> str:
 
 # uvu_edge_inst.cu is compiled once per (element type, channels per lane, shape); the shapes are those of uvu_edge.cuh
 EDGE_SOURCE = "uvu_edge_inst.cu"
-EDGE_LANES = (("float", 1), ("float", 2), ("float", 4), ("double", 1), ("double", 2))
+EDGE_LANES = (("float", 1), ("float", 2), ("float", 3), ("float", 4), ("double", 1), ("double", 2), ("double", 3))
 EDGE_SHAPES = 11
 
 

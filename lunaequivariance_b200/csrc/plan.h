@@ -165,7 +165,9 @@ struct EdgePlan {
   int shape = -1;      // index of the compiled shape, -1 if the plan has none or is kept from its kernels
   int ch = 0;          // channels per block
   EdgeLanes lanes;      // of the forward
-  EdgeLanes lanes_one;  // of backward calls that want one gradient, or dL/dx and dL/dw
+  EdgeLanes lanes_one;  // of backward calls that want dL/dy or dL/dw alone
+  EdgeLanes lanes_sums;  // of those that want dL/dx, alone or with dL/dw
+  EdgeLanes lanes_output;  // of output and dL/dw in one launch
   EdgeLanes lanes_all;  // of backward calls that want dL/dy and another gradient
   // [0] of the shape, [1] of the shape with x and out exchanged
   std::vector<double> prog_c[2], term_c[2], coef[2];

@@ -1,5 +1,6 @@
 // Which plans the edge kernels serve, the tables they read, and the choice of the compiled instance.
 #include "uvu_edge_bwd.cuh"
+#include "uvu_edge_fwd.cuh"
 
 #include <cmath>
 #include <utility>
@@ -9,41 +10,72 @@ namespace edgek {
 
 namespace {
 
-enum class EdgeUse { kForward, kOneGradient, kAllGradients };
-
-// Whether the kernel of all gradients spills registers by hundreds of bytes (a few bytes are common, and harmless).
+// The estimate of what a lane of the kernel needs.
+template <typename T, int CPL, typename S>
+constexpr int registers_of(EdgeUse use) {
+  using R = Transposed<S>;
+  using One = std::conditional_t<S::OD >= S::XD, R, S>;
+  switch (use) {
+    case EdgeUse::kForward: return EdgeFwd<T, CPL, S>::registers;
+    case EdgeUse::kSums: return EdgeBwd<T, CPL, S, true, true, false>::registers;
+    case EdgeUse::kOutputAndWeights: return EdgeBwd<T, CPL, R, true, true, false>::registers;
+    case EdgeUse::kAllGradients: return EdgeBwd<T, CPL, S, true, true, true>::registers;
+    default: return std::max(EdgeBwd<T, CPL, One, false, false, true>::registers, EdgeBwd<T, CPL, One, false, true, false>::registers);
+  }
+}
 template <typename T, int CPL, int... ID>
-bool spills(int shape, std::integer_sequence<int, ID...>) {
-  bool found = false;
-  ((found = found || (shape == ID && EdgeBwd<T, CPL, ShapeOf<ID>, true, true, true>::registers > 255)), ...);
+int registers_of(int shape, EdgeUse use, std::integer_sequence<int, ID...>) {
+  int found = 0;
+  ((found = shape == ID ? registers_of<T, CPL, ShapeOf<ID>>(use) : found), ...);
   return found;
 }
-bool spills(const luna_uvu_plan* plan, int shape, int cpl) {
-  constexpr std::make_integer_sequence<int, kEdgeShapes> all{};
-  if (plan->dtype == LUNA_F64) return cpl == 2 ? spills<double, 2>(shape, all) : spills<double, 1>(shape, all);
-  return cpl == 4 ? spills<float, 4>(shape, all) : (cpl == 2 ? spills<float, 2>(shape, all) : spills<float, 1>(shape, all));
-}
-
-template <typename T, int CPL, int... ID>
-bool paired(int shape, bool forward, std::integer_sequence<int, ID...>) {
-  bool found = false;
-  ((found = found || (shape == ID && edge_paired<T, CPL, ID>(forward))), ...);
-  return found;
-}
-bool paired(const luna_uvu_plan* plan, int shape, int cpl, bool forward) {
+int registers_of(const luna_uvu_plan* plan, int shape, EdgeUse use, int cpl) {
   constexpr std::make_integer_sequence<int, kEdgeShapes> all{};
   if (plan->dtype == LUNA_F64)
-    return cpl == 1 ? paired<double, 1>(shape, forward, all) : cpl == 2 && paired<double, 2>(shape, forward, all);
-  return cpl == 1 ? paired<float, 1>(shape, forward, all)
-                  : (cpl == 2 ? paired<float, 2>(shape, forward, all) : cpl == 4 && paired<float, 4>(shape, forward, all));
+    return cpl == 3 ? registers_of<double, 3>(shape, use, all)
+                    : (cpl == 2 ? registers_of<double, 2>(shape, use, all) : registers_of<double, 1>(shape, use, all));
+  if (cpl >= 3) return cpl == 4 ? registers_of<float, 4>(shape, use, all) : registers_of<float, 3>(shape, use, all);
+  return cpl == 2 ? registers_of<float, 2>(shape, use, all) : registers_of<float, 1>(shape, use, all);
+}
+
+template <typename T, int CPL, int... ID>
+bool paired(int shape, EdgeUse use, std::integer_sequence<int, ID...>) {
+  bool found = false;
+  ((found = found || (shape == ID && edge_paired<T, CPL, ID>(use))), ...);
+  return found;
+}
+bool paired(const luna_uvu_plan* plan, int shape, EdgeUse use, int cpl) {
+  constexpr std::make_integer_sequence<int, kEdgeShapes> all{};
+  if (plan->dtype == LUNA_F64)
+    return cpl == 1 ? paired<double, 1>(shape, use, all)
+                    : (cpl == 2 ? paired<double, 2>(shape, use, all) : cpl == 3 && paired<double, 3>(shape, use, all));
+  if (cpl >= 3) return cpl == 4 ? paired<float, 4>(shape, use, all) : cpl == 3 && paired<float, 3>(shape, use, all);
+  return cpl == 1 ? paired<float, 1>(shape, use, all) : cpl == 2 && paired<float, 2>(shape, use, all);
+}
+
+// Coupling-matrix entries of the shape.
+template <int... ID>
+int matrix_entries(int shape, std::integer_sequence<int, ID...>) {
+  int found = 0;
+  ((found = shape == ID ? ShapeOf<ID>::m_total : found), ...);
+  return found;
 }
 
 // Channels per lane and warps per team, or slices for blocks that no team takes.  A warp's pass over an edge costs about one
-// unit of fixed work plus one per channel of a lane, so 48 channels take one warp with two channels on 24 lanes, 96 one warp
-// with four on 24 lanes.  A kernel that spills counts half as much again: degrees (3, 3, 3) with the most channels per lane,
-// all gradients, which then spills 176 (FP32) or 276 bytes and more.  300 MB of weights, FP64: 96 channels 0.44 -> 0.41 ms with one
-// channel per lane, 224 channels 0.83 -> 0.54; FP32: 128 channels 0.33 -> 0.27 with two (2.6 GB: 2.03 -> 1.54), 256 channels 0.39 -> 0.30.
-// ch / 16 channels on each of a half warp's 16 lanes, two edges at a time, where that is compiled (edge_paired).
+// unit of fixed work plus one per channel of a lane, so 40 channels take one warp with two channels on 20 lanes, 96 one warp
+// with three on all of them.  A kernel that spills counts half as much again: degrees (3, 3, 3) with the most channels
+// per lane, all gradients, which then spills 176 (FP32) or 276 bytes and more.  300 MB of weights, FP64: 224 channels with one
+// channel per lane 0.83 -> 0.54 ms; FP32: 128 channels 0.33 -> 0.27 with two (2.6 GB: 2.03 -> 1.54), 256 channels 0.39 -> 0.30.
+// Three channels per lane, where four or two left a quarter of the lanes idle.  96 channels, forward / all gradients / dL/dy / dL/dw,
+// FP32: (2, 2, 2), 0.4 M edges 364 / 958 / 465 / 520 -> 323 / 759 / 426 / 434 us; (2, 3, 3), 0.4 M edges 653 / 1,611 / 852 / 922 ->
+// 550 / 1,439 / 790 / 718; FP64, two warps with two and one with three: (2, 2, 2), 0.2 M edges 361 / 1,050 / 566 / 567 -> 332 /
+// 763 / 426 / 450; (0, 1, 1), 0.4 M edges 217 / 580 / 408 / 348 -> 128 / 351 / 185 / 207.  It is not taken where its state is far above
+// the registers (FP64, (3, 3, 3), all gradients of 0.12 M edges 1.96 -> 3.27 ms), for more than two warps, for slices, and for two FP32
+// warps with long coupling matrices: 192 channels, forward / dL/dy (3, 3, 3) 408 / 523 -> 486 / 556 us, (2, 3, 3) 466 / 698 -> 495 /
+// 758, but (0, 2, 2) 332 / 560 -> 246 / 398.
+// ch / 16 channels on each of a half warp's 16 lanes, two edges at a time, where that is compiled (edge_paired).  48 channels, one edge
+// on 24 lanes and two edges with three channels per lane, 0.8 M edges: (1, 1, 1) 192 / 576 / 340 / 393 -> 165 / 352 / 194 / 252; (0, 3, 3)
+// 260 / 642 / 359 / 432 -> 187 / 463 / 252 / 287; (2, 2, 2), 0.52 M edges, 274 / 715 / 378 / 427 -> 260 / 683 / 301 / 301.
 EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool sliced) {
   const int ch = plan->edge.ch, elem = plan->dtype == LUNA_F64 ? 8 : 4;
   // one team with two stages must fit an SM's shared memory in either direction
@@ -52,20 +84,24 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool s
   const size_t rows = std::max(std::max(2 * W + O, 2 * (W + X)), std::max(X, O));
   EdgeLanes best;
   double best_cost = 0.0;
-  for (int cpl = plan->dtype == LUNA_F64 ? 2 : 4; cpl >= 1; cpl /= 2) {
+  for (int cpl = plan->dtype == LUNA_F64 ? 3 : 4; cpl >= 1; --cpl) {
     if (plan->tuning.lane_channels > 0 && cpl != plan->tuning.lane_channels) continue;
     const int parts = (ch + 32 * cpl - 1) / (32 * cpl);
     if (sliced ? ch % (32 * cpl) != 0 || parts > kEdgeMaxSlices
                : parts > capped_warps(plan->tuning, 8) || ch % (parts * cpl) != 0 || rows + parts * 8192 > room)
       continue;
-    const double cost = parts * (1 + cpl) * (use == EdgeUse::kAllGradients && spills(plan, shape, cpl) ? 1.5 : 1.0);
+    const int registers = registers_of(plan, shape, use, cpl);
+    if (cpl == 3 && (sliced || parts > 2 || registers > (use == EdgeUse::kForward ? 255 : 280) ||
+                     (parts == 2 && elem == 4 && matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 64)))
+      continue;
+    const double cost = parts * (1 + cpl) * ((use == EdgeUse::kAllGradients || cpl == 3) && registers > 255 ? 1.5 : 1.0);
     if (best.cpl != 0 && cost >= best_cost) continue;
     best_cost = cost;
     best = sliced ? EdgeLanes{cpl, 1, parts} : EdgeLanes{cpl, parts, 1};
   }
   const int half = ch / 16;
   if (!sliced && ch % 16 == 0 && (plan->tuning.lane_channels == 0 || plan->tuning.lane_channels == half) &&
-      paired(plan, shape, half, use == EdgeUse::kForward))
+      paired(plan, shape, use, half))
     return EdgeLanes{half, 1, 1, 2};
   return best;
 }
@@ -181,8 +217,10 @@ template <typename F>
 int with_instance(const luna_uvu_plan* plan, const EdgeLanes& lanes, F&& body) {
   const int shape = plan->edge.shape;
   if (plan->dtype == LUNA_F64)
-    return lanes.cpl == 2 ? with_shape<double, 2, 0>(shape, body) : with_shape<double, 1, 0>(shape, body);
+    return lanes.cpl == 3 ? with_shape<double, 3, 0>(shape, body)
+                          : (lanes.cpl == 2 ? with_shape<double, 2, 0>(shape, body) : with_shape<double, 1, 0>(shape, body));
   if (lanes.cpl == 4) return with_shape<float, 4, 0>(shape, body);
+  if (lanes.cpl == 3) return with_shape<float, 3, 0>(shape, body);
   return lanes.cpl == 2 ? with_shape<float, 2, 0>(shape, body) : with_shape<float, 1, 0>(shape, body);
 }
 
@@ -202,8 +240,12 @@ void analyse(luna_uvu_plan* plan) {
   if (sliced && !edge_sliced(shape)) return;
   plan->edge.lanes = choose_lanes(plan, shape, EdgeUse::kForward, sliced);
   plan->edge.lanes_one = choose_lanes(plan, shape, EdgeUse::kOneGradient, sliced);
+  plan->edge.lanes_sums = choose_lanes(plan, shape, EdgeUse::kSums, sliced);
+  plan->edge.lanes_output = choose_lanes(plan, shape, EdgeUse::kOutputAndWeights, sliced);
   plan->edge.lanes_all = choose_lanes(plan, shape, EdgeUse::kAllGradients, sliced);
-  if (plan->edge.lanes.cpl != 0) plan->edge.shape = shape;
+  for (const EdgeLanes* lanes : {&plan->edge.lanes, &plan->edge.lanes_one, &plan->edge.lanes_sums, &plan->edge.lanes_output, &plan->edge.lanes_all})
+    if (lanes->cpl == 0) return;
+  plan->edge.shape = shape;
 }
 
 int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
@@ -217,20 +259,20 @@ int backward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph
              const void* w, const void* g, void* gx, bool acc_x, void* gy, bool acc_y, void* gw, bool acc_w, void* scratch,
              int64_t scratch_bytes, cudaStream_t stream) {
   const EdgeBackwardArgs args{x, y, w, g, gx, gy, gw, acc_x, acc_y, acc_w, scratch, scratch_bytes, nullptr};
-  const EdgeLanes& lanes = gy && (gx || gw) ? plan->edge.lanes_all : plan->edge.lanes_one;
+  const EdgeLanes& lanes = gy && (gx || gw) ? plan->edge.lanes_all : (gx ? plan->edge.lanes_sums : plan->edge.lanes_one);
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
 }
 
 int output_and_weights(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
                        const void* w, const void* g, void* out, void* gw, cudaStream_t stream) {
   const EdgeBackwardArgs args{x, y, w, g, nullptr, nullptr, gw, false, false, false, nullptr, 0, out};
-  const EdgeLanes& lanes = plan->edge.lanes_one;
+  const EdgeLanes& lanes = plan->edge.lanes_output;
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.backward(plan, dt, graph, lanes, args, stream); });
 }
 
 bool joins_output(const luna_uvu_plan* plan) {
   bool joins = false;
-  with_instance(plan, plan->edge.lanes_one, [&](auto kernels) {
+  with_instance(plan, plan->edge.lanes_output, [&](auto kernels) {
     joins = kernels.joins_output();
     return LUNA_OK;
   });

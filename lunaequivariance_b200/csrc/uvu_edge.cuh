@@ -143,20 +143,28 @@ constexpr int kEdgeShapeMasks[kEdgeShapes][3] = {{1, 3, 3},  {1, 7, 7},   {1, 15
 constexpr bool edge_sliced(int id) { return id >= 3 && id <= 6; }
 template <int ID>
 using ShapeOf = Shape<kEdgeShapeMasks[ID][0], kEdgeShapeMasks[ID][1], kEdgeShapeMasks[ID][2]>;
+// What a launch computes, as far as the choice of its layout goes: one gradient is dL/dy or dL/dw alone, sums are dL/dx, alone or
+// with dL/dw.
+enum class EdgeUse { kForward, kOneGradient, kSums, kOutputAndWeights, kAllGradients };
+
 // Whether the kernels of 16 * CPL channels walk two edges at a time, with CPL channels on each lane of a half warp: what is
-// compiled and what is chosen.  One and two channels per lane, if the rows of two pairs leave room for eight warps.  With fewer it
+// compiled and what is chosen.  One to three channels per lane, if the rows of two pairs leave room for eight warps.  With fewer it
 // loses: FP64, 32 channels, degrees (2, 3, 3), six warps, all gradients of 0.4 M edges 1.30 -> 1.75 ms.  Four FP32 channels for shapes
 // whose paths all have a degree of zero and whose degrees end at 2.  The others have more arithmetic in an edge than beside it, or
 // too many registers: (2, 2, 2), 64 channels, all gradients of 0.24 M edges 0.345 -> 0.391 ms with two at a time; (0, 3, 3), forward of
 // 0.8 M edges 0.249 -> 0.475.  Of these the forward at degree 2 only: one edge and two, forward / all gradients / dL/dy / dL/dw, 0.8 M
 // edges: (1, 1, 1) 165 / 555 / 322 / 416 -> 174 / 380 / 194 / 260 us; (1, 1, 0) 143 / 476 / 330 / 250 -> 156 / 310 / 188 / 231; (0, 2, 2),
 // 1.05 M edges, 282 / 710 / 422 / 518 -> 215 / 478 / 250 / 332; (2, 2, 0) 233 / 545 / 370 / 424 -> 176 / 439 / 215 / 268.
+// Three channels per lane with six or seven warps: for one gradient alone, whose state is small.  48 channels, one edge and two,
+// dL/dy / dL/dw: (2, 3, 3), 0.4 M edges 505 / 519 -> 432 / 476 us; FP64 (0, 3, 3), 0.4 M edges, 336 / 287 -> 248 / 214; but forward
+// and all gradients of (3, 3, 3), 0.2 M edges, 289 / 756 -> 333 / 1,245, and FP64 (3, 3, 0), all, 661 -> 772.
 template <typename T, int CPL, int ID>
-constexpr bool edge_paired(bool forward) {
+constexpr bool edge_paired(EdgeUse use) {
   using S = ShapeOf<ID>;
   constexpr int top = top_degree(S::MX | S::MO), row = S::paths + (S::XD > S::OD ? S::XD : S::OD);
-  const bool four = sizeof(T) == 4 && S::m_total == 0 && (top == 2 || (top == 1 && !forward));
-  return (CPL <= 2 || four) && 4 * row * 16 * CPL * static_cast<int>(sizeof(T)) <= 24 * 1024;
+  constexpr int bytes = 4 * row * 16 * CPL * static_cast<int>(sizeof(T));
+  const bool four = CPL == 4 && sizeof(T) == 4 && S::m_total == 0 && (top == 2 || (top == 1 && use != EdgeUse::kForward));
+  return (CPL <= 3 || four) && bytes <= (CPL == 3 && use == EdgeUse::kOneGradient ? 31 : 24) * 1024;
 }
 
 // ---- launch arguments, type-erased ------------------------------------------------------------------------------------
@@ -427,27 +435,44 @@ __device__ __forceinline__ void edge_attributes(const T* buffer, T* y) {
 }
 
 // A lane's channels.  Packet q of a lane holds PK::W consecutive channels, and the packets of the warp's lanes lie side
-// by side: packet q of lane l starts at channel  own + q * stride  with  own = first + W * l  and  stride = W * lanes.
+// by side: packet q of lane l starts at channel  own + q * W * lanes  with  own = first + W * l.
 // Weights then arrive as ready-made packets, and the scalar loads that assemble the packets of a node row (channel-
 // major, 2l + 1 components) meet two-way bank conflicts at most (with four consecutive channels per lane: four-way).
+// Spread packets hold channels  own + (q * W + c) * lanes  with  own = first + l:  no conflicts, and a load for every weight.
+template <typename PK>
+__device__ __forceinline__ int lane_channel(int q, int c, int lanes) {
+  return PK::spread ? (q * PK::W + c) * lanes : q * PK::W * lanes + c;
+}
+template <typename PK>
+__device__ __forceinline__ int lane_first(int lane) {
+  return PK::spread ? lane : PK::W * lane;
+}
 template <typename PK, typename T>
-__device__ __forceinline__ void lane_load(const T* p, int stride, typename PK::V* out) {
+__device__ __forceinline__ void lane_load(const T* p, int lanes, typename PK::V* out) {
 #pragma unroll
   for (int q = 0; q < PK::NP; ++q) {
-    if constexpr (PK::W == 2)
-      out[q].v = *reinterpret_cast<const unsigned long long*>(p + q * stride);
-    else
-      out[q] = p[q * stride];
+    if constexpr (PK::W == 2 && !PK::spread) {
+      out[q].v = *reinterpret_cast<const unsigned long long*>(p + q * PK::W * lanes);
+    } else {
+      T vals[PK::W];
+#pragma unroll
+      for (int c = 0; c < PK::W; ++c) vals[c] = p[lane_channel<PK>(q, c, lanes)];
+      out[q] = make_packet(vals, typename PK::V{});
+    }
   }
 }
 template <typename PK, typename T>
-__device__ __forceinline__ void lane_store(T* p, int stride, const typename PK::V* in) {
+__device__ __forceinline__ void lane_store(T* p, int lanes, const typename PK::V* in) {
 #pragma unroll
   for (int q = 0; q < PK::NP; ++q) {
-    if constexpr (PK::W == 2)
-      *reinterpret_cast<unsigned long long*>(p + q * stride) = in[q].v;
-    else
-      p[q * stride] = in[q];
+    if constexpr (PK::W == 2 && !PK::spread) {
+      *reinterpret_cast<unsigned long long*>(p + q * PK::W * lanes) = in[q].v;
+    } else {
+      T vals[PK::W];
+      split_packet(in[q], vals);
+#pragma unroll
+      for (int c = 0; c < PK::W; ++c) p[lane_channel<PK>(q, c, lanes)] = vals[c];
+    }
   }
 }
 // Components of a node row's block of D components per channel -> packets [component][packet]; p: the block plus
@@ -455,7 +480,7 @@ __device__ __forceinline__ void lane_store(T* p, int stride, const typename PK::
 // taken from vector loads are put together again in front of every packed instruction that uses the pair (measured on
 // the 128-channel degree-(2,3,3) backward: 18.9 ms against 11.4).
 template <typename PK, typename T, int D>
-__device__ __forceinline__ void lane_load_block(const T* p, int stride, typename PK::V* out) {
+__device__ __forceinline__ void lane_load_block(const T* p, int lanes, typename PK::V* out) {
   using V = typename PK::V;
 #pragma unroll
   for (int q = 0; q < PK::NP; ++q)
@@ -463,13 +488,13 @@ __device__ __forceinline__ void lane_load_block(const T* p, int stride, typename
     for (int i = 0; i < D; ++i) {
       T vals[PK::W];
 #pragma unroll
-      for (int c = 0; c < PK::W; ++c) vals[c] = p[q * stride * D + c * D + i];
+      for (int c = 0; c < PK::W; ++c) vals[c] = p[lane_channel<PK>(q, c, lanes) * D + i];
       out[i * PK::NP + q] = make_packet(vals, V{});
     }
 }
 // Packets [component][packet] to such a block in memory, added to what is there if `add`.
 template <typename PK, typename T, int D>
-__device__ __forceinline__ void lane_store_block(T* p, int stride, const typename PK::V* in, bool add) {
+__device__ __forceinline__ void lane_store_block(T* p, int lanes, const typename PK::V* in, bool add) {
 #pragma unroll
   for (int q = 0; q < PK::NP; ++q) {
     T row[PK::W * D];
@@ -480,14 +505,18 @@ __device__ __forceinline__ void lane_store_block(T* p, int stride, const typenam
 #pragma unroll
       for (int c = 0; c < PK::W; ++c) row[c * D + i] = vals[c];
     }
-    T* to = p + q * stride * D;
-    if (add) {
-      T old[PK::W * D];
-      load_vectors<T, PK::W, D>(to, old);
+    constexpr int together = PK::spread ? 1 : PK::W;  // channels side by side
 #pragma unroll
-      for (int a = 0; a < PK::W * D; ++a) row[a] += old[a];
+    for (int c = 0; c < PK::W; c += together) {
+      T *to = p + lane_channel<PK>(q, c, lanes) * D, *from = row + c * D;
+      if (add) {
+        T old[together * D];
+        load_vectors<T, together, D>(to, old);
+#pragma unroll
+        for (int a = 0; a < together * D; ++a) from[a] += old[a];
+      }
+      store_vectors<T, together, D>(to, from);
     }
-    store_vectors<T, PK::W, D>(to, row);
   }
 }
 

@@ -263,12 +263,12 @@ __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const
 
 // A path of an edge, for a lane's channels: wq its weights in the stage, which the gradients replace if `keep`.
 template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
-__device__ __forceinline__ void backward_path(T* wq, int stride, bool keep, const V* xr, V* gxr, V* gy2, const V* g2,
+__device__ __forceinline__ void backward_path(T* wq, int lanes, bool keep, const V* xr, V* gxr, V* gy2, const V* g2,
                                               const T* mbuf, const T* term, const T* coef) {
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   V w2[NP], dot[NP];
-  lane_load<PK, T>(wq, stride, w2);
+  lane_load<PK, T>(wq, lanes, w2);
   if constexpr (ADD) {
 #pragma unroll
     for (int p = 0; p < NP; ++p) dot[p] = w2[p];
@@ -279,7 +279,7 @@ __device__ __forceinline__ void backward_path(T* wq, int stride, bool keep, cons
     edge_diagonal<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, coef[S::coff(l1, l2, l3)]);
   else
     edge_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, term);
-  if (WM && keep) lane_store<PK, T>(wq, stride, dot);  // the gradients leave with the row
+  if (WM && keep) lane_store<PK, T>(wq, lanes, dot);  // the gradients leave with the row
 }
 
 // FULL: one warp per edge and 32 * CPL channels, known to the compiler.  SLICED: these are a slice of wider blocks.  DST: rows
@@ -330,8 +330,8 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   __syncthreads();
 
   const int cpw = ch / team_warps;  // channels of this warp
-  const int lanes = FULL ? 32 : cpw / CPL, stride = PK::W * lanes;
-  const int own = FULL ? PK::W * lane : member * cpw + PK::W * min(lane, lanes - 1);  // first channel of this lane
+  const int lanes = FULL ? 32 : cpw / CPL;
+  const int own = FULL ? lane_first<PK>(lane) : member * cpw + lane_first<PK>(min(lane, lanes - 1));  // first channel of this lane
   const bool active = FULL || lane < lanes;
   const bool leader = member == 0 && lane == 0;
   const bool issuing = SLICED || leader;  // the pieces of a slice are copied by all lanes
@@ -399,13 +399,13 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
     constexpr int l3 = decltype(l3c)::value;
     constexpr int d3 = 2 * l3 + 1;
     V g2[d3 * NP];
-    lane_load_block<PK, T, d3>(gblock + own * d3, stride, g2);
+    lane_load_block<PK, T, d3>(gblock + own * d3, lanes, g2);
     static_for<0, 4>([&](auto l1c) {
       constexpr int l1 = decltype(l1c)::value;
       static_for<0, 4>([&](auto l2c) {
         constexpr int l2 = decltype(l2c)::value;
         if constexpr (S::ok(l1, l2, l3)) {
-          backward_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, stride, storing && active,
+          backward_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, lanes, storing && active,
                                                                 xr, gxr, gy2, g2, mbuf, P.term, P.coef);
         }
       });
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           constexpr int l1 = decltype(l1c)::value;
           if constexpr (S::has(S::MX, l1)) {
             constexpr int d = 2 * l1 + 1;
-            lane_load_block<PK, T, d>(P.x + static_cast<int64_t>(n) * x_row + row_ch * S::xoff(l1) + (first_ch + own) * d, stride, &xr[S::xoff(l1) * NP]);
+            lane_load_block<PK, T, d>(P.x + static_cast<int64_t>(n) * x_row + row_ch * S::xoff(l1) + (first_ch + own) * d, lanes, &xr[S::xoff(l1) * NP]);
           }
         });
         if (!active) {
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           static_for<0, 4>([&](auto l1c) {
             constexpr int l1 = decltype(l1c)::value, d = 2 * l1 + 1;
             if constexpr (S::has(S::MX, l1))
-              lane_store_block<PK, T, d>(to + block * S::xoff(l1) + at * d, stride, &gxr[S::xoff(l1) * NP],
+              lane_store_block<PK, T, d>(to + block * S::xoff(l1) + at * d, lanes, &gxr[S::xoff(l1) * NP],
                                          !rest && P.acc_x);
           });
         }

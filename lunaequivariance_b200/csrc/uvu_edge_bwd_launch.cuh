@@ -139,11 +139,12 @@ constexpr bool edge_joins_output() {
   return 2 * EdgeBwd<T, CPL, R, true, true, false>::max_warps > EdgeBwd<T, CPL, R, false, true, false>::max_warps;
 }
 
-template <typename T, int CPL, typename S, bool FULL, bool SLICED, bool PAIR>
+// ALL: whether there are kernels for more than one gradient.
+template <typename T, int CPL, typename S, bool FULL, bool SLICED, bool PAIR, bool ALL = true>
 int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                       const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
   const bool wx = a.gx != nullptr, ww = a.gw != nullptr, wy = a.gy != nullptr;
-  if constexpr (edge_joins_output<T, CPL, S>()) {
+  if constexpr (ALL && edge_joins_output<T, CPL, S>()) {
     if (a.out)
       return launch_edge_bwd<T, CPL, Transposed<S>, true, true, false, FULL, true, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
   }
@@ -157,9 +158,13 @@ int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const l
     return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED, PAIR>(plan, dt, graph, lanes, a, stream)
               : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
   }
-  if (wy) return launch_edge_bwd<T, CPL, S, true, true, true, FULL, false, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
-  if (wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
-  return LUNA_OK;
+  if constexpr (ALL) {
+    if (wy) return launch_edge_bwd<T, CPL, S, true, true, true, FULL, false, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
+    if (wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
+    return LUNA_OK;
+  } else {
+    return wx || wy || ww ? fail(LUNA_ERR_UNSUPPORTED, "no kernel of two edges at a time for these gradients") : LUNA_OK;
+  }
 }
 
 }  // namespace edgek

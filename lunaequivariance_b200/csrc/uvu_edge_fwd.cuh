@@ -39,22 +39,22 @@ template <typename T, int CPL, typename S>
 struct EdgeFwd {
   static constexpr int words = sizeof(T) / 4;
   static constexpr int m_elems = S::m_elems;
-  static constexpr int max_warps =
-      warps_for((S::OD + S::XD) * CPL * words + S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 + 44);
+  static constexpr int registers = (S::OD + S::XD) * CPL * words + S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 + 44;
+  static constexpr int max_warps = warps_for(registers);
   static constexpr size_t team_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
 };
 
 // out_k += sum_i M[i][k] * (x_i * w) for one path, over the entries of M that the pattern has.  xl / al: a lane's packets of
 // x and of the sums, of degrees l1 and l3; wq: its first weight; buffer: the edge's matrices.
 template <typename T, int CPL, typename S, int l1, int l2, int l3, typename V>
-__device__ __forceinline__ void forward_path(const T* wq, int stride, const T* buffer, const V* xl, V* al) {
+__device__ __forceinline__ void forward_path(const T* wq, int lanes, const T* buffer, const V* xl, V* al) {
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   using PT = CgPattern<l1, l2, l3>;
   const T* matrix = buffer + S::moff(l1, l2, l3);
   V w2[NP], xw[NP];
   T m[4];
-  lane_load<PK, T>(wq, stride, w2);
+  lane_load<PK, T>(wq, lanes, w2);
   static_for<0, PT::n>([&](auto tc) {
     constexpr int t = decltype(tc)::value;
     if constexpr (edge_new_entry<PT>(t)) {
@@ -70,13 +70,13 @@ __device__ __forceinline__ void forward_path(const T* wq, int stride, const T* b
 }
 // The paths with a degree of zero, c their coefficient: out_k += (c y w) x_k, (c w x) y_k or (c w) sum_i y_i x_i.
 template <typename T, int CPL, typename S, int l1, int l2, int l3, typename V>
-__device__ __forceinline__ void forward_diagonal(const T* wq, int stride, const T* buffer, T c, const V* xl, V* al) {
+__device__ __forceinline__ void forward_diagonal(const T* wq, int lanes, const T* buffer, T c, const V* xl, V* al) {
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   T y[8];
   edge_attributes<S, l2>(buffer, y);
   V w2[NP];
-  lane_load<PK, T>(wq, stride, w2);
+  lane_load<PK, T>(wq, lanes, w2);
   const V scale = bcast_packet(l2 == 0 ? c * y[0] : c, V{});
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
@@ -98,7 +98,7 @@ __device__ __forceinline__ void forward_diagonal(const T* wq, int stride, const 
 }
 // All paths of an edge, for a lane's channels.  ws: its first weight; xs: the edge's row of x.
 template <typename T, int CPL, typename S, typename V>
-__device__ __forceinline__ void forward_edge(const T* ws, const T* xs, int ch, int own, int stride, const T* buffer,
+__device__ __forceinline__ void forward_edge(const T* ws, const T* xs, int ch, int own, int lanes, const T* buffer,
                                              const T* coef, V* acc) {
   using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
@@ -107,7 +107,7 @@ __device__ __forceinline__ void forward_edge(const T* ws, const T* xs, int ch, i
     if constexpr (S::has(S::MX, l1)) {
       constexpr int d1 = 2 * l1 + 1;
       V xl[d1 * NP];
-      lane_load_block<PK, T, d1>(xs + ch * S::xoff(l1) + own * d1, stride, xl);
+      lane_load_block<PK, T, d1>(xs + ch * S::xoff(l1) + own * d1, lanes, xl);
       static_for<0, 4>([&](auto l3c) {
         constexpr int l3 = decltype(l3c)::value;
         static_for<0, 4>([&](auto l2c) {
@@ -116,9 +116,9 @@ __device__ __forceinline__ void forward_edge(const T* ws, const T* xs, int ch, i
             const T* wq = ws + S::rank(l1, l2, l3) * ch;
             V* al = &acc[S::ooff(l3) * NP];
             if constexpr (S::diagonal(l1, l2, l3))
-              forward_diagonal<T, CPL, S, l1, l2, l3>(wq, stride, buffer, coef[S::coff(l1, l2, l3)], xl, al);
+              forward_diagonal<T, CPL, S, l1, l2, l3>(wq, lanes, buffer, coef[S::coff(l1, l2, l3)], xl, al);
             else
-              forward_path<T, CPL, S, l1, l2, l3>(wq, stride, buffer, xl, al);
+              forward_path<T, CPL, S, l1, l2, l3>(wq, lanes, buffer, xl, al);
           }
         });
       });
@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   __syncthreads();
 
   const int cpw = ch / team_warps;  // channels of this warp
-  const int lanes = FULL ? 32 : cpw / CPL, stride = PK::W * lanes;
-  const int own = FULL ? PK::W * lane : member * cpw + PK::W * min(lane, lanes - 1);  // first channel of this lane
+  const int lanes = FULL ? 32 : cpw / CPL;
+  const int own = FULL ? lane_first<PK>(lane) : member * cpw + lane_first<PK>(min(lane, lanes - 1));  // first channel of this lane
   const bool active = FULL || lane < lanes;
   const bool leader = member == 0 && lane == 0;
   const bool issuing = SLICED || leader;  // the pieces of a slice are copied by all lanes
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         program.run(y_next, mbuf + (buf ^ 1) * K::m_elems, lane, member, team_warps);  // of the next edge; of no use after the last one
         if (lane < S::YD && e + 2 < e_end) y_next = P.y[static_cast<int64_t>(e + 2) * S::YD + lane];
         const T* m_now = mbuf + buf * K::m_elems;
-        forward_edge<T, CPL, S>(ws, xs, ch, own, stride, m_now, P.coef, acc);
+        forward_edge<T, CPL, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
         buf ^= 1;
         team_sync(team_warps, team);  // every lane is done with this stage and with the matrices
         if (issuing && e + stages < e_end) {
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         static_for<0, 4>([&](auto l3c) {
           constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
           if constexpr (S::has(S::MO, l3))
-            lane_store_block<PK, T, d3>(to + block * S::ooff(l3) + at * d3, stride, &acc[S::ooff(l3) * NP],
+            lane_store_block<PK, T, d3>(to + block * S::ooff(l3) + at * d3, lanes, &acc[S::ooff(l3) * NP],
                                         !rest && P.accumulate);
         });
       }

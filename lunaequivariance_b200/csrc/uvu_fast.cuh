@@ -334,7 +334,7 @@ __device__ __forceinline__ void load_ell(unsigned char* smem, const T* __restric
 // FP32 with an even number of channels per lane uses packed two-wide arithmetic; everything else the scalar path.
 template <typename T, int CPL>
 struct UsePairs {
-  static constexpr bool value = sizeof(T) == 4 && (CPL % 2 == 0);
+  static constexpr bool value = sizeof(T) == 4 && CPL > 1;
 };
 
 // One warp's share of the coupling-matrix computation when `parts` warps split the entries: warp `part` handles

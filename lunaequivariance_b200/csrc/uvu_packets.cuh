@@ -8,25 +8,39 @@ namespace fastk {
 
 // ---- arithmetic packets ---------------------------------------------------------------------------------------------
 // A lane's CPL channels are processed as NP packets of W channels: FP32 pairs with packed two-wide FMAs when CPL is
-// even, scalars otherwise.  A pair lives in one 64-bit register from the load to the last use (the packed instructions take 64-bit
+// even, a pair and a scalar when it is three, scalars otherwise.  `spread`: the channels of a packet are as far apart as the
+// warp has lanes, instead of side by side.  A pair lives in one 64-bit register from the load to the last use (the packed instructions take 64-bit
 // operands; keeping the halves as separate floats costs a register move per operand).
 struct Pair {
   unsigned long long v;
+};
+struct Triple {
+  unsigned long long v;
+  float s;
 };
 template <typename T, int CPL, bool PACKED>
 struct PkT {
   using V = T;
   static constexpr int W = 1, NP = CPL;
+  static constexpr bool spread = false;
 };
 template <>
 struct PkT<float, 2, true> {
   using V = Pair;
   static constexpr int W = 2, NP = 1;
+  static constexpr bool spread = false;
+};
+template <>
+struct PkT<float, 3, true> {
+  using V = Triple;
+  static constexpr int W = 3, NP = 1;
+  static constexpr bool spread = true;
 };
 template <>
 struct PkT<float, 4, true> {
   using V = Pair;
   static constexpr int W = 2, NP = 2;
+  static constexpr bool spread = false;
 };
 __device__ __forceinline__ Pair vfma(Pair a, Pair b, Pair c) {
   Pair d;
@@ -56,6 +70,17 @@ __device__ __forceinline__ float hsum(Pair a) {
   split_packet(a, v);
   return v[0] + v[1];
 }
+__device__ __forceinline__ Triple vfma(Triple a, Triple b, Triple c) {
+  return Triple{vfma(Pair{a.v}, Pair{b.v}, Pair{c.v}).v, fmaf(a.s, b.s, c.s)};
+}
+__device__ __forceinline__ Triple vmul(Triple a, Triple b) { return Triple{vmul(Pair{a.v}, Pair{b.v}).v, a.s * b.s}; }
+__device__ __forceinline__ Triple vadd(Triple a, Triple b) { return Triple{vadd(Pair{a.v}, Pair{b.v}).v, a.s + b.s}; }
+__device__ __forceinline__ Triple make_packet(const float* vals, Triple) { return Triple{make_packet(vals, Pair{}).v, vals[2]}; }
+__device__ __forceinline__ void split_packet(Triple a, float* vals) {
+  split_packet(Pair{a.v}, vals);
+  vals[2] = a.s;
+}
+__device__ __forceinline__ float hsum(Triple a) { return hsum(Pair{a.v}) + a.s; }
 __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float vmul(float a, float b) { return a * b; }
@@ -69,14 +94,17 @@ __device__ __forceinline__ double make_packet(const double* vals, double) { retu
 __device__ __forceinline__ void split_packet(float a, float* vals) { vals[0] = a; }
 __device__ __forceinline__ void split_packet(double a, double* vals) { vals[0] = a; }
 __device__ __forceinline__ Pair shfl_xor_packet(Pair a, int mask) { return Pair{__shfl_xor_sync(0xffffffffu, a.v, mask)}; }
+__device__ __forceinline__ Triple shfl_xor_packet(Triple a, int mask) {
+  return Triple{__shfl_xor_sync(0xffffffffu, a.v, mask), __shfl_xor_sync(0xffffffffu, a.s, mask)};
+}
 __device__ __forceinline__ float shfl_xor_packet(float a, int mask) { return __shfl_xor_sync(0xffffffffu, a, mask); }
 __device__ __forceinline__ double shfl_xor_packet(double a, int mask) { return __shfl_xor_sync(0xffffffffu, a, mask); }
 template <typename V>
 __device__ __forceinline__ V zero_packet() {
-  if constexpr (sizeof(V) == sizeof(Pair) && !std::is_floating_point<V>::value) {
-    return V{0ull};
-  } else {
+  if constexpr (std::is_floating_point<V>::value) {
     return V(0);
+  } else {
+    return V{};
   }
 }
 
@@ -119,6 +147,7 @@ __device__ __forceinline__ Pair bcast_packet(float m, Pair) {
   asm("mov.b64 %0, {%1, %1};" : "=l"(d.v) : "f"(m));
   return d;
 }
+__device__ __forceinline__ Triple bcast_packet(float m, Triple) { return Triple{bcast_packet(m, Pair{}).v, m}; }
 __device__ __forceinline__ float bcast_packet(float m, float) { return m; }
 __device__ __forceinline__ double bcast_packet(double m, double) { return m; }
 

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "uvu_edge_bwd.cuh"
+#include "uvu_pair_fwd.cuh"
 
 namespace luna {
 namespace edgek {
@@ -11,6 +12,7 @@ namespace edgek {
 template <typename T, int CPL, typename S, bool WX, bool WM, bool WY>
 struct PairBwd {
   using Edge = EdgeBwd<T, CPL, S, WX, WM, WY>;
+  using Packet = PkT<T, CPL, UsePairs<T, CPL>::value>;
   static constexpr int m_elems = WM ? S::m_elems : 0;  // of each half
   static constexpr int red_rows = Edge::red_rows, red_pass = Edge::red_pass, red_row = Edge::red_row;
   static constexpr int warp_elems = 2 * m_elems + (WY ? red_pass * red_row : 0);
@@ -29,8 +31,8 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   static_assert(!ADD || (WM && !WX && !WY), "the weights' place in a stage must be free");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, place = lane & 15;
-  constexpr int ch = 16 * CPL, stride = PK::W * 16, W = S::paths * ch, X = S::XD * ch, O = S::OD * ch, stage_elems = 2 * (W + O);
-  const int stages = P.stages, own = PK::W * place;
+  constexpr int ch = 16 * CPL, lanes = 16, W = S::paths * ch, X = S::XD * ch, O = S::OD * ch, half_elems = pair_half<PK>(W + O), stage_elems = 2 * half_elems;
+  const int stages = P.stages, own = lane_first<PK>(place);
 
   T* const base = reinterpret_cast<T*>(smem_raw);
   T* const ring = base + static_cast<size_t>(warp) * P.team_elems;
@@ -54,7 +56,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   const uint32_t w_bytes = P.need_w ? static_cast<uint32_t>(W * sizeof(T)) : 0u, g_bytes = static_cast<uint32_t>(O * sizeof(T));
 
   auto load_stage = [&](int e, int d, int st) {  // by the issuing lane of either half, of its edge; e < 0: none
-    T* to = ring + static_cast<size_t>(st) * stage_elems + half * (W + O);
+    T* to = ring + static_cast<size_t>(st) * stage_elems + half * half_elems;
     mbar_arrive_expect_tx(&full[st], e >= 0 ? w_bytes + g_bytes : 0u);
     if (e < 0) return;
     if (w_bytes) bulk_copy_g2s_hint(to, P.w + static_cast<int64_t>(e) * W, w_bytes, &full[st], l2_policy_evict_first());
@@ -73,13 +75,13 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   auto unit_body = [&](auto l3c, T* wrow) {
     constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
     V g2[d3 * NP];
-    lane_load_block<PK, T, d3>(wrow + W + ch * S::ooff(l3) + own * d3, stride, g2);
+    lane_load_block<PK, T, d3>(wrow + W + ch * S::ooff(l3) + own * d3, lanes, g2);
     static_for<0, 4>([&](auto l1c) {
       constexpr int l1 = decltype(l1c)::value;
       static_for<0, 4>([&](auto l2c) {
         constexpr int l2 = decltype(l2c)::value;
         if constexpr (S::ok(l1, l2, l3))
-          backward_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, stride, storing, xr, gxr,
+          backward_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, lanes, storing, xr, gxr,
                                                                 gy2, g2, mbuf, P.term, P.coef);
       });
     });
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           static_for<0, 4>([&](auto l1c) {
             constexpr int l1 = decltype(l1c)::value, d = 2 * l1 + 1;
             if constexpr (S::has(S::MX, l1))
-              lane_store_block<PK, T, d>(to + ch * S::xoff(l1) + own * d, stride, &gxr[S::xoff(l1) * NP], !rest && add);
+              lane_store_block<PK, T, d>(to + ch * S::xoff(l1) + own * d, lanes, &gxr[S::xoff(l1) * NP], !rest && add);
           });
         }
 #pragma unroll
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           constexpr int l1 = decltype(l1c)::value;
           if constexpr (S::has(S::MX, l1)) {
             constexpr int d = 2 * l1 + 1;
-            lane_load_block<PK, T, d>(P.x + static_cast<int64_t>(mine) * X + ch * S::xoff(l1) + own * d, stride, &xr[S::xoff(l1) * NP]);
+            lane_load_block<PK, T, d>(P.x + static_cast<int64_t>(mine) * X + ch * S::xoff(l1) + own * d, lanes, &xr[S::xoff(l1) * NP]);
           }
         });
       }
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
         if (lane == 0) atomicExch(P.status, 3);
         alive = false;
       }
-      T* const wrow = ring + static_cast<size_t>(st) * stage_elems + half * (W + O);
+      T* const wrow = ring + static_cast<size_t>(st) * stage_elems + half * half_elems;
       const bool valid = e0 >= 0;
       static_for<0, 4>([&](auto l3c) {
         constexpr int l3 = decltype(l3c)::value;
@@ -358,7 +360,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
 // K: the PairBwd of the kernel.
 template <typename T, typename S, typename K>
 EdgeLaunch pair_bwd_launch(const Tuning& tuning, int ch, int max_smem) {
-  const size_t stage = 2 * static_cast<size_t>(S::paths + S::OD) * ch * sizeof(T), row = static_cast<size_t>(S::XD) * ch * sizeof(T);
+  const size_t stage = 2 * static_cast<size_t>(pair_half<typename K::Packet>((S::paths + S::OD) * ch)) * sizeof(T), row = static_cast<size_t>(S::XD) * ch * sizeof(T);
   EdgeLaunch launch;
   for (int warps = capped_warps(tuning, K::max_warps); warps >= 1 && launch.warps == 0; --warps)
     for (int stages = 3; stages >= 2; --stages) {

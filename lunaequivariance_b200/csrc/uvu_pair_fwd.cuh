@@ -1,6 +1,6 @@
 // Forward kernel for narrow blocks: a warp walks two edges at a time, one on each half of its lanes.
 //
-// With 16 or 32 channels the arithmetic of an edge is a few dozen instructions per warp, and what an edge costs beside
+// With 16, 32 or 48 channels the arithmetic of an edge is a few dozen instructions per warp, and what an edge costs beside
 // it - waits, copies, addresses, the coupling matrices - is several times that.  Here a lane owns CPL channels of
 // half a warp, 16 * CPL channels in all, and both halves run the same instructions on an edge each.  One edge per warp and
 // two, degrees (2, 2, 2), 0.2 M edges, forward / all gradients: FP32, 32 channels 0.116 / 0.259 -> 0.105 / 0.216 ms, 16
@@ -19,6 +19,12 @@
 namespace luna {
 namespace edgek {
 
+// Elements of a stage that one half's rows take: with spread packets an odd multiple of 16, so that the halves' lanes read
+// different banks.
+template <typename PK>
+__host__ __device__ constexpr int pair_half(int elems) {
+  return PK::spread && elems % 32 == 0 ? elems + 16 : elems;
+}
 template <typename T, int CPL, typename S>
 struct PairFwd {
   static constexpr int words = sizeof(T) / 4;
@@ -34,8 +40,8 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
   constexpr int NP = PK::NP;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, place = lane & 15;
-  constexpr int ch = 16 * CPL, stride = PK::W * 16, W = S::paths * ch, X = S::XD * ch, O = S::OD * ch, stage_elems = 2 * (W + X);
-  const int stages = P.stages, own = PK::W * place;
+  constexpr int ch = 16 * CPL, lanes = 16, W = S::paths * ch, X = S::XD * ch, O = S::OD * ch, half_elems = pair_half<PK>(W + X), stage_elems = 2 * half_elems;
+  const int stages = P.stages, own = lane_first<PK>(place);
 
   T* const ring = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(warp) * P.ring_elems;
   T* const mbuf = reinterpret_cast<T*>(smem_raw) + static_cast<size_t>(P.teams) * P.ring_elems +
@@ -55,7 +61,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
   const bool issuing = place == 0;  // a half's copies are its first lane's
   const uint32_t w_bytes = static_cast<uint32_t>(W * sizeof(T)), x_bytes = static_cast<uint32_t>(X * sizeof(T));
   auto issue = [&](int e, int s_node, bool real, int s) {  // by the issuing lane of either half, of its edge
-    T* to = ring + static_cast<size_t>(s) * stage_elems + half * (W + X);
+    T* to = ring + static_cast<size_t>(s) * stage_elems + half * half_elems;
     mbar_arrive_expect_tx(&bars[s], real ? w_bytes + x_bytes : 0u);
     if (!real) return;
     bulk_copy_g2s_hint(to, P.w + static_cast<int64_t>(e) * W, w_bytes, &bars[s], l2_policy_evict_first());
@@ -84,7 +90,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
       static_for<0, 4>([&](auto l3c) {
         constexpr int l3 = decltype(l3c)::value, d3 = 2 * l3 + 1;
         if constexpr (S::has(S::MO, l3))
-          lane_store_block<PK, T, d3>(to + ch * S::ooff(l3) + own * d3, stride, &acc[S::ooff(l3) * NP], !rest && add);
+          lane_store_block<PK, T, d3>(to + ch * S::ooff(l3) + own * d3, lanes, &acc[S::ooff(l3) * NP], !rest && add);
       });
 #pragma unroll
       for (int a = 0; a < S::OD * NP; ++a) acc[a] = zero_packet<V>();
@@ -156,12 +162,12 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
         if (lane == 0) atomicExch(P.status, 1);
         alive = false;
       }
-      const T* ws = ring + static_cast<size_t>(s) * stage_elems + half * (W + X) + own;
+      const T* ws = ring + static_cast<size_t>(s) * stage_elems + half * half_elems + own;
       const T* xs = ws - own + W;
       program.run(y_next, mbuf + (buf ^ 1) * S::m_elems, place);  // of the next pair; of no use after the last one
       if (place < S::YD && mine + 4 < e_end) y_next = P.y[static_cast<int64_t>(mine + 4) * S::YD + place];
       const T* m_now = mbuf + buf * S::m_elems;
-      if (mine < e_end) forward_edge<T, CPL, S>(ws, xs, ch, own, stride, m_now, P.coef, acc);
+      if (mine < e_end) forward_edge<T, CPL, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
       buf ^= 1;
       __syncwarp();  // every lane is done with this stage and with the matrices
       if (issuing && e + 2 * stages < e_end) {
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
 
 template <typename T, int CPL, typename S>
 EdgeLaunch pair_fwd_launch(const Tuning& tuning, int ch, int max_smem) {
-  const size_t stage = 2 * static_cast<size_t>(S::paths + S::XD) * ch * sizeof(T), row = static_cast<size_t>(S::OD) * ch * sizeof(T);
+  const size_t stage = 2 * static_cast<size_t>(pair_half<PkT<T, CPL, UsePairs<T, CPL>::value>>((S::paths + S::XD) * ch)) * sizeof(T), row = static_cast<size_t>(S::OD) * ch * sizeof(T);
   EdgeLaunch launch;
   const int max_warps = capped_warps(tuning, PairFwd<T, CPL, S>::max_warps);
   for (int warps = max_warps; warps >= 1 && launch.warps == 0; --warps)

@@ -118,6 +118,16 @@ def one_gradient_alone(shape, mul, dtype, nodes, edges, skew, seed):
         assert_close(value, ref[key], dtype, f"{shape} x{mul} {dtype} {key} alone")
 
 
+# three channels per lane: two edges at a time (48), all lanes (96), idle lanes (66, 72), two warps per edge (102, 144)
+@pytest.mark.parametrize("shape,mul,dtype", [
+    *((shape, mul, dtype) for shape in range(len(SHAPES)) for mul in (48, 96) for dtype in (torch.float32, torch.float64)),
+    (4, 72, torch.float32), (1, 144, torch.float32), (4, 66, torch.float64), (4, 102, torch.float64), (3, 144, torch.float64)])
+def test_three_channels_per_lane(shape, mul, dtype):
+    check(SHAPES[shape], mul, dtype, 29, 400, 0.0, shape)  # long rows: shared by teams
+    one_gradient_alone(SHAPES[shape], mul, dtype, 150, 190, 1.5, shape + 50)  # short rows: tiles, many rows without edges
+    one_gradient_alone(SHAPES[shape], mul, dtype, 460, 2100, 0.0, shape + 90)  # equal parts
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("shape", range(len(SHAPES)))
 def test_one_gradient_alone(shape, dtype):
