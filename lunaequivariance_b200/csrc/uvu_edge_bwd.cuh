@@ -669,13 +669,10 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   if (!parts) {
     if (member == 0) leave_tiles(counters, total, lane);
   } else if constexpr (WX) {
-    __syncthreads();
-    const TeamPart part = kept[team];
-    if (want_x && part.closes()) {
-      T* const row = P.gx + static_cast<int64_t>(part.n) * x_row;
-      add_earlier_parts(part, P.src_rowptr[part.n], base, P.team_elems, team, P.teams, member * 32 + lane, team_warps * 32, X,
-                        [&](int a) { return row + (SLICED ? slice_element<S>(S::MX, a, ch, row_ch, first_ch) : a); });
-    }
+    if (want_x)
+      merge_parts(kept, P.teams, P.src_rowptr, base, P.team_elems, X, [&](int row, int a) {
+        return P.gx + static_cast<int64_t>(row) * x_row + (SLICED ? slice_element<S>(S::MX, a, ch, row_ch, first_ch) : a);
+      });
   }
   if (WM && issuing) bulk_wait_group_read_all();
   if (!alive) {  // let copies that are still in flight land before the CTA's shared memory is released

@@ -316,13 +316,9 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     unit = unit_after;
   }
   if (parts) {
-    __syncthreads();
-    const TeamPart part = kept[team];
-    if (part.closes()) {
-      T* const row = P.out + static_cast<int64_t>(part.n) * o_row;
-      add_earlier_parts(part, P.dst_rowptr[part.n], reinterpret_cast<const T*>(smem_raw), P.ring_elems, team, P.teams,
-                        member * 32 + lane, team_warps * 32, O, [&](int a) { return row + (SLICED ? slice_element<S>(S::MO, a, ch, row_ch, first_ch) : a); });
-    }
+    merge_parts(kept, P.teams, P.dst_rowptr, reinterpret_cast<const T*>(smem_raw), P.ring_elems, O, [&](int row, int a) {
+      return P.out + static_cast<int64_t>(row) * o_row + (SLICED ? slice_element<S>(S::MO, a, ch, row_ch, first_ch) : a);
+    });
   } else if (!grouped && member == 0) {
     leave_tiles(counters, total, lane);
   }

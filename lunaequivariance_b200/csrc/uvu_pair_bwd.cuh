@@ -345,12 +345,9 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   if (!parts) {
     leave_tiles(P.tile_counters, total, lane);
   } else if constexpr (WX) {
-    __syncthreads();
-    const TeamPart part = kept[warp];
-    if (want_x && part.closes()) {
-      T* const row = P.gx + static_cast<int64_t>(part.n) * X;
-      add_earlier_parts(part, P.src_rowptr[part.n], base, P.team_elems, warp, P.teams, lane, 32, X, [&](int a) { return row + a; });
-    }
+    if (want_x)
+      merge_parts(kept, P.teams, P.src_rowptr, base, P.team_elems, X,
+                  [&](int row, int a) { return P.gx + static_cast<int64_t>(row) * X + a; });
   }
   if (WM && issuing) bulk_wait_group_read_all();
   if (!alive)  // let copies that are still in flight land before the CTA's shared memory is released

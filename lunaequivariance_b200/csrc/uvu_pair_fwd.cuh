@@ -207,13 +207,8 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
     unit = unit_after;
   }
   if (parts) {
-    __syncthreads();
-    const TeamPart part = kept[warp];
-    if (part.closes()) {
-      T* const row = P.out + static_cast<int64_t>(part.n) * O;
-      add_earlier_parts(part, P.dst_rowptr[part.n], reinterpret_cast<const T*>(smem_raw), P.ring_elems, warp, P.teams,
-                        lane, 32, O, [&](int a) { return row + a; });
-    }
+    merge_parts(kept, P.teams, P.dst_rowptr, reinterpret_cast<const T*>(smem_raw), P.ring_elems, O,
+                [&](int row, int a) { return P.out + static_cast<int64_t>(row) * O + a; });
   } else if (!grouped) {
     leave_tiles(P.tile_counters, total, lane);
   }
