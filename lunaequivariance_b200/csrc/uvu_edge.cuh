@@ -475,6 +475,16 @@ __device__ __forceinline__ void edge_attributes(const T* buffer, T* y) {
 // Weights then arrive as ready-made packets, and the scalar loads that assemble the packets of a node row (channel-
 // major, 2l + 1 components) meet two-way bank conflicts at most (with four consecutive channels per lane: four-way).
 // Spread packets hold channels  own + (q * W + c) * lanes  with  own = first + l:  no conflicts, and a load for every weight.
+// Pairs are spread (edge_spread) where an edge's gathered row has at least twice as many components as its weight row has paths:
+// first layers backward, which gather g, and last layers forward, which gather x.  128 channels: (0, 3, 3), 1.05 M edges, all
+// gradients 1,169 -> 1,090 us, dL/dx with dL/dw 1,002 -> 947; (3, 3, 0), 0.4 M edges, forward 272 -> 244; (2, 2, 0) 182 -> 165.
+// Elsewhere the further loads of weights cost what the conflicts did: (2, 2, 2) and (2, 3, 3) within 2 %, (2, 2, 2) with 96
+// channels, dL/dw 526 -> 567.
+constexpr bool edge_spread(int gathered, int paths) { return gathered >= 2 * paths; }
+template <typename T, int CPL, bool SPREAD>
+struct EdgePacket : PkT<T, CPL, UsePairs<T, CPL>::value> {
+  static constexpr bool spread = SPREAD || PkT<T, CPL, UsePairs<T, CPL>::value>::spread;
+};
 template <typename PK>
 __device__ __forceinline__ int lane_channel(int q, int c, int lanes) {
   return PK::spread ? (q * PK::W + c) * lanes : q * PK::W * lanes + c;

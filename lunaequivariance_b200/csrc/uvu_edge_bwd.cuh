@@ -98,10 +98,9 @@ struct EdgeBwd {
 // One path for a lane's packets.  xl / gxl: the lane's x and gx packets of degree l1; g2: its g packets of degree l3;
 // w2: its weights; dot receives (ADD: is added) sum_i x_i s_i; gyl: the accumulators of degree l2.  The arithmetic of a row i is issued
 // in batches of independent instructions, so that the latency of one is covered by the others with few warps resident.
-template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
+template <typename T, typename PK, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
 __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* g2, const V* w2, V* dot, const T* mbuf,
                                           const T* term) {
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   using PT = CgPattern<l1, l2, l3>;
   constexpr int n = PT::n;
@@ -175,9 +174,8 @@ __device__ __forceinline__ void edge_path(const V* xl, V* gxl, V* gyl, const V* 
 // eleven paths of degrees (2, 2, 2) are like that, eight of the seventeen of (2, 3, 3).  Forward and backward with all paths in
 // edge_path, and like this: (2, 3, 3), 128 channels, 2.6 M edges 15.88 -> 15.33 ms; (3, 3, 3), 64 channels, 1.6 M edges 8.99
 // -> 8.54; (2, 2, 2), 64 channels, 5.2 M edges 10.23 -> 9.98; FP64 force step, 1.05 M edges 34.8 -> 33.9.
-template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
+template <typename T, typename PK, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
 __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const V* g2, const V* w2, V* dot, const T* mbuf, T c) {
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP, d = 2 * (l1 > l3 ? l1 : l3) + 1;
   T y[8];
   if constexpr (WM) edge_attributes<S, l2>(mbuf, y);
@@ -262,10 +260,9 @@ __device__ __forceinline__ void edge_diagonal(const V* xl, V* gxl, V* gyl, const
 }
 
 // A path of an edge, for a lane's channels: wq its weights in the stage, which the gradients replace if `keep`.
-template <typename T, int CPL, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
+template <typename T, typename PK, typename S, int l1, int l2, int l3, bool WX, bool WM, bool WY, bool ADD, typename V>
 __device__ __forceinline__ void backward_path(T* wq, int lanes, bool keep, const V* xr, V* gxr, V* gy2, const V* g2,
                                               const T* mbuf, const T* term, const T* coef) {
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   V w2[NP], dot[NP];
   lane_load<PK, T>(wq, lanes, w2);
@@ -276,9 +273,9 @@ __device__ __forceinline__ void backward_path(T* wq, int lanes, bool keep, const
   const V* xl = &xr[S::xoff(l1) * NP];
   V *gxl = &gxr[WX ? S::xoff(l1) * NP : 0], *gyl = &gy2[WY ? S::yoff(l2) : 0];
   if constexpr (S::diagonal(l1, l2, l3))
-    edge_diagonal<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, coef[S::coff(l1, l2, l3)]);
+    edge_diagonal<T, PK, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, coef[S::coff(l1, l2, l3)]);
   else
-    edge_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, term);
+    edge_path<T, PK, S, l1, l2, l3, WX, WM, WY, ADD, V>(xl, gxl, gyl, g2, w2, dot, mbuf, term);
   if (WM && keep) lane_store<PK, T>(wq, lanes, dot);  // the gradients leave with the row
 }
 
@@ -288,7 +285,7 @@ template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL,
 __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32, 1)
     edge_bwd_kernel(const __grid_constant__ EdgeBwdParams<T, EdgeBwd<T, CPL, S, WX, WM, WY>::terms> P) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  using PK = EdgePacket<T, CPL, edge_spread(S::OD, S::paths)>;
   using V = typename PK::V;
   constexpr int NP = PK::NP;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -405,7 +402,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       static_for<0, 4>([&](auto l2c) {
         constexpr int l2 = decltype(l2c)::value;
         if constexpr (S::ok(l1, l2, l3)) {
-          backward_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, lanes, storing && active,
+          backward_path<T, PK, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, lanes, storing && active,
                                                                 xr, gxr, gy2, g2, mbuf, P.term, P.coef);
         }
       });

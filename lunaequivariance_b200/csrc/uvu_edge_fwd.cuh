@@ -46,9 +46,8 @@ struct EdgeFwd {
 
 // out_k += sum_i M[i][k] * (x_i * w) for one path, over the entries of M that the pattern has.  xl / al: a lane's packets of
 // x and of the sums, of degrees l1 and l3; wq: its first weight; buffer: the edge's matrices.
-template <typename T, int CPL, typename S, int l1, int l2, int l3, typename V>
+template <typename T, typename PK, typename S, int l1, int l2, int l3, typename V>
 __device__ __forceinline__ void forward_path(const T* wq, int lanes, const T* buffer, const V* xl, V* al) {
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   using PT = CgPattern<l1, l2, l3>;
   const T* matrix = buffer + S::moff(l1, l2, l3);
@@ -69,9 +68,8 @@ __device__ __forceinline__ void forward_path(const T* wq, int lanes, const T* bu
   });
 }
 // The paths with a degree of zero, c their coefficient: out_k += (c y w) x_k, (c w x) y_k or (c w) sum_i y_i x_i.
-template <typename T, int CPL, typename S, int l1, int l2, int l3, typename V>
+template <typename T, typename PK, typename S, int l1, int l2, int l3, typename V>
 __device__ __forceinline__ void forward_diagonal(const T* wq, int lanes, const T* buffer, T c, const V* xl, V* al) {
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   T y[8];
   edge_attributes<S, l2>(buffer, y);
@@ -97,10 +95,9 @@ __device__ __forceinline__ void forward_diagonal(const T* wq, int lanes, const T
   }
 }
 // All paths of an edge, for a lane's channels.  ws: its first weight; xs: the edge's row of x.
-template <typename T, int CPL, typename S, typename V>
+template <typename T, typename PK, typename S, typename V>
 __device__ __forceinline__ void forward_edge(const T* ws, const T* xs, int ch, int own, int lanes, const T* buffer,
                                              const T* coef, V* acc) {
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
   constexpr int NP = PK::NP;
   static_for<0, 4>([&](auto l1c) {
     constexpr int l1 = decltype(l1c)::value;
@@ -116,9 +113,9 @@ __device__ __forceinline__ void forward_edge(const T* ws, const T* xs, int ch, i
             const T* wq = ws + S::rank(l1, l2, l3) * ch;
             V* al = &acc[S::ooff(l3) * NP];
             if constexpr (S::diagonal(l1, l2, l3))
-              forward_diagonal<T, CPL, S, l1, l2, l3>(wq, lanes, buffer, coef[S::coff(l1, l2, l3)], xl, al);
+              forward_diagonal<T, PK, S, l1, l2, l3>(wq, lanes, buffer, coef[S::coff(l1, l2, l3)], xl, al);
             else
-              forward_path<T, CPL, S, l1, l2, l3>(wq, lanes, buffer, xl, al);
+              forward_path<T, PK, S, l1, l2, l3>(wq, lanes, buffer, xl, al);
           }
         });
       });
@@ -131,7 +128,7 @@ template <typename T, int CPL, typename S, bool FULL, bool SLICED>
 __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
     edge_fwd_kernel(const __grid_constant__ EdgeFwdParams<T> P) {
   using K = EdgeFwd<T, CPL, S>;
-  using PK = PkT<T, CPL, UsePairs<T, CPL>::value>;
+  using PK = EdgePacket<T, CPL, edge_spread(S::XD, S::paths)>;
   using V = typename PK::V;
   constexpr int NP = PK::NP;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -274,7 +271,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
         program.run(y_next, mbuf + (buf ^ 1) * K::m_elems, lane, member, team_warps);  // of the next edge; of no use after the last one
         if (lane < S::YD && e + 2 < e_end) y_next = P.y[static_cast<int64_t>(e + 2) * S::YD + lane];
         const T* m_now = mbuf + buf * K::m_elems;
-        forward_edge<T, CPL, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
+        forward_edge<T, PK, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
         buf ^= 1;
         team_sync(team_warps, team);  // every lane is done with this stage and with the matrices
         if (issuing && e + stages < e_end) {

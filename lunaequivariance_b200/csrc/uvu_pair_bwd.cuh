@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
       static_for<0, 4>([&](auto l2c) {
         constexpr int l2 = decltype(l2c)::value;
         if constexpr (S::ok(l1, l2, l3))
-          backward_path<T, CPL, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, lanes, storing, xr, gxr,
+          backward_path<T, PK, S, l1, l2, l3, WX, WM, WY, ADD, V>(wrow + S::rank(l1, l2, l3) * ch + own, lanes, storing, xr, gxr,
                                                                 gy2, g2, mbuf, P.term, P.coef);
       });
     });

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
       program.run(y_next, mbuf + (buf ^ 1) * S::m_elems, place);  // of the next pair; of no use after the last one
       if (place < S::YD && mine + 4 < e_end) y_next = P.y[static_cast<int64_t>(mine + 4) * S::YD + place];
       const T* m_now = mbuf + buf * S::m_elems;
-      if (mine < e_end) forward_edge<T, CPL, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
+      if (mine < e_end) forward_edge<T, PK, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
       buf ^= 1;
       __syncwarp();  // every lane is done with this stage and with the matrices
       if (issuing && e + 2 * stages < e_end) {
