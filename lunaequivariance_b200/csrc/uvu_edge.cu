@@ -1,6 +1,5 @@
 // Which plans the edge kernels serve, the tables they read, and the choice of the compiled instance.
-#include "uvu_edge_bwd.cuh"
-#include "uvu_edge_fwd.cuh"
+#include "uvu_pair_bwd.cuh"
 
 #include <cmath>
 #include <utility>
@@ -66,6 +65,9 @@ int matrix_entries(int shape, std::integer_sequence<int, ID...>) {
 // with three on all of them.  A kernel that spills counts half as much again: degrees (3, 3, 3) with the most channels
 // per lane, all gradients, which then spills 176 (FP32) or 276 bytes and more.  300 MB of weights, FP64: 224 channels with one
 // channel per lane 0.83 -> 0.54 ms; FP32: 128 channels 0.33 -> 0.27 with two (2.6 GB: 2.03 -> 1.54), 256 channels 0.39 -> 0.30.
+// The forward with an estimate of more than 190 registers counts a third more: FP32 (3, 3, 3), 128 channels, two warps with two channels
+// per lane instead of one with four, 0.2 M edges 620 -> 583 us, 24,000 edges 134 -> 115; 256 channels, 60,000 edges, 420 -> 398.  (FP64
+// with 128 channels would lose by one per lane, 867 -> 972, and at a third more the choice stays at two.)
 // Three channels per lane, where four or two left a quarter of the lanes idle.  96 channels, forward / all gradients / dL/dy / dL/dw,
 // FP32: (2, 2, 2), 0.4 M edges 364 / 958 / 465 / 520 -> 323 / 759 / 426 / 434 us; (2, 3, 3), 0.4 M edges 653 / 1,611 / 852 / 922 ->
 // 550 / 1,439 / 790 / 718; FP64, two warps with two and one with three: (2, 2, 2), 0.2 M edges 361 / 1,050 / 566 / 567 -> 332 /
@@ -94,7 +96,10 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool s
     if (cpl == 3 && (sliced || parts > 2 || registers > (use == EdgeUse::kForward ? 255 : 280) ||
                      (parts == 2 && elem == 4 && matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 64)))
       continue;
-    const double cost = parts * (1 + cpl) * ((use == EdgeUse::kAllGradients || cpl == 3) && registers > 255 ? 1.5 : 1.0);
+    const double crowded = (use == EdgeUse::kAllGradients || cpl == 3) && registers > 255 ? 1.5
+                           : use == EdgeUse::kForward && registers > 190                   ? 1.3
+                                                                                           : 1.0;
+    const double cost = parts * (1 + cpl) * crowded;
     if (best.cpl != 0 && cost >= best_cost) continue;
     best_cost = cost;
     best = sliced ? EdgeLanes{cpl, 1, parts} : EdgeLanes{cpl, parts, 1};

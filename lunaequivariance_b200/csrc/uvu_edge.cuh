@@ -147,26 +147,6 @@ using ShapeOf = Shape<kEdgeShapeMasks[ID][0], kEdgeShapeMasks[ID][1], kEdgeShape
 // with dL/dw.
 enum class EdgeUse { kForward, kOneGradient, kSums, kOutputAndWeights, kAllGradients };
 
-// Whether the kernels of 16 * CPL channels walk two edges at a time, with CPL channels on each lane of a half warp: what is
-// compiled and what is chosen.  One to three channels per lane, if the rows of two pairs leave room for eight warps.  With fewer it
-// loses: FP64, 32 channels, degrees (2, 3, 3), six warps, all gradients of 0.4 M edges 1.30 -> 1.75 ms.  Four FP32 channels for shapes
-// whose paths all have a degree of zero and whose degrees end at 2.  The others have more arithmetic in an edge than beside it, or
-// too many registers: (2, 2, 2), 64 channels, all gradients of 0.24 M edges 0.345 -> 0.391 ms with two at a time; (0, 3, 3), forward of
-// 0.8 M edges 0.249 -> 0.475.  Of these the forward at degree 2 only: one edge and two, forward / all gradients / dL/dy / dL/dw, 0.8 M
-// edges: (1, 1, 1) 165 / 555 / 322 / 416 -> 174 / 380 / 194 / 260 us; (1, 1, 0) 143 / 476 / 330 / 250 -> 156 / 310 / 188 / 231; (0, 2, 2),
-// 1.05 M edges, 282 / 710 / 422 / 518 -> 215 / 478 / 250 / 332; (2, 2, 0) 233 / 545 / 370 / 424 -> 176 / 439 / 215 / 268.
-// Three channels per lane with six or seven warps: for one gradient alone, whose state is small.  48 channels, one edge and two,
-// dL/dy / dL/dw: (2, 3, 3), 0.4 M edges 505 / 519 -> 432 / 476 us; FP64 (0, 3, 3), 0.4 M edges, 336 / 287 -> 248 / 214; but forward
-// and all gradients of (3, 3, 3), 0.2 M edges, 289 / 756 -> 333 / 1,245, and FP64 (3, 3, 0), all, 661 -> 772.
-template <typename T, int CPL, int ID>
-constexpr bool edge_paired(EdgeUse use) {
-  using S = ShapeOf<ID>;
-  constexpr int top = top_degree(S::MX | S::MO), row = S::paths + (S::XD > S::OD ? S::XD : S::OD);
-  constexpr int bytes = 4 * row * 16 * CPL * static_cast<int>(sizeof(T));
-  const bool four = CPL == 4 && sizeof(T) == 4 && S::m_total == 0 && (top == 2 || (top == 1 && use != EdgeUse::kForward));
-  return (CPL <= 3 || four) && bytes <= (CPL == 3 && use == EdgeUse::kOneGradient ? 31 : 24) * 1024;
-}
-
 // ---- launch arguments, type-erased ------------------------------------------------------------------------------------
 struct EdgeForwardArgs {
   const void *x, *y, *w;

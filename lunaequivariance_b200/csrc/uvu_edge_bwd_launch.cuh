@@ -139,32 +139,36 @@ constexpr bool edge_joins_output() {
   return 2 * EdgeBwd<T, CPL, R, true, true, false>::max_warps > EdgeBwd<T, CPL, R, false, true, false>::max_warps;
 }
 
-// ALL: whether there are kernels for more than one gradient.
-template <typename T, int CPL, typename S, bool FULL, bool SLICED, bool PAIR, bool ALL = true>
+// ID: the shape's number, which tells with PAIR which uses have kernels of two edges at a time.
+template <typename T, int CPL, int ID, bool FULL, bool SLICED, bool PAIR>
 int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                       const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
+  using S = ShapeOf<ID>;
   const bool wx = a.gx != nullptr, ww = a.gw != nullptr, wy = a.gy != nullptr;
-  if constexpr (ALL && edge_joins_output<T, CPL, S>()) {
+  auto compiled = [](EdgeUse use) { return !PAIR || edge_paired<T, CPL, ID>(use); };
+  if constexpr (edge_joins_output<T, CPL, S>() && compiled(EdgeUse::kOutputAndWeights)) {
     if (a.out)
       return launch_edge_bwd<T, CPL, Transposed<S>, true, true, false, FULL, true, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
   }
   // One gradient per edge and none per row.  FP64, degrees (2, 3, 3), 128 channels, 1.05 M edges: rows by source 5.91 ms
   // (gw) and 6.44 ms (gy), by destination 5.36 and 5.95 ms.
-  if (!wx && ww != wy) {
-    constexpr bool dst = S::OD >= S::XD;
-    using R = std::conditional_t<dst, Transposed<S>, S>;
-    if (ww && a.acc_w)
-      return launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED, PAIR, true>(plan, dt, graph, lanes, a, stream);
-    return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED, PAIR>(plan, dt, graph, lanes, a, stream)
-              : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
+  if constexpr (compiled(EdgeUse::kOneGradient)) {
+    if (!a.out && !wx && ww != wy) {
+      constexpr bool dst = S::OD >= S::XD;
+      using R = std::conditional_t<dst, Transposed<S>, S>;
+      if (ww && a.acc_w)
+        return launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED, PAIR, true>(plan, dt, graph, lanes, a, stream);
+      return ww ? launch_edge_bwd<T, CPL, R, false, true, false, FULL, dst, SLICED, PAIR>(plan, dt, graph, lanes, a, stream)
+                : launch_edge_bwd<T, CPL, R, false, false, true, FULL, dst, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
+    }
   }
-  if constexpr (ALL) {
+  if constexpr (compiled(EdgeUse::kAllGradients)) {
     if (wy) return launch_edge_bwd<T, CPL, S, true, true, true, FULL, false, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
-    if (wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
-    return LUNA_OK;
-  } else {
-    return wx || wy || ww ? fail(LUNA_ERR_UNSUPPORTED, "no kernel of two edges at a time for these gradients") : LUNA_OK;
   }
+  if constexpr (compiled(EdgeUse::kSums)) {
+    if (!wy && wx) return launch_edge_bwd<T, CPL, S, true, true, false, FULL, false, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);
+  }
+  return wx || wy || ww || a.out ? fail(LUNA_ERR_UNSUPPORTED, "no kernel of this layout for these gradients") : LUNA_OK;
 }
 
 }  // namespace edgek

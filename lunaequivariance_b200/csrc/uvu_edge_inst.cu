@@ -26,18 +26,15 @@ template <>
 int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::backward(const luna_uvu_plan* plan, const DeviceTables& dt,
                                                                        const luna_graph* graph, const EdgeLanes& lanes, const EdgeBackwardArgs& a,
                                                                        cudaStream_t stream) {
-  using S = ShapeOf<LUNA_EDGE_SHAPE>;
   if constexpr (edge_sliced(LUNA_EDGE_SHAPE) && LUNA_EDGE_CPL != 3) {
-    if (lanes.slices > 1) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, false>(plan, dt, graph, lanes, a, stream);
+    if (lanes.slices > 1)
+      return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE, true, true, false>(plan, dt, graph, lanes, a, stream);
   }
-  constexpr bool one = edge_paired<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>(EdgeUse::kOneGradient);
-  constexpr bool all = edge_paired<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>(EdgeUse::kAllGradients);
-  if constexpr (one) {
-    if (lanes.edges == 2) return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, true, all>(plan, dt, graph, lanes, a, stream);
-  }
+  if (lanes.edges == 2)
+    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE, true, false, true>(plan, dt, graph, lanes, a, stream);
   if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, false>(plan, dt, graph, lanes, a, stream);
-  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false, false>(plan, dt, graph, lanes, a, stream);
+    return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE, true, false, false>(plan, dt, graph, lanes, a, stream);
+  return dispatch_edge_bwd<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE, false, false, false>(plan, dt, graph, lanes, a, stream);
 }
 
 template <>

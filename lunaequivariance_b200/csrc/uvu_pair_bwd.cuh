@@ -17,7 +17,8 @@ struct PairBwd {
   static constexpr int red_rows = Edge::red_rows, red_pass = Edge::red_pass, red_row = Edge::red_row;
   static constexpr int warp_elems = 2 * m_elems + (WY ? red_pass * red_row : 0);
   static constexpr int program_regs = WM ? 4 * S::m_rounds * Edge::words + S::m_rounds + 1 : 0;
-  static constexpr int max_warps = warps_for(Edge::state + program_regs + 44);
+  static constexpr int registers = Edge::state + program_regs + 44;
+  static constexpr int max_warps = warps_for(registers);
 };
 
 // 16 * CPL channels.  DST: rows by destination (S, x and g exchanged).  ADD: gw alone, added to; w names gw.
@@ -371,6 +372,40 @@ EdgeLaunch pair_bwd_launch(const Tuning& tuning, int ch, int max_smem) {
       break;
     }
   return launch;
+}
+
+// Whether the kernels of 16 * CPL channels walk two edges at a time, with CPL channels on each lane of a half warp: what is
+// compiled and what is chosen.  One to three channels per lane, if the rows of two pairs leave room for eight warps.  With fewer it
+// loses: FP64, 32 channels, degrees (2, 3, 3), six warps, all gradients of 0.4 M edges 1.30 -> 1.75 ms.  Four FP32 channels for shapes
+// whose paths all have a degree of zero and whose degrees end at 2.  The others have more arithmetic in an edge than beside it, or
+// too many registers: (2, 2, 2), 64 channels, all gradients of 0.24 M edges 0.345 -> 0.391 ms with two at a time; (0, 3, 3), forward of
+// 0.8 M edges 0.249 -> 0.475.  Of these the forward at degree 2 only: one edge and two, forward / all gradients / dL/dy / dL/dw, 0.8 M
+// edges: (1, 1, 1) 165 / 555 / 322 / 416 -> 174 / 380 / 194 / 260 us; (1, 1, 0) 143 / 476 / 330 / 250 -> 156 / 310 / 188 / 231; (0, 2, 2),
+// 1.05 M edges, 282 / 710 / 422 / 518 -> 215 / 478 / 250 / 332; (2, 2, 0) 233 / 545 / 370 / 424 -> 176 / 439 / 215 / 268.
+// Three channels per lane with six or seven warps: for one gradient alone, whose state is small.  48 channels, one edge and two,
+// dL/dy / dL/dw: (2, 3, 3), 0.4 M edges 505 / 519 -> 432 / 476 us; FP64 (0, 3, 3), 0.4 M edges, 336 / 287 -> 248 / 214; but forward
+// and all gradients of (3, 3, 3), 0.2 M edges, 289 / 756 -> 333 / 1,245, and FP64 (3, 3, 0), all, 661 -> 772.
+// Two channels per lane with eight warps, where one edge with one channel per lane has sixteen, or where the state is far above the
+// registers' share: shapes with coupling matrices, several gradients.  32 channels, two edges and one: FP32 (3, 3, 3), 0.4 M
+// edges, all gradients 1,123 -> 897 us, dL/dx with dL/dw 709 -> 602, output with dL/dw 700 -> 563; (2, 3, 3), all, 678 -> 595; FP64
+// (2, 2, 2), 0.4 M edges, 517 -> 488 and 504 -> 432, but all, eight warps and twelve, 617 -> 682.
+template <typename T, typename S, bool WY>
+constexpr bool pair_crowded() {
+  using Two = PairBwd<T, 2, S, true, true, WY>;
+  return Two::max_warps == 8 && (EdgeBwd<T, 1, S, true, true, WY>::max_warps >= 16 || Two::registers > 190);
+}
+template <typename T, int CPL, int ID>
+constexpr bool edge_paired(EdgeUse use) {
+  using S = ShapeOf<ID>;
+  if (CPL == 2 && S::m_total > 0) {
+    if (use == EdgeUse::kAllGradients && pair_crowded<T, S, true>()) return false;
+    if (use == EdgeUse::kSums && pair_crowded<T, S, false>()) return false;
+    if (use == EdgeUse::kOutputAndWeights && pair_crowded<T, Transposed<S>, false>()) return false;
+  }
+  constexpr int top = top_degree(S::MX | S::MO), row = S::paths + (S::XD > S::OD ? S::XD : S::OD);
+  constexpr int bytes = 4 * row * 16 * CPL * static_cast<int>(sizeof(T));
+  const bool four = CPL == 4 && sizeof(T) == 4 && S::m_total == 0 && (top == 2 || (top == 1 && use != EdgeUse::kForward));
+  return (CPL <= 3 || four) && bytes <= (CPL == 3 && use == EdgeUse::kOneGradient ? 31 : 24) * 1024;
 }
 
 }  // namespace edgek
