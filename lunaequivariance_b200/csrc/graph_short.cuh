@@ -15,7 +15,7 @@
 // A longer row sets the flag to kLongRow and the caller takes the general way.
 //
 // 1.05 M edges, 20,000 nodes, the five launches: 10, 14, 6, 9 and 9 us; the whole call, with the allocations before it and the
-// synchronisation at its end, 201 -> 105 us.  short_edges is not bound by its atomics (a copy of the same bytes takes 4.5 us);
+// synchronisation at its end, 201 -> 105 us, and 93 with launches that overlap (launch_early).  short_edges is not bound by its atomics (a copy of the same bytes takes 4.5 us);
 // short_counts is a chain of dependent steps, of which one block at the end does the last.  Blocks of 1,024 nodes halve that
 // block's sums but make short_nodes slower (6 -> 8 us) for nothing in total.
 #pragma once
@@ -73,6 +73,8 @@ __device__ __forceinline__ ShortNode short_node(const ShortTables& t, int64_t n)
 constexpr int kShortEdges = 4;  // per thread
 template <typename Index>
 __global__ void __launch_bounds__(256) short_edges(const Index* __restrict__ src, const Index* __restrict__ dst, ShortTables t) {
+  let_next_start();
+  wait_for_previous();
   const int64_t begin = static_cast<int64_t>(blockIdx.x) * (256 * kShortEdges) + threadIdx.x;
   Index s[kShortEdges], d[kShortEdges], before[kShortEdges], after[kShortEdges];
 #pragma unroll
@@ -138,6 +140,8 @@ __device__ __forceinline__ ShortSum short_scan(ShortSum mine, ShortSum* all, int
 }
 
 __global__ void __launch_bounds__(kShortBlock) short_counts(ShortTables t) {
+  let_next_start();
+  wait_for_previous();
   __shared__ int histogram[kShortSets * kShortKeys];
   __shared__ int scan[kShortWarps][3];
   __shared__ int finished;
@@ -209,6 +213,8 @@ __global__ void __launch_bounds__(kShortBlock) short_counts(ShortTables t) {
 }
 
 __global__ void __launch_bounds__(kShortBlock) short_nodes(ShortTables t) {
+  let_next_start();
+  wait_for_previous();
   __shared__ uint16_t before[kShortWarps][kShortKeys];  // nodes of a key in a warp, then in the warps before
   __shared__ int scan[kShortWarps][3];
   if (t.head[0] != 0) return;
@@ -264,6 +270,8 @@ __global__ void __launch_bounds__(kShortBlock) short_nodes(ShortTables t) {
 }
 
 __global__ void __launch_bounds__(256) short_scatter(ShortTables t) {
+  let_next_start();
+  wait_for_previous();
   if (t.head[0] != 0) return;
   const int64_t begin = static_cast<int64_t>(blockIdx.x) * (256 * kShortEdges) + threadIdx.x;
   int at[kShortEdges];
@@ -313,6 +321,8 @@ __device__ __forceinline__ void short_sort(int32_t* row, int edges, int lane) {
 }
 
 __global__ void __launch_bounds__(256) short_rows(ShortTables t) {
+  let_next_start();
+  wait_for_previous();
   if (t.head[0] != 0) return;
   const int lane = threadIdx.x & 31;
   const int64_t n = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5;
@@ -373,15 +383,15 @@ template <typename Index>
 int short_tables(const void* src, const void* dst, const ShortTables& t, size_t zeroed, cudaStream_t stream) {
   const unsigned edge_blocks = static_cast<unsigned>(ceil_div(t.edges, 256 * kShortEdges)), node_blocks = static_cast<unsigned>(t.blocks);
   LUNA_CUDA_CHECK(cudaMemsetAsync(t.head, 0, zeroed, stream));
-  short_edges<Index><<<edge_blocks, 256, 0, stream>>>(static_cast<const Index*>(src), static_cast<const Index*>(dst), t);
+  launch_early(short_edges<Index>, edge_blocks, 256, 0, stream, static_cast<const Index*>(src), static_cast<const Index*>(dst), t);
   LUNA_LAUNCH_CHECK("graph edge copies");
-  short_counts<<<node_blocks, kShortBlock, 0, stream>>>(t);
+  launch_early(short_counts, node_blocks, kShortBlock, 0, stream, t);
   LUNA_LAUNCH_CHECK("graph node counts");
-  short_nodes<<<node_blocks, kShortBlock, 0, stream>>>(t);
+  launch_early(short_nodes, node_blocks, kShortBlock, 0, stream, t);
   LUNA_LAUNCH_CHECK("graph node tables");
-  short_scatter<<<edge_blocks, 256, 0, stream>>>(t);
+  launch_early(short_scatter, edge_blocks, 256, 0, stream, t);
   LUNA_LAUNCH_CHECK("graph edge ids");
-  short_rows<<<static_cast<unsigned>(ceil_div(t.src_nodes, 8)), 256, 0, stream>>>(t);
+  launch_early(short_rows, static_cast<unsigned>(ceil_div(t.src_nodes, 8)), 256, 0, stream, t);
   LUNA_LAUNCH_CHECK("graph rows");
   return LUNA_OK;
 }

@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(kBlock)
 sh_kernel(const ShParams P, const T* __restrict__ v, const T* __restrict__ g, const T* __restrict__ rx,
           T* __restrict__ out0, T* __restrict__ out1, int64_t n) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  let_next_start();
   T* smem = reinterpret_cast<T*>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int C = P.C, CP = C | 1;
@@ -574,6 +575,7 @@ sh_canon_forward(const ShParams P, const T* __restrict__ v, T* __restrict__ out,
   constexpr int C = (LMAX + 1) * (LMAX + 1);
   using Tile = RowTile<T, C>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T* tile = reinterpret_cast<T*>(smem_raw) + warp * 32 * Tile::pitch;
   T* row = tile + lane * Tile::pitch;
@@ -628,6 +630,7 @@ sh_canon_backward(const ShParams P, const T* __restrict__ v, const T* __restrict
   constexpr int C = (LMAX + 1) * (LMAX + 1);
   using Tile = RowTile<T, C>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T* tiles = reinterpret_cast<T*>(smem_raw) + warp * 2 * 32 * Tile::pitch;
   const int64_t step = static_cast<int64_t>(gridDim.x) * kBlock;
@@ -681,6 +684,7 @@ __global__ void __launch_bounds__(kBlock)
 sh_canon_double(const ShParams P, const T* __restrict__ v, const T* __restrict__ g, const T* __restrict__ rx,
                 T* __restrict__ out0, T* __restrict__ out1, int64_t n) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  let_next_start();
   T* smem = reinterpret_cast<T*>(smem_raw);
   constexpr int C = (LMAX + 1) * (LMAX + 1), CP = C | 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

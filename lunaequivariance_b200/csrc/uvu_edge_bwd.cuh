@@ -289,6 +289,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   using V = typename PK::V;
   constexpr int NP = PK::NP;
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int team_warps = FULL ? 1 : P.team_warps;
   const int team = FULL ? warp : warp / team_warps, member = warp - team * team_warps;
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   MatrixProgram<T, S> program;
   if constexpr (WM) program.load(P.prog_c, P.prog_j, lane, 0, 1);
   __syncthreads();
+  wait_for_previous();
 
   const int cpw = ch / team_warps;  // channels of this warp
   const int lanes = FULL ? 32 : cpw / CPL;

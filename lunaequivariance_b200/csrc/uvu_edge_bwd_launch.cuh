@@ -120,7 +120,7 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
   if (rc != LUNA_OK) return rc;
   const dim3 grid(static_cast<unsigned>(cut.blocks), static_cast<unsigned>(lanes.slices));
-  kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
+  launch_early(kernel, grid, launch.warps * 32, launch.bytes, stream, P);
   LUNA_LAUNCH_CHECK("backward (edge family)");
   if (SLICED && WY) {
     reduce_gy_partial<T><<<static_cast<unsigned>(ceil_div(P.gy_part, 256)), 256, 0, stream>>>(

@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   using V = typename PK::V;
   constexpr int NP = PK::NP;
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int team_warps = FULL ? 1 : P.team_warps;
   const int team = FULL ? warp : warp / team_warps, member = warp - team * team_warps;
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
   MatrixProgram<T, S> program;
   program.load(P.prog_c, P.prog_j, lane, member, team_warps);
   __syncthreads();
+  wait_for_previous();
 
   const int cpw = ch / team_warps;  // channels of this warp
   const int lanes = FULL ? 32 : cpw / CPL;

@@ -54,7 +54,7 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
   if (rc != LUNA_OK) return rc;
   const dim3 grid(static_cast<unsigned>(split.blocks), static_cast<unsigned>(lanes.slices));
-  kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
+  launch_early(kernel, grid, launch.warps * 32, launch.bytes, stream, P);
   LUNA_LAUNCH_CHECK("forward (edge family)");
   return LUNA_OK;
 }

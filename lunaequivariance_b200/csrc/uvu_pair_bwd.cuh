@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   constexpr int NP = PK::NP;
   static_assert(!ADD || (WM && !WX && !WY), "the weights' place in a stage must be free");
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, place = lane & 15;
   constexpr int ch = 16 * CPL, lanes = 16, W = S::paths * ch, X = S::XD * ch, O = S::OD * ch, half_elems = pair_half<PK>(W + O), stage_elems = 2 * half_elems;
   const int stages = P.stages, own = lane_first<PK>(place);
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
   HalfMatrixProgram<T, S> program;
   if constexpr (WM) program.load(P.prog_c, P.prog_j, place);
   __syncthreads();
+  wait_for_previous();
 
   const bool issuing = place == 0;  // a half's copies are its first lane's
   const bool want_x = WX && P.gx != nullptr, storing = WM && P.gw != nullptr;

@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
   using V = typename PK::V;
   constexpr int NP = PK::NP;
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, place = lane & 15;
   constexpr int ch = 16 * CPL, lanes = 16, W = S::paths * ch, X = S::XD * ch, O = S::OD * ch, half_elems = pair_half<PK>(W + X), stage_elems = 2 * half_elems;
   const int stages = P.stages, own = lane_first<PK>(place);
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
   HalfMatrixProgram<T, S> program;
   program.load(P.prog_c, P.prog_j, place);
   __syncthreads();
+  wait_for_previous();
 
   const bool issuing = place == 0;  // a half's copies are its first lane's
   const uint32_t w_bytes = static_cast<uint32_t>(W * sizeof(T)), x_bytes = static_cast<uint32_t>(X * sizeof(T));
