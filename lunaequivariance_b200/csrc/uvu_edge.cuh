@@ -627,9 +627,17 @@ struct HalfMatrixProgram {
 };
 
 // Warps per CTA by the registers a lane is going to need (an estimate from the state it keeps): the launch bound caps
-// the registers at 65,536 / threads.
-__host__ __device__ constexpr int warps_for(int regs) {
-  return regs <= 60 ? 24 : (regs <= 120 ? 16 : (regs <= 150 ? 12 : 8));
+// the registers at 65,536 / threads.  slack: by how much the estimate is too high.
+__host__ __device__ constexpr int warps_for(int regs, int slack = 0) {
+  return regs <= 60 ? 24 : (regs <= 120 + slack ? 16 : (regs <= 150 + slack ? 12 : 8));
+}
+// Of the backward kernels, whose estimate has room for coupling matrices in it: lists without any need less, dL/dy alone, which
+// keeps neither gradients nor matrices, least.  Twelve warps and sixteen, 0.4 M edges: dL/dy alone, 128 channels, (3, 3, 0) 248 ->
+// 215 us, FP64 (0, 3, 3), 64 channels 334 -> 281; dL/dx with dL/dw, (2, 2, 0), 128 channels, 0.8 M edges 640 -> 555; output with
+// dL/dw, (0, 2, 2), 608 -> 537.  Above these limits it loses: all gradients of (2, 2, 0), 128 channels 716 -> 800.
+template <typename S>
+constexpr int slack_for(bool with_sums) {
+  return S::m_total != 0 ? 0 : (with_sums ? 10 : 35);
 }
 
 // Attributes a kernel needs set once per device, not on every launch.

@@ -75,7 +75,7 @@ struct EdgeBwd {
       (S::XD * CPL * (WX ? 2 : 1) + (WY ? S::YD * pair : 0) + (2 * S::LO + 1) * CPL) * words;
   static constexpr int program_regs = WM ? S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 : 0;
   static constexpr int registers = state + program_regs + 48;  // an estimate; beyond 255 it spills hundreds of bytes
-  static constexpr int max_warps = warps_for(registers);
+  static constexpr int max_warps = warps_for(registers, slack_for<S>(WM));
   // slots of g: the highest degree has one, the others share one
   static constexpr int slot_of(int l3) { return l3 == S::LO && S::ooff(S::LO) > 0 ? 1 : 0; }
   static constexpr int slots = slot_of(S::LO) + 1;

@@ -18,7 +18,7 @@ struct PairBwd {
   static constexpr int warp_elems = 2 * m_elems + (WY ? red_pass * red_row : 0);
   static constexpr int program_regs = WM ? 4 * S::m_rounds * Edge::words + S::m_rounds + 1 : 0;
   static constexpr int registers = Edge::state + program_regs + 44;
-  static constexpr int max_warps = warps_for(registers);
+  static constexpr int max_warps = warps_for(registers, slack_for<S>(WM));
 };
 
 // 16 * CPL channels.  DST: rows by destination (S, x and g exchanged).  ADD: gw alone, added to; w names gw.
