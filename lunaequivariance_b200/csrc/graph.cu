@@ -67,7 +67,7 @@ __global__ void init_bounds(Bounds* result) {
 // pointers).  Sums are taken modulo 2^32: only differences within a set, which are smaller, are used.
 // What bounds it is the number of dependent launches, 3 to 17 us each: 16 of them, 135 us on the device for 1.05 M edges
 // and 20,000 nodes, 201 us for the whole call.  Graphs whose rows all have at most 255 edges are built by counting
-// (graph_short.cuh) in 93; this is the way for longer rows, for luna_graph_build, and for graphs of over a million nodes.
+// (graph_short.cuh) in 88; this is the way for longer rows, for luna_graph_build, and for graphs of over a million nodes.
 struct TableSizes {
   int64_t nodes, src_nodes, edges;
   bool segments;

@@ -14,10 +14,11 @@
 //                  writes the row's pieces
 // A longer row sets the flag to kLongRow and the caller takes the general way.
 //
-// 1.05 M edges, 20,000 nodes, the five launches: 10, 14, 6, 9 and 9 us; the whole call, with the allocations before it and the
-// synchronisation at its end, 201 -> 105 us, and 93 with launches that overlap (launch_early).  short_edges is not bound by its atomics (a copy of the same bytes takes 4.5 us);
-// short_counts is a chain of dependent steps, of which one block at the end does the last.  Blocks of 1,024 nodes halve that
-// block's sums but make short_nodes slower (6 -> 8 us) for nothing in total.
+// 1.05 M edges, 20,000 nodes, the five launches: 10, 10, 6, 9 and 9 us; the whole call, with the allocations before it and the
+// synchronisation at its end, 201 -> 105 us, 93 with launches that overlap (launch_early), and 88 since the last block of
+// short_counts sums two columns to a thread and scans two orders at a time (14 us before).  short_edges is not bound by its atomics
+// (a copy of the same bytes takes 4.5 us); short_counts is a chain of dependent steps, of which one block does the last.  Blocks of
+// 1,024 nodes halve that block's sums but make short_nodes slower (6 -> 8 us).
 #pragma once
 
 #include <algorithm>
@@ -169,46 +170,61 @@ __global__ void __launch_bounds__(kShortBlock) short_counts(ShortTables t) {
   if (finished != static_cast<int>(t.blocks) - 1) return;
   __threadfence();
 
-  // the last block: what the blocks before each block have
-  auto running = [&](int32_t* column, int64_t stride) {
-    int sum = 0;
-    for (int64_t b = 0; b < t.blocks; b += 16) {
-      int part[16];
+  // the last block: what the blocks before each block have, two columns to a thread and 24 blocks of both at a time
+  constexpr int kColumns = kShortSets * kShortKeys + 3, kAtOnce = 24;
+  static_assert(kColumns <= 2 * kShortBlock, "a thread has two columns");
+  int32_t* column[2];
+  int stride[2], total[2] = {0, 0};
 #pragma unroll
-      for (int k = 0; k < 16; ++k) part[k] = b + k < t.blocks ? __ldcg(column + (b + k) * stride) : 0;
+  for (int c = 0; c < 2; ++c) {
+    const int i = static_cast<int>(threadIdx.x) + c * kShortBlock;
+    const bool keys = i < kShortSets * kShortKeys;
+    column[c] = i >= kColumns ? nullptr : (keys ? t.histogram + i : t.sums + (i - kShortSets * kShortKeys));
+    stride[c] = keys ? kShortSets * kShortKeys : 3;
+  }
+  for (int64_t b = 0; b < t.blocks; b += kAtOnce) {
+    int part[2][kAtOnce];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        if (b + k < t.blocks) column[(b + k) * stride] = sum;
-        sum += part[k];
+    for (int k = 0; k < kAtOnce; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) part[c][k] = column[c] && b + k < t.blocks ? __ldcg(column[c] + (b + k) * stride[c]) : 0;
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (column[c] && b + k < t.blocks) column[c][(b + k) * stride[c]] = total[c];
+        total[c] += part[c][k];
       }
-    }
-    return sum;
-  };
-  for (int i = threadIdx.x; i < kShortSets * kShortKeys + 3; i += kShortBlock) {
-    const int c = i - kShortSets * kShortKeys;
-    const int total = c < 0 ? running(t.histogram + i, kShortSets * kShortKeys) : running(t.sums + c, 3);
-    if (c < 0) histogram[i] = total;
-    if (c == 2) t.head[1] = total;
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int i = static_cast<int>(threadIdx.x) + c * kShortBlock;
+    if (i < kShortSets * kShortKeys) histogram[i] = total[c];
+    if (i == kColumns - 1) t.head[1] = total[c];
   }
   __syncthreads();
-  // keys: nodes before, and for the orders by degree the edges and the full pieces before
-  for (int s = 0; s < kShortSets; ++s) {
-    const int key = threadIdx.x, nodes = key < kShortKeys ? histogram[s * kShortKeys + key] : 0, degree = kShortRow - key;
-    const bool used = key < kShortKeys;
-    ShortSum totals;
-    const ShortSum before =
-        short_scan(ShortSum{{nodes, used ? nodes * degree : 0, used ? nodes * (degree >> 5) : 0}}, &totals, scan);
-    if (used) t.key_begin[s * kShortKeys + key] = before.v[0];
-    if (s == 0 && used) {
-      for (int k = 1; k < 4; ++k) {  // tier k ends with the row that brings the edges to k quarters
-        const int quarter = static_cast<int>(static_cast<int64_t>(k) * t.edges / 4);
-        if (quarter > before.v[1] && quarter <= before.v[1] + nodes * degree)
-          t.tiers[k - 1] = before.v[0] + (quarter - before.v[1] + degree - 1) / degree;
-        if (quarter == 0 && key == 0) t.tiers[k - 1] = 1;
-      }
+  // keys: nodes before, and for the orders by degree the edges and the full pieces before.  The first half of the threads has the
+  // first set, with the third set's nodes, and the second half the second set, from which the first one's totals are taken off.
+  static_assert(kShortBlock == 2 * kShortKeys, "a half of the threads has a key each");
+  const int set = static_cast<int>(threadIdx.x) / kShortKeys, key = static_cast<int>(threadIdx.x) % kShortKeys;
+  const int nodes = histogram[set * kShortKeys + key], degree = kShortRow - key;
+  const int weight = nodes * (set == 0 ? degree : degree >> 5);
+  ShortSum before = short_scan(ShortSum{{nodes, weight, set == 0 ? histogram[2 * kShortKeys + key] : 0}}, &all, scan);
+  if (set == 0) {
+    t.key_begin[key] = before.v[0];
+    t.key_begin[2 * kShortKeys + key] = before.v[2];
+    for (int k = 1; k < 4; ++k) {  // tier k ends with the row that brings the edges to k quarters
+      const int quarter = static_cast<int>(static_cast<int64_t>(k) * t.edges / 4);
+      if (quarter > before.v[1] && quarter <= before.v[1] + weight)
+        t.tiers[k - 1] = before.v[0] + (quarter - before.v[1] + degree - 1) / degree;
+      if (quarter == 0 && key == 0) t.tiers[k - 1] = 1;
     }
-    if (s == 1 && used) t.full_begin[key] = before.v[2];
-    if (s == 1 && key == kShortKeys) t.full_begin[kShortKeys] = totals.v[2];
+  } else {
+    before.v[0] -= static_cast<int>(t.nodes);
+    before.v[1] -= static_cast<int>(t.edges);  // of at most a hundred million (short_rows_likely)
+    t.key_begin[kShortKeys + key] = before.v[0];
+    t.full_begin[key] = before.v[1];
+    if (key == kShortKeys - 1) t.full_begin[kShortKeys] = before.v[1] + weight;
   }
 }
 
