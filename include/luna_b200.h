@@ -86,7 +86,7 @@ LUNA_API void luna_uvu_plan_destroy(luna_uvu_plan* plan);
  * counts that these are compiled for, or the staged kernels that read the path list from tables. */
 typedef enum {
   LUNA_PLAN_FAST_PATH = 0,      /* 1 if staged (bulk-copy) kernels apply to this configuration */
-  LUNA_PLAN_CHANNELS_PER_LANE = 1, /* of the forward kernel; 0 without staged kernels */
+  LUNA_PLAN_CHANNELS_PER_LANE = 1, /* of the forward kernel of small graphs (larger ones may have another layout); 0 without staged kernels */
   LUNA_PLAN_CHANNEL_CHUNKS = 2, /* parts of a block's channels that are launched side by side; 0 without staged kernels */
   LUNA_PLAN_FWD_SMEM_BYTES = 3, /* shared memory of a block, at most */
   LUNA_PLAN_BWD_SMEM_BYTES = 4, /* the same for all gradients */

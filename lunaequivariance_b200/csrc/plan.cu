@@ -397,6 +397,8 @@ int get_device_tables(luna_uvu_plan* plan, const DeviceTables** out) {
   dt.bytes = host.size();
   LUNA_CUDA_CHECK(cudaMalloc(&dt.buffer, dt.bytes));
   cudaError_t err = cudaMemcpy(dt.buffer, host.data(), dt.bytes, cudaMemcpyHostToDevice);
+  // a small copy from pageable memory may return before it has arrived, and kernels read the tables as soon as they start
+  if (err == cudaSuccess) err = cudaStreamSynchronize(cudaStreamLegacy);
   if (err != cudaSuccess) {
     cudaFree(dt.buffer);
     return fail(LUNA_ERR_CUDA, "table upload failed: %s", cudaGetErrorString(err));

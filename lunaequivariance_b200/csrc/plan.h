@@ -164,7 +164,8 @@ struct EdgeLanes {
 struct EdgePlan {
   int shape = -1;      // index of the compiled shape, -1 if the plan has none or is kept from its kernels
   int ch = 0;          // channels per block
-  EdgeLanes lanes;      // of the forward
+  EdgeLanes lanes;      // of the forward of few rows, which several teams share
+  EdgeLanes lanes_rows;  // of the forward otherwise
   EdgeLanes lanes_one;  // of backward calls that want dL/dy or dL/dw alone
   EdgeLanes lanes_sums;  // of those that want dL/dx, alone or with dL/dw
   EdgeLanes lanes_output;  // of output and dL/dw in one launch

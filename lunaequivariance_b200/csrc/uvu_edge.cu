@@ -78,7 +78,10 @@ int matrix_entries(int shape, std::integer_sequence<int, ID...>) {
 // ch / 16 channels on each of a half warp's 16 lanes, two edges at a time, where that is compiled (edge_paired).  48 channels, one edge
 // on 24 lanes and two edges with three channels per lane, 0.8 M edges: (1, 1, 1) 192 / 576 / 340 / 393 -> 165 / 352 / 194 / 252; (0, 3, 3)
 // 260 / 642 / 359 / 432 -> 187 / 463 / 252 / 287; (2, 2, 2), 0.52 M edges, 274 / 715 / 378 / 427 -> 260 / 683 / 301 / 301.
-EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool sliced) {
+// Not three channels per lane for the forward of few rows (`few`): of its thirteen teams no four or eight can share a row.  (2, 2, 2),
+// 48 channels, 24 nodes 6.7 us with one edge on 24 lanes and 24 with two edges, 300 nodes 18 and 38; 30,000 nodes 757 and 634.  Nor in
+// FP64 with coupling matrices, where seven teams fit: (2, 2, 2), 96 channels, 24 nodes 13 and 33, 440 nodes 42 and 69.
+EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool sliced, bool few = false) {
   const int ch = plan->edge.ch, elem = plan->dtype == LUNA_F64 ? 8 : 4;
   // one team with two stages must fit an SM's shared memory in either direction
   const size_t room = 200 * 1024, W = static_cast<size_t>(plan->W) * elem, X = static_cast<size_t>(plan->X) * elem,
@@ -93,6 +96,7 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool s
                : parts > capped_warps(plan->tuning, 8) || ch % (parts * cpl) != 0 || rows + parts * 8192 > room)
       continue;
     const int registers = registers_of(plan, shape, use, cpl);
+    if (cpl == 3 && few && elem == 8 && matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 0) continue;
     if (cpl == 3 && (sliced || parts > 2 || registers > (use == EdgeUse::kForward ? 255 : 280) ||
                      (parts == 2 && elem == 4 && matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 64)))
       continue;
@@ -105,7 +109,7 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool s
     best = sliced ? EdgeLanes{cpl, 1, parts} : EdgeLanes{cpl, parts, 1};
   }
   const int half = ch / 16;
-  if (!sliced && ch % 16 == 0 && (plan->tuning.lane_channels == 0 || plan->tuning.lane_channels == half) &&
+  if (!sliced && !(few && half == 3) && ch % 16 == 0 && (plan->tuning.lane_channels == 0 || plan->tuning.lane_channels == half) &&
       paired(plan, shape, use, half))
     return EdgeLanes{half, 1, 1, 2};
   return best;
@@ -243,12 +247,14 @@ void analyse(luna_uvu_plan* plan) {
   if (shape < 0) return;
   const bool sliced = choose_lanes(plan, shape, EdgeUse::kForward, false).cpl == 0;
   if (sliced && !edge_sliced(shape)) return;
-  plan->edge.lanes = choose_lanes(plan, shape, EdgeUse::kForward, sliced);
+  plan->edge.lanes = choose_lanes(plan, shape, EdgeUse::kForward, sliced, true);
+  plan->edge.lanes_rows = choose_lanes(plan, shape, EdgeUse::kForward, sliced);
+  if (plan->edge.lanes.cpl == 0) plan->edge.lanes = plan->edge.lanes_rows;  // counts that only three channels per lane divide
   plan->edge.lanes_one = choose_lanes(plan, shape, EdgeUse::kOneGradient, sliced);
   plan->edge.lanes_sums = choose_lanes(plan, shape, EdgeUse::kSums, sliced);
   plan->edge.lanes_output = choose_lanes(plan, shape, EdgeUse::kOutputAndWeights, sliced);
   plan->edge.lanes_all = choose_lanes(plan, shape, EdgeUse::kAllGradients, sliced);
-  for (const EdgeLanes* lanes : {&plan->edge.lanes, &plan->edge.lanes_one, &plan->edge.lanes_sums, &plan->edge.lanes_output, &plan->edge.lanes_all})
+  for (const EdgeLanes* lanes : {&plan->edge.lanes, &plan->edge.lanes_rows, &plan->edge.lanes_one, &plan->edge.lanes_sums, &plan->edge.lanes_output, &plan->edge.lanes_all})
     if (lanes->cpl == 0) return;
   plan->edge.shape = shape;
 }
@@ -256,7 +262,7 @@ void analyse(luna_uvu_plan* plan) {
 int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
             const void* w, void* out, bool accumulate, cudaStream_t stream) {
   const EdgeForwardArgs args{x, y, w, out, accumulate};
-  const EdgeLanes& lanes = plan->edge.lanes;
+  const EdgeLanes& lanes = few_rows(graph->num_nodes, dt.sm_count) ? plan->edge.lanes : plan->edge.lanes_rows;
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.forward(plan, dt, graph, lanes, args, stream); });
 }
 

@@ -217,12 +217,13 @@ constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
 // 2,083 nodes of 41 edges 80 / 160 -> 78 / 148 us, 4,000 of 30 98 / 201 -> 90 / 180; 48 channels, 10,001 of 52 290 / 777 -> 258 /
 // 711; 32 channels, 4,003 of 52 100 / 202 -> 88 / 176.  With 442 edges a team (64 channels, 20,000 nodes) the two are even, and
 // with 64 MB of gathered rows ((3, 3, 3), 128 channels, 8,000 nodes) parts lose: forward 0.98 -> 1.27 ms.
+inline bool few_rows(int64_t rows, int ctas) { return rows <= 3 * static_cast<int64_t>(ctas); }
 inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps, int64_t wanted_tile,
                             int at_once, int64_t gathered, bool may_group) {
   EdgeSplit s;
   const int64_t all = static_cast<int64_t>(sm_count) * teams;
   const double degree = static_cast<double>(edges) / static_cast<double>(std::max<int64_t>(rows, 1));
-  const bool few = may_group && rows <= 3 * static_cast<int64_t>(sm_count);
+  const bool few = may_group && few_rows(rows, sm_count);
   if (few && degree >= 4.0) {
     int want = 8;  // and at least two steps of a team in a part
     while (want > 1 && (want > teams || teams % want != 0 || degree < 2.0 * at_once * want)) want /= 2;

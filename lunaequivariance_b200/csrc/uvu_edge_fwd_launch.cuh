@@ -33,13 +33,19 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.row_ch = plan->edge.ch;
   P.team_warps = lanes.team_warps;
   P.accumulate = a.accumulate ? 1 : 0;
-  const EdgeLaunch launch = PAIR ? pair_fwd_launch<T, CPL, S>(plan->tuning, P.ch, dt.max_smem_optin)
+  EdgeLaunch launch = PAIR ? pair_fwd_launch<T, CPL, S>(plan->tuning, P.ch, dt.max_smem_optin)
                                  : edge_fwd_launch<T, CPL, S>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
   if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
   P.ring_elems = launch.team_elems;
   P.teams = launch.warps / lanes.team_warps;
   const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
+  // Teams that share rows come in twos, fours or eights: of seven or thirteen none could share one.  FP64 (2, 2, 2), 64 channels, ten teams
+  // in twos and eight in eights: 24 nodes 12.7 and 7.5 us, 440 nodes 31 and 34, so with the usual layouts only up to a row per CTA.
+  if (few_rows(graph->num_nodes, ctas) && P.teams > 4) {
+    P.teams -= P.teams > 8 && (CPL == 3 || graph->num_nodes <= ctas) ? P.teams % 4 : P.teams % 2;
+    launch.warps = P.teams * lanes.team_warps;
+  }
   const int64_t sources = graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;
   const EdgeSplit split =
       edge_split(graph->num_nodes, graph->num_edges, ctas, P.teams, lanes.team_warps, 64, lanes.edges,
