@@ -128,6 +128,14 @@ def test_three_channels_per_lane(shape, mul, dtype):
     one_gradient_alone(SHAPES[shape], mul, dtype, 460, 2100, 0.0, shape + 90)  # equal parts
 
 
+# three, seven, ten and thirteen teams fit: of a row per CTA, and of two
+@pytest.mark.parametrize("shape,mul,dtype", [(5, 128, torch.float32), (4, 96, torch.float64), (4, 64, torch.float64),
+                                             (6, 128, torch.float64), (2, 48, torch.float32), (6, 96, torch.float32)])
+def test_teams_of_few_rows(shape, mul, dtype):
+    check(SHAPES[shape], mul, dtype, 24, 552, 0.0, mul)
+    check(SHAPES[shape], mul, dtype, 230, 4100, 0.0, mul + 1)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("shape", range(len(SHAPES)))
 def test_one_gradient_alone(shape, dtype):

@@ -23,7 +23,15 @@ def _edges(nodes, source_rows, edges, hub, seed):
     return src, torch.sort(torch.randint(nodes, (edges,), generator=generator)).values
 
 
-def _compare(src, dst, nodes, source_rows):
+# one edge; fewer edges than quarters; rows of exactly 31, 32, 33 rows per warp; rows without edges; more source rows than
+# destinations and fewer
+@pytest.mark.parametrize("nodes,source_rows,edges,hub", [
+    (1, 1, 1, False), (3, 3, 2, False), (30, 30, 3, False), (31, 31, 992, False), (32, 32, 1024, True),
+    (62, 62, 4_000, True), (500, 500, 300, False), (64, 900, 5_001, False), (900, 7, 5_001, True), (20_011, 20_011, 200_003, True),
+])
+@pytest.mark.parametrize("index_dtype", [torch.int32, torch.int64])
+def test_tables(nodes, source_rows, edges, hub, index_dtype):
+    src, dst = (t.to(index_dtype) for t in _edges(nodes, source_rows, edges, hub, nodes + edges))
     other = None if source_rows == nodes else source_rows
     want = luna.make_graph(src, dst, nodes, num_src_nodes=other)
     got = luna.make_graph(src.cuda(), dst.cuda(), nodes, num_src_nodes=other)
@@ -35,16 +43,16 @@ def _compare(src, dst, nodes, source_rows):
     assert got.num_src_nodes == want.num_src_nodes and got.can_split == want.can_split
 
 
-# one edge; fewer edges than quarters; rows of exactly 31, 32, 33 rows per warp; rows without edges; more source rows than
-# destinations and fewer
-@pytest.mark.parametrize("nodes,source_rows,edges,hub", [
-    (1, 1, 1, False), (3, 3, 2, False), (30, 30, 3, False), (31, 31, 992, False), (32, 32, 1024, True),
-    (62, 62, 4_000, True), (500, 500, 300, False), (64, 900, 5_001, False), (900, 7, 5_001, True), (20_011, 20_011, 200_003, True),
-])
-@pytest.mark.parametrize("index_dtype", [torch.int32, torch.int64])
-def test_tables(nodes, source_rows, edges, hub, index_dtype):
-    src, dst = (t.to(index_dtype) for t in _edges(nodes, source_rows, edges, hub, nodes + edges))
-    _compare(src, dst, nodes, source_rows)
+def _compare(src, dst, nodes, source_rows):
+    other = None if source_rows == nodes else source_rows
+    want = luna.make_graph(src, dst, nodes, num_src_nodes=other)
+    got = luna.make_graph(src.cuda(), dst.cuda(), nodes, num_src_nodes=other)
+    for name in NAMES:
+        torch.testing.assert_close(getattr(got, name).cpu(), getattr(want, name), rtol=0, atol=0, msg=name)
+    for name in SEGMENTS:
+        torch.testing.assert_close(getattr(got.source_segments, name).cpu(), getattr(want.source_segments, name), rtol=0,
+                                   atol=0, msg=f"segment {name}")
+    assert got.num_src_nodes == want.num_src_nodes and got.can_split == want.can_split
 
 
 # Rows of up to 255 edges are counted into place, a longer one anywhere sends the graph to the general sorts: both sides of the
