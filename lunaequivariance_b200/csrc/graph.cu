@@ -256,26 +256,29 @@ ScratchLayout layout(TableSizes z) {
 
 unsigned grid(int64_t threads) { return static_cast<unsigned>(std::max<int64_t>(1, ceil_div(threads, kThreads))); }
 
-// Launches everything; *bad (in the scratch) tells whether the edge list was fit for it.
+// Launches everything; *bad (in the scratch) tells whether the edge list was fit for it.  `copied`: the narrow copies and the
+// identity are there already, and checked, and *bad is zero.
 template <typename Key>
 int build_tables(const void* src, const void* dst, int index_bits, const TableSizes& z, const luna_graph_out& out,
-                 const luna_graph_pieces* pieces, unsigned char* scratch, const ScratchLayout& l, cudaStream_t stream) {
+                 const luna_graph_pieces* pieces, unsigned char* scratch, const ScratchLayout& l, bool copied, cudaStream_t stream) {
   auto at = [&](size_t offset) { return reinterpret_cast<int32_t*>(scratch + offset); };
   int* bad = at(l.bad);
   Key *keys = reinterpret_cast<Key*>(scratch + l.keys), *keys_sorted = reinterpret_cast<Key*>(scratch + l.keys_sorted);
   uint32_t* scan = reinterpret_cast<uint32_t*>(scratch + l.scan);
   void* temp = scratch + l.cub_temp;
   size_t temp_bytes = l.cub_bytes;
-  LUNA_CUDA_CHECK(cudaMemsetAsync(bad, 0, sizeof(int), stream));
+  if (!copied) LUNA_CUDA_CHECK(cudaMemsetAsync(bad, 0, sizeof(int), stream));
   if (z.edges > 0) {
     int32_t* iota = pieces ? pieces->edge_ids_by_dst : at(l.iota);
-    if (index_bits == 64)
-      copy_edges<int64_t><<<grid(z.edges), kThreads, 0, stream>>>(static_cast<const int64_t*>(src),
-                                                                  static_cast<const int64_t*>(dst), z, out.src, out.dst, iota, bad);
-    else
-      copy_edges<int32_t><<<grid(z.edges), kThreads, 0, stream>>>(static_cast<const int32_t*>(src),
-                                                                  static_cast<const int32_t*>(dst), z, out.src, out.dst, iota, bad);
-    LUNA_LAUNCH_CHECK("graph edge copies");
+    if (!copied) {
+      if (index_bits == 64)
+        copy_edges<int64_t><<<grid(z.edges), kThreads, 0, stream>>>(static_cast<const int64_t*>(src),
+                                                                    static_cast<const int64_t*>(dst), z, out.src, out.dst, iota, bad);
+      else
+        copy_edges<int32_t><<<grid(z.edges), kThreads, 0, stream>>>(static_cast<const int32_t*>(src),
+                                                                    static_cast<const int32_t*>(dst), z, out.src, out.dst, iota, bad);
+      LUNA_LAUNCH_CHECK("graph edge copies");
+    }
     // stable grouping of edge ids by source
     LUNA_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, static_cast<const int32_t*>(out.src), at(l.src_sorted),
                                                     static_cast<const int32_t*>(iota), out.edge_ids_by_src, z.edges, 0,
@@ -382,8 +385,8 @@ extern "C" int luna_graph_build(const void* src, const void* dst, int index_bits
   if (rc != LUNA_OK) return rc;
   auto stream = static_cast<cudaStream_t>(stream_);
   auto* base = static_cast<unsigned char*>(scratch);
-  return wide_keys(z) ? build_tables<uint64_t>(src, dst, index_bits, z, *out, nullptr, base, l, stream)
-                      : build_tables<uint32_t>(src, dst, index_bits, z, *out, nullptr, base, l, stream);
+  return wide_keys(z) ? build_tables<uint64_t>(src, dst, index_bits, z, *out, nullptr, base, l, false, stream)
+                      : build_tables<uint32_t>(src, dst, index_bits, z, *out, nullptr, base, l, false, stream);
 }
 
 extern "C" int luna_graph_build_all(const void* src, const void* dst, int index_bits, int64_t num_nodes,
@@ -405,7 +408,8 @@ extern "C" int luna_graph_build_all(const void* src, const void* dst, int index_
     return fail(LUNA_ERR_INVALID_ARGUMENT, "segment tables missing");
   auto stream = static_cast<cudaStream_t>(stream_);
   auto* base = static_cast<unsigned char*>(scratch);
-  if (short_rows_likely(num_nodes, num_src_nodes, num_edges)) {
+  const bool copied = short_rows_likely(num_nodes, num_src_nodes, num_edges);
+  if (copied) {
     ShortTables t{};
     t.nodes = num_nodes;
     t.src_nodes = num_src_nodes;
@@ -429,19 +433,21 @@ extern "C" int luna_graph_build_all(const void* src, const void* dst, int index_
     const int launched = index_bits == 64 ? short_tables<int64_t>(src, dst, t, zeroed, stream)
                                           : short_tables<int32_t>(src, dst, t, zeroed, stream);
     if (launched != LUNA_OK) return launched;
-    int head[2] = {0, 0};  // flag and number of pieces
+    int head[kHeadWords] = {};
     LUNA_CUDA_CHECK(cudaMemcpyAsync(head, t.head, sizeof(head), cudaMemcpyDeviceToHost, stream));
     LUNA_CUDA_CHECK(cudaStreamSynchronize(stream));
-    *bad = head[0] == kUnfit;
-    *num_segments = head[0] == 0 ? head[1] : 0;
-    if (head[0] != kLongRow) return LUNA_OK;
+    *bad = head[kHeadUnfit];
+    *num_segments = *bad ? 0 : head[kHeadPieces];
+    if (*bad || !head[kHeadLongRow]) return LUNA_OK;
+    // the flag of unfit edges, which is zero, lies where that of the general kernels does, and the rest of the scratch is theirs
+    static_assert(kHeadUnfit == 0, "the general kernels' flag is the scratch's first word");
   }
-  const int built = wide_keys(z) ? build_tables<uint64_t>(src, dst, index_bits, z, *out, pieces, base, l, stream)
-                                 : build_tables<uint32_t>(src, dst, index_bits, z, *out, pieces, base, l, stream);
+  const int built = wide_keys(z) ? build_tables<uint64_t>(src, dst, index_bits, z, *out, pieces, base, l, copied, stream)
+                                 : build_tables<uint32_t>(src, dst, index_bits, z, *out, pieces, base, l, copied, stream);
   if (built != LUNA_OK) return built;
   int flag = 0;
   int32_t count = 0;
-  LUNA_CUDA_CHECK(cudaMemcpyAsync(&flag, base + l.bad, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  if (!copied) LUNA_CUDA_CHECK(cudaMemcpyAsync(&flag, base + l.bad, sizeof(int), cudaMemcpyDeviceToHost, stream));
   LUNA_CUDA_CHECK(cudaMemcpyAsync(&count, pieces->segment_rowptr + num_src_nodes, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
   LUNA_CUDA_CHECK(cudaStreamSynchronize(stream));
   *bad = flag;

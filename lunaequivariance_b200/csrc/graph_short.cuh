@@ -12,7 +12,8 @@
 //   short_scatter  edge ids to their sources' rows
 //   short_rows     a warp sorts a row's edge ids in registers (ascending, so the order in which they came does not matter) and
 //                  writes the row's pieces
-// A longer row sets the flag to kLongRow and the caller takes the general way.
+// A longer row sets a flag, at which the launches that follow do nothing, and the caller goes on with the sorts from the edges that
+// short_edges has copied and checked.
 //
 // 1.05 M edges, 20,000 nodes, the five launches: 10, 10, 6, 9 and 9 us; the whole call, with the allocations before it and the
 // synchronisation at its end, 201 -> 105 us, 93 with launches that overlap (launch_early), and 88 since the last block of
@@ -34,11 +35,12 @@ constexpr int kShortKeys = 256;
 constexpr int kShortSets = 3;  // orders: destinations, sources, source rows by their last piece
 constexpr int kShortBlock = 512;
 constexpr int kShortWarps = kShortBlock / 32;
-constexpr int kUnfit = 1, kLongRow = 2;  // bits of ShortTables::head[0]
+// ShortTables::head.  The flags are words of their own because one launch may set both.
+constexpr int kHeadUnfit = 0, kHeadPieces = 1, kHeadFinished = 2, kHeadLongRow = 3, kHeadWords = 4;
 
 struct ShortTables {
   int64_t nodes, src_nodes, edges, blocks;
-  int* head;  // flag, number of pieces, blocks that have finished; zero, like the next three, at the start
+  int* head;  // an index unfit, number of pieces, blocks that have finished, a long row; zero, like the next three, at the start
   int32_t *first, *last;  // [nodes] edges of a destination
   int32_t* count;         // [src_nodes] edges of a source
   uint16_t* place;        // [edges] within the source's row
@@ -50,6 +52,9 @@ struct ShortTables {
   int32_t *src, *dst, *iota, *dst_rowptr, *src_rowptr, *edge_ids, *node_order, *source_node_order, *tiers;
   int32_t *segment_nodes, *segment_begin, *segment_end, *segment_rowptr, *segment_order;
 };
+
+// Whether the edges are for others: unfit, or for the general kernels.
+__device__ __forceinline__ bool short_given_up(const ShortTables& t) { return (t.head[kHeadUnfit] | t.head[kHeadLongRow]) != 0; }
 
 struct ShortNode {
   int in, out, pieces;
@@ -86,26 +91,43 @@ __global__ void __launch_bounds__(256) short_edges(const Index* __restrict__ src
     before[k] = e > 0 && e < t.edges ? dst[e - 1] : -1;
     after[k] = e + 1 < t.edges ? dst[e + 1] : -1;
   }
-  int place[kShortEdges];
+  bool fit[kShortEdges];
 #pragma unroll
   for (int k = 0; k < kShortEdges; ++k) {
     const int64_t e = begin + 256 * k;
-    place[k] = -1;
-    if (e >= t.edges) continue;
-    if (s[k] < 0 || s[k] >= t.src_nodes || d[k] < 0 || d[k] >= t.nodes || (e > 0 && before[k] > d[k])) {
-      t.head[0] = kUnfit;  // the other bit is set by a later launch
-      continue;
-    }
-    place[k] = atomicAdd(t.count + s[k], 1);
+    const bool bad = s[k] < 0 || s[k] >= t.src_nodes || d[k] < 0 || d[k] >= t.nodes || (e > 0 && before[k] > d[k]);
+    if (e < t.edges && bad) t.head[kHeadUnfit] = 1;
+    fit[k] = e < t.edges && !bad;
+  }
+  // In a large graph a thread's first edge is counted, the copies are made meanwhile, and the others are counted if no row has turned
+  // out to be long: the atomics of a row with a good part of all edges wait for one another, 1.4 ns each.  1.05 M edges, 87,000 of them
+  // in one row, the whole call with the sorts that follow 354 -> 247 us; 64,000 edges are too few to be worth the second trip.
+  const bool wary = gridDim.x > 64;
+  int place[kShortEdges];
+#pragma unroll
+  for (int k = 0; k < kShortEdges; ++k) place[k] = fit[k] && (k == 0 || !wary) ? atomicAdd(t.count + s[k], 1) : -1;
+#pragma unroll
+  for (int k = 0; k < kShortEdges; ++k) {
+    const int64_t e = begin + 256 * k;
+    if (!fit[k]) continue;
     t.src[e] = static_cast<int32_t>(s[k]);
     t.dst[e] = static_cast<int32_t>(d[k]);
     t.iota[e] = static_cast<int32_t>(e);
     if (before[k] != d[k]) t.first[d[k]] = static_cast<int32_t>(e);
     if (after[k] != d[k]) t.last[d[k]] = static_cast<int32_t>(e + 1);
   }
+  if (wary) {
+    if (place[0] == kShortRow) t.head[kHeadLongRow] = 1;
+    if (__syncthreads_or(place[0] >= kShortRow || (threadIdx.x == 0 && __ldcg(t.head + kHeadLongRow) != 0))) return;
 #pragma unroll
-  for (int k = 0; k < kShortEdges; ++k)
+    for (int k = 1; k < kShortEdges; ++k)
+      if (fit[k]) place[k] = atomicAdd(t.count + s[k], 1);
+  }
+#pragma unroll
+  for (int k = 0; k < kShortEdges; ++k) {
     if (place[k] >= 0) t.place[begin + 256 * k] = static_cast<uint16_t>(place[k]);
+    if (place[k] == kShortRow) t.head[kHeadLongRow] = 1;  // short_counts would find it too, later
+  }
 }
 
 // Sums over the block's threads before this one, of three numbers; all: over all threads.
@@ -146,13 +168,13 @@ __global__ void __launch_bounds__(kShortBlock) short_counts(ShortTables t) {
   __shared__ int histogram[kShortSets * kShortKeys];
   __shared__ int scan[kShortWarps][3];
   __shared__ int finished;
-  if (__syncthreads_or(t.head[0] != 0)) return;  // unfit, or another block has found a long row
+  if (__syncthreads_or(short_given_up(t))) return;
   for (int i = threadIdx.x; i < kShortSets * kShortKeys; i += kShortBlock) histogram[i] = 0;
   __syncthreads();
   const ShortNode node = short_node(t, static_cast<int64_t>(blockIdx.x) * kShortBlock + threadIdx.x);
   const bool lost = __syncthreads_or(node.in > kShortRow || node.out > kShortRow) != 0;
   if (lost) {
-    if (threadIdx.x == 0) t.head[0] = kLongRow;
+    if (threadIdx.x == 0) t.head[kHeadLongRow] = 1;
     return;  // the other blocks' last one never comes
   }
 #pragma unroll
@@ -165,7 +187,7 @@ __global__ void __launch_bounds__(kShortBlock) short_counts(ShortTables t) {
   if (threadIdx.x < 3) t.sums[blockIdx.x * 3 + threadIdx.x] = all.v[threadIdx.x];
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) finished = atomicAdd(&t.head[2], 1);
+  if (threadIdx.x == 0) finished = atomicAdd(&t.head[kHeadFinished], 1);
   __syncthreads();
   if (finished != static_cast<int>(t.blocks) - 1) return;
   __threadfence();
@@ -200,7 +222,7 @@ __global__ void __launch_bounds__(kShortBlock) short_counts(ShortTables t) {
   for (int c = 0; c < 2; ++c) {
     const int i = static_cast<int>(threadIdx.x) + c * kShortBlock;
     if (i < kShortSets * kShortKeys) histogram[i] = total[c];
-    if (i == kColumns - 1) t.head[1] = total[c];
+    if (i == kColumns - 1) t.head[kHeadPieces] = total[c];
   }
   __syncthreads();
   // keys: nodes before, and for the orders by degree the edges and the full pieces before.  The first half of the threads has the
@@ -233,7 +255,7 @@ __global__ void __launch_bounds__(kShortBlock) short_nodes(ShortTables t) {
   wait_for_previous();
   __shared__ uint16_t before[kShortWarps][kShortKeys];  // nodes of a key in a warp, then in the warps before
   __shared__ int scan[kShortWarps][3];
-  if (t.head[0] != 0) return;
+  if (short_given_up(t)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t n = static_cast<int64_t>(blockIdx.x) * kShortBlock + threadIdx.x;
   const ShortNode node = short_node(t, n);
@@ -279,7 +301,7 @@ __global__ void __launch_bounds__(kShortBlock) short_nodes(ShortTables t) {
         t.full_at[n] = t.full_begin[key] + in_key * (node.out >> 5);
       }
       // the pieces that are shorter than 32 edges follow the full ones, those of rows without edges end the list
-      if (s == 2) t.part_at[n] = node.out == 0 ? t.head[1] - static_cast<int>(t.src_nodes - at) : t.full_begin[kShortKeys] + at;
+      if (s == 2) t.part_at[n] = node.out == 0 ? t.head[kHeadPieces] - static_cast<int>(t.src_nodes - at) : t.full_begin[kShortKeys] + at;
     }
     __syncthreads();
   }
@@ -288,7 +310,7 @@ __global__ void __launch_bounds__(kShortBlock) short_nodes(ShortTables t) {
 __global__ void __launch_bounds__(256) short_scatter(ShortTables t) {
   let_next_start();
   wait_for_previous();
-  if (t.head[0] != 0) return;
+  if (short_given_up(t)) return;
   const int64_t begin = static_cast<int64_t>(blockIdx.x) * (256 * kShortEdges) + threadIdx.x;
   int at[kShortEdges];
 #pragma unroll
@@ -339,7 +361,7 @@ __device__ __forceinline__ void short_sort(int32_t* row, int edges, int lane) {
 __global__ void __launch_bounds__(256) short_rows(ShortTables t) {
   let_next_start();
   wait_for_previous();
-  if (t.head[0] != 0) return;
+  if (short_given_up(t)) return;
   const int lane = threadIdx.x & 31;
   const int64_t n = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5;
   if (n >= t.src_nodes) return;
@@ -362,9 +384,10 @@ __global__ void __launch_bounds__(256) short_rows(ShortTables t) {
     short_sort<8>(t.edge_ids + row, edges, lane);
 }
 
-// A row of more than 255 edges costs the launches above and then the general ones, about half as much again.  Such rows are rare
-// where the average is a third of that, so up to there it is tried.  The limit of the nodes is that of the one block that sums
-// all blocks' histograms: 2,048 of them take it some 0.2 ms, as much as the general way has launches for.
+// A row of more than 255 edges costs the launches above, of which all but the first do nothing, and a synchronisation before the sorts
+// begin: one row of 300 edges, 20,000 nodes of 52 on average 199 -> 222 us, 200,000 of 8 258 -> 305; without that row 103 and 179.
+// Such rows are rare where the average is a third of that, so up to there it is tried.  The limit of the nodes is that of the one
+// block that sums all blocks' histograms: 2,048 of them take it some 0.2 ms, as much as the general way has launches for.
 constexpr int64_t kShortMostBlocks = 2048;
 inline bool short_rows_likely(int64_t nodes, int64_t src_nodes, int64_t edges) {
   return edges <= 96 * std::min(nodes, src_nodes) && std::max(nodes, src_nodes) <= kShortMostBlocks * kShortBlock;
@@ -379,7 +402,7 @@ inline size_t short_layout(ShortTables* t, unsigned char* scratch, size_t* zeroe
     cursor += (static_cast<size_t>(entries) * sizeof(Entry) + 15) / 16 * 16;
   };
   t->blocks = ceil_div(std::max(t->nodes, t->src_nodes), kShortBlock);
-  take(&t->head, 4);
+  take(&t->head, kHeadWords);
   take(&t->first, t->nodes);
   take(&t->last, t->nodes);
   take(&t->count, t->src_nodes);

@@ -71,6 +71,32 @@ def test_longest_row(longest, nodes, source_rows):
         _compare(ends[0][order], ends[1][order], nodes, source_rows)
 
 
+# More blocks of 512 nodes than the last one to count sums at a time: 24 blocks, one node more, and several turns.
+@pytest.mark.parametrize("nodes,source_rows,edges", [(12_288, 12_288, 90_001), (12_289, 12_289, 90_001), (20_011, 20_011, 200_003),
+                                                     (1_500, 30_011, 100_000), (100_003, 100_003, 300_001)])
+def test_many_blocks_of_nodes(nodes, source_rows, edges):
+    src, dst = _edges(nodes, source_rows, edges, False, nodes + edges)
+    assert max(src.bincount().max(), dst.bincount().max()) < 256
+    _compare(src, dst, nodes, source_rows)
+
+
+# A row that is too long for counting: the sorts begin with the edges that are copied and checked already.
+@pytest.mark.parametrize("by_source", [False, True])
+def test_long_row_is_copied_once(by_source):
+    src, dst = _edges(600, 600, 9_000, False, 3)
+    (src if by_source else dst)[:256] = 0
+    order = torch.argsort(dst, stable=True)
+    src, dst = src[order].cuda(), dst[order].cuda()
+    luna.make_graph(src, dst, 600)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        luna.make_graph(src, dst, 600)
+        torch.cuda.synchronize()
+    kernels = [event.name for event in profile.events() if event.device_type == torch.autograd.DeviceType.CUDA]
+    assert any("short_edges" in name for name in kernels) and any("segment_tables" in name for name in kernels), kernels
+    assert not any("copy_edges" in name for name in kernels), kernels
+
+
 @pytest.mark.parametrize("src,dst,match", [
     ([0, 4], [0, 1], "at least 5"), ([0, 1], [0, 4], "at least 5"), ([0, -1], [0, 1], "nonnegative"),
     ([0, 1], [1, 0], "sorted"), ([0, 1 << 32], [0, 1], "at least 4294967297"),
