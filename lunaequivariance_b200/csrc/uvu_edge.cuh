@@ -21,9 +21,10 @@
 // to whole rows, and every team of it an equal part of that, whatever the rows; a row that several teams share is summed
 // at the end, in the teams' order, through shared memory.  The forward of very few rows: `group` teams of a CTA share a row, each
 // a contiguous part of its edges, and the parts are summed in a fixed order through shared memory.  No sum depends
-// on which team was first.  A row's sum is one over its own edges, in their order, where tiles are handed out; in a group it is
-// cut by the row's length and `group`; in equal parts it is cut where a team's part ends, so by the lengths of other rows too.
-// So a piece of a graph gives the same rows to the bit where both launches hand out tiles, and else to rounding.
+// on which team was first.  A row's sum is one over its own edges, in their order, where tiles are handed out (two edges at a time:
+// that of the first, third, ... and that of the others); in a group it is cut by the row's length and `group`; in equal parts it is
+// cut where a team's part ends, so by the lengths of other rows too.  So a piece of a graph gives the same rows to the bit where
+// both launches hand out tiles, or both share rows in groups of one size (edge_split), and else to rounding.
 #pragma once
 
 #include <atomic>
@@ -212,19 +213,21 @@ constexpr int kNamedBarriers = 15;  // of a CTA, beside the one of __syncthreads
 // Parts of the edges are even to about a row per CTA; what they lose is order: a CTA's rows are its own, so the rows that all
 // CTAs gather at a time are spread over the whole graph.  So: as long as a team's part is short, and while the node rows that
 // are gathered (`gathered` bytes) stay in L2 whoever reads them.  Groups (`may_group`): while a CTA has three rows
-// or fewer, too few for even parts; pieces of such a graph that have the same group give the same sums.  Rows and edges
+// or fewer, too few for even parts.  The group is a matter of the kernel and of the edges per row, so pieces of such a graph that
+// have as many edges per row give the same sums.  Rows and edges
 // shared as before (groups of up to eight teams, then tiles) and in parts, forward / all gradients: (2, 2, 2), 64 channels,
 // 2,083 nodes of 41 edges 80 / 160 -> 78 / 148 us, 4,000 of 30 98 / 201 -> 90 / 180; 48 channels, 10,001 of 52 290 / 777 -> 258 /
 // 711; 32 channels, 4,003 of 52 100 / 202 -> 88 / 176.  With 442 edges a team (64 channels, 20,000 nodes) the two are even, and
 // with 64 MB of gathered rows ((3, 3, 3), 128 channels, 8,000 nodes) parts lose: forward 0.98 -> 1.27 ms.
 inline bool few_rows(int64_t rows, int ctas) { return rows <= 3 * static_cast<int64_t>(ctas); }
+inline bool shares_rows(int64_t rows, int64_t edges, int ctas) { return few_rows(rows, ctas) && edges >= 4 * rows; }
 inline EdgeSplit edge_split(int64_t rows, int64_t edges, int sm_count, int teams, int team_warps, int64_t wanted_tile,
                             int at_once, int64_t gathered, bool may_group) {
   EdgeSplit s;
   const int64_t all = static_cast<int64_t>(sm_count) * teams;
   const double degree = static_cast<double>(edges) / static_cast<double>(std::max<int64_t>(rows, 1));
   const bool few = may_group && few_rows(rows, sm_count);
-  if (few && degree >= 4.0) {
+  if (may_group && shares_rows(rows, edges, sm_count)) {
     int want = 8;  // and at least two steps of a team in a part
     while (want > 1 && (want > teams || teams % want != 0 || degree < 2.0 * at_once * want)) want /= 2;
     if (want > 1 && team_warps > 1 && teams + teams / want > kNamedBarriers) want = 1;

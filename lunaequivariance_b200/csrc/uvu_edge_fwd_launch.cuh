@@ -34,16 +34,18 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.team_warps = lanes.team_warps;
   P.accumulate = a.accumulate ? 1 : 0;
   EdgeLaunch launch = PAIR ? pair_fwd_launch<T, CPL, S>(plan->tuning, P.ch, dt.max_smem_optin)
-                                 : edge_fwd_launch<T, CPL, S>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
+                           : edge_fwd_launch<T, CPL, S>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
   if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
   P.ring_elems = launch.team_elems;
   P.teams = launch.warps / lanes.team_warps;
   const int ctas = SLICED ? slice_ctas(dt.sm_count, lanes.slices) : dt.sm_count;
-  // Teams that share rows come in twos, fours or eights: of seven or thirteen none could share one.  FP64 (2, 2, 2), 64 channels, ten teams
-  // in twos and eight in eights: 24 nodes 12.7 and 7.5 us, 440 nodes 31 and 34, so with the usual layouts only up to a row per CTA.
-  if (few_rows(graph->num_nodes, ctas) && P.teams > 4) {
-    P.teams -= P.teams > 8 && (CPL == 3 || graph->num_nodes <= ctas) ? P.teams % 4 : P.teams % 2;
+  // Teams that share rows come in twos, fours or eights: of seven or thirteen none could share one.  Whatever the number of rows, so that
+  // a piece of such a graph has the same groups.  Ten teams in twos and eight in eights, 24 / 100 / 300 / 440 nodes of 30 edges: FP64
+  // (2, 2, 2), 64 channels 16.8 / 20.9 / 22.8 / 26.1 and 7.9 / 9.2 / 22.0 / 23.6 us, (3, 3, 0) 10.2 / 12.6 / 13.9 / 14.7 and 5.8 / 6.6 / 15.0 /
+  // 16.3; FP32 (2, 3, 3), fourteen and twelve, 18.4 / 22.8 / 24.8 / 27.8 and 11.2 / 13.3 / 17.2 / 19.8.
+  if (shares_rows(graph->num_nodes, graph->num_edges, ctas) && P.teams > 4) {
+    P.teams -= P.teams > 8 ? P.teams % 4 : P.teams % 2;
     launch.warps = P.teams * lanes.team_warps;
   }
   const int64_t sources = graph->num_src_nodes > 0 ? graph->num_src_nodes : graph->num_nodes;

@@ -13,7 +13,7 @@ import lunaequivariance_b200 as luna
 from lunaequivariance_b200 import conv as conv_mod
 from lunaequivariance_b200 import sharded
 from lunaequivariance_b200.streaming import HostStreamedConv
-from tests.helpers import assert_close, config
+from tests.helpers import all_paths, assert_close, config, random_graph
 
 pytestmark = pytest.mark.gpu
 DEVICE = "cuda"
@@ -83,6 +83,35 @@ def test_pieces_of_a_graph_that_hands_out_tiles(cuts, same, monkeypatch):
         assert_close(out, ref["out"][begin:end].cpu(), torch.float32, f"rows {begin} to {end}")
         assert not same or torch.equal(out, ref["out"][begin:end])
     op.check_status()
+
+
+# Ten teams fit the shared memory in FP64, and eight, twelve or two at other widths: a row's parts do not depend on how many rows
+# a graph has, up to three per SM, as long as it has enough edges for them.
+@pytest.mark.parametrize("mul,degree,dtype", [(64, 2, torch.float64), (96, 2, torch.float64), (48, 2, torch.float32),
+                                              (96, 3, torch.float32), (48, 1, torch.float64)])
+def test_pieces_of_few_rows(mul, degree, dtype):
+    out, ref = _rows_of_pieces(mul, degree, dtype, 400, 400 * 36, (0, 30, 148, 149, 400))
+    assert torch.equal(out, ref)
+
+
+def _rows_of_pieces(mul, degree, dtype, nodes, edges, cuts):
+    features = "+".join(f"{mul}x{l}{'eo'[l % 2]}" for l in range(degree + 1))
+    attributes = "+".join(f"1x{l}{'eo'[l % 2]}" for l in range(degree + 1))
+    op = luna.TensorProductConv(features, attributes, features, all_paths(features, attributes, features),
+                                internal_weights=False, shared_weights=False, dtype=dtype).op
+    generator = torch.Generator().manual_seed(nodes + mul)
+    exact = edges // nodes if edges >= 36 * nodes else None  # rows of one length: their groups are the same in all pieces
+    src, dst = random_graph(nodes, edges, generator, exact_degree=exact)
+    graph = luna.make_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+    rand = lambda *shape: torch.randn(*shape, generator=generator, dtype=torch.float64).to(dtype).to(DEVICE)
+    x, y, w = rand(nodes, op.in1_dim), rand(edges, op.in2_dim), rand(edges, op.weight_numel)
+    ref = conv_mod.run_forward(op, x, y, w, graph)
+    out = torch.full_like(ref, float("nan"))
+    for begin, end in zip(cuts[:-1], cuts[1:]):
+        piece, e0, e1 = graph.destination_range(begin, end)
+        conv_mod.run_forward(op, x, y[e0:e1], w[e0:e1], piece, out=out[begin:end])
+    op.check_status()
+    return out, ref
 
 
 def test_add_gx_needs_a_tensor_and_out_shapes_are_checked():
