@@ -78,9 +78,11 @@ int matrix_entries(int shape, std::integer_sequence<int, ID...>) {
 // ch / 16 channels on each of a half warp's 16 lanes, two edges at a time, where that is compiled (edge_paired).  48 channels, one edge
 // on 24 lanes and two edges with three channels per lane, 0.8 M edges: (1, 1, 1) 192 / 576 / 340 / 393 -> 165 / 352 / 194 / 252; (0, 3, 3)
 // 260 / 642 / 359 / 432 -> 187 / 463 / 252 / 287; (2, 2, 2), 0.52 M edges, 274 / 715 / 378 / 427 -> 260 / 683 / 301 / 301.
-// Not three channels per lane for the forward of few rows (`few`): of its thirteen teams no four or eight can share a row.  (2, 2, 2),
-// 48 channels, 24 nodes 6.7 us with one edge on 24 lanes and 24 with two edges, 300 nodes 18 and 38; 30,000 nodes 757 and 634.  Nor in
-// FP64 with coupling matrices, where seven teams fit: (2, 2, 2), 96 channels, 24 nodes 13 and 33, 440 nodes 42 and 69.
+// The forward of few rows, whose teams share them (`few`), keeps the layout with the shorter way through an edge: its smallest graphs wait
+// for that.  24 / 100 / 300 / 440 nodes of 30 edges, 48 channels on 24 lanes, one edge, and three per lane, two edges: (2, 2, 2)
+// 7.0 / 8.0 / 13.9 / 16.4 and 7.6 / 8.6 / 10.8 / 12.2 us, (0, 3, 3) 5.4 / 6.0 / 10.2 / 11.2 and 6.5 / 7.2 / 8.1 / 8.4.  FP64 with coupling
+// matrices, 96 channels, two warps with two channels per lane and one with three: (2, 2, 2) 15.6 / 20.2 / 26.6 / 31.9 and 17.3 / 22.5 /
+// 26.5 / 30.7.
 EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool sliced, bool few = false) {
   const int ch = plan->edge.ch, elem = plan->dtype == LUNA_F64 ? 8 : 4;
   // one team with two stages must fit an SM's shared memory in either direction
@@ -262,7 +264,7 @@ void analyse(luna_uvu_plan* plan) {
 int forward(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph, const void* x, const void* y,
             const void* w, void* out, bool accumulate, cudaStream_t stream) {
   const EdgeForwardArgs args{x, y, w, out, accumulate};
-  const EdgeLanes& lanes = few_rows(graph->num_nodes, dt.sm_count) ? plan->edge.lanes : plan->edge.lanes_rows;
+  const EdgeLanes& lanes = shares_rows(graph->num_nodes, graph->num_edges, dt.sm_count) ? plan->edge.lanes : plan->edge.lanes_rows;
   return with_instance(plan, lanes, [&](auto kernels) { return kernels.forward(plan, dt, graph, lanes, args, stream); });
 }
 

@@ -94,6 +94,13 @@ def test_pieces_of_few_rows(mul, degree, dtype):
     assert torch.equal(out, ref)
 
 
+# With two edges per row every launch hands out tiles, however few the rows.
+@pytest.mark.parametrize("mul,degree,dtype", [(48, 2, torch.float32), (96, 2, torch.float64), (32, 2, torch.float32)])
+def test_pieces_of_a_sparse_graph(mul, degree, dtype):
+    out, ref = _rows_of_pieces(mul, degree, dtype, 3000, 6000, (0, 24, 400, 1500, 3000))
+    assert torch.equal(out, ref)
+
+
 def _rows_of_pieces(mul, degree, dtype, nodes, edges, cuts):
     features = "+".join(f"{mul}x{l}{'eo'[l % 2]}" for l in range(degree + 1))
     attributes = "+".join(f"1x{l}{'eo'[l % 2]}" for l in range(degree + 1))
