@@ -301,12 +301,12 @@ int canonical_l2(const luna_uvu_plan* plan) {
 }
 
 size_t smem_bytes(const luna_uvu_plan* plan, bool backward, int max_smem) {
-  const EdgeLanes& lanes = backward ? plan->edge.lanes_all : plan->edge.lanes;
   size_t bytes = 0;
-  with_instance(plan, lanes, [&](auto kernels) {
-    bytes = kernels.smem_bytes(plan, lanes, backward, max_smem);
-    return LUNA_OK;
-  });
+  for (const EdgeLanes* lanes : {backward ? &plan->edge.lanes_all : &plan->edge.lanes, backward ? &plan->edge.lanes_all : &plan->edge.lanes_rows})
+    with_instance(plan, *lanes, [&](auto kernels) {
+      bytes = std::max(bytes, kernels.smem_bytes(plan, *lanes, backward, max_smem));
+      return LUNA_OK;
+    });
   return bytes;
 }
 

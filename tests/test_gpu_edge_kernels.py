@@ -2,6 +2,7 @@
 that leave lanes idle or need several warps per edge, rows shared by several teams and rows handed out in tiles."""
 
 import dataclasses
+import json
 
 import pytest
 import torch
@@ -291,3 +292,26 @@ def test_parts_without_edges_behind_the_last_row(shape, mul):
         module.op.check_status()
         for key, value in dict(out=result, gx=gx, gy=gy, gw=gw).items():
             assert_close(value, ref[key], torch.float32, f"{SHAPES[shape]} x{mul} {nodes} nodes {key}")
+
+
+# The kernels of small graphs, of larger ones and of those that hand out tiles: the plan's figure bounds what any launch takes.
+@pytest.mark.parametrize("shape,mul,dtype", [(4, 48, torch.float32), (4, 96, torch.float64), (3, 48, torch.float64),
+                                             (5, 128, torch.float32), (4, 64, torch.float32), (3, 352, torch.float32)])
+def test_shared_memory_of_a_forward_block(shape, mul, dtype, tmp_path):
+    in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
+    op = luna.TensorProductConv(in1, in2, out, all_paths(in1, in2, out), internal_weights=False, shared_weights=False,
+                                dtype=dtype).op
+    sizes = []
+    for nodes, edges in ((24, 552), (700, 12_000), (900, 1_800)):
+        src, dst = skewed_graph(nodes, edges, torch.Generator().manual_seed(nodes), 0.0)
+        graph = luna.make_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+        x, y, w = (torch.zeros(*rows, dtype=dtype, device=DEVICE)
+                   for rows in ((nodes, op.in1_dim), (edges, op.in2_dim), (edges, op.weight_numel)))
+        torch.cuda.synchronize()
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+            conv_mod.run_forward(op, x, y, w, graph)
+            torch.cuda.synchronize()
+        profile.export_chrome_trace(str(tmp_path / "trace.json"))
+        events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+        sizes += [event["args"]["shared memory"] for event in events if "fwd_kernel" in event.get("name", "") and "args" in event]
+    assert len(sizes) == 3 and max(sizes) <= op._plan.query(3), sizes
