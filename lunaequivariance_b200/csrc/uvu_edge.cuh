@@ -42,6 +42,7 @@ constexpr int kEdgeMaxStages = 4;
 constexpr int kEdgeMaxSlices = kTileCounterWords / 2;
 constexpr int64_t kPartEdges = 256;          // of a team, at most
 constexpr int64_t kPartGathered = 24 << 20;  // bytes
+constexpr int64_t kEarlyWeights = 128 << 20;  // bytes, of launches that write dL/dw and start early
 constexpr int kEdgeMaxCoefs = 10;  // paths with a degree of zero
 
 // ---- shapes ---------------------------------------------------------------------------------------------------------

@@ -120,7 +120,14 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   const int rc = setup.once(reinterpret_cast<const void*>(kernel), dt.max_smem_optin);
   if (rc != LUNA_OK) return rc;
   const dim3 grid(static_cast<unsigned>(cut.blocks), static_cast<unsigned>(lanes.slices));
-  launch_early(kernel, grid, launch.warps * 32, launch.bytes, stream, P);
+  // An early start where weights come in and their gradients leave: beyond the size of L2 it costs more than the launch that it hides.
+  // Back to back, dL/dw alone, from 16 / 32 / 64 / 128 MB of weights on: FP32 -5 / -3 / -2 / +0.6 %, FP64 -5 / -2 / -1 / +1.3 %; (1, 1, 0),
+  // 48 FP64 channels, 0.26 M edges, 200 MB +16 %.  Launches that write no weight gradients are at no size slower on average.
+  const int64_t weights = P.num_edges * S::paths * plan->edge.ch * static_cast<int64_t>(sizeof(T));
+  if (a.gw == nullptr || weights <= kEarlyWeights)
+    launch_early(kernel, grid, launch.warps * 32, launch.bytes, stream, P);
+  else
+    kernel<<<grid, launch.warps * 32, launch.bytes, stream>>>(P);
   LUNA_LAUNCH_CHECK("backward (edge family)");
   if (SLICED && WY) {
     reduce_gy_partial<T><<<static_cast<unsigned>(ceil_div(P.gy_part, 256)), 256, 0, stream>>>(

@@ -139,3 +139,38 @@ def test_edge_kernels_behind_one_another(degree, mul, dtype, nodes, edges):
     op.check_status()
     for at, (a, b) in enumerate(zip(want, got)):
         assert torch.isfinite(a).all() and a.abs().max() > 0 and torch.equal(a, b), at
+
+
+class _EdgeData(ctypes.Structure):
+    _fields_ = [("from_port", ctypes.c_ubyte), ("to_port", ctypes.c_ubyte), ("type", ctypes.c_ubyte), ("reserved", ctypes.c_ubyte * 5)]
+
+
+def _early_starts(call):
+    """How many of two launches behind one another, captured in a graph, start before the launch ahead of them has ended."""
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+        call()
+    sources, targets, data, edges = (ctypes.c_void_p * 8)(), (ctypes.c_void_p * 8)(), (_EdgeData * 8)(), ctypes.c_size_t(8)
+    error = ctypes.CDLL("libcudart.so.12").cudaGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), sources, targets, data,
+                                                                ctypes.byref(edges))
+    assert error == 0 and edges.value == 1  # two nodes
+    return sum(data[edge].type == 1 for edge in range(edges.value))  # cudaGraphDependencyTypeProgrammatic
+
+
+# 128 MB of weights and a little more
+@pytest.mark.parametrize("edges,early", [(47_662, 1), (47_663, 0)])
+def test_large_weight_gradients_start_in_order(edges, early):
+    irreps, attributes = "64x0e+64x1o+64x2e", "1x0e+1x1o+1x2e"
+    module = luna.TensorProductConv(irreps, attributes, irreps, all_paths(irreps, attributes, irreps), internal_weights=False,
+                                    shared_weights=False, dtype=torch.float32)
+    op, nodes = module.op, 2_000
+    src, dst = random_graph(nodes, edges, torch.Generator().manual_seed(5))
+    graph = module.create_graph(src.cuda(), dst.cuda(), nodes)
+    x, y, w, g = (torch.zeros(*shape, device="cuda")
+                  for shape in ((nodes, op.in1_dim), (edges, op.in2_dim), (edges, op.weight_numel), (nodes, op.out_dim)))
+    out, gw = torch.empty_like(g), torch.empty_like(w)
+    assert _early_starts(lambda: conv_mod.run_forward(op, x, y, w, graph, out=out)) == 1
+    assert _early_starts(lambda: conv_mod.run_backward(op, x, y, w, g, graph, (False, False, True), out=(None, None, gw))) == early
