@@ -639,10 +639,13 @@ __host__ __device__ constexpr int warps_for(int regs, int slack = 0) {
 // Of the backward kernels, whose estimate has room for coupling matrices in it: lists without any need less, dL/dy alone, which
 // keeps neither gradients nor matrices, least.  Twelve warps and sixteen, 0.4 M edges: dL/dy alone, 128 channels, (3, 3, 0) 248 ->
 // 215 us, FP64 (0, 3, 3), 64 channels 334 -> 281; dL/dx with dL/dw, (2, 2, 0), 128 channels, 0.8 M edges 640 -> 555; output with
-// dL/dw, (0, 2, 2), 608 -> 537.  Above these limits it loses: all gradients of (2, 2, 0), 128 channels 716 -> 800.
-template <typename S>
-constexpr int slack_for(bool with_sums) {
-  return S::m_total != 0 ? 0 : (with_sums ? 10 : 35);
+// dL/dw, (0, 2, 2), 608 -> 537.  Above these limits it loses: all gradients of (2, 2, 0), 128 channels 716 -> 800.  So it does with two
+// edges at a time, which have no slack: (2, 2, 0), 64 channels, 0.26 M edges, dL/dx with dL/dw 116 -> 193 us, FP64, 48 channels, 60,000
+// edges 46 -> 54; and FP32 dL/dy alone with idle lanes (not `full`): (0, 3, 3), 80 channels, 600 and 15,000 edges +34 and +9 %.
+template <typename T, typename S>
+constexpr int slack_for(bool with_sums, bool full) {
+  if (S::m_total != 0) return 0;
+  return with_sums ? 10 : (full || sizeof(T) == 8 ? 35 : 0);
 }
 
 // Attributes a kernel needs set once per device, not on every launch.

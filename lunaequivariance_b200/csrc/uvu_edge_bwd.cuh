@@ -75,7 +75,8 @@ struct EdgeBwd {
       (S::XD * CPL * (WX ? 2 : 1) + (WY ? S::YD * pair : 0) + (2 * S::LO + 1) * CPL) * words;
   static constexpr int program_regs = WM ? S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 : 0;
   static constexpr int registers = state + program_regs + 48;  // an estimate; beyond 255 it spills hundreds of bytes
-  static constexpr int max_warps = warps_for(registers, slack_for<S>(WM));
+  template <bool FULL>
+  static constexpr int warps = warps_for(registers, slack_for<T, S>(WM, FULL));
   // slots of g: the highest degree has one, the others share one
   static constexpr int slot_of(int l3) { return l3 == S::LO && S::ooff(S::LO) > 0 ? 1 : 0; }
   static constexpr int slots = slot_of(S::LO) + 1;
@@ -282,7 +283,7 @@ __device__ __forceinline__ void backward_path(T* wq, int lanes, bool keep, const
 // FULL: one warp per edge and 32 * CPL channels, known to the compiler.  SLICED: these are a slice of wider blocks.  DST: rows
 // by destination (S, x and g exchanged).  ADD: gw alone, added to; w names gw.
 template <typename T, int CPL, typename S, bool WX, bool WM, bool WY, bool FULL, bool DST, bool SLICED, bool ADD>
-__global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::max_warps * 32, 1)
+__global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::template warps<FULL> * 32, 1)
     edge_bwd_kernel(const __grid_constant__ EdgeBwdParams<T, EdgeBwd<T, CPL, S, WX, WM, WY>::terms> P) {
   using K = EdgeBwd<T, CPL, S, WX, WM, WY>;
   using PK = EdgePacket<T, CPL, edge_spread(S::OD, S::paths)>;

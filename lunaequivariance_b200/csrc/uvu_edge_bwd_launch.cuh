@@ -8,12 +8,12 @@ namespace luna {
 namespace edgek {
 
 // K: the EdgeBwd of the kernel.
-template <typename T, typename S, typename K>
+template <typename T, typename S, typename K, bool FULL>
 EdgeLaunch edge_bwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch, int max_smem) {
   const size_t w_row = static_cast<size_t>(S::paths) * ch * sizeof(T);
   const size_t x_row = static_cast<size_t>(S::XD) * ch * sizeof(T), g_row = static_cast<size_t>(S::OD) * ch * sizeof(T);
   EdgeLaunch launch;
-  const int max_teams = capped_warps(tuning, K::max_warps) / lanes.team_warps;
+  const int max_teams = capped_warps(tuning, K::template warps<FULL>) / lanes.team_warps;
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
     for (int option = 0; option < 3; ++option) {  // three or two stages with g in them, or two and g by degree
       const int stages = option == 0 ? 3 : 2, split = option == 2;
@@ -82,7 +82,7 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   if constexpr (PAIR)
     launch = pair_bwd_launch<T, S, PairBwd<T, CPL, S, WX, WM, WY>>(plan->tuning, P.ch, dt.max_smem_optin);
   else
-    launch = edge_bwd_launch<T, S, K>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
+    launch = edge_bwd_launch<T, S, K, FULL>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
   if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
   P.team_elems = launch.team_elems;
@@ -143,7 +143,7 @@ int launch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
 template <typename T, int CPL, typename S>
 constexpr bool edge_joins_output() {
   using R = Transposed<S>;
-  return 2 * EdgeBwd<T, CPL, R, true, true, false>::max_warps > EdgeBwd<T, CPL, R, false, true, false>::max_warps;
+  return 2 * EdgeBwd<T, CPL, R, true, true, false>::template warps<true> > EdgeBwd<T, CPL, R, false, true, false>::template warps<true>;
 }
 
 // ID: the shape's number, which tells with PAIR which uses have kernels of two edges at a time.

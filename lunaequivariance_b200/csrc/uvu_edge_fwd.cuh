@@ -40,9 +40,10 @@ struct EdgeFwd {
   static constexpr int words = sizeof(T) / 4;
   static constexpr int m_elems = S::m_elems;
   static constexpr int registers = (S::OD + S::XD) * CPL * words + S::m_rounds * 2 * words + (S::m_rounds + 1) / 2 + 44;
-  // in FP64 with few matrices the estimate is a little high: (2, 2, 2), 64 channels, 0.42 M edges 469 -> 437 us with sixteen warps
-  // (FP32, 128 channels, which the same line would change, 402 -> 410)
-  static constexpr int max_warps = warps_for(registers, sizeof(T) == 8 && S::m_total <= 64 ? 5 : 0);
+  // FULL, in FP64 with few matrices: the estimate is a little high.  (2, 2, 2), 64 channels, 0.26 M edges 5 % faster with sixteen warps
+  // than with twelve, but 48 channels on 24 lanes 233 -> 256 us, 96 in two warps, 24 nodes, 16.0 -> 18.6.
+  template <bool FULL>
+  static constexpr int warps = warps_for(registers, FULL && sizeof(T) == 8 && S::m_total <= 64 ? 5 : 0);
   static constexpr size_t team_bytes = 2 * static_cast<size_t>(m_elems) * sizeof(T);
 };
 
@@ -143,7 +144,7 @@ static __device__ __noinline__ void merge_forward(const EdgeFwdParams<T>& P) {
 
 // FULL: one warp per edge and 32 * CPL channels, known to the compiler.  SLICED: these are a slice of wider blocks.
 template <typename T, int CPL, typename S, bool FULL, bool SLICED>
-__global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
+__global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::template warps<FULL> * 32, 1)
     edge_fwd_kernel(const __grid_constant__ EdgeFwdParams<T> P) {
   using K = EdgeFwd<T, CPL, S>;
   using PK = EdgePacket<T, CPL, edge_spread(S::XD, S::paths)>;
@@ -342,13 +343,13 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::max_warps * 32, 1)
 }
 
 // As many teams as fit the shared memory with three stages each (two, if they are then more).
-template <typename T, int CPL, typename S>
+template <typename T, int CPL, typename S, bool FULL>
 EdgeLaunch edge_fwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch, int max_smem) {
   using K = EdgeFwd<T, CPL, S>;
   const size_t stage = static_cast<size_t>(S::paths + S::XD) * ch * sizeof(T);
   const size_t row = static_cast<size_t>(S::OD) * ch * sizeof(T);
   EdgeLaunch launch;
-  const int max_teams = capped_warps(tuning, K::max_warps) / lanes.team_warps;
+  const int max_teams = capped_warps(tuning, K::template warps<FULL>) / lanes.team_warps;
   for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
     for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
       const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;

@@ -34,7 +34,7 @@ int launch_edge_fwd(const luna_uvu_plan* plan, const DeviceTables& dt, const lun
   P.team_warps = lanes.team_warps;
   P.accumulate = a.accumulate ? 1 : 0;
   EdgeLaunch launch = PAIR ? pair_fwd_launch<T, CPL, S>(plan->tuning, P.ch, dt.max_smem_optin)
-                           : edge_fwd_launch<T, CPL, S>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
+                           : edge_fwd_launch<T, CPL, S, FULL>(plan->tuning, lanes, P.ch, dt.max_smem_optin);
   if (launch.warps == 0) return fail(LUNA_ERR_UNSUPPORTED, "the rows of an edge do not fit the shared memory of this device");
   P.stages = launch.stages;
   P.ring_elems = launch.team_elems;

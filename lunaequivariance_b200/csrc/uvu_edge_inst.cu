@@ -50,9 +50,11 @@ size_t EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::smem_bytes(cons
   if (lanes.edges == 2)
     return backward ? pair_bwd_launch<LUNA_EDGE_T, S, PairBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>>(plan->tuning, ch, max_smem).bytes
                     : pair_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, ch, max_smem).bytes;
-  if (!backward) return edge_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S>(plan->tuning, lanes, ch, max_smem).bytes;
+  if (!backward)
+    return ch == 32 * LUNA_EDGE_CPL ? edge_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true>(plan->tuning, lanes, ch, max_smem).bytes
+                                    : edge_fwd_launch<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false>(plan->tuning, lanes, ch, max_smem).bytes;
   using K = EdgeBwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, true, true>;
-  return edge_bwd_launch<LUNA_EDGE_T, S, K>(plan->tuning, lanes, ch, max_smem).bytes;
+  return edge_bwd_launch<LUNA_EDGE_T, S, K, true>(plan->tuning, lanes, ch, max_smem).bytes;
 }
 
 }  // namespace edgek

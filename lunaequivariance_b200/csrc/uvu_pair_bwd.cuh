@@ -18,7 +18,7 @@ struct PairBwd {
   static constexpr int warp_elems = 2 * m_elems + (WY ? red_pass * red_row : 0);
   static constexpr int program_regs = WM ? 4 * S::m_rounds * Edge::words + S::m_rounds + 1 : 0;
   static constexpr int registers = Edge::state + program_regs + 44;
-  static constexpr int max_warps = warps_for(registers, slack_for<S>(WM));
+  static constexpr int max_warps = warps_for(registers);
 };
 
 // 16 * CPL channels.  DST: rows by destination (S, x and g exchanged).  ADD: gw alone, added to; w names gw.
@@ -394,7 +394,7 @@ EdgeLaunch pair_bwd_launch(const Tuning& tuning, int ch, int max_smem) {
 template <typename T, typename S, bool WY>
 constexpr bool pair_crowded() {
   using Two = PairBwd<T, 2, S, true, true, WY>;
-  return Two::max_warps == 8 && (EdgeBwd<T, 1, S, true, true, WY>::max_warps >= 16 || Two::registers > 190);
+  return Two::max_warps == 8 && (EdgeBwd<T, 1, S, true, true, WY>::template warps<true> >= 16 || Two::registers > 190);
 }
 template <typename T, int CPL, int ID>
 constexpr bool edge_paired(EdgeUse use) {

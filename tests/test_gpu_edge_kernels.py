@@ -3,6 +3,7 @@ that leave lanes idle or need several warps per edge, rows shared by several tea
 
 import dataclasses
 import json
+import re
 
 import pytest
 import torch
@@ -294,6 +295,28 @@ def test_parts_without_edges_behind_the_last_row(shape, mul):
             assert_close(value, ref[key], torch.float32, f"{SHAPES[shape]} x{mul} {nodes} nodes {key}")
 
 
+def launches(op, dtype, nodes, edges, which, tmp_path):
+    """(kernel, channels per lane, warps and shared memory of a block) of the edge kernels that a call launches."""
+    src, dst = skewed_graph(nodes, edges, torch.Generator().manual_seed(nodes), 0.0)
+    graph = luna.make_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+    x, y, w, g = (torch.zeros(*rows, dtype=dtype, device=DEVICE)
+                  for rows in ((nodes, op.in1_dim), (edges, op.in2_dim), (edges, op.weight_numel), (nodes, op.out_dim)))
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        if which == "forward":
+            conv_mod.run_forward(op, x, y, w, graph)
+        else:
+            conv_mod.run_backward(op, x, y, w, g, graph, tuple(key in which for key in "xyw"))
+        torch.cuda.synchronize()
+    profile.export_chrome_trace(str(tmp_path / "trace.json"))
+    found = []
+    for event in json.loads((tmp_path / "trace.json").read_text())["traceEvents"]:
+        match = re.search(r"(edge|pair)_(?:fwd|bwd)_kernel<(?:float|double), (\d)", event.get("name", ""))
+        if match and "shared memory" in event.get("args", {}):
+            found.append((match[1], int(match[2]), event["args"]["block"][0] // 32, event["args"]["shared memory"]))
+    return found
+
+
 # The kernels of small graphs, of larger ones and of those that hand out tiles: the plan's figure bounds what any launch takes.
 @pytest.mark.parametrize("shape,mul,dtype", [(4, 48, torch.float32), (4, 96, torch.float64), (3, 48, torch.float64),
                                              (5, 128, torch.float32), (4, 64, torch.float32), (3, 352, torch.float32)])
@@ -301,17 +324,21 @@ def test_shared_memory_of_a_forward_block(shape, mul, dtype, tmp_path):
     in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
     op = luna.TensorProductConv(in1, in2, out, all_paths(in1, in2, out), internal_weights=False, shared_weights=False,
                                 dtype=dtype).op
-    sizes = []
     for nodes, edges in ((24, 552), (700, 12_000), (900, 1_800)):
-        src, dst = skewed_graph(nodes, edges, torch.Generator().manual_seed(nodes), 0.0)
-        graph = luna.make_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
-        x, y, w = (torch.zeros(*rows, dtype=dtype, device=DEVICE)
-                   for rows in ((nodes, op.in1_dim), (edges, op.in2_dim), (edges, op.weight_numel)))
-        torch.cuda.synchronize()
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
-            conv_mod.run_forward(op, x, y, w, graph)
-            torch.cuda.synchronize()
-        profile.export_chrome_trace(str(tmp_path / "trace.json"))
-        events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
-        sizes += [event["args"]["shared memory"] for event in events if "fwd_kernel" in event.get("name", "") and "args" in event]
-    assert len(sizes) == 3 and max(sizes) <= op._plan.query(3), sizes
+        (launch,) = launches(op, dtype, nodes, edges, "forward", tmp_path)
+        assert launch[3] <= op._plan.query(3), (nodes, launch)
+
+
+# Layouts that are slower than the ones beside them are not chosen.
+@pytest.mark.parametrize("shape,mul,dtype,which,kernel,lane_channels,warps", [
+    # an estimate of registers that is taken to be too high
+    (8, 64, torch.float32, "xw", "pair", 4, [12]), (8, 48, torch.float64, "xw", "pair", 3, [8]),
+    (2, 80, torch.float32, "y", "edge", 4, [12]), (2, 128, torch.float32, "y", "edge", 4, [16]),
+    (4, 48, torch.float64, "forward", "edge", 2, [12]),
+])
+def test_layout_of_a_launch(shape, mul, dtype, which, kernel, lane_channels, warps, tmp_path):
+    in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
+    op = luna.TensorProductConv(in1, in2, out, all_paths(in1, in2, out), internal_weights=False, shared_weights=False,
+                                dtype=dtype).op
+    (launch,) = launches(op, dtype, 700, 12_000, which, tmp_path)
+    assert launch[:2] == (kernel, lane_channels) and launch[2] in (warps or [launch[2]]), launch
