@@ -66,15 +66,18 @@ int matrix_entries(int shape, std::integer_sequence<int, ID...>) {
 // per lane, all gradients, which then spills 176 (FP32) or 276 bytes and more.  300 MB of weights, FP64: 224 channels with one
 // channel per lane 0.83 -> 0.54 ms; FP32: 128 channels 0.33 -> 0.27 with two (2.6 GB: 2.03 -> 1.54), 256 channels 0.39 -> 0.30.
 // The forward with an estimate of more than 190 registers counts a third more: FP32 (3, 3, 3), 128 channels, two warps with two channels
-// per lane instead of one with four, 0.2 M edges 620 -> 583 us, 24,000 edges 134 -> 115; 256 channels, 60,000 edges, 420 -> 398.  (FP64
-// with 128 channels would lose by one per lane, 867 -> 972, and at a third more the choice stays at two.)
+// per lane instead of one with four, 0.2 M edges 620 -> 583 us, 24,000 edges 134 -> 115; 256 channels, 60,000 edges, 420 -> 398.  Not where
+// two channels would leave lanes idle: 80 channels, 24 nodes 18.6 -> 25.7 us, 60,000 edges 158 -> 167; 160, five warps with one channel
+// instead of two with four, 27 -> 61 and 292 -> 311.  (FP64 with 128 channels would lose by one per lane, 867 -> 972, and at a third more
+// the choice stays at two.)
 // Three channels per lane, where four or two left a quarter of the lanes idle.  96 channels, forward / all gradients / dL/dy / dL/dw,
 // FP32: (2, 2, 2), 0.4 M edges 364 / 958 / 465 / 520 -> 323 / 759 / 426 / 434 us; (2, 3, 3), 0.4 M edges 653 / 1,611 / 852 / 922 ->
 // 550 / 1,439 / 790 / 718; FP64, two warps with two and one with three: (2, 2, 2), 0.2 M edges 361 / 1,050 / 566 / 567 -> 332 /
 // 763 / 426 / 450; (0, 1, 1), 0.4 M edges 217 / 580 / 408 / 348 -> 128 / 351 / 185 / 207.  It is not taken where its state is far above
 // the registers (FP64, (3, 3, 3), all gradients of 0.12 M edges 1.96 -> 3.27 ms), for more than two warps, for slices, and for two FP32
 // warps with long coupling matrices: 192 channels, forward / dL/dy (3, 3, 3) 408 / 523 -> 486 / 556 us, (2, 3, 3) 466 / 698 -> 495 /
-// 758, but (0, 2, 2) 332 / 560 -> 246 / 398.
+// 758, but (0, 2, 2) 332 / 560 -> 246 / 398.  Nor for two FP64 warps of estimates above 220: 192 channels, 60,000 edges, (3, 3, 3), dL/dy /
+// dL/dw 796 / 955 -> 843 / 1,022 us, (2, 3, 3), dL/dx with dL/dw 697 -> 760; below, (2, 3, 3), dL/dy / dL/dw 562 / 650 -> 523 / 559.
 // ch / 16 channels on each of a half warp's 16 lanes, two edges at a time, where that is compiled (edge_paired).  48 channels, one edge
 // on 24 lanes and two edges with three channels per lane, 0.8 M edges: (1, 1, 1) 192 / 576 / 340 / 393 -> 165 / 352 / 194 / 252; (0, 3, 3)
 // 260 / 642 / 359 / 432 -> 187 / 463 / 252 / 287; (2, 2, 2), 0.52 M edges, 274 / 715 / 378 / 427 -> 260 / 683 / 301 / 301.
@@ -100,11 +103,11 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool s
     const int registers = registers_of(plan, shape, use, cpl);
     if (cpl == 3 && few && elem == 8 && matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 0) continue;
     if (cpl == 3 && (sliced || parts > 2 || registers > (use == EdgeUse::kForward ? 255 : 280) ||
-                     (parts == 2 && elem == 4 && matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 64)))
+                     (parts == 2 && (elem == 8 ? registers > 220 : matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 64))))
       continue;
     const double crowded = (use == EdgeUse::kAllGradients || cpl == 3) && registers > 255 ? 1.5
-                           : use == EdgeUse::kForward && registers > 190                   ? 1.3
-                                                                                           : 1.0;
+                           : use == EdgeUse::kForward && registers > 190 && (elem == 8 || ch % 64 == 0) ? 1.3
+                                                                                                         : 1.0;
     const double cost = parts * (1 + cpl) * crowded;
     if (best.cpl != 0 && cost >= best_cost) continue;
     best_cost = cost;

@@ -335,6 +335,10 @@ def test_shared_memory_of_a_forward_block(shape, mul, dtype, tmp_path):
     (8, 64, torch.float32, "xw", "pair", 4, [12]), (8, 48, torch.float64, "xw", "pair", 3, [8]),
     (2, 80, torch.float32, "y", "edge", 4, [12]), (2, 128, torch.float32, "y", "edge", 4, [16]),
     (4, 48, torch.float64, "forward", "edge", 2, [12]),
+    # idle lanes, and states that are too large, of the layout with less work
+    (5, 80, torch.float32, "forward", "edge", 4, None), (5, 160, torch.float32, "forward", "edge", 4, None),
+    (5, 128, torch.float32, "forward", "edge", 2, None), (5, 192, torch.float64, "y", "edge", 2, None),
+    (6, 192, torch.float64, "xw", "edge", 2, None), (6, 192, torch.float64, "w", "edge", 3, None),
 ])
 def test_layout_of_a_launch(shape, mul, dtype, which, kernel, lane_channels, warps, tmp_path):
     in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
