@@ -350,7 +350,11 @@ EdgeLaunch edge_fwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
   const size_t row = static_cast<size_t>(S::OD) * ch * sizeof(T);
   EdgeLaunch launch;
   const int max_teams = capped_warps(tuning, K::template warps<FULL>) / lanes.team_warps;
-  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams)
+  for (int teams = max_teams; teams >= 1 && launch.warps == 0; --teams) {
+    // With more than twenty teams of three channels per lane and the long gathered rows of (1, 1, 0) the plain loads of attributes and
+    // indices wait behind the bulk copies: 96 channels, 0.26 M edges, 16 / 20 / 22 / 24 teams 59 / 55 / 94 / 121 us.  (0, 1, 1), half as many bytes
+    // in flight, 59 / 53 / 53 / 50.
+    if (CPL == 3 && teams > 16 && 3 * max_teams * stage > 150 * 1024) continue;
     for (int stages = teams * 2 > max_teams ? 3 : kEdgeMaxStages; stages >= 2; --stages) {
       const size_t ring = (std::max(stages * stage, row) + 127) / 128 * 128;
       const size_t bytes = teams * (ring + K::team_bytes + kEdgeMaxStages * sizeof(uint64_t) + sizeof(unsigned) + sizeof(TeamPart));
@@ -361,6 +365,7 @@ EdgeLaunch edge_fwd_launch(const Tuning& tuning, const EdgeLanes& lanes, int ch,
       launch.team_elems = static_cast<int>(ring / sizeof(T));
       break;
     }
+  }
   return launch;
 }
 

@@ -339,6 +339,8 @@ def test_shared_memory_of_a_forward_block(shape, mul, dtype, tmp_path):
     (5, 80, torch.float32, "forward", "edge", 4, None), (5, 160, torch.float32, "forward", "edge", 4, None),
     (5, 128, torch.float32, "forward", "edge", 2, None), (5, 192, torch.float64, "y", "edge", 2, None),
     (6, 192, torch.float64, "xw", "edge", 2, None), (6, 192, torch.float64, "w", "edge", 3, None),
+    # too many bulk copies under way
+    (7, 96, torch.float32, "forward", "edge", 3, [16]), (0, 96, torch.float32, "forward", "edge", 3, [24]),
 ])
 def test_layout_of_a_launch(shape, mul, dtype, which, kernel, lane_channels, warps, tmp_path):
     in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
