@@ -9,19 +9,6 @@ namespace edgek {
 
 namespace {
 
-// The estimate of what a lane of the kernel needs.
-template <typename T, int CPL, typename S>
-constexpr int registers_of(EdgeUse use) {
-  using R = Transposed<S>;
-  using One = std::conditional_t<S::OD >= S::XD, R, S>;
-  switch (use) {
-    case EdgeUse::kForward: return EdgeFwd<T, CPL, S>::registers;
-    case EdgeUse::kSums: return EdgeBwd<T, CPL, S, true, true, false>::registers;
-    case EdgeUse::kOutputAndWeights: return EdgeBwd<T, CPL, R, true, true, false>::registers;
-    case EdgeUse::kAllGradients: return EdgeBwd<T, CPL, S, true, true, true>::registers;
-    default: return std::max(EdgeBwd<T, CPL, One, false, false, true>::registers, EdgeBwd<T, CPL, One, false, true, false>::registers);
-  }
-}
 template <typename T, int CPL, int... ID>
 int registers_of(int shape, EdgeUse use, std::integer_sequence<int, ID...>) {
   int found = 0;
@@ -50,6 +37,18 @@ bool paired(const luna_uvu_plan* plan, int shape, EdgeUse use, int cpl) {
                     : (cpl == 2 ? paired<double, 2>(shape, use, all) : cpl == 3 && paired<double, 3>(shape, use, all));
   if (cpl >= 3) return cpl == 4 ? paired<float, 4>(shape, use, all) : cpl == 3 && paired<float, 3>(shape, use, all);
   return cpl == 1 ? paired<float, 1>(shape, use, all) : cpl == 2 && paired<float, 2>(shape, use, all);
+}
+
+// Whether one edge at a time with three channels per lane is compiled.
+template <typename T, int... ID>
+bool three(int shape, EdgeUse use, std::integer_sequence<int, ID...>) {
+  bool found = false;
+  ((found = found || (shape == ID && edge_alone<T, 3, ID>(use))), ...);
+  return found;
+}
+bool three(const luna_uvu_plan* plan, int shape, EdgeUse use) {
+  constexpr std::make_integer_sequence<int, kEdgeShapes> all{};
+  return plan->dtype == LUNA_F64 ? three<double>(shape, use, all) : three<float>(shape, use, all);
 }
 
 // Coupling-matrix entries of the shape.
@@ -102,7 +101,7 @@ EdgeLanes choose_lanes(const luna_uvu_plan* plan, int shape, EdgeUse use, bool s
       continue;
     const int registers = registers_of(plan, shape, use, cpl);
     if (cpl == 3 && few && elem == 8 && matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 0) continue;
-    if (cpl == 3 && (sliced || parts > 2 || registers > (use == EdgeUse::kForward ? 255 : 280) ||
+    if (cpl == 3 && (sliced || parts > 2 || !three(plan, shape, use) ||
                      (parts == 2 && (elem == 8 ? registers > 220 : matrix_entries(shape, std::make_integer_sequence<int, kEdgeShapes>{}) > 64))))
       continue;
     const double crowded = (use == EdgeUse::kAllGradients || cpl == 3) && registers > 255 ? 1.5

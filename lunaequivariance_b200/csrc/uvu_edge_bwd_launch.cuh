@@ -146,13 +146,13 @@ constexpr bool edge_joins_output() {
   return 2 * EdgeBwd<T, CPL, R, true, true, false>::template warps<true> > EdgeBwd<T, CPL, R, false, true, false>::template warps<true>;
 }
 
-// ID: the shape's number, which tells with PAIR which uses have kernels of two edges at a time.
+// ID: the shape's number, which tells with CPL and PAIR which uses have kernels.
 template <typename T, int CPL, int ID, bool FULL, bool SLICED, bool PAIR>
 int dispatch_edge_bwd(const luna_uvu_plan* plan, const DeviceTables& dt, const luna_graph* graph,
                       const EdgeLanes& lanes, const EdgeBackwardArgs& a, cudaStream_t stream) {
   using S = ShapeOf<ID>;
   const bool wx = a.gx != nullptr, ww = a.gw != nullptr, wy = a.gy != nullptr;
-  auto compiled = [](EdgeUse use) { return !PAIR || edge_paired<T, CPL, ID>(use); };
+  auto compiled = [](EdgeUse use) { return SLICED || (PAIR ? edge_paired<T, CPL, ID>(use) : edge_alone<T, CPL, ID>(use)); };
   if constexpr (edge_joins_output<T, CPL, S>() && compiled(EdgeUse::kOutputAndWeights)) {
     if (a.out)
       return launch_edge_bwd<T, CPL, Transposed<S>, true, true, false, FULL, true, SLICED, PAIR>(plan, dt, graph, lanes, a, stream);

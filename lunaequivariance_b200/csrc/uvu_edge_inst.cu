@@ -17,9 +17,13 @@ int EdgeKernels<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>::forward(const luna
   if constexpr (edge_paired<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>(EdgeUse::kForward)) {
     if (lanes.edges == 2) return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, true>(plan, dt, graph, lanes, a, stream);
   }
-  if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
-    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, false>(plan, dt, graph, lanes, a, stream);
-  return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false, false>(plan, dt, graph, lanes, a, stream);
+  if constexpr (edge_alone<LUNA_EDGE_T, LUNA_EDGE_CPL, LUNA_EDGE_SHAPE>(EdgeUse::kForward)) {
+    if (plan->edge.ch == 32 * LUNA_EDGE_CPL)
+      return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, true, false, false>(plan, dt, graph, lanes, a, stream);
+    return launch_edge_fwd<LUNA_EDGE_T, LUNA_EDGE_CPL, S, false, false, false>(plan, dt, graph, lanes, a, stream);
+  } else {
+    return fail(LUNA_ERR_UNSUPPORTED, "no forward kernel of this layout");
+  }
 }
 
 template <>

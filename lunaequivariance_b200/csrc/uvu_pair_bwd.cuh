@@ -410,5 +410,25 @@ constexpr bool edge_paired(EdgeUse use) {
   return (CPL <= 3 || four) && bytes <= (CPL == 3 && use == EdgeUse::kOneGradient ? 31 : 24) * 1024;
 }
 
+// The estimate of what a lane of the kernel needs.
+template <typename T, int CPL, typename S>
+constexpr int registers_of(EdgeUse use) {
+  using R = Transposed<S>;
+  using One = std::conditional_t<S::OD >= S::XD, R, S>;
+  switch (use) {
+    case EdgeUse::kForward: return EdgeFwd<T, CPL, S>::registers;
+    case EdgeUse::kSums: return EdgeBwd<T, CPL, S, true, true, false>::registers;
+    case EdgeUse::kOutputAndWeights: return EdgeBwd<T, CPL, R, true, true, false>::registers;
+    case EdgeUse::kAllGradients: return EdgeBwd<T, CPL, S, true, true, true>::registers;
+    default: return std::max(EdgeBwd<T, CPL, One, false, false, true>::registers, EdgeBwd<T, CPL, One, false, true, false>::registers);
+  }
+}
+// Whether the kernels of one edge at a time are compiled for teams (for slices: edge_sliced).  Three channels per lane are not where the
+// state is far above the registers: FP64 (3, 3, 3) but for one gradient alone, and (2, 3, 3) for output with dL/dw.
+template <typename T, int CPL, int ID>
+constexpr bool edge_alone(EdgeUse use) {
+  return CPL != 3 || registers_of<T, CPL, ShapeOf<ID>>(use) <= (use == EdgeUse::kForward ? 255 : 280);
+}
+
 }  // namespace edgek
 }  // namespace luna
