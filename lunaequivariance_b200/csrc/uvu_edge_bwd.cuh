@@ -531,6 +531,7 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::template warps
             unit_body(l3c, (split ? gslots : wrow + W) + ch * S::ooff(l3), wrow);
             if constexpr (l3 != S::LO && S::ooff(l3) + 2 * l3 + 1 == K::slot_begin(slot + 1)) {
               if (split) {  // the slot is done with; the last one is refilled at the end of the edge
+                fence_async_shared();
                 team_sync(team_warps, team);
                 if (issuing && more) load_slot(std::integral_constant<int, slot>{}, d1);
               }
@@ -544,8 +545,8 @@ __global__ void __launch_bounds__(EdgeBwd<T, CPL, S, WX, WM, WY>::template warps
             }
           }
         });
-        if (storing) fence_async_shared();  // gradient writes, before the bulk store reads the stage
-        team_sync(team_warps, team);      // every lane is done with the stage, the last slot and the scalars
+        fence_async_shared();         // gradient writes, before the bulk store reads the stage, and reads, before it is refilled
+        team_sync(team_warps, team);  // every lane is done with the stage, the last slot and the scalars
         if (issuing) {
           if (split && more) load_slot(std::integral_constant<int, K::slots - 1>{}, d1);
           if (storing) {

@@ -294,7 +294,8 @@ __global__ void __launch_bounds__(EdgeFwd<T, CPL, S>::template warps<FULL> * 32,
         const T* m_now = mbuf + buf * K::m_elems;
         forward_edge<T, PK, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
         buf ^= 1;
-        team_sync(team_warps, team);  // every lane is done with this stage and with the matrices
+        fence_async_shared();         // what was read of this stage, before it is refilled
+        team_sync(team_warps, team);  // every lane is done with it and with the matrices
         if (issuing && e + stages < e_end) {
           issue(e + stages, src_ahead, s);
           if (e + stages + 1 < e_end) src_ahead = P.src[e + stages + 1];

@@ -317,7 +317,8 @@ __global__ void __launch_bounds__(MAXW * 32, MINB) fast_bwd_kernel(const __grid_
       return false;
     }
     unit_body(l3c, slots + static_cast<size_t>(s) * slot_elems);
-    __syncwarp();  // every lane is done with this slot
+    fence_async_shared();  // what was read of this slot, before it is refilled
+    __syncwarp();          // every lane is done with it
     if (u + R < total_units) {
       int next = kind + R, de = 0;
       if (next >= nk) {

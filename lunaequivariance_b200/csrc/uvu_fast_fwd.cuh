@@ -207,7 +207,8 @@ __global__ void __launch_bounds__(kFwdMaxWarps * 32, 1) fast_fwd_kernel(const __
             path_body(l1c, l3c, wl + F.w_soff[q], mbuf + F.m_off[q], xl, al);
         });
       });
-      __syncwarp();  // every lane is done with this stage, mbuf and ybuf
+      fence_async_shared();  // what was read of this stage, before it is refilled
+      __syncwarp();          // every lane is done with it, mbuf and ybuf
       const int src_now = src_ahead;
       if (e + stages + 1 < e_end) src_ahead = P.src[e + stages + 1];
       if (e + stages < e_end) issue(e + stages, src_now, s);

@@ -249,8 +249,8 @@ __global__ void __launch_bounds__(PairBwd<T, CPL, S, WX, WM, WY>::max_warps * 32
           }
         }
       });
-      if (storing) fence_async_shared();  // gradient writes, before the bulk store reads the stage
-      __syncwarp();                       // every lane is done with the stage and the matrices
+      fence_async_shared();  // gradient writes, before the bulk store reads the stage, and reads, before it is refilled
+      __syncwarp();          // every lane is done with the stage and the matrices
       if (issuing) {
         if (storing) {
           if (valid) {

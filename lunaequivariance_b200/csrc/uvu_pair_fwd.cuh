@@ -171,7 +171,8 @@ __global__ void __launch_bounds__(PairFwd<T, CPL, S>::max_warps * 32, 1)
       const T* m_now = mbuf + buf * S::m_elems;
       if (mine < e_end) forward_edge<T, PK, S>(ws, xs, ch, own, lanes, m_now, P.coef, acc);
       buf ^= 1;
-      __syncwarp();  // every lane is done with this stage and with the matrices
+      fence_async_shared();  // what was read of this stage, before it is refilled
+      __syncwarp();          // every lane is done with it and with the matrices
       if (issuing && e + 2 * stages < e_end) {
         issue(mine + 2 * stages, src_ahead, mine + 2 * stages < e_end, s);
         if (mine + 2 * stages + 2 < e_end) src_ahead = P.src[mine + 2 * stages + 2];

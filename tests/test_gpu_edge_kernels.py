@@ -348,3 +348,24 @@ def test_layout_of_a_launch(shape, mul, dtype, which, kernel, lane_channels, war
                                 dtype=dtype).op
     (launch,) = launches(op, dtype, 700, 12_000, which, tmp_path)
     assert launch[:2] == (kernel, lane_channels) and launch[2] in (warps or [launch[2]]), launch
+
+
+# One warp per edge and several, rows by source and by destination: the smallest work for a stage of all kernels, whose last read
+# comes straight before the row that replaces it.
+@pytest.mark.parametrize("shape,mul,nodes,edges", [(2, 224, 2453, 27_901), (9, 128, 3524, 18_953), (9, 60, 1514, 104_166)])
+def test_a_stage_is_read_before_it_is_refilled(shape, mul, nodes, edges):
+    in1, in2, out = irreps(mul, SHAPES[shape][0]), irreps(1, SHAPES[shape][1]), irreps(mul, SHAPES[shape][2])
+    op = luna.TensorProductConv(in1, in2, out, all_paths(in1, in2, out), internal_weights=False, shared_weights=False,
+                                dtype=torch.float64).op
+    src, dst = skewed_graph(nodes, edges, torch.Generator().manual_seed(5), 0.0)
+    graph = luna.make_graph(src.to(DEVICE), dst.to(DEVICE), nodes)
+    generator = torch.Generator(device=DEVICE).manual_seed(5)
+    x, y, w, g = (torch.randn(*rows, generator=generator, dtype=torch.float64, device=DEVICE)
+                  for rows in ((nodes, op.in1_dim), (edges, op.in2_dim), (edges, op.weight_numel), (nodes, op.out_dim)))
+    _, want, _ = conv_mod.run_backward(op, x, y, w, g, graph)
+    results = [torch.empty_like(want) for _ in range(120)]
+    for gy in results:
+        conv_mod.run_backward(op, x, y, w, g, graph, (False, True, False), out=(None, gy, None))
+    op.check_status()
+    assert_close(results[0], want.cpu(), torch.float64, "dL/dy alone")
+    assert all(torch.equal(gy, results[0]) for gy in results)
