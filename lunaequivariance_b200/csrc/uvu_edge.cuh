@@ -507,7 +507,7 @@ __device__ __forceinline__ void lane_store(T* p, int lanes, const typename PK::V
   }
 }
 // Components of a node row's block of D components per channel -> packets [component][packet]; p: the block plus
-// own * D, stride as above.  Scalar loads on purpose: the two halves then land in the pair's registers, while halves
+// own * D, `lanes` as above.  Scalar loads on purpose: the two halves then land in the pair's registers, while halves
 // taken from vector loads are put together again in front of every packed instruction that uses the pair (measured on
 // the 128-channel degree-(2,3,3) backward: 18.9 ms against 11.4).
 template <typename PK, typename T, int D>

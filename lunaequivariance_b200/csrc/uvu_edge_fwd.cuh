@@ -2,7 +2,7 @@
 //
 // Per edge the warp turns the edge attributes into the coupling matrices M^p[i][k] = sum_j C^p_ijk y_j (the entries the
 // coupling tensors leave zero for every y are skipped, at compile time), a lane multiplies them into its channels:
-// out_k += sum_i M[i][k] * (x_i * w).  FP32 with an even number of channels per lane runs on packed two-wide FMAs.
+// out_k += sum_i M[i][k] * (x_i * w).  FP32 with more than one channel per lane runs on packed two-wide FMAs (three: a pair and a scalar).
 // The matrices of the next edge are made while the current edge is computed: its attributes sit one per lane and reach
 // the lane that needs them by shuffles, so nothing waits for shared memory in between.
 #pragma once
